@@ -42,10 +42,11 @@ size_t align_up(size_t x) { return (x + 255) & ~(size_t)255; }
 // Workspace a job needs for kc maps per chunk, laid out as [W buffers][WS][EB].
 struct JobLayout {
   int kc, nbuf;
-  size_t w_bytes, ws_off, eb_off, lb_off, total;
+  size_t w_bytes, ws_off, fl_off, eb_off, lb_off, total;
 };
 
-JobLayout job_layout(const fsht_plan* p, const fsht_job& j, int kc) {
+// tc: with the digit tiles of the tensor-core FP64 contraction.
+JobLayout job_layout(const fsht_plan* p, const fsht_job& j, int kc, bool tc = false) {
   JobLayout L;
   L.kc = kc;
   const bool pol = j.kind == FSHT_JOB_QU2EB || j.kind == FSHT_JOB_EB2QU;
@@ -53,6 +54,7 @@ JobLayout job_layout(const fsht_plan* p, const fsht_job& j, int kc) {
   const size_t per_map = (size_t)(p->lmax + 1) * p->nnorth * 2 * sizeof(double2);
   L.w_bytes = per_map * L.nbuf * kc;
   L.ws_off = align_up(L.w_bytes);
+  L.fl_off = L.ws_off;
   L.eb_off = L.ws_off;
   L.lb_off = L.ws_off;
   L.total = L.ws_off;
@@ -61,6 +63,12 @@ JobLayout job_layout(const fsht_plan* p, const fsht_job& j, int kc) {
     const size_t f = pol2 ? 2 : 1;   // spin 2: tiles of Q and U (or E and B)
     L.eb_off = align_up(L.ws_off + f * fsht_split_ws_bytes(p, kc));
     L.lb_off = align_up(L.eb_off + f * fsht_split_eb_bytes(p, kc));
+    L.total = align_up(L.lb_off + p->lbuf_bytes);
+  } else if (tc) {
+    const int nf = pol ? 2 : 1;
+    L.fl_off = align_up(L.ws_off + fsht_tc_ws_bytes(p, kc, nf));
+    L.eb_off = align_up(L.fl_off + fsht_tc_flag_bytes(p, kc));
+    L.lb_off = align_up(L.eb_off + fsht_tc_eb_bytes(p, kc));
     L.total = align_up(L.lb_off + p->lbuf_bytes);
   }
   return L;
@@ -74,9 +82,21 @@ double job_cost(const fsht_job& j) {
 
 int run_job(const fsht_plan* base, const fsht_job& j, unsigned char* arena, size_t arena_bytes,
             cudaStream_t s) {
+  // FP64 jobs take the tensor-core contraction when its digit tiles fit beside the phase
+  // matrices of a whole 64-map group (or of every map), else the FMA kernels, which need none
+  const bool pol = j.kind == FSHT_JOB_QU2EB || j.kind == FSHT_JOB_EB2QU;
+  bool tc = base->tc64 && (!pol || base->d_poltab);
   int kc = j.nmaps;
-  while (kc > 1 && job_layout(base, j, kc).total > arena_bytes) --kc;
-  const JobLayout L = job_layout(base, j, kc);
+  if (tc) {
+    while (kc > 1 && job_layout(base, j, kc, true).total > arena_bytes)
+      kc = kc > 64 ? (kc - 1) / 64 * 64 : kc - 1;
+    if (job_layout(base, j, kc, true).total > arena_bytes || (kc < j.nmaps && kc < 64)) {
+      tc = false;
+      kc = j.nmaps;
+    }
+  }
+  while (kc > 1 && job_layout(base, j, kc, tc).total > arena_bytes) --kc;
+  const JobLayout L = job_layout(base, j, kc, tc);
   if (L.total > arena_bytes) {
     fsht_set_error("batch job (nside %d, lmax %d) needs %zu bytes of workspace per slot, above "
                    "the slot's %zu", j.nside, j.lmax, L.total, arena_bytes);
@@ -92,6 +112,8 @@ int run_job(const fsht_plan* base, const fsht_job& j, unsigned char* arena, size
   jp.d_ws = arena + L.ws_off;
   jp.d_eb = reinterpret_cast<int*>(arena + L.eb_off);
   jp.d_lbuf = arena + L.lb_off;
+  jp.tc64 = tc ? 1 : 0;
+  jp.d_tcflag = reinterpret_cast<int*>(arena + L.fl_off);
   jp.prof = nullptr;
   switch (j.kind) {
     case FSHT_JOB_T2ALM: return fsht_t2alm(&jp, j.in0, j.out0, j.nmaps, 0, 0);

@@ -188,6 +188,12 @@ struct fsht_plan {
   int gemm_ctas;
   int wave_qmax;                   // most orders in one wave
   FshtPolRow* d_poltab;            // spin-2 plans only, same triangular index as d_lamtab
+  // FP64 plans: 1 when the contraction may run on the tensor cores (legendre_fp64_tc.cu); it
+  // shares the split form's tables, staging buffers, waves and streams.  d_tcflag: per (order,
+  // 64-map group of the chunk) four flags of columns left to the FMA kernels.
+  int tc64;
+  int* d_tcflag;
+  FshtLamRow* d_lamtab2;           // their spin-2 recursion rows (d_poltab: integer factors)
 };
 
 // ---------------------------------------------------------------- status codes
@@ -263,10 +269,32 @@ int fsht_launch_fourier_residual(fsht_plan* p, const double2* X, double2* GR, in
 int fsht_launch_ring_skip(fsht_plan* p, cudaStream_t s);
 // Legendre contraction, FP64.  alm layout: [col][l][k] with ld = nmaps total,
 // k offset k0.  which: bit0 = E (or T), bit1 = B.
+// flags (may be null): only the orders and 64-map groups flagged there (p->d_tcflag).
 int fsht_launch_analysis_fp64(fsht_plan* p, int spin, const double2* WQ,
                               const double2* WU, double* almE, double* almB,
                               int nmaps_total, int k0, int kc, int accumulate,
-                              int which, cudaStream_t s);
+                              int which, cudaStream_t s, const int* flags = nullptr);
+// The same contraction as exact digit products on the tensor cores (FP64 plans with tc64).
+// Per wave w: slice (phases or alm -> digit tiles WS, exponents EB), lambda (-> lbuf), gemm
+// (dir 0: into alm, dir 1: into the phase matrices).  A null second field means spin 0.
+bool fsht_tc_supported(const fsht_plan* p);
+int fsht_tc_tables_init(fsht_plan* p);
+size_t fsht_tc_ws_bytes(const fsht_plan* p, int kc, int nf);
+size_t fsht_tc_eb_bytes(const fsht_plan* p, int kc);
+size_t fsht_tc_flag_bytes(const fsht_plan* p, int kc);
+int fsht_launch_tc_slice(fsht_plan* p, int w, const double2* W0, const double2* W1,
+                         unsigned char* WS, int* EB, int kc, cudaStream_t s);
+int fsht_launch_tc_slice_alm(fsht_plan* p, int w, const double* alm0, const double* alm1,
+                             unsigned char* WS, int* EB, int nmaps_total, int k0, int kc,
+                             cudaStream_t s);
+int fsht_launch_tc_lambda(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s);
+int fsht_launch_tc_lambda_pol(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s);
+int fsht_launch_tc_lambdaT(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s);
+int fsht_launch_tc_lambdaT_pol(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s);
+int fsht_launch_tc_gemm(fsht_plan* p, int w, int dir, int spin, const unsigned char* WS,
+                        const int* EB, const unsigned char* lbuf, double* out0, double* out1,
+                        int nmaps_total, int k0, int kc, int accumulate, int which,
+                        cudaStream_t s);
 // Split-precision form.  WS / EB: digit tiles and column exponents of one wave of m.
 size_t fsht_split_ws_bytes(const fsht_plan* p, int kc);
 size_t fsht_split_eb_bytes(const fsht_plan* p, int kc);
@@ -276,6 +304,8 @@ size_t fsht_split_eb_bytes(const fsht_plan* p, int kc);
 // writes the wave's lambda digit tiles into lbuf, gemm contracts them into alm (stores, or
 // adds when accumulate).
 int fsht_split_tables_init(fsht_plan* p);
+// Tile offsets per order and the waves of m, for digit tiles of `unit` bytes per k-step.
+int fsht_wave_tables_init(fsht_plan* p, size_t unit);
 int fsht_launch_split_slice(fsht_plan* p, int w, const double2* W, unsigned char* WS, int* EB,
                             int kc, cudaStream_t s);
 int fsht_launch_split_lambda(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s);
@@ -308,4 +338,5 @@ int fsht_launch_split_synth(fsht_plan* p, int w, const unsigned char* WS, const 
                             const unsigned char* lbuf, double2* W, int kc, cudaStream_t s);
 int fsht_launch_synthesis_fp64(fsht_plan* p, int spin, const double* almE,
                                const double* almB, double2* WQ, double2* WU,
-                               int nmaps_total, int k0, int kc, cudaStream_t s);
+                               int nmaps_total, int k0, int kc, cudaStream_t s,
+                               const int* flags = nullptr);

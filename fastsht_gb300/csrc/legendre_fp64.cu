@@ -21,6 +21,7 @@
 // accumulator tile in registers and reads shared-memory tiles laid out so that a
 // warp's loads are conflict-free.
 #include "common.cuh"
+#include "legendre_rec.cuh"
 
 namespace {
 
@@ -58,56 +59,6 @@ __device__ __forceinline__ void rec_seed(double sth, double pref, int m, double&
   cur = ldexp(rm, (int)(re - 600LL * e));
 }
 
-__device__ __forceinline__ void rec_step(double& cur, double& prev, int& e, double a_cth,
-                                         double b) {
-  const double nx = a_cth * cur - b * prev;
-  prev = cur;
-  cur = nx;
-  if (e < 0 && fabs(cur) > 0x1p300) {
-    cur *= 0x1p-600;
-    prev *= 0x1p-600;
-    ++e;
-  }
-}
-
-// Spin-2 lambda1/lambda2 from lambda_l (cur) and lambda_{l-1} (prev) on one ring
-// (get_plm_recursive.f90:101-125).
-struct PolRing {
-  double cth, b_w, two_on_s2, c_w, diag1, diag2;
-};
-__device__ __forceinline__ PolRing pol_ring(double cth, double sth, int m) {
-  PolRing r;
-  const double s2 = sth * sth;
-  r.cth = cth;
-  r.b_w = cth / s2;
-  r.two_on_s2 = 2.0 / s2;
-  r.c_w = (double)m / s2;
-  r.diag1 = 0.5 - 1.0 / s2;
-  r.diag2 = cth / s2;
-  return r;
-}
-__device__ __forceinline__ double normal_l(int l) {
-  if (l < 2) return 0.0;
-  return 1.0 / sqrt((double)(l + 2) * (double)(l + 1) * (double)l * (double)(l - 1));
-}
-__device__ __forceinline__ double lam_fact(int l, int m) {
-  const int m1 = m > 1 ? m : 1;
-  if (l <= m1) return 0.0;
-  return 2.0 * sqrt((double)(2 * l + 1) / (double)(2 * l - 1) * (double)((long long)l * l - (long long)m * m));
-}
-__device__ __forceinline__ void pol_lambda(const PolRing& r, int l, int m, double cur, double prev,
-                                           double lf, double nl, double& l1, double& l2) {
-  if (l == m) {
-    const double nm = (double)(2LL * m * (1 - m)) * nl;
-    l1 = nm * cur * r.diag1;
-    l2 = nm * cur * r.diag2;
-  } else {
-    l1 = (prev * lf * r.b_w - cur * (r.two_on_s2 * (double)((long long)l - (long long)m * m) +
-                                     (double)l * ((double)l - 1.0))) * nl;
-    l2 = (prev * lf - cur * (2.0 * r.cth * ((double)l - 1.0))) * r.c_w * nl;
-  }
-}
-
 // ====================================================================== analysis
 struct AnaArgs {
   int nside, lmax, nnorth;
@@ -125,7 +76,17 @@ struct AnaArgs {
   double scale;        // pa (T) or -pa (spin 2)
   int accumulate;
   int which;           // bit0: E/T, bit1: B
+  const int* flags;    // null, or only the flagged (order, 64-map group): four ints each
+  int ngroups;
 };
+
+// Whether (m, the 64-map group at kt0) is left to these kernels (no flags: everything is).
+__device__ __forceinline__ bool flagged(const int* flags, int ngroups, int m, int kt0) {
+  if (!flags) return true;
+  const int4 f =
+      *reinterpret_cast<const int4*>(flags + ((long long)m * ngroups + (kt0 >> 6)) * 4);
+  return (f.x | f.y | f.z | f.w) != 0;
+}
 
 // Tile shape: QN map slots per thread (16 QN maps per CTA: 64 by default, 32 for small
 // batches) and RC rings per chunk (16 for spin 0 and 8 for spin 2 by default); the autotuner
@@ -167,6 +128,7 @@ __global__ void __launch_bounds__(NT) k_analysis_fp64(AnaArgs a) {
     const int m = pass == 0 ? (int)blockIdx.x : a.lmax - (int)blockIdx.x;
     if (pass == 1 && m == (int)blockIdx.x) break;
     if (m < 0) break;
+    if (!flagged(a.flags, a.ngroups, m, kt0)) continue;
     (void)npair;
     const int i0 = a.ring_i0[m];
     const int nr = a.nnorth - i0;
@@ -335,6 +297,8 @@ struct SynArgs {
   double2* WQ;          // {G_N, G_S} per (m, ring, map); T or Q
   double2* WU;
   int kc;
+  const int* flags;     // as in AnaArgs
+  int ngroups;
 };
 
 template <int SPIN>
@@ -370,6 +334,7 @@ __global__ void __launch_bounds__(NT) k_synthesis_fp64(SynArgs a) {
     if (pass == 1 && m == (int)blockIdx.x) break;
     const int i0 = a.ring_i0[m];
     if (ib + RCS <= i0) continue;          // no ring of this chunk is kept for m
+    if (!flagged(a.flags, a.ngroups, m, kt0)) continue;
     // recursion state for ring ib + tid (warp 0)
     double cur = 0.0, prev = 0.0;
     int e = -1;
@@ -551,8 +516,10 @@ int launch_ana(const AnaArgs& a, int npair, int nnorth, int kc, cudaStream_t s) 
 
 int fsht_launch_analysis_fp64(fsht_plan* p, int spin, const double2* WQ, const double2* WU,
                               double* almE, double* almB, int nmaps_total, int k0, int kc,
-                              int accumulate, int which, cudaStream_t s) {
+                              int accumulate, int which, cudaStream_t s, const int* flags) {
   AnaArgs a;
+  a.flags = flags;
+  a.ngroups = (kc + 63) / 64;
   a.nside = p->nside;
   a.lmax = p->lmax;
   a.nnorth = p->nnorth;
@@ -592,8 +559,10 @@ int fsht_launch_analysis_fp64(fsht_plan* p, int spin, const double2* WQ, const d
 
 int fsht_launch_synthesis_fp64(fsht_plan* p, int spin, const double* almE, const double* almB,
                                double2* WQ, double2* WU, int nmaps_total, int k0, int kc,
-                               cudaStream_t s) {
+                               cudaStream_t s, const int* flags) {
   SynArgs a;
+  a.flags = flags;
+  a.ngroups = (kc + 63) / 64;
   a.nside = p->nside;
   a.lmax = p->lmax;
   a.nnorth = p->nnorth;

@@ -1069,12 +1069,17 @@ int fsht_split_tables_init(fsht_plan* p) {
   const int lmax = p->lmax;
   const size_t ntab = (size_t)tri_off(lmax + 1, lmax);
   FSHT_CUDA_TRY(cudaMalloc(&p->d_lamtab, sizeof(FshtLamRow) * (ntab ? ntab : 1)));
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_off, sizeof(long long) * (lmax + 2)));
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_offT, sizeof(long long) * (lmax + 2)));
   k_lam_table<<<(lmax + 1 + 127) / 128, 128, 0, p->stream>>>(lmax, p->d_lamtab);
   FSHT_LAUNCH_CHECK();
-  // per q (pair order): 16 KB units of m(q)'s analysis tiles (l-rows) and synthesis tiles
-  // (ring rows)
+  return fsht_wave_tables_init(p, (size_t)kSlices * kATileBytes);
+}
+
+int fsht_wave_tables_init(fsht_plan* p, size_t unit) {
+  const int lmax = p->lmax;
+  FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_off, sizeof(long long) * (lmax + 2)));
+  FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_offT, sizeof(long long) * (lmax + 2)));
+  // per q (pair order): `unit`-byte k-steps of m(q)'s analysis tiles (l-rows) and synthesis
+  // tiles (ring rows)
   std::vector<long long> off(lmax + 2, 0), offT(lmax + 2, 0);
   std::vector<int> ntl(lmax + 1), nkm(lmax + 1), nrb(lmax + 1), nkl(lmax + 1);
   for (int q = 0; q <= lmax; ++q) {
@@ -1087,7 +1092,6 @@ int fsht_split_tables_init(fsht_plan* p) {
     off[q + 1] = off[q] + 2LL * ntl[q] * nkm[q];
     offT[q + 1] = offT[q] + 2LL * nrb[q] * nkl[q];
   }
-  const size_t unit = (size_t)kSlices * kATileBytes;
   const size_t cap_units = kLbufCap / unit;
   // spin-2 plans stage lambda1 and lambda2: twice the analysis tiles
   const long long fa = p->pol ? 2 : 1;

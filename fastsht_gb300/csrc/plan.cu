@@ -120,6 +120,9 @@ void free_plan_memory(fsht_plan* p) {
   cudaFree(p->d_eb);
   cudaFree(p->d_lamtab);
   cudaFree(p->d_lam_off);
+  cudaFree(p->d_lam_offT);
+  cudaFree(p->d_tcflag);
+  cudaFree(p->d_lamtab2);
   cudaFree(p->d_lbuf);
   cudaFree(p->d_lbuf2);
   for (int i = 0; i < 6; ++i)
@@ -146,6 +149,16 @@ void free_plan_memory(fsht_plan* p) {
     delete p->prof;
     p->prof = nullptr;
   }
+}
+
+void drop_tc_buffers(fsht_plan* p) {
+  cudaFree(p->d_ws);
+  cudaFree(p->d_eb);
+  cudaFree(p->d_tcflag);
+  cudaFree(p->d_lbuf);
+  cudaFree(p->d_lbuf2);
+  p->d_ws = p->d_lbuf = p->d_lbuf2 = nullptr;
+  p->d_eb = p->d_tcflag = nullptr;
 }
 
 // theta of the first pixel of north ring i (HEALPix pix2loc, as used through
@@ -316,6 +329,10 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   if (precision == FSHT_PREC_SPLIT && (rc = fsht_split_tables_init(p))) return fail(rc);
   if (precision == FSHT_PREC_SPLIT && p->pol && (rc = fsht_split_pol_tables_init(p)))
     return fail(rc);
+  if (precision == FSHT_PREC_FP64 && fsht_tc_supported(p)) {
+    if ((rc = fsht_tc_tables_init(p))) return fail(rc);
+    p->tc64 = 1;
+  }
   // ---- workspace: nbuf phase matrices of kchunk maps (+ the sliced copy for the
   // split form, sized in groups of 128 maps)
   const size_t limit = workspace_limit_bytes
@@ -324,6 +341,11 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   const size_t per_map = per_map_buffer_bytes(p) * p->nbuf;
   // digit-tile buffers of the split form: two waves in flight of T, or of Q and U (four)
   const size_t f_ws = p->pol ? 4 : 2;
+  const int tc_nf = p->pol ? 2 : 1;
+  auto need_tc = [&](size_t k) -> size_t {     // two waves in flight, as in the split form
+    return per_map * k + 2 * (fsht_tc_ws_bytes(p, (int)k, tc_nf) + fsht_tc_eb_bytes(p, (int)k)) +
+           fsht_tc_flag_bytes(p, (int)k) + 2 * p->lbuf_bytes;
+  };
   auto need = [&](size_t k) -> size_t {
     size_t b = per_map * k;
     if (precision == FSHT_PREC_SPLIT)   // digit tiles and their exponents, two lambda buffers
@@ -338,6 +360,32 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     fsht_set_error("workspace limit %zu bytes is below one map's %zu bytes", limit, need(1));
     return fail(FSHT_EINVAL);
   }
+  if (p->tc64 && !tables_only) {
+    // The digit tiles share the workspace limit with the phase matrices: whole 64-map groups.
+    // A limit that leaves them less than one group (and fewer maps than the FMA kernels' chunk)
+    // keeps the FMA kernels, which need no tiles.
+    size_t kt = (size_t)nmaps_max;
+    while (kt > 1 && need_tc(kt) > limit) kt = kt > 64 ? (kt - 1) / 64 * 64 : kt - 1;
+    if (need_tc(kt) > limit || (kt < kc && kt < 64)) {
+      p->tc64 = 0;
+    } else {
+      // two digit-tile buffers, exponents, flags, two lambda buffers; without room for them on
+      // the device the FMA kernels run
+      const size_t ws = 2 * fsht_tc_ws_bytes(p, (int)kt, tc_nf);
+      const size_t eb = 2 * fsht_tc_eb_bytes(p, (int)kt);
+      if (cudaMalloc(&p->d_ws, ws) != cudaSuccess || cudaMalloc(&p->d_eb, eb) != cudaSuccess ||
+          cudaMalloc(&p->d_tcflag, fsht_tc_flag_bytes(p, (int)kt)) != cudaSuccess ||
+          cudaMalloc(&p->d_lbuf, p->lbuf_bytes) != cudaSuccess ||
+          cudaMalloc(&p->d_lbuf2, p->lbuf_bytes) != cudaSuccess) {
+        cudaGetLastError();
+        drop_tc_buffers(p);
+        p->tc64 = 0;
+      } else {
+        p->ws_bytes = ws;
+        kc = kt;
+      }
+    }
+  }
   p->kchunk = tables_only ? 0 : (int)kc;
   p->work_bytes = tables_only ? 0 : per_map * kc;
   if (!tables_only && (rc = dalloc((void**)&p->d_work, p->work_bytes))) return fail(rc);
@@ -346,13 +394,15 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     fsht_set_error("memset: %s", cudaGetErrorString(ce));
     return fail(FSHT_ECUDA);
   }
-  if (precision == FSHT_PREC_SPLIT && !tables_only) {
-    const size_t f = f_ws;
-    p->ws_bytes = f * fsht_split_ws_bytes(p, p->kchunk);
-    if ((rc = dalloc((void**)&p->d_ws, p->ws_bytes))) return fail(rc);
-    if ((rc = dalloc((void**)&p->d_eb, f * fsht_split_eb_bytes(p, p->kchunk)))) return fail(rc);
-    if ((rc = dalloc((void**)&p->d_lbuf, p->lbuf_bytes))) return fail(rc);
-    if ((rc = dalloc((void**)&p->d_lbuf2, p->lbuf_bytes))) return fail(rc);
+  if ((precision == FSHT_PREC_SPLIT || p->tc64) && !tables_only) {
+    if (!p->tc64) {
+      const size_t f = f_ws;
+      p->ws_bytes = f * fsht_split_ws_bytes(p, p->kchunk);
+      if ((rc = dalloc((void**)&p->d_ws, p->ws_bytes))) return fail(rc);
+      if ((rc = dalloc((void**)&p->d_eb, f * fsht_split_eb_bytes(p, p->kchunk)))) return fail(rc);
+      if ((rc = dalloc((void**)&p->d_lbuf, p->lbuf_bytes))) return fail(rc);
+      if ((rc = dalloc((void**)&p->d_lbuf2, p->lbuf_bytes))) return fail(rc);
+    }
     if ((ce = cudaStreamCreateWithFlags(&p->aux, cudaStreamNonBlocking)) != cudaSuccess) {
       fsht_set_error("auxiliary stream: %s", cudaGetErrorString(ce));
       return fail(FSHT_ECUDA);
@@ -373,6 +423,8 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
         return fail(FSHT_ECUDA);
       }
     }
+  }
+  if (precision == FSHT_PREC_SPLIT && !tables_only) {
     int least = 0, greatest = 0;
     if ((ce = cudaDeviceGetStreamPriorityRange(&least, &greatest)) != cudaSuccess ||
         (ce = cudaStreamCreateWithPriority(&p->hp_main, cudaStreamNonBlocking, greatest)) !=
@@ -601,6 +653,11 @@ int fsht_plan_check(fsht_plan* p) {
 typedef int (*LamLaunch)(fsht_plan*, int, unsigned char*, cudaStream_t);
 enum { kEvFork = 0, kEvJoin = 1, kEvTiles = 2, kEvDone = 4 };
 
+// Whether a call of this plan takes the tensor-core form of the FP64 contraction.
+static bool use_tc(const fsht_plan* p, int spin) {
+  return p->tc64 && p->d_lbuf && p->d_tcflag && (spin == 0 || p->d_poltab);
+}
+
 static unsigned char* lam_buf(fsht_plan* p, int w) {
   return (p->aux && (w & 1)) ? p->d_lbuf2 : p->d_lbuf;
 }
@@ -789,6 +846,96 @@ static int split_synthesis(fsht_plan* p, const double* alm, double2* W, int nmap
   return lam_finish(p);
 }
 
+// ----------------------------------------------------------------- FP64 contraction
+// One chunk's FP64 analysis (spin 0: W0 -> alm0; spin 2: W0 = Q, W1 = U -> alm0 = E, alm1 = B,
+// which: bit0 E, bit1 B): the tensor-core digit products in the wave pipeline of the split form
+// (lambda tiles two waves ahead, slicing one wave ahead), then the FMA kernel over what the
+// slicing flagged; or the FMA kernel alone.
+static int fp64_analysis(fsht_plan* p, int spin, const double2* W0, const double2* W1,
+                         double* alm0, double* alm1, int nmaps, int c0, int kc, int accumulate,
+                         int which, bool started = false) {
+  if (!use_tc(p, spin)) {
+    FSHT_PROF(FSHT_KCAT_ANALYSIS);
+    return fsht_launch_analysis_fp64(p, spin, W0, W1, alm0, alm1, nmaps, c0, kc, accumulate,
+                                     which, p->stream);
+  }
+  const LamLaunch lam = spin == 2 ? fsht_launch_tc_lambda_pol : fsht_launch_tc_lambda;
+  if (!started) FSHT_TRY(lam_start(p, lam));
+  const bool ahead = p->aux2 != nullptr && p->aux != nullptr;
+  const size_t ws1 = fsht_tc_ws_bytes(p, kc, spin == 2 ? 2 : 1);
+  const size_t eb1 = fsht_tc_eb_bytes(p, kc) / sizeof(int);
+  auto ws_of = [&](int w) { return p->d_ws + (ahead ? (size_t)(w & 1) * ws1 : 0); };
+  auto eb_of = [&](int w) { return p->d_eb + (ahead ? (size_t)(w & 1) * eb1 : 0); };
+  auto slice_on = [&](int w, cudaStream_t st) -> int {
+    FSHT_PROF_ON(FSHT_KCAT_SLICE, st);
+    return fsht_launch_tc_slice(p, w, W0, spin == 2 ? W1 : nullptr, ws_of(w), eb_of(w), kc, st);
+  };
+  if (ahead) {
+    FSHT_CUDA_TRY(cudaEventRecord(p->evs[0], p->stream));
+    FSHT_CUDA_TRY(cudaStreamWaitEvent(p->aux2, p->evs[0], 0));
+    FSHT_TRY(slice_on(0, p->aux2));
+    FSHT_CUDA_TRY(cudaEventRecord(p->evs[2], p->aux2));
+  }
+  for (int w = 0; w < p->nwaves; ++w) {
+    if (!ahead) {
+      FSHT_TRY(slice_on(w, p->stream));
+    } else {
+      if (w + 1 < p->nwaves) {
+        if (w >= 1)
+          FSHT_CUDA_TRY(cudaStreamWaitEvent(p->aux2, p->ev[kEvDone + ((w + 1) & 1)], 0));
+        FSHT_TRY(slice_on(w + 1, p->aux2));
+        FSHT_CUDA_TRY(cudaEventRecord(p->evs[2 + ((w + 1) & 1)], p->aux2));
+      }
+      FSHT_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->evs[2 + (w & 1)], 0));
+    }
+    unsigned char* lb = nullptr;
+    FSHT_TRY(lam_ready(p, lam, w, &lb));
+    {
+      FSHT_PROF(FSHT_KCAT_ANALYSIS);
+      FSHT_TRY(fsht_launch_tc_gemm(p, w, 0, spin, ws_of(w), eb_of(w), lb, alm0, alm1, nmaps, c0,
+                                   kc, accumulate, which, p->stream));
+    }
+    FSHT_TRY(lam_done(p, lam, w));
+  }
+  if (ahead) {
+    FSHT_CUDA_TRY(cudaEventRecord(p->evs[1], p->aux2));
+    FSHT_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->evs[1], 0));
+  }
+  FSHT_TRY(lam_finish(p));
+  return fsht_launch_analysis_fp64(p, spin, W0, W1, alm0, alm1, nmaps, c0, kc, accumulate, which,
+                                   p->stream, p->d_tcflag);
+}
+
+// One chunk's FP64 synthesis into {G_N, G_S} of W0 (and W1), by the same two routes.
+static int fp64_synthesis(fsht_plan* p, int spin, const double* alm0, const double* alm1,
+                          double2* W0, double2* W1, int nmaps, int c0, int kc) {
+  if (!use_tc(p, spin)) {
+    FSHT_PROF(FSHT_KCAT_SYNTHESIS);
+    return fsht_launch_synthesis_fp64(p, spin, alm0, alm1, W0, W1, nmaps, c0, kc, p->stream);
+  }
+  const LamLaunch lam = spin == 2 ? fsht_launch_tc_lambdaT_pol : fsht_launch_tc_lambdaT;
+  FSHT_TRY(lam_start(p, lam));
+  for (int w = 0; w < p->nwaves; ++w) {
+    {
+      FSHT_PROF(FSHT_KCAT_SLICE);
+      FSHT_TRY(fsht_launch_tc_slice_alm(p, w, alm0, spin == 2 ? alm1 : nullptr, p->d_ws, p->d_eb,
+                                        nmaps, c0, kc, p->stream));
+    }
+    unsigned char* lb = nullptr;
+    FSHT_TRY(lam_ready(p, lam, w, &lb));
+    {
+      FSHT_PROF(FSHT_KCAT_SYNTHESIS);
+      FSHT_TRY(fsht_launch_tc_gemm(p, w, 1, spin, p->d_ws, p->d_eb, lb,
+                                   reinterpret_cast<double*>(W0), reinterpret_cast<double*>(W1),
+                                   nmaps, c0, kc, 0, 3, p->stream));
+    }
+    FSHT_TRY(lam_done(p, lam, w));
+  }
+  FSHT_TRY(lam_finish(p));
+  return fsht_launch_synthesis_fp64(p, spin, alm0, alm1, W0, W1, nmaps, c0, kc, p->stream,
+                                    p->d_tcflag);
+}
+
 int fsht_run_stage(fsht_plan* p, int stage, const void* in, void* out, int nmaps) {
   FSHT_TRY(check_call(p, nmaps, in, out));
   if (nmaps > p->kchunk) {
@@ -908,7 +1055,9 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
       hx->cdone.assign(p->lmax + 1, 0);
     }
     // the first lambda tiles are computed on the auxiliary stream during the FFT
+    const bool tc = !split && use_tc(p, 0);
     if (split) FSHT_TRY(lam_start(p, fsht_launch_split_lambda));
+    if (tc) FSHT_TRY(lam_start(p, fsht_launch_tc_lambda));
     // the chunk's maps as the FFT reads them: device buffer, or host memory read in place
     const double* cmaps = (hx && hx->direct ? hx->direct : maps) + (size_t)c0 * p->npix;
     if (!hx || hx->direct) {
@@ -947,26 +1096,14 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
       }
     } else {
       double2* W1 = work_buf(p, 1, kc);
-      {
-        FSHT_PROF(FSHT_KCAT_ANALYSIS);
-        FSHT_TRY(fsht_launch_analysis_fp64(p, 0, W0, nullptr, alm, nullptr, nmaps, c0, kc, 0, 1,
-                                           p->stream));
-      }
+      FSHT_TRY(fp64_analysis(p, 0, W0, nullptr, alm, nullptr, nmaps, c0, kc, 0, 1, tc));
       for (int it = 0; it < niter; ++it) {
-        {
-          FSHT_PROF(FSHT_KCAT_SYNTHESIS);
-          FSHT_TRY(fsht_launch_synthesis_fp64(p, 0, alm, nullptr, W1, nullptr, nmaps, c0, kc,
-                                              p->stream));
-        }
+        FSHT_TRY(fp64_synthesis(p, 0, alm, nullptr, W1, nullptr, nmaps, c0, kc));
         {
           FSHT_PROF(FSHT_KCAT_RESIDUAL);
           FSHT_TRY(fsht_launch_fourier_residual(p, W0, W1, kc, method, p->stream));
         }
-        {
-          FSHT_PROF(FSHT_KCAT_ANALYSIS);
-          FSHT_TRY(fsht_launch_analysis_fp64(p, 0, W1, nullptr, alm, nullptr, nmaps, c0, kc, 1,
-                                             1, p->stream));
-        }
+        FSHT_TRY(fp64_analysis(p, 0, W1, nullptr, alm, nullptr, nmaps, c0, kc, 1, 1));
       }
     }
     // whatever the waves did not return yet (all of it for FP64 or niter > 0)
@@ -1024,9 +1161,7 @@ int fsht_alm2t(fsht_plan* p, const double* alm, double* maps, int nmaps) {
     if (p->precision == FSHT_PREC_SPLIT) {
       FSHT_TRY(split_synthesis(p, alm, W0, nmaps, c0, kc));
     } else {
-      FSHT_PROF(FSHT_KCAT_SYNTHESIS);
-      FSHT_TRY(fsht_launch_synthesis_fp64(p, 0, alm, nullptr, W0, nullptr, nmaps, c0, kc,
-                                          p->stream));
+      FSHT_TRY(fp64_synthesis(p, 0, alm, nullptr, W0, nullptr, nmaps, c0, kc));
     }
     {
       FSHT_PROF(FSHT_KCAT_FFT_INV);
@@ -1042,11 +1177,8 @@ int fsht_alm2t(fsht_plan* p, const double* alm, double* maps, int nmaps) {
 static int pol_analysis(fsht_plan* p, const double2* WQ, const double2* WU, double* almE,
                         double* almB, int nmaps, int c0, int kc, int accumulate, int which,
                         bool started = false) {
-  if (p->precision != FSHT_PREC_SPLIT) {
-    FSHT_PROF(FSHT_KCAT_ANALYSIS);
-    return fsht_launch_analysis_fp64(p, 2, WQ, WU, almE, almB, nmaps, c0, kc, accumulate, which,
-                                     p->stream);
-  }
+  if (p->precision != FSHT_PREC_SPLIT)
+    return fp64_analysis(p, 2, WQ, WU, almE, almB, nmaps, c0, kc, accumulate, which, started);
   if (!p->d_poltab) {
     fsht_set_error("spin-2 split analysis needs a plan created with FSHT_FLAG_POL");
     return FSHT_EUNSUPPORTED;
@@ -1112,10 +1244,8 @@ static int pol_analysis(fsht_plan* p, const double2* WQ, const double2* WU, doub
 // split form's tiles and waves.
 static int pol_synthesis(fsht_plan* p, const double* almE, const double* almB, double2* WQ,
                          double2* WU, int nmaps, int c0, int kc) {
-  if (p->precision != FSHT_PREC_SPLIT) {
-    FSHT_PROF(FSHT_KCAT_SYNTHESIS);
-    return fsht_launch_synthesis_fp64(p, 2, almE, almB, WQ, WU, nmaps, c0, kc, p->stream);
-  }
+  if (p->precision != FSHT_PREC_SPLIT)
+    return fp64_synthesis(p, 2, almE, almB, WQ, WU, nmaps, c0, kc);
   if (!p->d_poltab) {
     fsht_set_error("spin-2 split synthesis needs a plan created with FSHT_FLAG_POL");
     return FSHT_EUNSUPPORTED;
@@ -1151,8 +1281,10 @@ static int qu_analysis(fsht_plan* p, const double* Q, const double* U, double* a
     const int kc = nmaps - c0 < p->kchunk ? nmaps - c0 : p->kchunk;
     double2* WQ = work_buf(p, 0, kc);
     double2* WU = work_buf(p, 1, kc);
-    const bool pre = p->precision == FSHT_PREC_SPLIT && p->d_poltab;
-    if (pre) FSHT_TRY(lam_start(p, fsht_launch_split_lambda_pol));   // overlaps the FFTs
+    const bool split = p->precision == FSHT_PREC_SPLIT;
+    const bool pre = split ? p->d_poltab != nullptr : use_tc(p, 2);
+    if (pre)                                                         // overlaps the FFTs
+      FSHT_TRY(lam_start(p, split ? fsht_launch_split_lambda_pol : fsht_launch_tc_lambda_pol));
     {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
       FSHT_TRY(fsht_launch_ring_fft_fwd(p, Q + (size_t)c0 * p->npix, p->npix, kc, WQ, p->stream));

@@ -311,87 +311,88 @@ __global__ void __launch_bounds__(512, 2) k_ring_fft_inv(InvArgs a) {
 // on exit.  prefix = 0 ("old" method, t2alm_iter_old): Y sums all m'.  prefix = 1
 // ("new" method, t2alm_iter, sht_main.f90:171-264): the reference forms each
 // order's residual right after its own synthesis, so Y only holds m' <= m.
-// Thread per half-spectrum bin p in [0, n/2]: it owns every m that lands in p or
-// n - p, walks them in ascending order and needs no shared spectrum.
+// Every m that lands in bin p or n - p is p + a n or a n - p, and e^{i n phi0} = (-1)^s is
+// real, so with Z_p = sum (-1)^{a s} {G_m or conj G_m} the residual needs no phases:
+//   F^R_m = F^X_m - n (-1)^{a s} {Z_p or conj Z_p}
+// (p = 0 and n/2 are their own mirrors: Z is folded with its conjugate).  That leaves about 12
+// FP64 operations per entry of 40; FP64 runs at two per clock per SM.
+// A warp owns one bin, its lanes maps: every access is one contiguous KB of 32-byte entries
+// (with bins on the lanes each entry was a sector of its own, nnorth kc 32 B apart).  100 maps
+// at nside 128 / lmax 383 move 0.94 GB.
 struct ResArgs {
   const double2* X;
   double2* GR;
-  int kc, maps_per_block;
-  int nside, lmax, nnorth, ring_base, prefix;
+  int kc;
+  int nside, lmax, nnorth, prefix;
   const FshtRingFFT* rfs;
   const int* ring_i0;
 };
 
-__global__ void __launch_bounds__(512) k_fourier_residual(ResArgs a) {
-  extern __shared__ double2 smem[];
-  const int i = a.ring_base + blockIdx.x;
+constexpr int kResBins = 8;      // bins (warps) per CTA
+
+__global__ void __launch_bounds__(32 * kResBins) k_fourier_residual(ResArgs a) {
+  const int i = blockIdx.x;
   const int n = a.rfs[i].n;
-  double2* phf = smem;   // lmax+1: exp(+i m phi0)
-  const int tid = threadIdx.x, nt = blockDim.x;
   const bool equator = (i == a.nnorth - 1);
   const int sflag = ring_phase_flag(a.nside, i);
-  int mtop = a.lmax;
-  while (mtop >= 0 && a.ring_i0[mtop] > i) --mtop;
-  for (int m = tid; m <= mtop; m += nt) {
-    double s = 0.0, c = 1.0;
-    if (sflag) {
-      long long r = (long long)m % (2LL * n);
-      sincospi((double)r / (double)n, &s, &c);
-    }
-    phf[m] = make_double2(c, s);
+  // highest kept order (ring_i0 is non-decreasing in m)
+  int lo = -1, hi = a.lmax;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (a.ring_i0[mid] > i) hi = mid - 1;
+    else lo = mid;
   }
-  __syncthreads();
+  const int mtop = lo;
+  const int p = blockIdx.y * kResBins + (threadIdx.x >> 5);
+  if (p > n / 2 || p > mtop) return;
+  const bool self = p == 0 || 2 * p == n;       // the bin is its own mirror
   const long long stride_m = (long long)a.nnorth * a.kc * 2;
-  const int k_begin = blockIdx.y * a.maps_per_block;
-  const int k_end = min(a.kc, k_begin + a.maps_per_block);
-  const int half = n / 2;
   const double dn = (double)n;
-  for (int k = k_begin; k < k_end; ++k) {
+  // order t of the ascending list: p, n - p, n + p, 2n - p, ... (p, n + p, ... when self)
+  auto order = [&](int t) { return self ? p + t * n : ((t + 1) >> 1) * n + ((t & 1) ? -p : p); };
+  // multiple of n, for the sign (-1)^{a s}
+  auto wraps = [&](int t) { return self ? t : (t + 1) >> 1; };
+  for (int k = threadIdx.x & 31; k < a.kc; k += 32) {
     const long long base = ((long long)i * a.kc + k) * 2;
-    for (int p = tid; p <= half; p += nt) {
-      const int pn = (n - p) % n;     // the mirrored bin (p itself for p = 0, n/2)
-      // ascending merge of {p + t n} and {pn + t n}; when p == pn one list
-      int ma = p, mb = (pn == p) ? INT_MAX : pn;
-      double2 yN = make_double2(0.0, 0.0), yS = make_double2(0.0, 0.0);
-      // pass 0 (old method only): totals; pass 1: emit residuals (accumulating
-      // the prefix first when prefix = 1)
-      for (int pass = a.prefix ? 1 : 0; pass < 2; ++pass) {
-        int ua = ma, ub = mb;
-        while (true) {
-          const int m = min(ua, ub);
-          if (m > mtop) break;
-          const bool inA = (m == ua);
-          if (inA) ua += n; else ub += n;
-          const double2* g = a.GR + base + (long long)m * stride_m;
-          const double c = (m == 0) ? 0.5 : 1.0;
-          const double2 hN = cscale(cmul(phf[m], g[0]), c);
-          const double2 hS = equator ? make_double2(0.0, 0.0) : cscale(cmul(phf[m], g[1]), c);
-          const int q = m % n;
-          // this m adds to bin p: h if q == p, conj(h) if q == n - p (both when p == pn)
-          if (pass == 0 || a.prefix) {
-            if (q == p) { yN = cadd(yN, hN); yS = cadd(yS, hS); }
-            if (q == pn) { yN = cadd(yN, cconj(hN)); yS = cadd(yS, cconj(hS)); }
-          }
-          if (pass == 1) {
-            // Y[q] = Y[p] when q == p, conj(Y[p]) otherwise
-            const double2 vN = (q == p) ? yN : cconj(yN);
-            const double2 vS = (q == p) ? yS : cconj(yS);
-            const double2 e = cconj(phf[m]);
-            const double2 rN = cscale(cmul(e, vN), dn);
-            const double2* x = a.X + base + (long long)m * stride_m;
-            double2* o = a.GR + base + (long long)m * stride_m;
-            const double2 x0 = x[0], x1 = x[1];
-            if (equator) {
-              o[0] = csub(x0, rN);
-              o[1] = csub(x1, rN);
-            } else {
-              const double2 rS = cscale(cmul(e, vS), dn);
-              o[0] = csub(x0, cadd(rN, rS));
-              o[1] = csub(x1, csub(rN, rS));
-            }
-          }
+    double2 zN = make_double2(0.0, 0.0), zS = make_double2(0.0, 0.0);
+    auto add = [&](int t, double2 gN, double2 gS) {
+      double sg = (sflag && (wraps(t) & 1)) ? -1.0 : 1.0;
+      const double sy = (!self && (t & 1)) ? -sg : sg;       // conj for a n - p
+      if (self) {
+        // h + conj h: 2 Re(e^{i p phi0} G): p = 0, or n/2 with e^{i p phi0} = i^s
+        if (p == 0) {
+          if (t > 0) sg *= 2.0;                              // c_0 = 1/2 for m = 0
+          zN.x = fma(sg, gN.x, zN.x);
+          zS.x = fma(sg, gS.x, zS.x);
+        } else if (sflag) {
+          zN.y = fma(2.0 * sg, gN.y, zN.y);                  // conj(i) Re(i G) = i Im G
+          zS.y = fma(2.0 * sg, gS.y, zS.y);
+        } else {
+          zN.x = fma(2.0 * sg, gN.x, zN.x);
+          zS.x = fma(2.0 * sg, gS.x, zS.x);
         }
+        return;
       }
+      zN = make_double2(fma(sg, gN.x, zN.x), fma(sy, gN.y, zN.y));
+      zS = make_double2(fma(sg, gS.x, zS.x), fma(sy, gS.y, zS.y));
+    };
+    if (!a.prefix) {
+      // old method: the bin's totals over all orders first
+      for (int t = 0, m; (m = order(t)) <= mtop; ++t) {
+        const double2* g = a.GR + base + (long long)m * stride_m;
+        add(t, g[0], equator ? make_double2(0.0, 0.0) : g[1]);
+      }
+    }
+    for (int t = 0, m; (m = order(t)) <= mtop; ++t) {
+      const double2* x = a.X + base + (long long)m * stride_m;
+      double2* o = a.GR + base + (long long)m * stride_m;
+      const double2 x0 = x[0], x1 = x[1];
+      if (a.prefix) add(t, o[0], equator ? make_double2(0.0, 0.0) : o[1]);
+      const double sg = (sflag && (wraps(t) & 1)) ? -dn : dn;
+      const double sy = (!self && (t & 1)) ? -sg : sg;
+      const double2 sum = cadd(zN, zS), dif = csub(zN, zS);   // zS = 0 on the equator
+      o[0] = make_double2(fma(-sg, sum.x, x0.x), fma(-sy, sum.y, x0.y));
+      o[1] = make_double2(fma(-sg, dif.x, x1.x), fma(-sy, dif.y, x1.y));
     }
   }
 }
@@ -699,14 +700,12 @@ int fsht_launch_fourier_residual(fsht_plan* p, const double2* X, double2* GR, in
   a.nside = p->nside;
   a.lmax = p->lmax;
   a.nnorth = p->nnorth;
-  a.ring_base = 0;
   a.prefix = prefix;
   a.rfs = p->d_rfft;
   a.ring_i0 = p->d_ring_i0;
-  a.maps_per_block = p->fft_mpb > 0 ? p->fft_mpb : maps_per_block_for(kc, p->nnorth);
-  dim3 grid(p->nnorth, (kc + a.maps_per_block - 1) / a.maps_per_block);
-  FSHT_TRY(fsht_smem_limit((const void*)k_fourier_residual, (size_t)(p->fft_smem)));
-  k_fourier_residual<<<grid, p->fft_threads > 0 ? p->fft_threads : 512, p->fft_smem, s>>>(a);
+  const int bins = (p->lmax < 2 * p->nside ? p->lmax : 2 * p->nside) + 1;
+  const dim3 grid(p->nnorth, (bins + kResBins - 1) / kResBins);
+  k_fourier_residual<<<grid, 32 * kResBins, 0, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }
