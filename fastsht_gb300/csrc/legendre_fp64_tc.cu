@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(128 * NF) k_tc_slice_alm(TcSliceAArgs a) {
 }
 
 // ------------------------------------------------------------------ contraction
-// Persistent, one CTA per SM.  A unit is a 128-column (64 maps x Re/Im, the UMMA M side = TMEM
+// Persistent, one CTA per SM, units from the queue of split_common.cuh.  A unit is a 128-column (64 maps x Re/Im, the UMMA M side = TMEM
 // lanes) x N-row tile: N <= 128 l-rows of one parity (DIR 0, analysis) or rings (DIR 1,
 // synthesis), over one or two phases of one or two segments:
 //   DIR 0          one phase;  spin 2: lambda1 against the field, lambda2 against i x the other
@@ -640,7 +640,7 @@ constexpr uint32_t kTcStageBytes = 2 * kHalfBytes;              // 32 KB
 constexpr size_t kTcSmem = (size_t)kTcStages * kTcStageBytes;
 
 struct TcGemmArgs {
-  int lmax, nnorth, ngroups, q0, ntmax, nunits;
+  int lmax, nnorth, ngroups, q0, q1, ntmax, nunits;
   int nfield, field0;          // spin 2: fields of this call (E/Q = 0, B/U = 1)
   int accumulate, unit_bits, eag;
   size_t row_bytes;
@@ -683,7 +683,7 @@ __device__ __forceinline__ TcUnit tc_unit(const TcGemmArgs& a, int u) {
     r >>= 1;
   }
   w.t = r % a.ntmax;
-  w.qi = r / a.ntmax;
+  w.qi = wave_order(a.q0, a.q1, r / a.ntmax) - a.q0;
   w.m = m_of_q(a.q0 + w.qi, a.lmax);
   const int i0 = a.ring_i0[w.m];
   const int K = a.nnorth - i0;
@@ -757,10 +757,11 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
   constexpr int NPH = DIR == 0 ? 1 : 2, NSEG = SPIN == 2 ? 2 : 1;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ TcSmemHdr h;
-  __shared__ double s_fac[kRows];
+  __shared__ UnitQueue uq;
+  __shared__ double s_fac[kEpiThreads / 32][64];      // per epilogue warp: its rows' factors
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = tc::warp_index();
   volatile int* abort = &h.abort;
   if (tid == 0) {
     for (int s = 0; s < kTcStages; ++s) {
@@ -772,6 +773,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
       tc::mbar_init(&h.tempty[s], kEpiThreads);
     }
     tc::mbar_init(&h.fin, 1);
+    uq_init(uq, kEpiThreads + 32);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -784,25 +786,21 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
   uint32_t n_loaded = 0;
   if (tid == kEpiThreads) {
     uint32_t i = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
+    uq_walk(uq, a.nunits, 0, abort, [&](int u) -> bool {
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
-      if (w.nk == 0) continue;
-      for (int s = 0; s < NPH * NSEG && ok; ++s) {
+      if (w.nk == 0) return true;
+      for (int s = 0; s < NPH * NSEG; ++s) {
         const unsigned char *cols, *rows;
         int sign;
         tc_segment<DIR, SPIN>(a, w, s / NSEG, s % NSEG, cols, rows, sign);
-        for (int k0 = 0; k0 < w.nk && ok; k0 += kPartK) {
+        for (int k0 = 0; k0 < w.nk; k0 += kPartK) {
           const int nk = min(w.nk - k0, kPartK);
           // pass 0: the low half (planes 0..3) of each k-step; pass 1: both halves
           for (int j = 0; j < 3 * nk; ++j, ++i) {
             const int k = k0 + (j < nk ? j : (j - nk) >> 1);
             const uint32_t half = j < nk ? 0 : (uint32_t)((j - nk) & 1);
             const uint32_t st = i % kTcStages;
-            if (!tc::mbar_wait(&h.empty[st], ((i / kTcStages) & 1) ^ 1, abort)) {
-              ok = false;
-              break;
-            }
+            if (!tc::mbar_wait(&h.empty[st], ((i / kTcStages) & 1) ^ 1, abort)) return false;
             unsigned char* dst = smem + st * kTcStageBytes;
             tc::mbar_arrive_expect_tx(&h.full[st], kTcStageBytes);
             tc::bulk_g2s(dst, cols + (size_t)k * kStepBytes + half * kHalfBytes, kHalfBytes,
@@ -813,12 +811,15 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
           }
         }
       }
-    }
-  } else if (tid == kEpiThreads + 32) {
+      return true;
+    });
+  } else if (warp == kEpiThreads / 32 + 1) {
     const uint32_t s_u = tc::smem_u32(smem);
     uint32_t i = 0, use = 0;       // stages consumed, passes issued (one use of every slot each)
     bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
+    for (uint32_t n = 0; ok; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (!__all_sync(0xffffffffu, u >= 0)) break;
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
       if (w.nk == 0) continue;
       const uint32_t idesc = tc::umma_idesc_bf16(kRows, w.N);
@@ -832,7 +833,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
               break;
             }
             tc::tc_fence_after();
-            const uint32_t ca = s_u + st * kTcStageBytes, ra = ca + kHalfBytes;
+            const uint64_t ca = tc::umma_desc(s_u + st * kTcStageBytes, 128, 256);
+            const uint64_t ra = tc::umma_desc_add(ca, kHalfBytes);
 #pragma unroll
             for (int lev = 0; lev < 4; ++lev) {
               if (k == 0 && use > 0) {
@@ -844,12 +846,12 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
               }
 #pragma unroll
               for (int aa = 0; aa <= lev; ++aa)
-                tc::umma_bf16(tmem + lev * kCols, tc::umma_desc(ca + aa * kPlaneBytes, 128, 256),
-                              tc::umma_desc(ra + (lev - aa) * kPlaneBytes, 128, 256), idesc,
-                              (k > 0 || aa > 0) ? 1u : 0u);
-              if (k == nk - 1) tc::umma_commit(&h.tfull[lev]);
+                tc::umma_bf16_warp(tmem + lev * kCols, tc::umma_desc_add(ca, aa * kPlaneBytes),
+                                   tc::umma_desc_add(ra, (lev - aa) * kPlaneBytes), idesc,
+                                   (k > 0 || aa > 0) ? 1u : 0u);
+              if (k == nk - 1) tc::umma_commit_warp(&h.tfull[lev]);
             }
-            if (ok) tc::umma_commit(&h.empty[st]);
+            if (ok) tc::umma_commit_warp(&h.empty[st]);
           }
           ++use;
           for (int k = 0; k < nk && ok; ++k, i += 2) {           // pass 1
@@ -860,9 +862,11 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
               break;
             }
             tc::tc_fence_after();
-            const uint32_t ca = s_u + st * kTcStageBytes, cb = s_u + st1 * kTcStageBytes;
-            auto plane = [&](int d) { return d < 4 ? ca + d * kPlaneBytes
-                                                   : cb + (d - 4) * kPlaneBytes; };
+            const uint64_t ca = tc::umma_desc(s_u + st * kTcStageBytes, 128, 256);
+            const uint64_t cb = tc::umma_desc(s_u + st1 * kTcStageBytes, 128, 256);
+            auto plane = [&](int d) {
+              return tc::umma_desc_add(d < 4 ? ca : cb, (uint32_t)(d & 3) * kPlaneBytes);
+            };
 #pragma unroll
             for (int lev = 4; lev < 8; ++lev) {
               if (k == 0) {
@@ -874,14 +878,14 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
               }
 #pragma unroll
               for (int aa = 0; aa <= lev; ++aa)
-                tc::umma_bf16(tmem + (lev - 4) * kCols, tc::umma_desc(plane(aa), 128, 256),
-                              tc::umma_desc(plane(lev - aa) + kHalfBytes, 128, 256), idesc,
-                              (k > 0 || aa > 0) ? 1u : 0u);
-              if (k == nk - 1) tc::umma_commit(&h.tfull[lev - 4]);
+                tc::umma_bf16_warp(tmem + (lev - 4) * kCols, plane(aa),
+                                   tc::umma_desc_add(plane(lev - aa), kHalfBytes), idesc,
+                                   (k > 0 || aa > 0) ? 1u : 0u);
+              if (k == nk - 1) tc::umma_commit_warp(&h.tfull[lev - 4]);
             }
             if (ok) {
-              tc::umma_commit(&h.empty[st]);
-              tc::umma_commit(&h.empty[st1]);
+              tc::umma_commit_warp(&h.empty[st]);
+              tc::umma_commit_warp(&h.empty[st1]);
             }
           }
           ++use;
@@ -889,8 +893,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
       }
     }
   } else if (tid < kEpiThreads) {
-    // epilogue: no early exit (the named barriers want all 256 threads); after an expired wait
-    // the remaining slots are walked without work
+    // epilogue: each warp works alone (no barrier among them); after an expired wait the
+    // remaining slots are walked without work
     const int lane = tid & 31;
     const int c = ((warp & 3) << 5) + lane;              // tile column: 2 map + comp
     const int comp = c & 1;
@@ -900,18 +904,20 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
     // level weights 2^(unit_bits - 8 s) as (float factor, integer multiplier): the level-0 sum
     // goes into the high word, the others by 32 x 32 -> 64-bit multiply-adds with <= 2^30
     uint32_t use = 0;
-    for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
+    for (uint32_t n = 0;; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (!__all_sync(0xffffffffu, u >= 0)) break;
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
       if (w.nk == 0) continue;
       const int map = w.g * kGroupMaps + (c >> 1);
       const int nrow = min(64, w.nrows - rbeg);
       if (DIR == 0) {
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-        if (tid < kRows) {
-          const int l = w.row0 + 2 * tid;
-          s_fac[tid] = l <= a.lmax ? a.tab[tri_off(w.m, a.lmax) + (l - w.m)].dm * a.pa : 0.0;
+        __syncwarp();
+        for (int j = lane; j < 64; j += 32) {
+          const int l = w.row0 + 2 * (rbeg + j);
+          s_fac[warp][j] = l <= a.lmax ? a.tab[tri_off(w.m, a.lmax) + (l - w.m)].dm * a.pa : 0.0;
         }
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+        __syncwarp();
       }
       const int4 fl = *reinterpret_cast<const int4*>(a.flags +
                                                      ((long long)w.m * a.ngroups + w.g) * 4);
@@ -964,7 +970,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
 #pragma unroll
           for (int j = 0; j < 64; ++j) {
             if (j >= nrow) break;
-            const double v = i64_scaled(acc[j], e) * s_fac[rbeg + j];
+            const double v = i64_scaled(acc[j], e) * s_fac[warp][j];
             double* d = dst + (long long)(2 * j) * a.ld;
             *d = a.accumulate ? *d + v : v;
           }
@@ -991,8 +997,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
   }
   // the UMMA issuer waits for its last products before TMEM is released, the loader for its
   // last copies
-  if (tid == kEpiThreads + 32) {
-    tc::umma_commit(&h.fin);
+  if (warp == kEpiThreads / 32 + 1) {
+    tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
   }
@@ -1037,20 +1043,10 @@ int tc_bits_synthesis(const fsht_plan* p) {
   return std::min(46, 51 - ceil_log2((2LL * (p->lmax / 2 + 1) + 4) / 5 + 1));
 }
 
-int sm_count(int* nsm) {
-  int dev = 0;
-  FSHT_CUDA_TRY(cudaGetDevice(&dev));
-  FSHT_CUDA_TRY(cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev));
-  return FSHT_OK;
-}
-
 template <int DIR, int SPIN>
 int launch_tc_gemm(const TcGemmArgs& a, cudaStream_t s) {
   FSHT_TRY(fsht_smem_limit((const void*)k_tc_gemm<DIR, SPIN>, kTcSmem));
-  int nsm = 0;
-  FSHT_TRY(sm_count(&nsm));
-  const int grid = a.nunits < nsm ? a.nunits : nsm;
-  if (grid > 0) k_tc_gemm<DIR, SPIN><<<grid, kThreadsG, kTcSmem, s>>>(a);
+  if (a.nunits > 0) k_tc_gemm<DIR, SPIN><<<a.nunits, kThreadsG, kTcSmem, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }
@@ -1188,6 +1184,7 @@ int fsht_launch_tc_gemm(fsht_plan* p, int w, int dir, int spin, const unsigned c
   a.nnorth = p->nnorth;
   a.ngroups = tc_groups(kc);
   a.q0 = wv[0];
+  a.q1 = wv[1];
   a.ntmax = dir == 0 ? wv[2] : wv[4];
   a.nfield = 1;
   a.field0 = 0;

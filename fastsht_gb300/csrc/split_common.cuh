@@ -78,6 +78,94 @@ __host__ __device__ __forceinline__ long long tri_off(int m, int lmax) {
   return (long long)m * (2LL * lmax + 3 - m) / 2;
 }
 
+// The r-th order (as a pair-order index) of the wave [q0, q1) by ascending m: the work of an
+// order falls with m (fewer l, fewer kept rings), so units handed out in this order end on
+// small ones.
+__device__ __forceinline__ int wave_order(int q0, int q1, int r) {
+  const int e0 = q0 + (q0 & 1);                          // first even index: m = q / 2
+  const int ne = q1 > e0 ? (q1 - e0 + 1) / 2 : 0;
+  if (r < ne) return e0 + 2 * r;
+  const int o1 = (q1 & 1) ? q1 - 2 : q1 - 1;             // last odd index: m = lmax - q / 2
+  return o1 - 2 * (r - ne);
+}
+
+// Work units of a contraction CTA.  The grid has one CTA per unit; a running CTA takes over the
+// next unstarted one (cluster launch control) instead of walking a fixed stride, so the units
+// spread over the SMs by their actual cost, also while other kernels hold some SMs.  (A fixed
+// stride of 152 resonated with the unit order: the busiest SM had 2.0 times the mean work at
+// nside 256, and k_tc_gemm's SMs were active 61 % of its time.)  stride > 0 keeps the fixed
+// walk, for launches capped to some SMs.  The copy thread asks for the next unit while it loads
+// the current one and passes indices through a small ring; -1 ends it.
+constexpr int kUq = 4;
+struct __align__(16) UnitQueue {
+  uint4 resp;
+  uint64_t clc, full[kUq], empty[kUq];
+  int unit[kUq];
+};
+
+__device__ __forceinline__ void uq_init(UnitQueue& q, uint32_t takers) {
+  tc::mbar_init(&q.clc, 1);
+  for (int i = 0; i < kUq; ++i) {
+    tc::mbar_init(&q.full[i], 1);
+    tc::mbar_init(&q.empty[i], takers);
+  }
+}
+// Copy thread: pass on unit u (the n-th, -1: no more).
+__device__ __forceinline__ bool uq_put(UnitQueue& q, uint32_t n, int u, volatile int* abort) {
+  if (!tc::mbar_wait(&q.empty[n % kUq], ((n / kUq) & 1) ^ 1, abort)) return false;
+  *const_cast<volatile int*>(&q.unit[n % kUq]) = u;
+  tc::mbar_arrive(&q.full[n % kUq]);
+  return true;
+}
+// Every other role's threads: the n-th unit, or -1 (also after an expired wait).
+__device__ __forceinline__ int uq_take(UnitQueue& q, uint32_t n, volatile int* abort) {
+  if (!tc::mbar_wait(&q.full[n % kUq], (n / kUq) & 1, abort)) return -1;
+  const int u = *const_cast<volatile int*>(&q.unit[n % kUq]);
+  tc::mbar_arrive(&q.empty[n % kUq]);
+  return u;
+}
+// Copy thread: ask for the next unit / the answer to the n-th request (-1: none left).
+__device__ __forceinline__ void uq_request(UnitQueue& q) {
+  tc::mbar_arrive_expect_tx(&q.clc, 16);
+  tc::clc_try_cancel(&q.resp, &q.clc);
+}
+__device__ __forceinline__ int uq_answer(UnitQueue& q, uint32_t n, volatile int* abort) {
+  if (!tc::mbar_wait(&q.clc, n & 1, abort)) return -1;
+  const int u = tc::clc_first_cta(&q.resp);
+  tc::fence_proxy_async();
+  return u;
+}
+// The whole walk of the copy thread: f(u) loads unit u and returns false on an expired wait.
+// On every path the last request has been answered (or its bounded wait has run out).
+template <typename F>
+__device__ __forceinline__ void uq_walk(UnitQueue& q, int nunits, int stride, volatile int* abort,
+                                        F f) {
+  int u = blockIdx.x;
+  uint32_t n = 0;
+  while (true) {
+    if (stride == 0) uq_request(q);
+    const bool ok = uq_put(q, n, u, abort) && f(u);
+    int next;
+    if (stride == 0) {
+      if (!ok) {
+        for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
+          if (tc::mbar_try_wait(&q.clc, n & 1)) break;
+        return;
+      }
+      next = uq_answer(q, n, abort);
+    } else {
+      if (!ok) return;
+      next = u + stride < nunits ? u + stride : -1;
+    }
+    ++n;
+    if (next < 0) {
+      uq_put(q, n, -1, abort);
+      return;
+    }
+    u = next;
+  }
+}
+
 // per wave: q0, q1, max l-tiles, max ring K-chunks (analysis), max 128-ring blocks,
 // max l-steps, max l K-chunks (synthesis)
 constexpr int kWaveInts = 7;

@@ -65,6 +65,28 @@ __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Cluster launch control: ask to take over the next CTA of the grid that has not started (the
+// 16-byte answer completes on bar), and its blockIdx.x, or -1 when there is none left.
+__device__ __forceinline__ void clc_try_cancel(uint4* resp, uint64_t* bar) {
+  asm volatile(
+      "clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 "
+      "[%0], [%1];" ::"r"(smem_u32(resp)),
+      "r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ int clc_first_cta(const uint4* resp) {
+  uint32_t x, ok;
+  asm volatile(
+      "{\n.reg .pred p;\n.reg .b128 r;\nld.shared.b128 r, [%2];\n"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n"
+      "selp.u32 %1, 1, 0, p;\nmov.u32 %0, 0;\n"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %0, r;\n}"
+      : "=r"(x), "=r"(ok)
+      : "r"(smem_u32(resp))
+      : "memory");
+  return ok ? (int)x : -1;
+}
+
 // ------------------------------------------------------------------ UMMA
 // Shared-memory matrix descriptor, no swizzle, K-major core matrices (8 rows x 16 B):
 // lbo = byte stride between core matrices adjacent along K, sbo = along M/N.
@@ -87,6 +109,33 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
       "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// The same from a whole warp, which elects the issuing lane: in warp-uniform code the
+// descriptors stay in uniform registers, where a branch to a single thread makes every operand
+// of every product a move into them (about 200 clocks per product of 62 on the tensor pipe, in
+// k_tc_gemm).
+__device__ __forceinline__ void umma_bf16_warp(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                               uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p, q;\nsetp.ne.b32 p, %4, 0;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// A descriptor moved by `bytes` (a multiple of 16) of shared memory.
+__device__ __forceinline__ uint64_t umma_desc_add(uint64_t desc, uint32_t bytes) {
+  return desc + (bytes >> 4);
+}
+// Warp index in a form the compiler knows to be warp-uniform.
+__device__ __forceinline__ int warp_index() {
+  return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
+}
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
+  asm volatile(
+      "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}" ::"r"(
+          smem_u32(bar))
       : "memory");
 }
 // Arrive on bar when every previously issued tcgen05.mma of this thread completes.
