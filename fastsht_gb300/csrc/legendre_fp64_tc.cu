@@ -5,10 +5,10 @@
 // exact integer products.  Both operands become 62-bit fixed-point numbers against a power-of-two
 // scale, cut into eight balanced base-256 digits (|d0| <= 64, |d1..7| <= 128) that BF16 holds
 // exactly.  The 36 digit products of level a + b <= 7 run as BF16 UMMAs with FP32 accumulation,
-// one accumulator per level: over the 192 summands of a part the sums of levels 0..4 stay
-// below 2^24 whatever the digits are (at most (s + 1) 192 2^14), so they are exact integers;
-// levels 5..7 carry weights from 2^-40 of the leading product down, where an FP32 rounding is
-// far below FP64's.  The epilogue adds every level into one 64-bit integer per output element
+// one accumulator per level: over the 256 summands of a part the sums of levels 0..4 stay
+// within 2^24 whatever the digits are (level s >= 1: 256 (2 2^13 + (s - 1) 2^14)), so they are
+// exact integers; levels 5..7 carry weights from 2^-40 of the leading product down, where an
+// FP32 rounding is far below FP64's.  The epilogue adds every level into one 64-bit integer per output element
 // (unit 2^-unit_bits), so no FP64 instruction runs before the last conversion and the order of
 // the parts does not matter.
 //
@@ -35,7 +35,7 @@ constexpr int kPlanes = 8;
 constexpr uint32_t kPlaneBytes = kRows * kKStep * 2;              // 4 KB: 128 rows x 16 summands
 constexpr uint32_t kStepBytes = kPlanes * kPlaneBytes;            // 32 KB per operand and k-step
 constexpr uint32_t kHalfBytes = kStepBytes / 2;                   // four planes
-constexpr int kPartK = 12;                                        // k-steps per part (192 summands)
+constexpr int kPartK = 16;                                        // k-steps per part (256 summands)
 constexpr unsigned long long kBias = 0x8080808080808080ull;
 constexpr int kFixBits = 62;       // |v| < 2^E becomes |X| < 2^62
 constexpr int kMaxExp = 900;       // column maxima beyond 2^+-900 go to the FMA kernels
@@ -635,6 +635,7 @@ __global__ void __launch_bounds__(128 * NF) k_tc_slice_alm(TcSliceAArgs a) {
 // copies (16 KB of each operand per stage), warp 9 lane 0: UMMAs.
 // The map columns are on the lanes, so a warp's alm stores are two 128-byte segments and its
 // phase-matrix stores whole {Re, Im} pairs, with no staging through shared memory.
+constexpr int kTcThreads = kEpiThreads + 96;     // epilogue, copy thread's warp, two UMMA warps
 constexpr int kTcStages = 6;
 constexpr uint32_t kTcStageBytes = 2 * kHalfBytes;              // 32 KB
 constexpr size_t kTcSmem = (size_t)kTcStages * kTcStageBytes;
@@ -725,11 +726,16 @@ __device__ __forceinline__ void tc_segment(const TcGemmArgs& a, const TcUnit& w,
           (size_t)((sg * 2 + lpar) * w.nt + w.t) * w.nk) * kStepBytes;
 }
 
-// acc += level sums of one slot, 64 rows per thread: LEV0 adds weight 2^(32 + x) as the high
-// word, other levels the rounded f L (integer, |f L| < 2^31) times m.
-template <bool LEV0>
-__device__ __forceinline__ void tc_drain(uint32_t taddr, int nrow, float f, int mul,
-                                         long long (&acc)[64]) {
+// acc += level sums L of one slot, 64 rows per thread: f L (an integer, or rounded to one) times
+// mul, in the high word (HI) or as a 32 x 32 + 64-bit multiply-add.  The integer comes out of
+// the mantissa of f L + 1.5 2^23, so a sum costs a float FMA, a maximum and the multiply-add (the
+// conversion instruction and its 64-bit handling took three times as long, with the UMMA warps
+// waiting); the bias 0x4B400000 stays in acc until the end of the unit.  Sums of 2^22 and more,
+// which need extreme digits throughout, take the conversion.
+constexpr uint32_t kMagic = 0x4B400000u;
+template <bool HI>
+__device__ __forceinline__ void tc_drain(uint32_t taddr, int nrow, float f, uint32_t mul,
+                                         unsigned long long (&acc)[64]) {
 #pragma unroll
   for (int c = 0; c < 64; c += 32) {
     if (c >= nrow) break;
@@ -737,23 +743,30 @@ __device__ __forceinline__ void tc_drain(uint32_t taddr, int nrow, float f, int 
     tc::tmem_ld16(taddr + c, v0);
     tc::tmem_ld16(taddr + c + 16, v1);
     tc::tmem_wait_ld();
+    float mx = 0.f;
+    auto L = [&](int j) { return __uint_as_float(j < 16 ? v0[j & 15] : v1[j & 15]); };
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float L = __uint_as_float(j < 16 ? v0[j & 15] : v1[j & 15]);
-      if (LEV0) {
-        const uint32_t hi = (uint32_t)((unsigned long long)acc[c + j] >> 32) +
-                            (uint32_t)__float2int_rn(L) * (uint32_t)mul;
-        acc[c + j] =
-            (long long)(((unsigned long long)hi << 32) | (unsigned long long)(uint32_t)acc[c + j]);
-      } else {
-        acc[c + j] += (long long)__float2int_rn(L * f) * (long long)mul;
-      }
+    for (int j = 0; j < 32; ++j) mx = fmaxf(mx, fabsf(L(j)));
+    const bool big = __any_sync(0xffffffffu, mx * fabsf(f) >= 0x1p22f);
+    auto put = [&](int j, uint32_t n) {
+      if (HI)
+        acc[c + j] = ((unsigned long long)((uint32_t)(acc[c + j] >> 32) + n * mul) << 32) |
+                     (uint32_t)acc[c + j];
+      else
+        acc[c + j] += (unsigned long long)n * mul;
+    };
+    if (!big) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) put(j, __float_as_uint(fmaf(L(j), f, 12582912.f)));
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) put(j, (uint32_t)__float2int_rn(L(j) * f) + kMagic);
     }
   }
 }
 
 template <int DIR, int SPIN>
-__global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
+__global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
   constexpr int NPH = DIR == 0 ? 1 : 2, NSEG = SPIN == 2 ? 2 : 1;
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ TcSmemHdr h;
@@ -766,14 +779,14 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
   if (tid == 0) {
     for (int s = 0; s < kTcStages; ++s) {
       tc::mbar_init(&h.full[s], 1);
-      tc::mbar_init(&h.empty[s], 1);
+      tc::mbar_init(&h.empty[s], 2);                     // both UMMA warps
     }
     for (int s = 0; s < 4; ++s) {
       tc::mbar_init(&h.tfull[s], 1);
-      tc::mbar_init(&h.tempty[s], kEpiThreads);
+      tc::mbar_init(&h.tempty[s], kEpiThreads / 32);
     }
-    tc::mbar_init(&h.fin, 1);
-    uq_init(uq, kEpiThreads + 32);
+    tc::mbar_init(&h.fin, 2);
+    uq_init(uq, kEpiThreads / 32 + 2);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -813,22 +826,26 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
       }
       return true;
     });
-  } else if (warp == kEpiThreads / 32 + 1) {
-    const uint32_t s_u = tc::smem_u32(smem);
+  } else if (warp > kEpiThreads / 32) {
+    // UMMA warps: slots 0 and 3, and slots 1 and 2 (5 of 10 and 13 of 26 products each)
+    const int side = warp - kEpiThreads / 32 - 1;
+    const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
+    const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
     uint32_t i = 0, use = 0;       // stages consumed, passes issued (one use of every slot each)
     bool ok = true;
     for (uint32_t n = 0; ok; ++n) {
       const int u = uq_take(uq, n, abort);
-      if (!__all_sync(0xffffffffu, u >= 0)) break;
+      if (u < 0) break;
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
-      if (w.nk == 0) continue;
-      const uint32_t idesc = tc::umma_idesc_bf16(kRows, w.N);
+      // (the shuffles tell the compiler that these are warp-uniform)
+      const int unk = tc::uniform(w.nk);
+      const uint32_t idesc = tc::umma_idesc_bf16(kRows, tc::uniform(w.N));
       for (int s = 0; s < NPH * NSEG && ok; ++s) {
-        for (int k0 = 0; k0 < w.nk && ok; k0 += kPartK) {
-          const int nk = min(w.nk - k0, kPartK);
+        for (int k0 = 0; k0 < unk && ok; k0 += kPartK) {
+          const int nk = min(unk - k0, kPartK);
           for (int k = 0; k < nk && ok; ++k, ++i) {              // pass 0
             const uint32_t st = i % kTcStages;
-            if (!tc::mbar_wait(&h.full[st], (i / kTcStages) & 1, abort)) {
+            if (!tc::mbar_wait_warp(&h.full[st], (i / kTcStages) & 1, abort)) {
               ok = false;
               break;
             }
@@ -837,8 +854,9 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
             const uint64_t ra = tc::umma_desc_add(ca, kHalfBytes);
 #pragma unroll
             for (int lev = 0; lev < 4; ++lev) {
+              if ((lev == 0 || lev == 3) != (side == 0)) continue;
               if (k == 0 && use > 0) {
-                if (!tc::mbar_wait(&h.tempty[lev], (use - 1) & 1, abort)) {
+                if (!tc::mbar_wait_warp(&h.tempty[lev], (use - 1) & 1, abort)) {
                   ok = false;
                   break;
                 }
@@ -846,7 +864,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
               }
 #pragma unroll
               for (int aa = 0; aa <= lev; ++aa)
-                tc::umma_bf16_warp(tmem + lev * kCols, tc::umma_desc_add(ca, aa * kPlaneBytes),
+                tc::umma_bf16_warp(utmem + lev * kCols, tc::umma_desc_add(ca, aa * kPlaneBytes),
                                    tc::umma_desc_add(ra, (lev - aa) * kPlaneBytes), idesc,
                                    (k > 0 || aa > 0) ? 1u : 0u);
               if (k == nk - 1) tc::umma_commit_warp(&h.tfull[lev]);
@@ -856,8 +874,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
           ++use;
           for (int k = 0; k < nk && ok; ++k, i += 2) {           // pass 1
             const uint32_t st = i % kTcStages, st1 = (i + 1) % kTcStages;
-            if (!tc::mbar_wait(&h.full[st], (i / kTcStages) & 1, abort) ||
-                !tc::mbar_wait(&h.full[st1], ((i + 1) / kTcStages) & 1, abort)) {
+            if (!tc::mbar_wait_warp(&h.full[st], (i / kTcStages) & 1, abort) ||
+                !tc::mbar_wait_warp(&h.full[st1], ((i + 1) / kTcStages) & 1, abort)) {
               ok = false;
               break;
             }
@@ -869,8 +887,9 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
             };
 #pragma unroll
             for (int lev = 4; lev < 8; ++lev) {
+              if ((lev == 4 || lev == 7) != (side == 0)) continue;
               if (k == 0) {
-                if (!tc::mbar_wait(&h.tempty[lev - 4], (use - 1) & 1, abort)) {
+                if (!tc::mbar_wait_warp(&h.tempty[lev - 4], (use - 1) & 1, abort)) {
                   ok = false;
                   break;
                 }
@@ -878,7 +897,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
               }
 #pragma unroll
               for (int aa = 0; aa <= lev; ++aa)
-                tc::umma_bf16_warp(tmem + (lev - 4) * kCols, plane(aa),
+                tc::umma_bf16_warp(utmem + (lev - 4) * kCols, plane(aa),
                                    tc::umma_desc_add(plane(lev - aa), kHalfBytes), idesc,
                                    (k > 0 || aa > 0) ? 1u : 0u);
               if (k == nk - 1) tc::umma_commit_warp(&h.tfull[lev - 4]);
@@ -901,12 +920,12 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
     const int rbeg = (warp >> 2) * 64;                   // this warp's half of the rows
     const uint32_t tbase = tmem + ((uint32_t)((warp & 3) << 5) << 16) + rbeg;
     const long long L1 = a.lmax + 1;
-    // level weights 2^(unit_bits - 8 s) as (float factor, integer multiplier): the level-0 sum
-    // goes into the high word, the others by 32 x 32 -> 64-bit multiply-adds with <= 2^30
+    // level weights 2^wt, wt = unit_bits - 8 s, as (float factor, integer multiplier): 2^32 and up
+    // in the high word, the others with multipliers <= 2^30
     uint32_t use = 0;
     for (uint32_t n = 0;; ++n) {
       const int u = uq_take(uq, n, abort);
-      if (!__all_sync(0xffffffffu, u >= 0)) break;
+      if (u < 0) break;
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
       if (w.nk == 0) continue;
       const int map = w.g * kGroupMaps + (c >> 1);
@@ -927,7 +946,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
       for (int ph = 0; ph < NPH; ++ph) {
         const int par = DIR == 0 ? w.p : ph;
         const int eb = a.EB[(((long long)w.qi * 2 + par) * a.ngroups + w.g) * kCols + c];
-        long long acc[64];
+        unsigned long long acc[64], bias = 0;
 #pragma unroll
         for (int j = 0; j < 64; ++j) acc[j] = 0;
 #pragma unroll 1
@@ -942,21 +961,22 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
 #pragma unroll 1
             for (int lev = 0; lev < 8; ++lev) {
               const int slot = lev & 3;
-              bool ok = tc::mbar_wait(&h.tfull[slot], use & 1, abort);
-              ok = __all_sync(0xffffffffu, ok);
+              const bool ok = tc::mbar_wait_warp(&h.tfull[slot], use & 1, abort);
               if (slot == 3) ++use;
               if (!ok) continue;
               tc::tc_fence_after();
               const int wt = a.unit_bits - 8 * lev;      // weight 2^wt of this level
-              if (lev == 0) {
-                tc_drain<true>(tbase, nrow, 1.f, sign * (1 << (wt - 32)), acc);
+              if (wt >= 32) {
+                tc_drain<true>(tbase + slot * kCols, nrow, (float)sign, 1u << (wt - 32), acc);
+                bias += (unsigned long long)kMagic << wt;
               } else {
                 const int me = min(max(wt, 0), 30);
-                tc_drain<false>(tbase + slot * kCols, nrow, ldexpf(1.f, wt - me),
-                                sign * (1 << me), acc);
+                tc_drain<false>(tbase + slot * kCols, nrow, sign * ldexpf(1.f, wt - me), 1u << me,
+                                acc);
+                bias += (unsigned long long)kMagic << me;
               }
               tc::tc_fence_before();
-              tc::mbar_arrive(&h.tempty[slot]);
+              tc::mbar_arrive_warp(&h.tempty[slot]);
             }
           }
         }
@@ -970,7 +990,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
 #pragma unroll
           for (int j = 0; j < 64; ++j) {
             if (j >= nrow) break;
-            const double v = i64_scaled(acc[j], e) * s_fac[warp][j];
+            const double v = i64_scaled((long long)(acc[j] - bias), e) * s_fac[warp][j];
             double* d = dst + (long long)(2 * j) * a.ld;
             *d = a.accumulate ? *d + v : v;
           }
@@ -982,7 +1002,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
 #pragma unroll
           for (int j = 0; j < 64; ++j) {
             if (j >= nrow) break;
-            const double v = i64_scaled(acc[j], e);
+            const double v = i64_scaled((long long)(acc[j] - bias), e);
             if (ph == 0) {
               dst[j * rs] = v;
             } else {
@@ -997,7 +1017,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_tc_gemm(TcGemmArgs a) {
   }
   // the UMMA issuer waits for its last products before TMEM is released, the loader for its
   // last copies
-  if (warp == kEpiThreads / 32 + 1) {
+  if (warp > kEpiThreads / 32) {
     tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
@@ -1046,7 +1066,7 @@ int tc_bits_synthesis(const fsht_plan* p) {
 template <int DIR, int SPIN>
 int launch_tc_gemm(const TcGemmArgs& a, cudaStream_t s) {
   FSHT_TRY(fsht_smem_limit((const void*)k_tc_gemm<DIR, SPIN>, kTcSmem));
-  if (a.nunits > 0) k_tc_gemm<DIR, SPIN><<<a.nunits, kThreadsG, kTcSmem, s>>>(a);
+  if (a.nunits > 0) k_tc_gemm<DIR, SPIN><<<a.nunits, kTcThreads, kTcSmem, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }

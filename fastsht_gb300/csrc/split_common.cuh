@@ -103,7 +103,7 @@ struct __align__(16) UnitQueue {
   int unit[kUq];
 };
 
-__device__ __forceinline__ void uq_init(UnitQueue& q, uint32_t takers) {
+__device__ __forceinline__ void uq_init(UnitQueue& q, uint32_t takers /* warps */) {
   tc::mbar_init(&q.clc, 1);
   for (int i = 0; i < kUq; ++i) {
     tc::mbar_init(&q.full[i], 1);
@@ -117,11 +117,11 @@ __device__ __forceinline__ bool uq_put(UnitQueue& q, uint32_t n, int u, volatile
   tc::mbar_arrive(&q.full[n % kUq]);
   return true;
 }
-// Every other role's threads: the n-th unit, or -1 (also after an expired wait).
+// Every other role, by whole warps: the n-th unit, or -1 (also after an expired wait).
 __device__ __forceinline__ int uq_take(UnitQueue& q, uint32_t n, volatile int* abort) {
-  if (!tc::mbar_wait(&q.full[n % kUq], (n / kUq) & 1, abort)) return -1;
+  if (!tc::mbar_wait_warp(&q.full[n % kUq], (n / kUq) & 1, abort)) return -1;
   const int u = *const_cast<volatile int*>(&q.unit[n % kUq]);
-  tc::mbar_arrive(&q.empty[n % kUq]);
+  tc::mbar_arrive_warp(&q.empty[n % kUq]);
   return u;
 }
 // Copy thread: ask for the next unit / the answer to the n-th request (-1: none left).

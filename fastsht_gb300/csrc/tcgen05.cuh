@@ -50,6 +50,31 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return false;
 }
 
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The same for a converged warp on a latency-critical hand-over: a spin on test_wait, which does
+// not suspend the warp, before the suspending wait.
+constexpr uint32_t kSpinPolls = 4096;
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
+                                               volatile int* abort) {
+  for (uint32_t it = 0; it < kSpinPolls; ++it)
+    if (__all_sync(0xffffffffu, mbar_test_wait(bar, parity))) return true;
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort));
+}
+// One arrival for the warp, after everything its lanes did before.
+__device__ __forceinline__ void mbar_arrive_warp(uint64_t* bar) {
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+
 // 1-D bulk copy global -> shared, completion signalled on an mbarrier (TMA engine).
 // dst, src and bytes must be multiples of 16.
 __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t bytes,
@@ -127,10 +152,9 @@ __device__ __forceinline__ void umma_bf16_warp(uint32_t d_tmem, uint64_t adesc, 
 __device__ __forceinline__ uint64_t umma_desc_add(uint64_t desc, uint32_t bytes) {
   return desc + (bytes >> 4);
 }
-// Warp index in a form the compiler knows to be warp-uniform.
-__device__ __forceinline__ int warp_index() {
-  return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0);
-}
+// A warp-uniform value in a form that the compiler knows to be uniform.
+__device__ __forceinline__ int uniform(int v) { return __shfl_sync(0xffffffffu, v, 0); }
+__device__ __forceinline__ int warp_index() { return uniform((int)(threadIdx.x >> 5)); }
 __device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
   asm volatile(
       "{\n.reg .pred q;\nelect.sync _|q, 0xffffffff;\n"
