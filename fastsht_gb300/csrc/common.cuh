@@ -103,6 +103,16 @@ struct FshtPolRow {
   double c1, c2, c3, c4;
 };
 
+// A north ring whose transform runs as matrix products (legendre_fp64_tc.cu).  Offsets are in
+// 32 KB k-steps from the start of the ring's wave.
+struct FshtDftRing {
+  int ring, q, s;       // n = 4 q samples at (2 j + s) pi / n
+  int nk, nrt;          // k-steps and 128-row tiles of each of its four matrices
+  int first;            // 1: its wave's matrices of (q, s) are made for this entry
+  int mtop;             // highest kept order
+  long long off_c, off_t, off_cos;
+};
+
 struct fsht_plan {
   int nside, lmax, nring, nnorth;  // nnorth = 2*nside (north rings incl. equator)
   long long npix;
@@ -193,6 +203,11 @@ struct fsht_plan {
   // 64-map group of the chunk) four flags of columns left to the FMA kernels.
   int tc64;
   int* d_tcflag;
+  // their matrix-form ring transforms: rings below dft_end (0: none), in waves
+  FshtDftRing* d_dft;
+  long long* d_dft_cos;
+  int* h_dft_waves;
+  int ndft_waves, dft_end;
   FshtLamRow* d_lamtab2;           // their spin-2 recursion rows (d_poltab: integer factors)
 };
 
@@ -252,10 +267,12 @@ int fsht_launch_ring_fft_fwd(fsht_plan* p, const double* maps, long long map_str
 int fsht_fft_df_tables_init(fsht_plan* p);
 int fsht_launch_ring_fft_fwd_df(fsht_plan* p, const double* maps, long long map_stride,
                                 int kc, int k0, int kb, double2* W, cudaStream_t s);
+// (ring0: only north rings from ring0 on.)
 // The forward transform of maps [k0, k0 + kb) of a chunk of kc maps (W keeps the chunk's
 // map stride kc), for transfers that land in parts.
 int fsht_launch_ring_fft_fwd_part(fsht_plan* p, const double* maps, long long map_stride,
-                                  int kc, int k0, int kb, double2* W, cudaStream_t s);
+                                  int kc, int k0, int kb, double2* W, cudaStream_t s,
+                                  int ring0 = 0);
 // Pair-order range [q0, q1) of the orders in wave w of a split-precision plan.
 void fsht_split_wave_range(const fsht_plan* p, int w, int* q0, int* q1);
 int fsht_launch_ring_fft_inv_df(fsht_plan* p, const double2* W, double* maps,
@@ -263,7 +280,7 @@ int fsht_launch_ring_fft_inv_df(fsht_plan* p, const double2* W, double* maps,
 // Maps per CTA of the ring-FFT launches when the autotuner has not set one.
 int fsht_fft_maps_per_block(int kc, int nrings);
 int fsht_launch_ring_fft_inv(fsht_plan* p, const double2* W, double* maps,
-                             long long map_stride, int kc, cudaStream_t s);
+                             long long map_stride, int kc, cudaStream_t s, int ring0 = 0);
 int fsht_launch_fourier_residual(fsht_plan* p, const double2* X, double2* GR, int kc,
                                  int prefix, cudaStream_t s);
 int fsht_launch_ring_skip(fsht_plan* p, cudaStream_t s);
@@ -277,6 +294,11 @@ int fsht_launch_analysis_fp64(fsht_plan* p, int spin, const double2* WQ,
 // The same contraction as exact digit products on the tensor cores (FP64 plans with tc64).
 // Per wave w: slice (phases or alm -> digit tiles WS, exponents EB), lambda (-> lbuf), gemm
 // (dir 0: into alm, dir 1: into the phase matrices).  A null second field means spin 0.
+int fsht_dft_tables_init(fsht_plan* p);
+int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, int kc, int k0,
+                        int cnt, double2* W, cudaStream_t s);
+int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride, int kc,
+                        cudaStream_t s);
 bool fsht_tc_supported(const fsht_plan* p);
 int fsht_tc_tables_init(fsht_plan* p);
 size_t fsht_tc_ws_bytes(const fsht_plan* p, int kc, int nf);

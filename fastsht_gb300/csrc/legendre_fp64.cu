@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(NT) k_analysis_fp64(AnaArgs a) {
                 lam1[tid * LC + j] = ok ? cur : 0.0;
               } else {
                 double l1 = 0.0, l2 = 0.0;
-                if (ok) pol_lambda(pr, l, m, cur, prev, s_lf[j], s_nl[j], l1, l2);
+                if (ok) pol_lambda(pr, pol_l(l, m), cur, prev, s_lf[j], s_nl[j], l1, l2);
                 lam1[tid * LC + j] = l1;
                 lam2[tid * LC + j] = l2;
               }
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(NT) k_synthesis_fp64(SynArgs a) {
             lam1[tid][j] = ok ? cur : 0.0;
           } else {
             double l1 = 0.0, l2 = 0.0;
-            if (ok) pol_lambda(pr, l, m, cur, prev, s_lf[j], s_nl[j], l1, l2);
+            if (ok) pol_lambda(pr, pol_l(l, m), cur, prev, s_lf[j], s_nl[j], l1, l2);
             lam1[tid][j] = l1;
             lam2[tid][j] = l2;
           }

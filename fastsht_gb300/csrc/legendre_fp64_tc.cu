@@ -28,6 +28,8 @@
 
 #include <algorithm>
 #include <cmath>
+#include <new>
+#include <vector>
 
 namespace {
 
@@ -99,18 +101,47 @@ __device__ __forceinline__ void store_planes(unsigned char* dst, unsigned char* 
   put(7, plane_of<7>(y));
 }
 
-// a 2^e as the nearest FP64, with integer instructions; zero below the normal range.
-__device__ __forceinline__ double i64_scaled(long long a, int e) {
-  unsigned long long u = (unsigned long long)(a < 0 ? -a : a);
+// The output stays off the FP64 pipe too (an FP64 addition per value was 15 clocks a warp, and
+// bound the output of the ring transforms): sums are combined as integers and rounded once.
+// Magnitude u (bit 63 - lz leading) 2^e as the nearest FP64.
+__device__ __forceinline__ double u64_scaled(unsigned long long u, bool neg, int e) {
   if (u == 0) return 0.0;
   const int lz = __clzll((long long)u);
   u <<= lz;
   const unsigned long long r = (u >> 11) + ((u >> 10) & 1);       // 2^52 .. 2^53
-  const int ex = 63 - lz + e + 1023;
-  if (ex <= 0) return 0.0;
-  unsigned long long b = ((unsigned long long)ex << 52) + (r - (1ull << 52));
-  b |= a < 0 ? 1ull << 63 : 0ull;
-  return __longlong_as_double((long long)b);
+  int ex = 63 - lz + e + 1023;
+  const unsigned long long sign = neg ? 1ull << 63 : 0ull;
+  if (ex >= 2047) return __longlong_as_double((long long)(sign | 0x7FF0000000000000ull));
+  const bool low = ex <= 0;                                        // subnormal or zero
+  if (low) ex = max(ex + 128, 1);
+  const double v = __longlong_as_double(
+      (long long)((((unsigned long long)ex << 52) + (r - (1ull << 52))) | sign));
+  return low ? v * 0x1p-128 : v;
+}
+__device__ __forceinline__ double i64_scaled(long long a, int e) {
+  return u64_scaled((unsigned long long)(a < 0 ? -a : a), a < 0, e);
+}
+// a f 2^e for a factor f as (64-bit mantissa fm with its top bit set, sign, exponent: f = +-fm
+// 2^fe): the high half of the product, truncated at 2^-62 of it.
+struct TcFac {
+  unsigned long long fm;
+  int fe, neg;
+};
+__device__ __forceinline__ TcFac tc_fac(double f) {
+  TcFac t;
+  const unsigned long long b = (unsigned long long)__double_as_longlong(f);
+  const int ex = (int)(b >> 52) & 0x7FF;
+  t.fm = ex ? ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 11 : 0ull;
+  t.fe = ex - 1023 - 63;
+  t.neg = (long long)b < 0;
+  return t;
+}
+__device__ __forceinline__ double i64_scaled_mul(long long a, const TcFac& f, int e) {
+  unsigned long long u = (unsigned long long)(a < 0 ? -a : a);
+  if (u == 0) return 0.0;
+  const int lz = __clzll((long long)u);
+  u = __umul64hi(u << lz, f.fm);                                  // times 2^(64 - lz)
+  return u64_scaled(u, (a < 0) != (f.neg != 0), e + f.fe + 64 - lz);
 }
 
 // ------------------------------------------------------------------ tables
@@ -346,14 +377,15 @@ __device__ __forceinline__ void tc_step(TcRing& r, double beta) {
 // The values of step j (l = m + j) as biased fixed point against the row exponent (k: 62 minus
 // it, plus Dx for spin 0).
 template <int SPIN>
-__device__ __forceinline__ void tc_value(TcRing& r, int j, int m, double beta, const FshtPolRow& c,
-                                         int k, unsigned long long& y1, unsigned long long& y2) {
+__device__ __forceinline__ void tc_value(TcRing& r, int j, double beta, const FshtPolRow& c,
+                                         const PolL& pl, int k, unsigned long long& y1,
+                                         unsigned long long& y2) {
   if (SPIN == 2) {
     if (j > 0) rec_step(r.s1, r.s2, r.et, c.c1 * r.x, c.c2);
     y1 = y2 = kBias;
     if (r.et != 0) return;
     double l1, l2;
-    pol_lambda(r.pol, m + j, m, r.s1, r.s2, c.c3, c.c4, l1, l2);
+    pol_lambda(r.pol, pl, r.s1, r.s2, c.c3, c.c4, l1, l2);
     y1 = fixed_biased(l1, k);
     y2 = fixed_biased(l2, k);
   } else {
@@ -389,6 +421,7 @@ __global__ void __launch_bounds__(128) k_tc_lambda(TcLamArgs a) {
   __shared__ double s_beta[LB];
   __shared__ int s_k[LB];
   __shared__ FshtPolRow s_c[SPIN == 2 ? LB : 1];
+  __shared__ PolL s_l[SPIN == 2 ? LB : 1];
   const int q = a.q0 + blockIdx.x;
   const int m = m_of_q(q, a.lmax);
   const int i0 = a.ring_i0[m];
@@ -413,7 +446,10 @@ __global__ void __launch_bounds__(128) k_tc_lambda(TcLamArgs a) {
       const FshtLamRow rw = tab[lb + tid];
       s_beta[tid] = rw.beta;
       s_k[tid] = rw.dx + kFixBits - a.eag;
-      if (SPIN == 2) s_c[tid] = ptab[lb + tid];
+      if (SPIN == 2) {
+        s_c[tid] = ptab[lb + tid];
+        s_l[tid] = pol_l(m + lb + tid, m);
+      }
     }
     __syncthreads();
     if (SPIN == 0) tc_rescale(R);
@@ -422,7 +458,8 @@ __global__ void __launch_bounds__(128) k_tc_lambda(TcLamArgs a) {
       const int j = lb + jj;
       unsigned long long y1 = kBias, y2 = kBias;
       if (j < nl && valid)
-        tc_value<SPIN>(R, j, m, s_beta[jj], s_c[SPIN == 2 ? jj : 0], s_k[jj], y1, y2);
+        tc_value<SPIN>(R, j, s_beta[jj], s_c[SPIN == 2 ? jj : 0], s_l[SPIN == 2 ? jj : 0],
+                       s_k[jj], y1, y2);
       S[0][jj & 1][jj >> 1][tid] = y1;
       if (SPIN == 2) S[NT - 1][jj & 1][jj >> 1][tid] = y2;
     }
@@ -465,6 +502,7 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
   __shared__ double s_beta[LB];
   __shared__ int s_k[LB];
   __shared__ FshtPolRow s_c[SPIN == 2 ? LB : 1];
+  __shared__ PolL s_l[SPIN == 2 ? LB : 1];
   const int q = a.q0 + blockIdx.x;
   const int m = m_of_q(q, a.lmax);
   const int i0 = a.ring_i0[m];
@@ -490,7 +528,10 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
       const FshtLamRow rw = tab[lb + tid];
       s_beta[tid] = rw.beta;
       s_k[tid] = kFixBits - rw.erow;
-      if (SPIN == 2) s_c[tid] = ptab[lb + tid];
+      if (SPIN == 2) {
+        s_c[tid] = ptab[lb + tid];
+        s_l[tid] = pol_l(m + lb + tid, m);
+      }
     }
     __syncthreads();
     if (SPIN == 0) tc_rescale(R);
@@ -500,7 +541,8 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
       const int j = lb + jj;
       unsigned long long y1 = kBias, y2 = kBias;
       if (j < nl && valid)
-        tc_value<SPIN>(R, j, m, s_beta[jj], s_c[SPIN == 2 ? jj : 0], s_k[jj], y1, y2);
+        tc_value<SPIN>(R, j, s_beta[jj], s_c[SPIN == 2 ? jj : 0], s_l[SPIN == 2 ? jj : 0],
+                       s_k[jj], y1, y2);
       y[0][jj & 1][jj >> 1] = y1;
       if (SPIN == 2) y[NT - 1][jj & 1][jj >> 1] = y2;
     }
@@ -518,9 +560,9 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
 }
 
 // ------------------------------------------------------------------ alm -> digits
-// grid (q in wave, group), 128 threads per field = (comp, map): v = a_lm Dm 2^EA(l), tile column
-// c = 2 map + comp, 16 l of one parity per k-step.  T: an exponent per (column, parity), since
-// the two parities are separate sums; E/B (NF = 2): one per map and order, plain and i v copies.
+// grid (q in wave, group), 256 threads per field = (half of the l steps, comp, map): v = a_lm Dm
+// 2^EA(l), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an exponent per
+// column; E/B (NF = 2): one per map and order, plain and i v copies.
 struct TcSliceAArgs {
   const double* alm[2];
   int ld, k0, kc, lmax, ngroups, q0;
@@ -532,22 +574,23 @@ struct TcSliceAArgs {
 };
 
 template <int NF>
-__global__ void __launch_bounds__(128 * NF) k_tc_slice_alm(TcSliceAArgs a) {
-  __shared__ unsigned long long s_mx[2 * NF][64];
+__global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
+  __shared__ unsigned long long s_mx[2 * NF][2][2][64];        // [field, half][parity][comp][map]
   const int qi = blockIdx.x, g = blockIdx.y;
   const int m = m_of_q(a.q0 + qi, a.lmax);
-  const int f = NF == 1 ? 0 : (int)(threadIdx.x >> 7);
-  const int kl = threadIdx.x & 63, comp = (threadIdx.x >> 6) & 1;
+  const int f = NF == 1 ? 0 : (int)(threadIdx.x >> 8);
+  const int kl = threadIdx.x & 63, comp = (threadIdx.x >> 6) & 1, half = (threadIdx.x >> 7) & 1;
   const int k = g * kGroupMaps + kl;
   const int c = 2 * kl + comp;
   const bool valid = k < a.kc && !(comp == 1 && m == 0);
   const long long L1 = a.lmax + 1;
-  const int nkl = ((a.lmax - m) / 2 + 1 + kKStep - 1) / kKStep;
+  const int nh = 2 * (((a.lmax - m) / 2 + 1 + kKStep - 1) / kKStep);   // blocks of eight l
+  const int h0 = half ? nh / 2 : 0, h1 = half ? nh : nh / 2;
   const FshtLamRow* tab = a.tab + tri_off(m, a.lmax);
   const double* col = a.alm[f] + a.k0 + k +
                       (comp == 0 ? (long long)m * L1 + m : (L1 - m) * L1) * a.ld;
   auto cnt_of = [&](int p) { return a.lmax - m - p >= 0 ? (a.lmax - m - p) / 2 + 1 : 0; };
-  // bits of |a Dm| 2^EA(l); values too small for the exponent sum count as zero (the flag of a
+  // bits of |a Dm| 2^EA(l); values too small for the exponent sum count as tiny (the flag of a
   // tiny column maximum sends the whole column to the FMA kernel)
   auto key_of = [&](double w, int ea) -> unsigned long long {
     const unsigned long long b =
@@ -556,39 +599,36 @@ __global__ void __launch_bounds__(128 * NF) k_tc_slice_alm(TcSliceAArgs a) {
     if ((b >> 52) > 2000) return 0x7FF0000000000000ull;
     return b + ((unsigned long long)(long long)ea << 52);
   };
-  bool flag = false;
-  unsigned long long mxp[2];
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     unsigned long long mx = 0;
     if (valid) {
-      const int cnt = cnt_of(p);
+      const int e1 = min(cnt_of(p), h1 * 8);
 #pragma unroll 8
-      for (int idx = 0; idx < cnt; ++idx) {
+      for (int idx = h0 * 8; idx < e1; ++idx) {
         const int j = p + 2 * idx;
         const FshtLamRow rw = tab[j];
-        mx = max(mx, key_of(col[(long long)j * a.ld] * rw.dm, rw.erow + rw.dx));
+        mx = max(mx, key_of(__ldg(&col[(long long)j * a.ld]) * rw.dm, rw.erow + rw.dx));
       }
     }
-    mxp[p] = mx;
+    s_mx[2 * f + half][p][comp][kl] = mx;
   }
-  if (NF == 2) {
-    __syncthreads();
-    s_mx[f * 2 + comp][kl] = max(mxp[0], mxp[1]);
-    __syncthreads();
-    unsigned long long mx = 0;
-#pragma unroll
-    for (int h = 0; h < 2 * NF; ++h) mx = max(mx, s_mx[h][kl]);
-    mxp[0] = mxp[1] = mx;
-  }
+  __syncthreads();
+  bool flag = false;
   int Ep[2];
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
-    const int ef = (int)(mxp[p] >> 52);
-    const bool odd_range = mxp[p] != 0 && (ef < 1023 - kMaxExp || ef > 1023 + kMaxExp);
+    unsigned long long mx = 0;
+#pragma unroll
+    for (int h = 0; h < 2 * NF; ++h)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (NF == 2 || (u & 1) == comp) mx = max(mx, s_mx[h][u >> 1][u & 1][kl]);
+    const int ef = (int)(mx >> 52);
+    const bool odd_range = mx != 0 && (ef < 1023 - kMaxExp || ef > 1023 + kMaxExp);
     flag |= odd_range;
-    Ep[p] = (mxp[p] == 0 || odd_range) ? kEmptyExp : ef - 1022;
-    if (f == 0) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = Ep[p];
+    Ep[p] = (mx == 0 || odd_range) ? kEmptyExp : ef - 1022;
+    if (f == 0 && !half) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = Ep[p];
   }
   const int any = __syncthreads_or(flag ? 1 : 0);
   if (threadIdx.x < 4) a.flags[((long long)m * a.ngroups + g) * 4 + threadIdx.x] = any;
@@ -601,22 +641,282 @@ __global__ void __launch_bounds__(128 * NF) k_tc_slice_alm(TcSliceAArgs a) {
         a.WS + (((size_t)(qi * 2 + p) * a.ngroups + g) * NC + 2 * f) * a.row_bytes;
     unsigned char* dst = base + (c >> 3) * 256 + (c & 7) * 16;
     unsigned char* rot = base + a.row_bytes + (cr >> 3) * 256 + (cr & 7) * 16;
-    for (int h = 0; h < 2 * nkl; ++h) {
+    for (int h = h0; h < h1; ++h) {
+      double v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int idx = h * 8 + j;
+        v[j] = valid && idx < cnt ? __ldg(&col[(long long)(p + 2 * idx) * a.ld]) : 0.0;
+      }
       unsigned long long y[8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int idx = h * 8 + j;
         y[j] = kBias;
-        if (valid && idx < cnt && E != kEmptyExp) {
+        if (idx < cnt && E != kEmptyExp) {
           const FshtLamRow rw = tab[p + 2 * idx];
-          y[j] = fixed_biased(col[(long long)(p + 2 * idx) * a.ld] * rw.dm,
-                              rw.erow + rw.dx + kFixBits - E);
+          y[j] = fixed_biased(v[j] * rw.dm, rw.erow + rw.dx + kFixBits - E);
         }
       }
       store_planes<NF == 2>(dst + (size_t)(h >> 1) * kStepBytes + (h & 1) * 128,
                             rot + (size_t)(h >> 1) * kStepBytes + (h & 1) * 128, comp == 1, y);
     }
   }
+}
+
+// ------------------------------------------------------------------ ring transforms
+// The DFT of a ring as four real matrix products.  A ring of n = 4 q pixels has its samples at
+// (2 j + s) pi / n (s = 1: cap rings and every other belt ring).  Folded about 0 and pi / 2,
+//   F_r = sum_j [x_j +- x_{-j} +- x_{pi-j} +- x_{pi+j}] {cos, sin}(r (2 j + s) pi / n),
+// even and odd r and cos and sin take one sign pattern each: four q x q products (s = 0: up to
+// q + 1) instead of one n x n, 8 q^2 flop per real ring.  Bins r <= n/2 serve every order
+// a n +- r, by (-1)^{a s} and a conjugate.  As digit products that is 0.12 ms per map for all
+// cap rings of nside 1024 at the tensor rate, where Bluestein transforms on the FP64 pipe (two
+// FFTs of 2 n points or more per ring) took 0.90 ms.  The belt's power-of-two rings cost q^2
+// too, and from nside 512 on the FFT is the cheaper form there (kDftBeltMax).
+// Types: 0 cos r even, 1 cos r odd, 2 sin r even (from 2), 3 sin r odd; row rho of a type is
+// r = 2 rho + {0, 1, 2, 1}.
+__device__ __forceinline__ int dft_r(int type, int rho) {
+  return 2 * rho + (type == 0 ? 0 : type == 2 ? 2 : 1);
+}
+__device__ __forceinline__ int dft_rows(const FshtDftRing& d, int type) {
+  return d.q + ((d.s == 0 && type == 0) ? 1 : 0);
+}
+
+// cos(pi t / n) 2^61, t <= n/2, of every class (q, s) (plan creation).
+__global__ void k_dft_cos(const FshtDftRing* rings, long long* cosv) {
+  const FshtDftRing d = rings[blockIdx.x];
+  if (!d.first) return;
+  const int n = 4 * d.q;
+  for (int t = threadIdx.x; t <= n / 2; t += blockDim.x)
+    cosv[d.off_cos + t] = (long long)(cospi((double)t / (double)n) * 0x1p61);
+}
+
+struct DftTrigArgs {
+  const FshtDftRing* rings;     // of the wave
+  const long long* cosv;
+  unsigned char* lbuf;
+};
+
+// Matrix tiles: rows x 16 summands; forward rows rho and summands j, inverse the other way
+// round.  grid (ring of the wave, 4 types x row tile), 256 threads = (row, half of the k-step).
+// The class's cosines sit in shared memory; the angle r (2 j + s) mod 2 n moves by a constant
+// step along a row.
+template <bool INV>
+__global__ void __launch_bounds__(256) k_dft_trig(DftTrigArgs a) {
+  extern __shared__ long long s_cos[];
+  const FshtDftRing d = a.rings[blockIdx.x];
+  const int type = blockIdx.y & 3, t = blockIdx.y >> 2;
+  if (!d.first || t >= d.nrt) return;
+  const int n = 4 * d.q;
+  for (int u = threadIdx.x; u <= n / 2; u += 256) s_cos[u] = a.cosv[d.off_cos + u];
+  __syncthreads();
+  const int r8 = threadIdx.x & 7, half = (threadIdx.x >> 3) & 1, rg = threadIdx.x >> 4;
+  const int row = t * kRows + rg * 8 + r8;
+  const int nr = dft_rows(d, type), nj = d.q + (d.s == 0 ? 1 : 0);
+  const int rows = INV ? nj : nr, ks = INV ? nr : nj;
+  unsigned char* dst = a.lbuf +
+                       (size_t)(d.off_t + (long long)(type * d.nrt + t) * d.nk) * kStepBytes +
+                       rg * 256 + half * 128 + r8 * 16;
+  // angle index of summand 0 and its step
+  const int r0 = INV ? dft_r(type, 0) : dft_r(type, row);
+  const int j0 = INV ? row : 0;
+  int step = INV ? 2 * (2 * j0 + d.s) : 2 * r0;
+  step %= 2 * n;
+  int idx = (int)(((long long)r0 * (2 * j0 + d.s) + (long long)step * (half * 8)) % (2 * n));
+  if (type >= 2) idx = (idx + 2 * n - n / 2) % (2 * n);       // sin t = cos(t - pi / 2)
+  const int skip = (int)(((long long)step * 8) % (2 * n));
+  for (int k = 0; k < d.nk; ++k) {
+    unsigned long long y[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      int v = min(idx, 2 * n - idx);                          // 0 .. n
+      const bool neg = v > n / 2;
+      if (neg) v = n - v;
+      long long x = s_cos[v];
+      if (neg) x = -x;
+      const int kk = k * kKStep + half * 8 + e;
+      y[e] = (row < rows && kk < ks) ? (unsigned long long)x + kBias : kBias;
+      idx += step;
+      if (idx >= 2 * n) idx -= 2 * n;
+    }
+    idx += skip;
+    if (idx >= 2 * n) idx -= 2 * n;
+    store_planes<false>(dst + (size_t)k * kStepBytes, nullptr, false, y);
+  }
+}
+
+struct DftSliceArgs {
+  const FshtDftRing* rings;
+  int ngroups;
+  unsigned char* WS;
+  int* EB;                      // per (ring of the wave, group, column)
+  // forward: map k of this launch at maps + k map_stride
+  const double* maps;
+  long long map_stride;
+  int nside, nring, cnt;
+  // inverse
+  const double2* W;
+  int kc, nnorth;
+};
+constexpr int kNanExp = kEmptyExp - 1;     // column with a non-finite sample: NaN out
+
+// A fixed-point value without the digit bias.
+__device__ __forceinline__ long long fixed_i64(double v, int k) {
+  return (long long)(fixed_biased(v, k) - kBias);
+}
+__device__ __forceinline__ int dft_exp(unsigned long long mx) {
+  const int ef = (int)(mx >> 52);
+  if (mx == 0 || ef == 0) return kEmptyExp;
+  return ef == 0x7FF ? kNanExp : ef - 1022;
+}
+
+// Ring samples -> folded digit tiles.  grid (ring of the wave, 4 maps), 256 threads = (column of
+// 8: map, north | south; 32 chunks of 8 samples): a warp reads 256 contiguous bytes per map and
+// writes whole 128-byte core matrices.  The ring's samples against its maximum with two bits to
+// spare, so the folds are exact integer sums.
+__global__ void __launch_bounds__(256) k_dft_slice(DftSliceArgs a) {
+  __shared__ unsigned long long s_mx[8][8];
+  const FshtDftRing d = a.rings[blockIdx.x];
+  const int n = 4 * d.q;
+  const int col = threadIdx.x & 7, chunk = threadIdx.x >> 3;
+  const int map = blockIdx.y * 4 + (col >> 1), h = col & 1;
+  const int ip = a.nring - 1 - d.ring;
+  const bool valid = map < a.cnt && !(h == 1 && ip == d.ring);
+  const double* x = a.maps + (long long)map * a.map_stride +
+                    ring_start(a.nside, h ? ip : d.ring);
+  unsigned long long mx = 0;
+  if (valid)
+    for (int j0 = chunk * 8; j0 < n; j0 += 256) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        if (j0 + e < n)
+          mx = max(mx, (unsigned long long)__double_as_longlong(__ldg(&x[j0 + e])) &
+                           0x7FFFFFFFFFFFFFFFull);
+    }
+  // one exponent for the map's two rings: their sum and difference are formed as integers
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+  if ((threadIdx.x & 31) < 8) s_mx[threadIdx.x >> 5][col] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w][col]);
+  const int E = dft_exp(mx);
+  const bool live = valid && E > kEmptyExp;
+  const int g = map >> 6, c = 2 * (map & 63) + h;
+  if (map >= a.cnt) return;
+  if (chunk == 0)
+    a.EB[((long long)blockIdx.x * a.ngroups + g) * kCols + c] = E > kEmptyExp ? E + 2 : E;
+  const int nj = d.q + (d.s == 0 ? 1 : 0);
+  unsigned char* dst = a.WS + (size_t)(d.off_c * a.ngroups) * kStepBytes +
+                       (size_t)g * d.nk * kStepBytes + (c >> 3) * 256 + (c & 7) * 16;
+  const size_t tstride = (size_t)a.ngroups * d.nk * kStepBytes;
+  const int kf = kFixBits - 2 - E;
+  for (int hc = chunk; hc < 2 * d.nk; hc += 32) {
+    unsigned long long y[4][8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const int j = hc * 8 + e;
+      long long x0 = 0, x1 = 0, x2 = 0, x3 = 0;
+      if (live && j < nj) {
+        const bool lo = d.s == 0 && j == 0, hi = d.s == 0 && j == d.q;   // samples on an axis
+        x0 = fixed_i64(__ldg(&x[j]), kf);
+        if (!lo) x1 = fixed_i64(__ldg(&x[n - d.s - j]), kf);
+        if (!hi) x2 = fixed_i64(__ldg(&x[n / 2 - d.s - j]), kf);
+        if (!lo && !hi) x3 = fixed_i64(__ldg(&x[n / 2 + j]), kf);
+      }
+      const long long u = x0 + x1, u2 = x2 + x3, v = x0 - x1, v2 = x2 - x3;
+      y[0][e] = (unsigned long long)(u + u2) + kBias;
+      y[1][e] = (unsigned long long)(u - u2) + kBias;
+      y[2][e] = (unsigned long long)(v - v2) + kBias;
+      y[3][e] = (unsigned long long)(v + v2) + kBias;
+    }
+#pragma unroll
+    for (int ty = 0; ty < 4; ++ty)
+      store_planes<false>(dst + ty * tstride + (size_t)(hc >> 1) * kStepBytes + (hc & 1) * 128,
+                          nullptr, false, y[ty]);
+  }
+}
+
+// c (-1)^{a s} sums of G over the orders of bin r: x = sum_r A_r cos - B_r sin.  Most bins have
+// the orders r and n - r at most, loaded without a loop so that several bins are in flight.
+__device__ __forceinline__ double2 dft_bin(const double2* __restrict__ g, long long stride_m,
+                                           const FshtDftRing& d, int r) {
+  const int n = 4 * d.q;
+  const bool self = r == 0 || 2 * r == n;
+  const double2 zero = make_double2(0.0, 0.0);
+  const double2 z0 = r <= d.mtop ? g[(long long)r * stride_m] : zero;
+  const double2 z1 = !self && n - r <= d.mtop ? g[(long long)(n - r) * stride_m] : zero;
+  const double w0 = r == 0 ? 1.0 : 2.0, w1 = d.s ? -2.0 : 2.0;
+  double2 v = make_double2(fma(w1, z1.x, w0 * z0.x), fma(-w1, z1.y, w0 * z0.y));
+  double sg = w1;
+  for (int m = n + r; m <= d.mtop; m += n) {         // a n + r and (a + 1) n - r
+    const double2 z = g[(long long)m * stride_m];
+    v.x = fma(sg, z.x, v.x);
+    v.y = fma(sg, z.y, v.y);
+    if (d.s) sg = -sg;
+    const int m1 = m + n - 2 * r;
+    if (!self && m1 <= d.mtop) {
+      const double2 y = g[(long long)m1 * stride_m];
+      v.x = fma(sg, y.x, v.x);
+      v.y = fma(-sg, y.y, v.y);
+    }
+  }
+  return v;
+}
+
+// {G_N, G_S} -> digit tiles of A (cos types) and B (sin types).  grid (ring of the wave, 16 maps),
+// lanes = columns (map, north | south): a warp reads 512 contiguous bytes per order.
+__global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
+  __shared__ unsigned long long s_mx[8][32];
+  const FshtDftRing d = a.rings[blockIdx.x];
+  const int n = 4 * d.q;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int map = blockIdx.y * 16 + (lane >> 1), h = lane & 1;
+  const bool valid = map < a.kc && !(h == 1 && d.ring == a.nnorth - 1);
+  const long long stride_m = (long long)a.nnorth * a.kc * 2;
+  const double2* g = a.W + ((long long)d.ring * a.kc + (map < a.kc ? map : 0)) * 2 + h;
+  unsigned long long mx = 0;
+  if (valid)
+#pragma unroll 4
+    for (int r = warp; r <= n / 2; r += 8) {
+      const double2 v = dft_bin(g, stride_m, d, r);
+      const unsigned long long bx =
+          (unsigned long long)__double_as_longlong(v.x) & 0x7FFFFFFFFFFFFFFFull;
+      const unsigned long long by =
+          (unsigned long long)__double_as_longlong(v.y) & 0x7FFFFFFFFFFFFFFFull;
+      mx = max(mx, max(bx, by));
+    }
+  s_mx[warp][lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w][lane]);
+  const int E = dft_exp(mx);
+  const bool live = valid && E > kEmptyExp;
+  const int grp = map >> 6, c = 2 * (map & 63) + h;
+  if (map >= a.kc) return;
+  if (warp == 0) a.EB[((long long)blockIdx.x * a.ngroups + grp) * kCols + c] = E;
+  unsigned char* dst = a.WS + (size_t)(d.off_c * a.ngroups) * kStepBytes +
+                       (size_t)grp * d.nk * kStepBytes + (c >> 3) * 256 + (c & 7) * 16;
+  const size_t tstride = (size_t)a.ngroups * d.nk * kStepBytes;
+  for (int hc = warp; hc < 2 * d.nk; hc += 8)
+#pragma unroll 1
+    for (int ty = 0; ty < 4; ++ty) {
+      const int nr = dft_rows(d, ty);
+      unsigned long long y[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int rho = hc * 8 + e;
+        y[e] = kBias;
+        if (live && rho < nr) {
+          const double2 v = dft_bin(g, stride_m, d, dft_r(ty, rho));
+          y[e] = fixed_biased(ty < 2 ? v.x : v.y, kFixBits - E);
+        }
+      }
+      store_planes<false>(dst + ty * tstride + (size_t)(hc >> 1) * kStepBytes + (hc & 1) * 128,
+                          nullptr, false, y);
+    }
 }
 
 // ------------------------------------------------------------------ contraction
@@ -631,11 +931,15 @@ __global__ void __launch_bounds__(128 * NF) k_tc_slice_alm(TcSliceAArgs a) {
 // levels 0..3 (digit planes 0..3) and levels 4..7 (all planes).  A level's accumulator is drained
 // into the 64-bit integers as soon as its last product is done, while the products of the other
 // levels still run, and is handed back alone: the four slots have their own barriers.
-// Warps 0-7: epilogue (two per TMEM lane quarter, one per half of the rows), warp 8 lane 0:
-// copies (16 KB of each operand per stage), warp 9 lane 0: UMMAs.
+// One lane copies (16 KB of each operand per stage), two warps issue the UMMAs.
 // The map columns are on the lanes, so a warp's alm stores are two 128-byte segments and its
 // phase-matrix stores whole {Re, Im} pairs, with no staging through shared memory.
-constexpr int kTcThreads = kEpiThreads + 96;     // epilogue, copy thread's warp, two UMMA warps
+// Sixteen epilogue warps (four per TMEM lane quarter, one per 32 accumulator columns: 32 64-bit
+// sums a thread), then the copy thread's warp and two UMMA warps.  With eight warps and 64 sums a
+// thread the drains and the output ran at the latency of two warps per scheduler.
+constexpr int kTcEpi = 512, kTcEpiWarps = kTcEpi / 32;
+constexpr int kTcAcc = 32;
+constexpr int kTcThreads = kTcEpi + 96;
 constexpr int kTcStages = 6;
 constexpr uint32_t kTcStageBytes = 2 * kHalfBytes;              // 32 KB
 constexpr size_t kTcSmem = (size_t)kTcStages * kTcStageBytes;
@@ -656,6 +960,10 @@ struct TcGemmArgs {
   int ld, k0, kc;
   double pa;                   // DIR 0: factor of the sums
   int* err;
+  // ring transforms (DIR 2, 3): the rings of the wave, map k_off + k of W / map k of maps
+  const FshtDftRing* rings;
+  long long map_stride;
+  int nside, nring, k_off, w_kc;
 };
 
 struct __align__(8) TcSmemHdr {
@@ -666,6 +974,7 @@ struct __align__(8) TcSmemHdr {
 
 struct TcUnit {
   int g, field, p, t, qi, m, nk, nt, row0, nrows, N;
+  FshtDftRing d;               // DIR 2, 3
 };
 
 template <int DIR, int SPIN>
@@ -674,6 +983,31 @@ __device__ __forceinline__ TcUnit tc_unit(const TcGemmArgs& a, int u) {
   w.g = u % a.ngroups;
   int r = u / a.ngroups;
   w.field = 0;
+  if (DIR >= 2) {
+    w.p = 0;
+    if (DIR == 2) {
+      w.p = r & 3;                                         // type
+      r >>= 2;
+    }
+    w.t = r % a.ntmax;
+    w.qi = r / a.ntmax;
+    w.d = a.rings[w.qi];
+    w.m = w.d.ring;
+    w.nt = w.d.nrt;
+    w.row0 = w.t * kRows;
+    if (DIR == 2) {
+      // rows rho whose bin r some kept order reaches
+      const int r0 = dft_r(w.p, 0);
+      const int need = w.d.mtop >= r0 ? (w.d.mtop - r0) / 2 + 1 : 0;
+      w.nrows = max(0, min(kRows, min(dft_rows(w.d, w.p), need) - w.row0));
+      w.N = (w.nrows + 15) & ~15;
+    } else {
+      w.nrows = max(0, min(kRows, w.d.q + (w.d.s == 0 ? 1 : 0) - w.row0));
+      w.N = (2 * min(kGroupMaps, a.kc - w.g * kGroupMaps) + 15) & ~15;   // map columns
+    }
+    w.nk = w.nrows > 0 ? w.d.nk : 0;
+    return w;
+  }
   if (SPIN == 2) {
     w.field = a.field0 + r % a.nfield;
     r /= a.nfield;
@@ -709,6 +1043,14 @@ __device__ __forceinline__ void tc_segment(const TcGemmArgs& a, const TcUnit& w,
                                            const unsigned char*& cols, const unsigned char*& rows,
                                            int& sign) {
   constexpr int NT = SPIN == 2 ? 2 : 1, NC = SPIN == 2 ? 4 : 1;
+  if (DIR >= 2) {
+    const int type = DIR == 2 ? w.p : ph;
+    sign = 1;
+    cols = a.WS + (size_t)(w.d.off_c * a.ngroups + (long long)(type * a.ngroups + w.g) * w.d.nk) *
+                      kStepBytes;
+    rows = a.lbuf + (size_t)(w.d.off_t + (long long)(type * w.d.nrt + w.t) * w.d.nk) * kStepBytes;
+    return;
+  }
   const int par = DIR == 0 ? (w.p ^ sg) : (ph ^ sg);
   const int lpar = DIR == 0 ? w.p : par;                 // parity of the lambda rows / l
   int copy = 0;
@@ -726,7 +1068,7 @@ __device__ __forceinline__ void tc_segment(const TcGemmArgs& a, const TcUnit& w,
           (size_t)((sg * 2 + lpar) * w.nt + w.t) * w.nk) * kStepBytes;
 }
 
-// acc += level sums L of one slot, 64 rows per thread: f L (an integer, or rounded to one) times
+// acc += level sums L of one slot, 32 columns per thread: f L (an integer, or rounded to one) times
 // mul, in the high word (HI) or as a 32 x 32 + 64-bit multiply-add.  The integer comes out of
 // the mantissa of f L + 1.5 2^23, so a sum costs a float FMA, a maximum and the multiply-add (the
 // conversion instruction and its 64-bit handling took three times as long, with the UMMA warps
@@ -735,18 +1077,16 @@ __device__ __forceinline__ void tc_segment(const TcGemmArgs& a, const TcUnit& w,
 constexpr uint32_t kMagic = 0x4B400000u;
 template <bool HI>
 __device__ __forceinline__ void tc_drain(uint32_t taddr, int nrow, float f, uint32_t mul,
-                                         unsigned long long (&acc)[64]) {
+                                         unsigned long long (&acc)[kTcAcc]) {
 #pragma unroll
-  for (int c = 0; c < 64; c += 32) {
+  for (int c = 0; c < kTcAcc; c += 16) {
     if (c >= nrow) break;
-    uint32_t v0[16], v1[16];
-    tc::tmem_ld16(taddr + c, v0);
-    tc::tmem_ld16(taddr + c + 16, v1);
+    uint32_t v[16];
+    tc::tmem_ld16(taddr + c, v);
     tc::tmem_wait_ld();
     float mx = 0.f;
-    auto L = [&](int j) { return __uint_as_float(j < 16 ? v0[j & 15] : v1[j & 15]); };
 #pragma unroll
-    for (int j = 0; j < 32; ++j) mx = fmaxf(mx, fabsf(L(j)));
+    for (int j = 0; j < 16; ++j) mx = fmaxf(mx, fabsf(__uint_as_float(v[j])));
     const bool big = __any_sync(0xffffffffu, mx * fabsf(f) >= 0x1p22f);
     auto put = [&](int j, uint32_t n) {
       if (HI)
@@ -757,21 +1097,157 @@ __device__ __forceinline__ void tc_drain(uint32_t taddr, int nrow, float f, uint
     };
     if (!big) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) put(j, __float_as_uint(fmaf(L(j), f, 12582912.f)));
+      for (int j = 0; j < 16; ++j)
+        put(j, __float_as_uint(fmaf(__uint_as_float(v[j]), f, 12582912.f)));
     } else {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) put(j, (uint32_t)__float2int_rn(L(j) * f) + kMagic);
+      for (int j = 0; j < 16; ++j)
+        put(j, (uint32_t)__float2int_rn(__uint_as_float(v[j]) * f) + kMagic);
+    }
+  }
+}
+
+// Finished sums n0 .. n0 + cnt - 1 of column c (TMEM lane) of the unit's tile (DIR 3: matrix row
+// c, map columns n); every lane of the warp calls it.  What is read back is read before anything
+// is written, so the loads are in flight together.
+template <int DIR, int SPIN, int kOut>
+__device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int ph, bool store,
+                                       int c, int n0, int cnt, int map, int eb, int e,
+                                       const long long (&sum)[kOut], const TcFac* fac) {
+  const int comp = c & 1;
+  double v[kOut];
+  if (DIR == 0) {
+    if (!store) return;
+    const long long L1 = a.lmax + 1;
+    const long long row = comp == 0 ? (long long)w.m * L1 + w.row0 + 2 * n0
+                                    : (L1 - w.m) * L1 + (w.row0 - w.m) + 2 * n0;
+    double* d = a.out[SPIN == 2 ? w.field : 0] + row * a.ld + a.k0 + map;
+    const long long ds = 2LL * a.ld;
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) v[j] = a.accumulate && j < cnt ? d[j * ds] : 0.0;
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+      const double x = i64_scaled_mul(sum[j], fac[j], e);
+      if (j < cnt) d[j * ds] = a.accumulate ? v[j] + x : x;
+    }
+  } else if (DIR == 1) {
+    if (!store) return;
+    double* d = a.out[SPIN == 2 ? w.field : 0] +
+                (((long long)w.m * a.nnorth + w.row0 + n0) * a.kc + map) * 4 + comp;
+    const long long ds = (long long)a.kc * 4;
+    if (ph == 0) {                   // A waits, as its integer, in the slot of the same thread
+#pragma unroll
+      for (int j = 0; j < kOut; ++j)
+        if (j < cnt) d[j * ds] = __longlong_as_double(sum[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) v[j] = j < cnt ? d[j * ds] : 0.0;
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) {
+        const long long A = __double_as_longlong(v[j]);
+        if (j < cnt) {
+          d[j * ds] = i64_scaled(A + sum[j], e);
+          d[j * ds + 2] = i64_scaled(A - sum[j], e);
+        }
+      }
+    }
+  } else if (DIR == 2) {
+    // {S, D} = F_N +- F_S from the lane pair (the map's north and south), then every kept order
+    // a n +- r of bin r
+    const int nr = 4 * w.d.q, cmp = w.p >= 2;
+    double* d = a.out[0] + (((long long)w.m * a.w_kc + a.k_off + map) * 2 + comp) * 2;
+    const long long ms = (long long)a.nnorth * a.w_kc * 4;
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+      const long long o = __shfl_xor_sync(0xffffffffu, sum[j], 1);
+      v[j] = i64_scaled(comp == 0 ? sum[j] + o : o - sum[j], e);
+      if (eb == kNanExp) v[j] = __longlong_as_double(0x7FF8000000000000ll);
+    }
+    if (!store) return;
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+      if (j >= cnt) break;
+      const int r = dft_r(w.p, w.row0 + n0 + j);
+      const bool self = r == 0 || 2 * r == nr;
+      double sg = cmp ? -v[j] : v[j];              // Im F = -(sin sum)
+      for (int m0 = 0; m0 - r <= w.d.mtop; m0 += nr) {
+        if (m0 > 0 && !self) d[(long long)(m0 - r) * ms + cmp] = cmp ? -sg : sg;
+        if (m0 + r <= w.d.mtop) {
+          d[(long long)(m0 + r) * ms + cmp] = sg;
+          // the parts that no row computes: Im at r = 0, and with s = 1 Re at n / 2
+          if (r == 0) d[(long long)m0 * ms + 1] = sg - sg;
+          if (w.d.s && w.p == 2 && 2 * r == nr) d[(long long)(m0 + r) * ms] = sg - sg;
+        }
+        if (w.d.s) sg = -sg;
+      }
+    }
+  } else {
+    // phases: e, o, se, so (cos even, cos odd, sin even, sin odd sums at sample j); the four
+    // mirrored samples hold them until so is there:
+    //   x_j = P - T, x_{-j} = P + T, x_{pi-j} = M + V, x_{pi+j} = M - V
+    //   P, M = e +- o, T = se + so, V = se - so
+    // (on the axis x_{-0} is x_0, and both sin sums are zero)
+    const int nr = 4 * w.d.q, j0 = w.row0 + c;
+    if (!store || (ph >= 2 && w.d.s == 0 && j0 == 0)) return;
+    const bool equator = w.m == a.nnorth - 1;
+    double* x = a.out[0] + (long long)(w.g * kGroupMaps) * a.map_stride;
+    const long long on = ring_start(a.nside, w.m), os = ring_start(a.nside, a.nring - 1 - w.m);
+    const int i1 = nr - w.d.s - j0, i2 = nr / 2 - w.d.s - j0, i3 = nr / 2 + j0;
+    auto base = [&](int j) {
+      return x + (long long)((n0 + j) >> 1) * a.map_stride + (((n0 + j) & 1) ? os : on);
+    };
+    auto live = [&](int j) { return j < cnt && !(equator && ((n0 + j) & 1)); };
+    double p[kOut], q[kOut];
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+      v[j] = ph >= 1 && live(j) ? base(j)[j0] : 0.0;
+      p[j] = ph == 3 && live(j) ? base(j)[i2] : 0.0;
+      q[j] = ph == 3 && live(j) ? base(j)[i1] : 0.0;
+    }
+    auto bits = [](double t) { return __double_as_longlong(t); };
+    auto keep = [](long long t) { return __longlong_as_double(t); };
+#pragma unroll
+    for (int j = 0; j < kOut; ++j) {
+      if (!live(j)) continue;
+      const int ec = fac[j].fe;
+      double* b = base(j);
+      if (ph == 0) {
+        b[j0] = keep(sum[j]);
+      } else if (ph == 1) {
+        b[j0] = keep(bits(v[j]) + sum[j]);
+        b[i2] = keep(bits(v[j]) - sum[j]);
+        if (w.d.s == 0 && j0 == 0) {                       // no later phase
+          b[j0] = ec == kNanExp ? keep(0x7FF8000000000000ll)
+                                : i64_scaled(bits(v[j]) + sum[j], ec + e);
+          b[i2] = ec == kNanExp ? keep(0x7FF8000000000000ll)
+                                : i64_scaled(bits(v[j]) - sum[j], ec + e);
+        }
+      } else if (ph == 2) {
+        b[i1] = keep(sum[j]);
+      } else {
+        const long long T = bits(q[j]) + sum[j], V = bits(q[j]) - sum[j];
+        const long long P = bits(v[j]), M = bits(p[j]);
+        auto out = [&](long long t) {
+          return ec == kNanExp ? keep(0x7FF8000000000000ll) : i64_scaled(t, ec + e);
+        };
+        b[j0] = out(P - T);
+        b[i1] = out(P + T);
+        b[i2] = out(M + V);
+        b[i3] = out(M - V);
+      }
     }
   }
 }
 
 template <int DIR, int SPIN>
 __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
-  constexpr int NPH = DIR == 0 ? 1 : 2, NSEG = SPIN == 2 ? 2 : 1;
+  constexpr int NPH = DIR == 0 || DIR == 2 ? 1 : DIR == 1 ? 2 : 4, NSEG = SPIN == 2 ? 2 : 1;
+  constexpr bool SWAP = DIR == 3;      // matrix rows on the TMEM lanes, map columns as N
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ TcSmemHdr h;
   __shared__ UnitQueue uq;
-  __shared__ double s_fac[kEpiThreads / 32][64];      // per epilogue warp: its rows' factors
+  // per epilogue warp: its rows' factors (DIR 0), its columns' exponents (DIR 3: fe)
+  __shared__ TcFac s_fac[kTcEpiWarps][kTcAcc];
 
   const int tid = threadIdx.x;
   const int warp = tc::warp_index();
@@ -783,10 +1259,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
     }
     for (int s = 0; s < 4; ++s) {
       tc::mbar_init(&h.tfull[s], 1);
-      tc::mbar_init(&h.tempty[s], kEpiThreads / 32);
+      tc::mbar_init(&h.tempty[s], kTcEpiWarps);
     }
     tc::mbar_init(&h.fin, 2);
-    uq_init(uq, kEpiThreads / 32 + 2);
+    uq_init(uq, kTcEpiWarps + 2);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -797,7 +1273,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
   const uint32_t tmem = h.tmem;
 
   uint32_t n_loaded = 0;
-  if (tid == kEpiThreads) {
+  if (tid == kTcEpi) {
     uint32_t i = 0;
     uq_walk(uq, a.nunits, 0, abort, [&](int u) -> bool {
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
@@ -826,9 +1302,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
       }
       return true;
     });
-  } else if (warp > kEpiThreads / 32) {
+  } else if (warp > kTcEpiWarps) {
     // UMMA warps: slots 0 and 3, and slots 1 and 2 (5 of 10 and 13 of 26 products each)
-    const int side = warp - kEpiThreads / 32 - 1;
+    const int side = warp - kTcEpiWarps - 1;
     const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
     const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
     uint32_t i = 0, use = 0;       // stages consumed, passes issued (one use of every slot each)
@@ -850,8 +1326,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
               break;
             }
             tc::tc_fence_after();
-            const uint64_t ca = tc::umma_desc(s_u + st * kTcStageBytes, 128, 256);
-            const uint64_t ra = tc::umma_desc_add(ca, kHalfBytes);
+            const uint64_t c0 = tc::umma_desc(s_u + st * kTcStageBytes, 128, 256);
+            const uint64_t c1 = tc::umma_desc_add(c0, kHalfBytes);
+            const uint64_t ca = SWAP ? c1 : c0, ra = SWAP ? c0 : c1;
 #pragma unroll
             for (int lev = 0; lev < 4; ++lev) {
               if ((lev == 0 || lev == 3) != (side == 0)) continue;
@@ -882,8 +1359,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
             tc::tc_fence_after();
             const uint64_t ca = tc::umma_desc(s_u + st * kTcStageBytes, 128, 256);
             const uint64_t cb = tc::umma_desc(s_u + st1 * kTcStageBytes, 128, 256);
-            auto plane = [&](int d) {
-              return tc::umma_desc_add(d < 4 ? ca : cb, (uint32_t)(d & 3) * kPlaneBytes);
+            // plane d of the UMMA's first (M) operand and of its second
+            auto plane = [&](int d, bool second) {
+              return tc::umma_desc_add(d < 4 ? ca : cb, (uint32_t)(d & 3) * kPlaneBytes +
+                                                            (second != SWAP ? kHalfBytes : 0));
             };
 #pragma unroll
             for (int lev = 4; lev < 8; ++lev) {
@@ -897,8 +1376,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
               }
 #pragma unroll
               for (int aa = 0; aa <= lev; ++aa)
-                tc::umma_bf16_warp(utmem + (lev - 4) * kCols, plane(aa),
-                                   tc::umma_desc_add(plane(lev - aa), kHalfBytes), idesc,
+                tc::umma_bf16_warp(utmem + (lev - 4) * kCols, plane(aa, false),
+                                   plane(lev - aa, true), idesc,
                                    (k > 0 || aa > 0) ? 1u : 0u);
               if (k == nk - 1) tc::umma_commit_warp(&h.tfull[lev - 4]);
             }
@@ -911,15 +1390,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
         }
       }
     }
-  } else if (tid < kEpiThreads) {
+  } else if (tid < kTcEpi) {
     // epilogue: each warp works alone (no barrier among them); after an expired wait the
     // remaining slots are walked without work
     const int lane = tid & 31;
     const int c = ((warp & 3) << 5) + lane;              // tile column: 2 map + comp
     const int comp = c & 1;
-    const int rbeg = (warp >> 2) * 64;                   // this warp's half of the rows
+    const int rbeg = (warp >> 2) * kTcAcc;               // this warp's quarter of the columns
     const uint32_t tbase = tmem + ((uint32_t)((warp & 3) << 5) << 16) + rbeg;
-    const long long L1 = a.lmax + 1;
     // level weights 2^wt, wt = unit_bits - 8 s, as (float factor, integer multiplier): 2^32 and up
     // in the high word, the others with multipliers <= 2^30
     uint32_t use = 0;
@@ -929,26 +1407,40 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
       if (w.nk == 0) continue;
       const int map = w.g * kGroupMaps + (c >> 1);
-      const int nrow = min(64, w.nrows - rbeg);
+      const int ncol = 2 * min(kGroupMaps, a.kc - w.g * kGroupMaps);
+      const int nrow = min(kTcAcc, (SWAP ? ncol : w.nrows) - rbeg);   // TMEM columns of this warp
       if (DIR == 0) {
         __syncwarp();
-        for (int j = lane; j < 64; j += 32) {
-          const int l = w.row0 + 2 * (rbeg + j);
-          s_fac[warp][j] = l <= a.lmax ? a.tab[tri_off(w.m, a.lmax) + (l - w.m)].dm * a.pa : 0.0;
+        {
+          const int l = w.row0 + 2 * (rbeg + lane);
+          s_fac[warp][lane] =
+              tc_fac(l <= a.lmax ? a.tab[tri_off(w.m, a.lmax) + (l - w.m)].dm * a.pa : 0.0);
         }
         __syncwarp();
       }
-      const int4 fl = *reinterpret_cast<const int4*>(a.flags +
-                                                     ((long long)w.m * a.ngroups + w.g) * 4);
-      const bool store = (fl.x | fl.y | fl.z | fl.w) == 0 && map < a.kc &&
-                         (DIR == 1 || !(comp == 1 && w.m == 0));
+      bool store = map < a.kc;
+      if (DIR < 2) {
+        const int4 fl = *reinterpret_cast<const int4*>(a.flags +
+                                                       ((long long)w.m * a.ngroups + w.g) * 4);
+        store = (fl.x | fl.y | fl.z | fl.w) == 0 && map < a.kc &&
+                (DIR == 1 || !(comp == 1 && w.m == 0));
+      }
+      if (DIR == 3) {
+        __syncwarp();
+        s_fac[warp][lane].fe = a.EB[((long long)w.qi * a.ngroups + w.g) * kCols + rbeg + lane];
+        __syncwarp();
+        store = c < w.nrows;                               // the lane's matrix row
+      }
 #pragma unroll 1
       for (int ph = 0; ph < NPH; ++ph) {
         const int par = DIR == 0 ? w.p : ph;
-        const int eb = a.EB[(((long long)w.qi * 2 + par) * a.ngroups + w.g) * kCols + c];
-        unsigned long long acc[64], bias = 0;
+        const int eb =
+            DIR == 3 ? 0
+                     : a.EB[((DIR == 2 ? (long long)w.qi : (long long)w.qi * 2 + par) * a.ngroups +
+                             w.g) * kCols + c];
+        unsigned long long acc[kTcAcc], bias = 0;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) acc[j] = 0;
+        for (int j = 0; j < kTcAcc; ++j) acc[j] = 0;
 #pragma unroll 1
         for (int sg = 0; sg < NSEG; ++sg) {
           int sign = 1;
@@ -980,49 +1472,32 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
             }
           }
         }
-        // the phase's sums out
-        const int e = eb - 12 - a.unit_bits + (DIR == 0 ? a.eag : 0);
-        if (!store) continue;
-        if (DIR == 0) {
-          double* out = a.out[SPIN == 2 ? w.field : 0] + a.k0 + map;
-          double* dst = out + (comp == 0 ? (long long)w.m * L1 + w.row0 + 2 * rbeg
-                                         : (L1 - w.m) * L1 + (w.row0 - w.m) + 2 * rbeg) * a.ld;
+        // the phase's sums out, a few at a time: the output code exists once and the registers
+        // move down to it (unrolled over all sums it ran at the instruction fetch rate, one value
+        // at a time at the latency of a load)
+        const int e = eb - 12 - a.unit_bits + (DIR == 0 ? a.eag : DIR >= 2 ? 1 : 0);
+        constexpr int kOut = 4;
+#pragma unroll 1
+        for (int c0 = 0; c0 < nrow; c0 += kOut) {
+          long long sum[kOut];
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            if (j >= nrow) break;
-            const double v = i64_scaled((long long)(acc[j] - bias), e) * s_fac[warp][j];
-            double* d = dst + (long long)(2 * j) * a.ld;
-            *d = a.accumulate ? *d + v : v;
-          }
-        } else {
-          double* dst = a.out[SPIN == 2 ? w.field : 0] +
-                        (((long long)w.m * a.nnorth + w.row0 + rbeg) * a.kc + map) * 4 + comp;
-          const long long rs = (long long)a.kc * 4;
-          // phase 0 leaves A in the north slot; the same thread reads it back in phase 1
+          for (int j = 0; j < kOut; ++j) sum[j] = (long long)(acc[j] - bias);
 #pragma unroll
-          for (int j = 0; j < 64; ++j) {
-            if (j >= nrow) break;
-            const double v = i64_scaled((long long)(acc[j] - bias), e);
-            if (ph == 0) {
-              dst[j * rs] = v;
-            } else {
-              const double A = dst[j * rs];
-              dst[j * rs] = A + v;
-              dst[j * rs + 2] = A - v;
-            }
-          }
+          for (int j = 0; j + kOut < kTcAcc; ++j) acc[j] = acc[j + kOut];
+          tc_out<DIR, SPIN, kOut>(a, w, ph, store, c, rbeg + c0, min(kOut, nrow - c0), map, eb, e, sum,
+                            &s_fac[warp][c0]);
         }
       }
     }
   }
   // the UMMA issuer waits for its last products before TMEM is released, the loader for its
   // last copies
-  if (warp > kEpiThreads / 32) {
+  if (warp > kTcEpiWarps) {
     tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
   }
-  if (tid == kEpiThreads) {
+  if (tid == kTcEpi) {
     for (uint32_t d = 0; d < (uint32_t)kTcStages && d < n_loaded; ++d) {
       const uint32_t i = n_loaded - 1 - d;
       for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
@@ -1055,12 +1530,13 @@ int ceil_log2(long long x) {
 // Integer units: sums in digit units are below 2^12 times the sum of |row| / scale, and the 64-bit
 // sum has 63 bits.  Analysis: sum over the north rings of |lambda| (spin 2: |lambda1| + |lambda2|)
 // is below 0.85 nside for every l and m (tests/test_tc_bounds.py), against 2^EAG.  Synthesis: the
-// sum over l of one parity of |lambda| 2^-EA(l) is below 0.4 (lmax/2 + 1) for the same reason.
+// sum over l of one parity of |lambda| 2^-EA(l) is below 0.4 (lmax/2 + 1) for the same reason, and
+// the two parities are added and subtracted.
 int tc_bits_analysis(const fsht_plan* p) {
   return std::min(46, 51 - ceil_log2(p->nside) + tc_eag(p->lmax));
 }
 int tc_bits_synthesis(const fsht_plan* p) {
-  return std::min(46, 51 - ceil_log2((2LL * (p->lmax / 2 + 1) + 4) / 5 + 1));
+  return std::min(46, 50 - ceil_log2((2LL * (p->lmax / 2 + 1) + 4) / 5 + 1));
 }
 
 template <int DIR, int SPIN>
@@ -1146,9 +1622,9 @@ int fsht_launch_tc_slice_alm(fsht_plan* p, int w, const double* alm0, const doub
   a.flags = p->d_tcflag;
   const dim3 grid(wv[1] - wv[0], a.ngroups);
   if (alm1)
-    k_tc_slice_alm<2><<<grid, 256, 0, s>>>(a);
+    k_tc_slice_alm<2><<<grid, 512, 0, s>>>(a);
   else
-    k_tc_slice_alm<1><<<grid, 128, 0, s>>>(a);
+    k_tc_slice_alm<1><<<grid, 256, 0, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }
@@ -1234,4 +1710,202 @@ int fsht_launch_tc_gemm(fsht_plan* p, int w, int dir, int spin, const unsigned c
   if (dir == 0)
     return spin == 0 ? launch_tc_gemm<0, 0>(a, s) : launch_tc_gemm<0, 2>(a, s);
   return spin == 0 ? launch_tc_gemm<1, 0>(a, s) : launch_tc_gemm<1, 2>(a, s);
+}
+
+// ------------------------------------------------------------------ ring transforms, host side
+namespace {
+// The belt takes the matrix form up to this nside: its products grow with nside^3 in all, the
+// power-of-two FFT's passes with nside^2 log nside.
+constexpr int kDftBeltMax = 256;
+constexpr int kDftWaveInts = 5;     // first entry, end, most row tiles, largest q, digit k-steps
+
+// Sums of q / 2 + 1 products against the cosines' 2^1; north and south, or the four mirrored
+// samples, are added and subtracted.
+int dft_bits(int qmax, int extra) { return std::min(46, 51 - extra - ceil_log2(qmax / 2 + 2)); }
+
+DftSliceArgs dft_slice_args(const fsht_plan* p, const int* wv, int ngroups) {
+  DftSliceArgs a{};
+  a.rings = p->d_dft + wv[0];
+  a.ngroups = ngroups;
+  a.WS = p->d_ws;
+  a.EB = p->d_eb;
+  a.nside = p->nside;
+  a.nring = p->nring;
+  a.nnorth = p->nnorth;
+  return a;
+}
+
+template <bool INV>
+int launch_dft_trig(fsht_plan* p, const int* wv, cudaStream_t s) {
+  DftTrigArgs a;
+  a.rings = p->d_dft + wv[0];
+  a.cosv = p->d_dft_cos;
+  a.lbuf = p->d_lbuf;
+  const size_t sm = sizeof(long long) * (2 * (size_t)wv[3] + 1);
+  FSHT_TRY(fsht_smem_limit((const void*)k_dft_trig<INV>, sm));
+  k_dft_trig<INV><<<dim3(wv[1] - wv[0], 4 * wv[2]), 256, sm, s>>>(a);
+  FSHT_LAUNCH_CHECK();
+  return FSHT_OK;
+}
+
+TcGemmArgs dft_gemm_args(const fsht_plan* p, const int* wv, int ngroups, int cnt, int extra) {
+  TcGemmArgs a{};
+  a.ngroups = ngroups;
+  a.ntmax = wv[2];
+  a.nnorth = p->nnorth;
+  a.unit_bits = dft_bits(p->nside, extra);
+  a.lbuf = p->d_lbuf;
+  a.WS = p->d_ws;
+  a.EB = p->d_eb;
+  a.kc = cnt;
+  a.err = p->d_err;
+  a.rings = p->d_dft + wv[0];
+  a.nside = p->nside;
+  a.nring = p->nring;
+  return a;
+}
+}  // namespace
+
+// The rings of the matrix form in waves whose matrix tiles fit the lambda staging buffer and
+// whose digit tiles fit one 64-map group's share of the contraction's; belt rings of one phase
+// share their matrices.
+int fsht_dft_tables_init(fsht_plan* p) {
+  const int ns = p->nside;
+  const int end = ns <= kDftBeltMax ? 2 * ns : ns - 1;
+  p->dft_end = 0;
+  std::vector<FshtDftRing> rings;
+  std::vector<int> order;
+  for (int i = ns - 2; i >= 0; --i) order.push_back(i);            // caps, large first
+  if (end > ns)
+    for (int s = 1; s >= 0; --s)
+      for (int i = ns - 1; i < 2 * ns; ++i)
+        if (ring_phase_flag(ns, i) == s) order.push_back(i);
+  // the staging buffer holds at least the largest ring's matrices, and all of a small plan's
+  const long long unit = kStepBytes;
+  const long long nkm = (ns + 16) / 16, nrm = (ns + 128) / 128;
+  const long long want = std::max<long long>(4 * nkm * nrm, std::min<long long>(2048, 2LL * ns * ns / 16));
+  p->lbuf_bytes = std::max<size_t>(p->lbuf_bytes, (size_t)(want * unit));
+  const long long cap_t = (long long)(p->lbuf_bytes / unit);
+  const long long cap_c = (long long)(fsht_tc_ws_bytes(p, 1, 1) / unit);
+  const int cap_r = 2 * p->wave_qmax;
+  std::vector<int> waves;
+  long long ut = 0, uc = 0, ucos = 0;
+  int w0 = 0, nrt = 0, qm = 0;
+  std::vector<long long> cls(2, -1), clsc(2, -1);                  // belt classes of this wave
+  auto close = [&](int e) {
+    if (e > w0) {
+      const int wv[kDftWaveInts] = {w0, e, nrt, qm, (int)uc};
+      waves.insert(waves.end(), wv, wv + kDftWaveInts);
+    }
+    w0 = e;
+    ut = uc = 0;
+    nrt = qm = 0;
+    cls[0] = cls[1] = -1;
+  };
+  for (int i : order) {
+    FshtDftRing d{};
+    d.ring = i;
+    d.q = std::min(i + 1, ns);
+    d.s = ring_phase_flag(ns, i);
+    d.nk = (d.q + (d.s == 0) + kKStep - 1) / kKStep;
+    d.nrt = (d.q + (d.s == 0) + kRows - 1) / kRows;
+    d.mtop = -1;
+    for (int m = p->lmax; m >= 0; --m)
+      if (p->h_ring_i0[m] <= i) {
+        d.mtop = m;
+        break;
+      }
+    const bool belt = d.q == ns;
+    const long long tsteps = 4LL * d.nrt * d.nk, csteps = 4LL * d.nk;
+    if (tsteps > cap_t || csteps > cap_c) return FSHT_OK;          // no matrix form
+    bool fresh = !belt || cls[d.s] < 0;
+    if (ut + (fresh ? tsteps : 0) > cap_t || uc + csteps > cap_c ||
+        (int)rings.size() - w0 >= cap_r) {
+      close((int)rings.size());
+      fresh = true;
+    }
+    d.first = fresh ? 1 : 0;
+    if (fresh) {
+      d.off_t = ut;
+      ut += tsteps;
+      if (belt) cls[d.s] = d.off_t;
+    } else {
+      d.off_t = cls[d.s];
+    }
+    if (belt && clsc[d.s] >= 0) {
+      d.off_cos = clsc[d.s];
+    } else {
+      d.off_cos = ucos;
+      ucos += 2LL * d.q + 1;
+      if (belt) clsc[d.s] = d.off_cos;
+    }
+    d.off_c = uc;
+    uc += csteps;
+    nrt = std::max(nrt, d.nrt);
+    qm = std::max(qm, d.q);
+    rings.push_back(d);
+  }
+  close((int)rings.size());
+  if (rings.empty()) return FSHT_OK;
+  p->ndft_waves = (int)waves.size() / kDftWaveInts;
+  p->h_dft_waves = new (std::nothrow) int[waves.size()];
+  if (!p->h_dft_waves) {
+    fsht_set_error("host allocation failed");
+    return FSHT_ENOMEM;
+  }
+  std::copy(waves.begin(), waves.end(), p->h_dft_waves);
+  FSHT_CUDA_TRY(cudaMalloc(&p->d_dft, sizeof(FshtDftRing) * rings.size()));
+  FSHT_CUDA_TRY(cudaMalloc(&p->d_dft_cos, sizeof(long long) * ucos));
+  FSHT_CUDA_TRY(cudaMemcpyAsync(p->d_dft, rings.data(), sizeof(FshtDftRing) * rings.size(),
+                                cudaMemcpyHostToDevice, p->stream));
+  k_dft_cos<<<(unsigned)rings.size(), 256, 0, p->stream>>>(p->d_dft, p->d_dft_cos);
+  FSHT_LAUNCH_CHECK();
+  FSHT_CUDA_TRY(cudaStreamSynchronize(p->stream));                 // the list is a local vector
+  p->dft_end = end;
+  return FSHT_OK;
+}
+
+// Maps [k0, k0 + cnt) of a chunk of kc maps (maps: the chunk's base) -> their {S, D} of rings
+// below dft_end.
+int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, int kc, int k0,
+                        int cnt, double2* W, cudaStream_t s) {
+  const int ngroups = tc_groups(cnt);
+  for (int w = 0; w < p->ndft_waves; ++w) {
+    const int* wv = p->h_dft_waves + kDftWaveInts * w;
+    FSHT_TRY(launch_dft_trig<false>(p, wv, s));
+    DftSliceArgs sa = dft_slice_args(p, wv, ngroups);
+    sa.maps = maps + (long long)k0 * map_stride;
+    sa.map_stride = map_stride;
+    sa.cnt = cnt;
+    k_dft_slice<<<dim3(wv[1] - wv[0], (cnt + 3) / 4), 256, 0, s>>>(sa);
+    FSHT_LAUNCH_CHECK();
+    TcGemmArgs a = dft_gemm_args(p, wv, ngroups, cnt, 1);
+    a.k_off = k0;
+    a.w_kc = kc;
+    a.out[0] = reinterpret_cast<double*>(W);
+    a.nunits = ngroups * 4 * a.ntmax * (wv[1] - wv[0]);
+    FSHT_TRY((launch_tc_gemm<2, 0>(a, s)));
+  }
+  return FSHT_OK;
+}
+
+// {G_N, G_S} of rings below dft_end -> their pixels.
+int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride, int kc,
+                        cudaStream_t s) {
+  const int ngroups = tc_groups(kc);
+  for (int w = 0; w < p->ndft_waves; ++w) {
+    const int* wv = p->h_dft_waves + kDftWaveInts * w;
+    FSHT_TRY(launch_dft_trig<true>(p, wv, s));
+    DftSliceArgs sa = dft_slice_args(p, wv, ngroups);
+    sa.W = W;
+    sa.kc = kc;
+    k_dft_slice_inv<<<dim3(wv[1] - wv[0], (kc + 15) / 16), 256, 0, s>>>(sa);
+    FSHT_LAUNCH_CHECK();
+    TcGemmArgs a = dft_gemm_args(p, wv, ngroups, kc, 2);
+    a.map_stride = map_stride;
+    a.out[0] = maps;
+    a.nunits = ngroups * a.ntmax * (wv[1] - wv[0]);
+    FSHT_TRY((launch_tc_gemm<3, 0>(a, s)));
+  }
+  return FSHT_OK;
 }

@@ -44,16 +44,29 @@ __device__ __forceinline__ double lam_fact(int l, int m) {
   if (l <= m1) return 0.0;
   return 2.0 * sqrt((double)(2 * l + 1) / (double)(2 * l - 1) * (double)((long long)l * l - (long long)m * m));
 }
-__device__ __forceinline__ void pol_lambda(const PolRing& r, int l, int m, double cur, double prev,
+// The ring-independent factors of step l (integers, exact in FP64; nm = 2 m (1 - m) at l = m).
+struct PolL {
+  double lm, ll, l1, nm;
+  bool diag;
+};
+__device__ __forceinline__ PolL pol_l(int l, int m) {
+  PolL p;
+  p.lm = (double)((long long)l - (long long)m * m);
+  p.ll = (double)l * ((double)l - 1.0);
+  p.l1 = (double)l - 1.0;
+  p.nm = (double)(2LL * m * (1 - m));
+  p.diag = l == m;
+  return p;
+}
+__device__ __forceinline__ void pol_lambda(const PolRing& r, const PolL& p, double cur, double prev,
                                            double lf, double nl, double& l1, double& l2) {
-  if (l == m) {
-    const double nm = (double)(2LL * m * (1 - m)) * nl;
+  if (p.diag) {
+    const double nm = p.nm * nl;
     l1 = nm * cur * r.diag1;
     l2 = nm * cur * r.diag2;
   } else {
-    l1 = (prev * lf * r.b_w - cur * (r.two_on_s2 * (double)((long long)l - (long long)m * m) +
-                                     (double)l * ((double)l - 1.0))) * nl;
-    l2 = (prev * lf - cur * (2.0 * r.cth * ((double)l - 1.0))) * r.c_w * nl;
+    l1 = (prev * lf * r.b_w - cur * (r.two_on_s2 * p.lm + p.ll)) * nl;
+    l2 = (prev * lf - cur * (2.0 * r.cth * p.l1)) * r.c_w * nl;
   }
 }
 

@@ -123,6 +123,9 @@ void free_plan_memory(fsht_plan* p) {
   cudaFree(p->d_lam_offT);
   cudaFree(p->d_tcflag);
   cudaFree(p->d_lamtab2);
+  cudaFree(p->d_dft);
+  cudaFree(p->d_dft_cos);
+  delete[] p->h_dft_waves;
   cudaFree(p->d_lbuf);
   cudaFree(p->d_lbuf2);
   for (int i = 0; i < 6; ++i)
@@ -331,6 +334,7 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     return fail(rc);
   if (precision == FSHT_PREC_FP64 && fsht_tc_supported(p)) {
     if ((rc = fsht_tc_tables_init(p))) return fail(rc);
+    if ((rc = fsht_dft_tables_init(p))) return fail(rc);
     p->tc64 = 1;
   }
   // ---- workspace: nbuf phase matrices of kchunk maps (+ the sliced copy for the
@@ -656,6 +660,30 @@ enum { kEvFork = 0, kEvJoin = 1, kEvTiles = 2, kEvDone = 4 };
 // Whether a call of this plan takes the tensor-core form of the FP64 contraction.
 static bool use_tc(const fsht_plan* p, int spin) {
   return p->tc64 && p->d_lbuf && p->d_tcflag && (spin == 0 || p->d_poltab);
+}
+
+// Whether a chunk of kc device-resident maps takes the matrix form of the ring transforms for the
+// rings below dft_end (it uses the contraction's buffers).
+static bool use_dft(const fsht_plan* p, int kc) {
+  return use_tc(p, 0) && p->dft_end > 0 && kc >= 1;
+}
+
+// Ring transforms of a whole chunk: matrix form below dft_end where it applies, FFT above.
+static int ring_fwd(fsht_plan* p, const double* maps, int kc, double2* W) {
+  int ring0 = 0;
+  if (use_dft(p, kc)) {
+    FSHT_TRY(fsht_launch_dft_fwd(p, maps, p->npix, kc, 0, kc, W, p->stream));
+    ring0 = p->dft_end;
+  }
+  return fsht_launch_ring_fft_fwd_part(p, maps, p->npix, kc, 0, kc, W, p->stream, ring0);
+}
+static int ring_inv(fsht_plan* p, const double2* W, double* maps, int kc) {
+  int ring0 = 0;
+  if (use_dft(p, kc)) {
+    FSHT_TRY(fsht_launch_dft_inv(p, W, maps, p->npix, kc, p->stream));
+    ring0 = p->dft_end;
+  }
+  return fsht_launch_ring_fft_inv(p, W, maps, p->npix, kc, p->stream, ring0);
 }
 
 static unsigned char* lam_buf(fsht_plan* p, int w) {
@@ -1055,12 +1083,16 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
       hx->cdone.assign(p->lmax + 1, 0);
     }
     // the first lambda tiles are computed on the auxiliary stream during the FFT
-    const bool tc = !split && use_tc(p, 0);
+    // (not beside the matrix form of the FFT, which uses the tiles' buffers)
+    const bool tc = !split && use_tc(p, 0) && ((hx && hx->direct) || !use_dft(p, kc));
     if (split) FSHT_TRY(lam_start(p, fsht_launch_split_lambda));
     if (tc) FSHT_TRY(lam_start(p, fsht_launch_tc_lambda));
     // the chunk's maps as the FFT reads them: device buffer, or host memory read in place
     const double* cmaps = (hx && hx->direct ? hx->direct : maps) + (size_t)c0 * p->npix;
-    if (!hx || hx->direct) {
+    if (!hx && !split) {
+      FSHT_PROF(FSHT_KCAT_FFT_FWD);
+      FSHT_TRY(ring_fwd(p, cmaps, kc, W0));
+    } else if (!hx || hx->direct) {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
       // (page-locked maps mapped into the device's address space are read over the host link
       // as the transform goes, every value once, with no staging copy)
@@ -1078,7 +1110,13 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
         FSHT_CUDA_TRY(cudaEventRecord(p->evx[1], p->xfer));
         FSHT_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->evx[1], 0));
         FSHT_PROF(FSHT_KCAT_FFT_FWD);
-        FSHT_TRY(fsht_launch_ring_fft_fwd_part(p, cmaps, p->npix, kc, k0, cnt, W0, p->stream));
+        int ring0 = 0;
+        if (use_dft(p, kc)) {
+          FSHT_TRY(fsht_launch_dft_fwd(p, cmaps, p->npix, kc, k0, cnt, W0, p->stream));
+          ring0 = p->dft_end;
+        }
+        FSHT_TRY(fsht_launch_ring_fft_fwd_part(p, cmaps, p->npix, kc, k0, cnt, W0, p->stream,
+                                               ring0));
       }
     }
     if (split) {
@@ -1165,7 +1203,7 @@ int fsht_alm2t(fsht_plan* p, const double* alm, double* maps, int nmaps) {
     }
     {
       FSHT_PROF(FSHT_KCAT_FFT_INV);
-      FSHT_TRY(fsht_launch_ring_fft_inv(p, W0, maps + (size_t)c0 * p->npix, p->npix, kc, p->stream));
+      FSHT_TRY(ring_inv(p, W0, maps + (size_t)c0 * p->npix, kc));
     }
   }
   return FSHT_OK;
@@ -1282,16 +1320,16 @@ static int qu_analysis(fsht_plan* p, const double* Q, const double* U, double* a
     double2* WQ = work_buf(p, 0, kc);
     double2* WU = work_buf(p, 1, kc);
     const bool split = p->precision == FSHT_PREC_SPLIT;
-    const bool pre = split ? p->d_poltab != nullptr : use_tc(p, 2);
+    const bool pre = split ? p->d_poltab != nullptr : use_tc(p, 2) && !use_dft(p, kc);
     if (pre)                                                         // overlaps the FFTs
       FSHT_TRY(lam_start(p, split ? fsht_launch_split_lambda_pol : fsht_launch_tc_lambda_pol));
     {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
-      FSHT_TRY(fsht_launch_ring_fft_fwd(p, Q + (size_t)c0 * p->npix, p->npix, kc, WQ, p->stream));
+      FSHT_TRY(ring_fwd(p, Q + (size_t)c0 * p->npix, kc, WQ));
     }
     {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
-      FSHT_TRY(fsht_launch_ring_fft_fwd(p, U + (size_t)c0 * p->npix, p->npix, kc, WU, p->stream));
+      FSHT_TRY(ring_fwd(p, U + (size_t)c0 * p->npix, kc, WU));
     }
     FSHT_TRY(pol_analysis(p, WQ, WU, almE, almB, nmaps, c0, kc, 0, which, pre));
     if (niter > 0) {
@@ -1357,11 +1395,11 @@ int fsht_eb2qu(fsht_plan* p, const double* almE, const double* almB, double* Q, 
     FSHT_TRY(pol_synthesis(p, almE, almB, WQ, WU, nmaps, c0, kc));
     {
       FSHT_PROF(FSHT_KCAT_FFT_INV);
-      FSHT_TRY(fsht_launch_ring_fft_inv(p, WQ, Q + (size_t)c0 * p->npix, p->npix, kc, p->stream));
+      FSHT_TRY(ring_inv(p, WQ, Q + (size_t)c0 * p->npix, kc));
     }
     {
       FSHT_PROF(FSHT_KCAT_FFT_INV);
-      FSHT_TRY(fsht_launch_ring_fft_inv(p, WU, U + (size_t)c0 * p->npix, p->npix, kc, p->stream));
+      FSHT_TRY(ring_inv(p, WU, U + (size_t)c0 * p->npix, kc));
     }
   }
   return FSHT_OK;

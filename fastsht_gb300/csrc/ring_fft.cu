@@ -628,7 +628,7 @@ int fsht_launch_ring_fft_fwd(fsht_plan* p, const double* maps, long long map_str
 }
 
 int fsht_launch_ring_fft_fwd_part(fsht_plan* p, const double* maps, long long map_stride, int kc,
-                                  int k0, int kb, double2* W, cudaStream_t s) {
+                                  int k0, int kb, double2* W, cudaStream_t s, int ring0) {
   if (p->d_tw_df) return fsht_launch_ring_fft_fwd_df(p, maps, map_stride, kc, k0, kb, W, s);
   FwdArgs a;
   a.maps = maps;
@@ -652,8 +652,10 @@ int fsht_launch_ring_fft_fwd_part(fsht_plan* p, const double* maps, long long ma
   FSHT_TRY(fsht_smem_limit((const void*)k_ring_fft_fwd, (size_t)(p->fft_smem)));
   for (int sgi = 0; sgi < p->fft_nseg; ++sgi) {
     const long long* sg = p->fft_seg + 3 * sgi;
-    a.ring_base = (int)sg[0];
-    dim3 grid((unsigned)(sg[1] - sg[0]), (kb + a.maps_per_block - 1) / a.maps_per_block);
+    const int r0 = sg[0] > ring0 ? (int)sg[0] : ring0;
+    if (r0 >= sg[1]) continue;
+    a.ring_base = r0;
+    dim3 grid((unsigned)(sg[1] - r0), (kb + a.maps_per_block - 1) / a.maps_per_block);
     k_ring_fft_fwd<<<grid, p->fft_threads > 0 ? p->fft_threads : 512, (size_t)sg[2], s>>>(a);
     FSHT_LAUNCH_CHECK();
   }
@@ -661,7 +663,7 @@ int fsht_launch_ring_fft_fwd_part(fsht_plan* p, const double* maps, long long ma
 }
 
 int fsht_launch_ring_fft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride,
-                             int kc, cudaStream_t s) {
+                             int kc, cudaStream_t s, int ring0) {
   if (p->d_tw_df) return fsht_launch_ring_fft_inv_df(p, W, maps, map_stride, kc, s);
   InvArgs a;
   a.W = W;
@@ -683,8 +685,10 @@ int fsht_launch_ring_fft_inv(fsht_plan* p, const double2* W, double* maps, long 
   FSHT_TRY(fsht_smem_limit((const void*)k_ring_fft_inv, (size_t)(p->fft_smem)));
   for (int sgi = 0; sgi < p->fft_nseg; ++sgi) {
     const long long* sg = p->fft_seg + 3 * sgi;
-    a.ring_base = (int)sg[0];
-    dim3 grid((unsigned)(sg[1] - sg[0]), (kc + a.maps_per_block - 1) / a.maps_per_block);
+    const int r0 = sg[0] > ring0 ? (int)sg[0] : ring0;
+    if (r0 >= sg[1]) continue;
+    a.ring_base = r0;
+    dim3 grid((unsigned)(sg[1] - r0), (kc + a.maps_per_block - 1) / a.maps_per_block);
     k_ring_fft_inv<<<grid, p->fft_threads > 0 ? p->fft_threads : 512, (size_t)sg[2], s>>>(a);
     FSHT_LAUNCH_CHECK();
   }
