@@ -419,8 +419,13 @@ extern "C" int fsht_batch_create(const fsht_job* jobs, int njobs, int nslots,
     auto it = key_plan.find(key);
     if (it == key_plan.end()) {
       fsht_plan* p = nullptr;
-      // tables only (spin-2 tables too in the split form); the slots hold the workspaces
-      const int flags = FSHT_FLAG_TABLES_ONLY | (j.precision == FSHT_PREC_SPLIT ? FSHT_FLAG_POL : 0);
+      // tables only (spin-2 tables too in the split form and for Q/U jobs); the slots hold the
+      // workspaces
+      bool pol = j.precision == FSHT_PREC_SPLIT;
+      for (int k = i; k < njobs; ++k)
+        pol |= (jobs[k].kind == FSHT_JOB_QU2EB || jobs[k].kind == FSHT_JOB_EB2QU) &&
+               std::make_tuple(jobs[k].nside, jobs[k].lmax, jobs[k].precision) == key;
+      const int flags = FSHT_FLAG_TABLES_ONLY | (pol ? FSHT_FLAG_POL : 0);
       int rc = fsht_plan_create(j.nside, j.lmax, 1, flags, j.precision, 0, b->stream, &p);
       if (rc) return fail(rc);
       b->plans.push_back(p);

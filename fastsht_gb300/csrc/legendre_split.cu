@@ -335,7 +335,8 @@ constexpr int kPartSteps = kKChunk / kKStep;   // most k-steps per part (levels 
 constexpr size_t kSmemG = (size_t)kStagesG * kStageBytesG + kStgBytes;
 
 struct GemmArgs {
-  int lmax, nnorth, ngroups, q0, ntmax, accumulate, nunits;
+  int lmax, nnorth, ngroups, q0, q1, ntmax, accumulate, nunits;
+  int stride;            // > 0: fixed walk of the units (a grid capped to some SMs)
   int part_steps;        // k-steps per ring part, <= kPartSteps (the plan's tile choice)
   size_t row_bytes;
   const int* ring_i0;
@@ -368,7 +369,7 @@ __device__ __forceinline__ GemmUnit gemm_unit(const GemmArgs& a, int u) {
   w.p = r & 1;
   r >>= 1;
   w.t = r % a.ntmax;
-  w.qi = r / a.ntmax;
+  w.qi = wave_order(a.q0, a.q1, r / a.ntmax) - a.q0;
   w.m = m_of_q(a.q0 + w.qi, a.lmax);
   const int K = a.nnorth - a.ring_i0[w.m];
   w.ntiles = (a.lmax - w.m + 1 + 2 * kRows - 1) / (2 * kRows);
@@ -380,19 +381,21 @@ __device__ __forceinline__ GemmUnit gemm_unit(const GemmArgs& a, int u) {
 __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ GemmSmemHdr h;
-  __shared__ int s_ce[kCols];          // column exponents (eb - 12) of the current unit
+  __shared__ UnitQueue uq;
+  __shared__ int s_ce[kEpiWarps][kCols / 2];   // per warp: its columns' exponents (eb - 12)
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = tc::warp_index();
   volatile int* abort = &h.abort;
   if (tid == 0) {
     for (int s = 0; s < kStagesG; ++s) {
       tc::mbar_init(&h.full[s], 1);
-      tc::mbar_init(&h.empty[s], 1);
+      tc::mbar_init(&h.empty[s], 2);                       // both UMMA warps
     }
-    tc::mbar_init(&h.tfull, 1);
-    tc::mbar_init(&h.tempty, kEpiThreads);
-    tc::mbar_init(&h.fin, 1);
+    tc::mbar_init(&h.tfull, 2);
+    tc::mbar_init(&h.tempty, kEpiWarps);
+    tc::mbar_init(&h.fin, 2);
+    uq_init(uq, kEpiWarps + 2);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -406,21 +409,17 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
   if (tid == kEpiThreads) {
     // producer: the k-step ring runs on across parts and units
     uint32_t i = 0;
-    for (int u = blockIdx.x; u < a.nunits && !*abort; u += gridDim.x) {
+    uq_walk(uq, a.nunits, a.stride, abort, [&](int u) -> bool {
       const GemmUnit w = gemm_unit(a, u);
-      if (w.nks == 0) continue;
+      if (w.nks == 0) return true;
       const unsigned char* asrc =
           a.lbuf + (size_t)(a.lam_off[a.q0 + w.qi] - a.lam_off[a.q0]) * kSlices * kATileBytes +
           (size_t)(w.p * w.ntiles + w.t) * w.nks * kSlices * kATileBytes;
       const unsigned char* bsrc =
           a.WS + (((size_t)w.qi * 2 + w.p) * a.ngroups + w.g) * a.row_bytes;
-      bool ok = true;
       for (int k = 0; k < w.nks; ++k, ++i) {
         const uint32_t st = i % kStagesG;
-        if (!tc::mbar_wait(&h.empty[st], ((i / kStagesG) & 1) ^ 1, abort)) {
-          ok = false;
-          break;
-        }
+        if (!tc::mbar_wait(&h.empty[st], ((i / kStagesG) & 1) ^ 1, abort)) return false;
         unsigned char* dst = smem + st * kStageBytesG;
         tc::mbar_arrive_expect_tx(&h.full[st], kStageBytesG);
         tc::bulk_g2s(dst, asrc + (size_t)k * kSlices * kATileBytes, kSlices * kATileBytes,
@@ -429,52 +428,47 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
                      kSlices * kBTileBytes, &h.full[st]);
         ++n_loaded;
       }
-      if (!ok) break;
-    }
-  } else if (tid == kEpiThreads + 32) {
-    // UMMA issuer
+      return true;
+    });
+  } else if (warp > kEpiWarps) {
+    // UMMA warps
+    const int side = warp - kEpiWarps - 1;
     const uint32_t idesc = tc::umma_idesc_bf16(kRows, kCols);
-    const uint32_t s_u = tc::smem_u32(smem);
+    const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
+    const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
     uint32_t i = 0, np = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
-      const GemmUnit w = gemm_unit(a, u);
-      for (int ks0 = 0; ks0 < w.nks && ok; ks0 += a.part_steps, ++np) {
+    for (uint32_t n = 0; ok; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
+      const int nks = tc::uniform(gemm_unit(a, u).nks);
+      for (int ks0 = 0; ks0 < nks && ok; ks0 += a.part_steps, ++np) {
         // the epilogue of the previous part has read the accumulators
-        if (np > 0 && !tc::mbar_wait(&h.tempty, (np - 1) & 1, abort)) {
+        if (np > 0 && !tc::mbar_wait_warp(&h.tempty, (np - 1) & 1, abort)) {
           ok = false;
           break;
         }
         tc::tc_fence_after();
-        const int nk = min(w.nks - ks0, a.part_steps);
+        const int nk = min(nks - ks0, a.part_steps);
         for (int k = 0; k < nk; ++k, ++i) {
           const uint32_t st = i % kStagesG;
-          if (!tc::mbar_wait(&h.full[st], (i / kStagesG) & 1, abort)) {
+          if (!tc::mbar_wait_warp(&h.full[st], (i / kStagesG) & 1, abort)) {
             ok = false;
             break;
           }
           tc::tc_fence_after();
-          const uint32_t abase = s_u + st * kStageBytesG;
-          const uint32_t bbase = abase + kSlices * kATileBytes;
-#pragma unroll
-          for (int lev = 0; lev <= 3; ++lev) {
-#pragma unroll
-            for (int aa = 0; aa <= lev; ++aa) {
-              const uint64_t ad = tc::umma_desc(abase + aa * kATileBytes, 128, 256);
-              const uint64_t bd = tc::umma_desc(bbase + (lev - aa) * kBTileBytes, 128, 256);
-              tc::umma_bf16(tmem + lev * kCols, ad, bd, idesc, (k > 0 || aa > 0) ? 1u : 0u);
-            }
-          }
-          tc::umma_commit(&h.empty[st]);
+          const uint64_t ad = tc::umma_desc(s_u + st * kStageBytesG, 128, 256);
+          split_step<false, false>(side, utmem, ad, tc::umma_desc_add(ad, kSlices * kATileBytes), idesc,
+                            k == 0);
+          tc::umma_commit_warp(&h.empty[st]);
         }
-        if (ok) tc::umma_commit(&h.tfull);
+        if (ok) tc::umma_commit_warp(&h.tfull);
       }
     }
   } else if (tid < kEpiThreads) {
     // epilogue (warps 0-7): TMEM -> alm, row = TMEM lane (warp % 4 picks the lane quarter,
-    // warp / 4 the half of the columns).  No early exit: the epilogue threads must meet at
-    // every named barrier, so after an expired wait (abort) the remaining parts are walked
-    // without work.
+    // warp / 4 the half of the columns).  Each warp works alone; after an expired wait (abort)
+    // the remaining parts are walked without work.
     const int lane = tid & 31;
     const int row0 = (warp & 3) << 5;              // this warp's 32 rows (its TMEM lane quarter)
     const int row = row0 + lane;
@@ -485,18 +479,18 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
     double* stg = reinterpret_cast<double*>(smem + (size_t)kStagesG * kStageBytesG) +
                   (size_t)warp * kStgWarpDoubles;
     uint32_t np = 0;
-    for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
+    for (uint32_t n = 0;; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
       const GemmUnit w = gemm_unit(a, u);
       if (w.nks == 0) continue;
       // this unit's column exponents and this thread's row factor
-      {
-        const int eb =
-            tid < kCols ? a.EB[(((long long)w.qi * 2 + w.p) * a.ngroups + w.g) * kCols + tid] : 0;
-        // the previous unit's readers of s_ce are done (named barrier of the epilogue threads)
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-        if (tid < kCols) s_ce[tid] = (eb == kEmptyExp) ? kEmptyExp : eb - 12;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      __syncwarp();
+      for (int c = lane; c < kCols / 2; c += 32) {
+        const int eb = a.EB[(((long long)w.qi * 2 + w.p) * a.ngroups + w.g) * kCols + cbeg + c];
+        s_ce[warp][c] = (eb == kEmptyExp) ? kEmptyExp : eb - 12;
       }
+      __syncwarp();
       const int l = w.lt0 + w.p + 2 * row;
       const bool rowok = l <= a.lmax;
       float rh = 0.f, rl = 0.f;
@@ -507,8 +501,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
         re = rw.erow + rw.dx;
       }
       for (int ks0 = 0; ks0 < w.nks; ks0 += a.part_steps) {
-        bool ok = tc::mbar_wait(&h.tfull, np & 1, abort);
-        ok = __all_sync(0xffffffffu, ok);      // tcgen05.ld below is warp-collective
+        const bool ok = tc::mbar_wait_warp(&h.tfull, np & 1, abort);
         ++np;
         if (!ok) continue;
         tc::tc_fence_after();
@@ -534,7 +527,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
             combine_levels_pair(v0[j], v1[j], v2[j], v3[j], hh[c + j], ll[c + j]);
         }
         tc::tc_fence_before();
-        tc::mbar_arrive(&h.tempty);
+        tc::mbar_arrive_warp(&h.tempty);
 #pragma unroll
         for (int cr = 0; cr < kCols / 2; cr += 16) {
           const int c0 = cbeg + cr;
@@ -542,7 +535,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
 #pragma unroll
           for (int j = 0; j < 16; ++j)
             stg[stg_at(lane, j)] =
-                rowok ? pair_scaled(hh[cr + j], ll[cr + j], rh, rl, re + s_ce[c0 + j]) : 0.0;
+                rowok ? pair_scaled(hh[cr + j], ll[cr + j], rh, rl, re + s_ce[warp][cr + j]) : 0.0;
           __syncwarp();
           // the block back out by rows: lanes 0-15 one row, 16-31 the next, 16 maps each.
           // Adds go out as fire-and-forget reductions (no load latency in the epilogue); one
@@ -572,8 +565,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
   }
   // drain: the UMMA issuer waits for its last products before TMEM is released, and the
   // loader for its last copies
-  if (tid == kEpiThreads + 32) {
-    tc::umma_commit(&h.fin);
+  if (warp > kEpiWarps) {
+    tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
   }
@@ -784,7 +777,7 @@ __global__ void __launch_bounds__(128) k_slice_alm(SliceAArgs a) {
 // TMEM accumulators (E first, written as G_N = G_S = E; then O, added to G_N and subtracted
 // from G_S by the same threads).  Roles as in k_split_gemm.
 struct SynthArgs {
-  int lmax, nnorth, ngroups, q0, nrbmax, eag, nunits;
+  int lmax, nnorth, ngroups, q0, q1, nrbmax, eag, nunits;
   size_t row_bytes;
   const int* ring_i0;
   const long long* lam_offT;
@@ -816,7 +809,7 @@ __device__ __forceinline__ SynthUnit synth_unit(const SynthArgs& a, int u) {
   w.g = u % a.ngroups;
   int r = u / a.ngroups;
   w.rb = r % a.nrbmax;
-  w.qi = r / a.nrbmax;
+  w.qi = wave_order(a.q0, a.q1, r / a.nrbmax) - a.q0;
   w.m = m_of_q(a.q0 + w.qi, a.lmax);
   w.i0 = a.ring_i0[w.m];
   w.K = a.nnorth - w.i0;
@@ -835,19 +828,20 @@ __device__ __forceinline__ SynthUnit synth_unit(const SynthArgs& a, int u) {
 __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ SynthSmemHdr h;
-  __shared__ int s_ce[2][kCols];       // column exponents EAG + eb - 12 per parity
+  __shared__ UnitQueue uq;
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = tc::warp_index();
   volatile int* abort = &h.abort;
   if (tid == 0) {
     for (int s = 0; s < kStagesS; ++s) {
       tc::mbar_init(&h.full[s], 1);
-      tc::mbar_init(&h.empty[s], 1);
+      tc::mbar_init(&h.empty[s], 2);                       // both UMMA warps
     }
-    tc::mbar_init(&h.tfull, 1);
-    tc::mbar_init(&h.tempty, kEpiThreads);
-    tc::mbar_init(&h.fin, 1);
+    tc::mbar_init(&h.tfull, 2);
+    tc::mbar_init(&h.tempty, kEpiWarps);
+    tc::mbar_init(&h.fin, 2);
+    uq_init(uq, kEpiWarps + 2);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -860,21 +854,17 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
   uint32_t n_loaded = 0;
   if (tid == kEpiThreads) {
     uint32_t i = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
+    uq_walk(uq, a.nunits, 0, abort, [&](int u) -> bool {
       const SynthUnit w = synth_unit(a, u);
-      if (w.nkl == 0) continue;
+      if (w.nkl == 0) return true;
       const unsigned char* abase =
           a.lbuf + (size_t)(a.lam_offT[a.q0 + w.qi] - a.lam_offT[a.q0]) * kSlices * kATileBytes;
-      for (int kl0 = 0; kl0 < w.nkl && ok; kl0 += kPartStepsS) {
+      for (int kl0 = 0; kl0 < w.nkl; kl0 += kPartStepsS) {
         const int nk = min(w.nkl - kl0, kPartStepsS);
-        for (int par = 0; par < 2 && ok; ++par) {
+        for (int par = 0; par < 2; ++par) {
           for (int kk = kl0; kk < kl0 + nk; ++kk, ++i) {
             const uint32_t st = i % kStagesS;
-            if (!tc::mbar_wait(&h.empty[st], ((i / kStagesS) & 1) ^ 1, abort)) {
-              ok = false;
-              break;
-            }
+            if (!tc::mbar_wait(&h.empty[st], ((i / kStagesS) & 1) ^ 1, abort)) return false;
             unsigned char* dst = smem + st * kStageBytesS;
             const unsigned char* asrc =
                 abase + ((size_t)(par * w.nrb + w.rb) * w.nkl + kk) * kSlices * kATileBytes;
@@ -888,115 +878,116 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
           }
         }
       }
-    }
-  } else if (tid == kEpiThreads + 32) {
+      return true;
+    });
+  } else if (warp > kEpiWarps) {
+    // UMMA warps: lambda tiles (rings) as the second operand, alm tiles as the first, so that the
+    // map columns are on the TMEM lanes
+    const int side = warp - kEpiWarps - 1;
     const uint32_t idesc = tc::umma_idesc_bf16(kRows, kCols);
-    const uint32_t s_u = tc::smem_u32(smem);
+    const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
+    const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
     uint32_t i = 0, np = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
-      const SynthUnit w = synth_unit(a, u);
-      for (int kl0 = 0; kl0 < w.nkl && ok; kl0 += kPartStepsS) {
-        const int nk = min(w.nkl - kl0, kPartStepsS);
+    for (uint32_t n = 0; ok; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
+      const int nkl = tc::uniform(synth_unit(a, u).nkl);
+      for (int kl0 = 0; kl0 < nkl && ok; kl0 += kPartStepsS) {
+        const int nk = min(nkl - kl0, kPartStepsS);
         for (int par = 0; par < 2 && ok; ++par, ++np) {
-          if (np > 0 && !tc::mbar_wait(&h.tempty, (np - 1) & 1, abort)) {
+          if (np > 0 && !tc::mbar_wait_warp(&h.tempty, (np - 1) & 1, abort)) {
             ok = false;
             break;
           }
           tc::tc_fence_after();
           for (int k = 0; k < nk; ++k, ++i) {
             const uint32_t st = i % kStagesS;
-            if (!tc::mbar_wait(&h.full[st], (i / kStagesS) & 1, abort)) {
+            if (!tc::mbar_wait_warp(&h.full[st], (i / kStagesS) & 1, abort)) {
               ok = false;
               break;
             }
             tc::tc_fence_after();
-            const uint32_t abase = s_u + st * kStageBytesS;
-            const uint32_t bbase = abase + kSlices * kATileBytes;
-#pragma unroll
-            for (int lev = 0; lev <= 3; ++lev) {
-#pragma unroll
-              for (int aa = 0; aa <= lev; ++aa) {
-                const uint64_t ad = tc::umma_desc(abase + aa * kATileBytes, 128, 256);
-                const uint64_t bd = tc::umma_desc(bbase + (lev - aa) * kBTileBytes, 128, 256);
-                tc::umma_bf16(tmem + lev * kCols, ad, bd, idesc, (k > 0 || aa > 0) ? 1u : 0u);
-              }
-            }
-            // level 4 (a1 b3, a2 b2, a3 b1) into the level-3 accumulator via the 2^-8 planes:
-            // with lambda against one scale its digits are often small, and dropping level 4
-            // would cost ~2e-7
-#pragma unroll
-            for (int aa = 1; aa <= 3; ++aa) {
-              const uint64_t ad = tc::umma_desc(abase + aa * kATileBytes, 128, 256);
-              const uint64_t bd =
-                  tc::umma_desc(bbase + (kSlices - 1 + (4 - aa)) * kBTileBytes, 128, 256);
-              tc::umma_bf16(tmem + 3 * kCols, ad, bd, idesc, 1u);
-            }
-            tc::umma_commit(&h.empty[st]);
+            const uint64_t ad = tc::umma_desc(s_u + st * kStageBytesS, 128, 256);
+            // (level 4, a1 b3, a2 b2, a3 b1, folded into the level-3 accumulator via the 2^-8
+            // planes: with lambda against one scale its digits are often small, and dropping
+            // level 4 would cost ~2e-7)
+            split_step<true, true>(side, utmem, ad, tc::umma_desc_add(ad, kSlices * kATileBytes), idesc,
+                             k == 0);
+            tc::umma_commit_warp(&h.empty[st]);
           }
-          if (ok) tc::umma_commit(&h.tfull);
+          if (ok) tc::umma_commit_warp(&h.tfull);
         }
       }
     }
   } else if (tid < kEpiThreads) {
-    // No early exit: the epilogue threads must meet at every named barrier.
-    const int row = ((warp & 3) << 5) + (tid & 31);
-    const int cbeg = (warp >> 2) * (kCols / 2);
-    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) << 5) << 16);
+    // Each warp works alone: TMEM lane = map column (its quarter), half of the rings.  The even
+    // sum E waits in the north slot, the odd one is added and subtracted by the same thread.
+    const int lane = tid & 31;
+    const int c = ((warp & 3) << 5) + lane;            // column: comp * 64 + map
+    const int comp = c >> 6;
+    const int rbeg = (warp >> 2) * (kCols / 2);
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) << 5) << 16) + rbeg;
+    const long long rs = (long long)a.kc * 4;          // doubles from ring to ring
     uint32_t np = 0;
-    for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
+    for (uint32_t n = 0;; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
       const SynthUnit w = synth_unit(a, u);
       if (w.nkl == 0) continue;
-      {
-        int e[2] = {0, 0};
-        if (tid < kCols)
-          for (int pp = 0; pp < 2; ++pp)
-            e[pp] = a.EB[(((long long)w.qi * 2 + pp) * a.ngroups + w.g) * kCols + tid];
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-        if (tid < kCols)
-          for (int pp = 0; pp < 2; ++pp)
-            s_ce[pp][tid] = (e[pp] == kEmptyExp) ? kEmptyExp : a.eag + e[pp] - 12;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      const int k = w.g * kGroupMaps + (c & 63);
+      const bool ok_col = k < a.kc;
+      int ce[2];
+#pragma unroll
+      for (int pp = 0; pp < 2; ++pp) {
+        const int e = a.EB[(((long long)w.qi * 2 + pp) * a.ngroups + w.g) * kCols + c];
+        ce[pp] = (e == kEmptyExp) ? kEmptyExp : a.eag + e - 12;
       }
-      const int rr = w.rb * kSCRings + row;
-      const bool rowok = rr < w.K;
-      const int i = w.i0 + rr;
+      const int nrow = min(kCols / 2, w.K - w.rb * kSCRings - rbeg);
+      double* base = a.W +
+                     (((long long)w.m * a.nnorth + w.i0 + w.rb * kSCRings + rbeg) * a.kc +
+                      (ok_col ? k : 0)) * 4 + comp;
       for (int kl0 = 0; kl0 < w.nkl; kl0 += kPartStepsS) {
+#pragma unroll 1
         for (int par = 0; par < 2; ++par) {
-          bool ok = tc::mbar_wait(&h.tfull, np & 1, abort);
-          ok = __all_sync(0xffffffffu, ok);
+          const bool ok = tc::mbar_wait_warp(&h.tfull, np & 1, abort);
           ++np;
           if (!ok) continue;
           tc::tc_fence_after();
-          const bool first = kl0 == 0 && par == 0;
-          for (int c0 = cbeg; c0 < cbeg + kCols / 2; c0 += 16) {
+          // mode 0: E stored in the north slot; 1: E read back, N = E + O, S = E - O; 2: a later
+          // part added to both
+          const int mode = kl0 > 0 ? 2 : par;
+          const int cexp = par ? ce[1] : ce[0];
+#pragma unroll
+          for (int c0 = 0; c0 < kCols / 2; c0 += 16) {
             uint32_t v0[16], v1[16], v2[16], v3[16];
             tc::tmem_ld16(lane_base + 0 * kCols + c0, v0);
             tc::tmem_ld16(lane_base + 1 * kCols + c0, v1);
             tc::tmem_ld16(lane_base + 2 * kCols + c0, v2);
             tc::tmem_ld16(lane_base + 3 * kCols + c0, v3);
             tc::tmem_wait_ld();
-            if (c0 == cbeg + kCols / 2 - 16) {
+            if (c0 == kCols / 2 - 16) {
               tc::tc_fence_before();
-              tc::mbar_arrive(&h.tempty);
+              tc::mbar_arrive_warp(&h.tempty);
             }
-            const int comp = c0 >> 6;
+            if (!ok_col) continue;
+            double* d = base + (long long)c0 * rs;
+            double n0[16], s0[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              const int c = c0 + j;
-              const int k = w.g * kGroupMaps + (c & 63);
-              if (rowok && k < a.kc) {
-                const double v =
-                    levels_scaled(v0[j], v1[j], v2[j], v3[j], 1.f, 0.f, s_ce[par][c]);
-                double* gn = a.W + ((((long long)w.m * a.nnorth + i) * a.kc + k) * 2) * 2 + comp;
-                double* gs = gn + 2;
-                if (first) {
-                  *gn = v;
-                  *gs = v;
-                } else {
-                  atomicAdd(gn, v);
-                  atomicAdd(gs, par ? -v : v);
-                }
+              const bool in = c0 + j < nrow;
+              n0[j] = mode > 0 && in ? d[j * rs] : 0.0;
+              s0[j] = mode == 2 && in ? d[j * rs + 2] : n0[j];
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (c0 + j >= nrow) continue;
+              const double v = levels_scaled(v0[j], v1[j], v2[j], v3[j], 1.f, 0.f, cexp);
+              if (mode == 0) {
+                d[j * rs] = v;
+              } else {
+                d[j * rs] = n0[j] + v;
+                d[j * rs + 2] = par ? s0[j] - v : s0[j] + v;
               }
             }
           }
@@ -1004,8 +995,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
       }
     }
   }
-  if (tid == kEpiThreads + 32) {
-    tc::umma_commit(&h.fin);
+  if (warp > kEpiWarps) {
+    tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
   }
@@ -1171,6 +1162,7 @@ int fsht_launch_split_gemm(fsht_plan* p, int w, const unsigned char* WS, const i
   a.row_bytes = ws_row_bytes(p->lmax, p->nnorth);
   a.accumulate = accumulate;
   a.q0 = wv[0];
+  a.q1 = wv[1];
   a.ntmax = wv[2];
   a.ring_i0 = p->d_ring_i0;
   a.lam_off = p->d_lam_off;
@@ -1188,12 +1180,10 @@ int fsht_launch_split_gemm(fsht_plan* p, int w, const unsigned char* WS, const i
   a.nunits = a.ngroups * 2 * a.ntmax * (wv[1] - wv[0]);
   const size_t sm = kSmemG;
   FSHT_TRY(fsht_smem_limit((const void*)k_split_gemm, (size_t)(sm)));
-  int dev = 0, nsm = 0;
-  FSHT_CUDA_TRY(cudaGetDevice(&dev));
-  FSHT_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  // persistent: one CTA per SM, or fewer while another kernel needs SMs beside it
-  const int cap = (p->gemm_ctas > 0 && p->gemm_ctas < nsm) ? p->gemm_ctas : nsm;
-  const int grid = a.nunits < cap ? a.nunits : cap;
+  // a CTA per unit (the running ones take the others over), or a fixed walk by fewer CTAs while
+  // another kernel needs SMs beside it
+  a.stride = p->gemm_ctas > 0 ? p->gemm_ctas : 0;
+  const int grid = (a.stride > 0 && a.stride < a.nunits) ? a.stride : a.nunits;
   if (grid > 0) k_split_gemm<<<grid, kThreadsG, sm, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
@@ -1250,6 +1240,7 @@ int fsht_launch_split_synth(fsht_plan* p, int w, const unsigned char* WS, const 
   a.ngroups = (kc + kGroupMaps - 1) / kGroupMaps;
   a.row_bytes = ws_row_bytes(p->lmax, p->nnorth);
   a.q0 = wv[0];
+  a.q1 = wv[1];
   a.nrbmax = wv[4];
   a.eag = eag_of(p->lmax);
   a.nunits = a.ngroups * a.nrbmax * (wv[1] - wv[0]);
@@ -1263,11 +1254,7 @@ int fsht_launch_split_synth(fsht_plan* p, int w, const unsigned char* WS, const 
   a.err = p->d_err;
   const size_t sm = (size_t)kStagesS * kStageBytesS;
   FSHT_TRY(fsht_smem_limit((const void*)k_split_synth, (size_t)(sm)));
-  int dev = 0, nsm = 0;
-  FSHT_CUDA_TRY(cudaGetDevice(&dev));
-  FSHT_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const int grid = a.nunits < nsm ? a.nunits : nsm;
-  if (grid > 0) k_split_synth<<<grid, kThreadsG, sm, s>>>(a);
+  if (a.nunits > 0) k_split_synth<<<a.nunits, kThreadsG, sm, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }

@@ -231,7 +231,7 @@ constexpr uint32_t kStageBytesP = 2 * kSlices * kATileBytes;    // 32 KB: A then
 constexpr int kPartStepsP = kKChunk / kKStep;
 
 struct GemmPArgs {
-  int lmax, nnorth, ngroups, q0, ntmax, accumulate, which, nunits;
+  int lmax, nnorth, ngroups, q0, q1, ntmax, accumulate, which, nunits;
   int part_steps;        // k-steps per ring part, <= kPartStepsP (the plan's tile choice)
   size_t row_bytes;
   const int* ring_i0;
@@ -269,7 +269,7 @@ __device__ __forceinline__ GemmPUnit gemm_pol_unit(const GemmPArgs& a, int u) {
   w.p = r & 1;
   r >>= 1;
   w.t = r % a.ntmax;
-  w.qi = r / a.ntmax;
+  w.qi = wave_order(a.q0, a.q1, r / a.ntmax) - a.q0;
   w.m = m_of_q(a.q0 + w.qi, a.lmax);
   const int K = a.nnorth - a.ring_i0[w.m];
   w.ntiles = (a.lmax - w.m + 1 + 2 * kRows - 1) / (2 * kRows);
@@ -281,19 +281,22 @@ __device__ __forceinline__ GemmPUnit gemm_pol_unit(const GemmPArgs& a, int u) {
 __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ GemmPSmemHdr h;
-  __shared__ int s_ce[2][kCols];       // column exponents (e - 12) per pass of the unit
+  __shared__ UnitQueue uq;
+  // per warp: the exponents (e - 12) of the columns it reads in each pass of the unit
+  __shared__ short s_ce[kEpiWarps][2][kCols / 2];
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = tc::warp_index();
   volatile int* abort = &h.abort;
   if (tid == 0) {
     for (int s = 0; s < kStagesP; ++s) {
       tc::mbar_init(&h.full[s], 1);
-      tc::mbar_init(&h.empty[s], 1);
+      tc::mbar_init(&h.empty[s], 2);                       // both UMMA warps
     }
-    tc::mbar_init(&h.tfull, 1);
-    tc::mbar_init(&h.tempty, kEpiThreads);
-    tc::mbar_init(&h.fin, 1);
+    tc::mbar_init(&h.tfull, 2);
+    tc::mbar_init(&h.tempty, kEpiWarps);
+    tc::mbar_init(&h.fin, 2);
+    uq_init(uq, kEpiWarps + 2);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -308,24 +311,20 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
     // producer: per part, the lambda1 k-steps (B = the field's own map) then the lambda2
     // k-steps (B = the other map, opposite parity)
     uint32_t i = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
+    uq_walk(uq, a.nunits, 0, abort, [&](int u) -> bool {
       const GemmPUnit w = gemm_pol_unit(a, u);
-      if (w.nks == 0) continue;
+      if (w.nks == 0) return true;
       const unsigned char* lam =
           a.lbuf + (size_t)(2 * (a.lam_off[a.q0 + w.qi] - a.lam_off[a.q0])) * kSlices * kATileBytes;
       const unsigned char* ws[2] = {w.field == 0 ? a.WSQ : a.WSU, w.field == 0 ? a.WSU : a.WSQ};
       const int bpar[2] = {w.p, 1 - w.p};
-      for (int ks0 = 0; ks0 < w.nks && ok; ks0 += a.part_steps) {
+      for (int ks0 = 0; ks0 < w.nks; ks0 += a.part_steps) {
         const int nk = min(w.nks - ks0, a.part_steps);
-        for (int part = 0; part < 2 && ok; ++part) {
+        for (int part = 0; part < 2; ++part) {
           for (int k = 0; k < nk; ++k, ++i) {
             const int ks = ks0 + k;
             const uint32_t st = i % kStagesP;
-            if (!tc::mbar_wait(&h.empty[st], ((i / kStagesP) & 1) ^ 1, abort)) {
-              ok = false;
-              break;
-            }
+            if (!tc::mbar_wait(&h.empty[st], ((i / kStagesP) & 1) ^ 1, abort)) return false;
             unsigned char* dst = smem + st * kStageBytesP;
             const unsigned char* asrc =
                 lam + (((size_t)(w.p * w.ntiles + w.t) * 2 + part) * w.nks + ks) * kSlices *
@@ -340,51 +339,48 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
           }
         }
       }
-    }
-  } else if (tid == kEpiThreads + 32) {
-    // UMMA issuer: one accumulation pass per (part of k-steps, lambda1 | lambda2)
+      return true;
+    });
+  } else if (warp > kEpiWarps) {
+    // UMMA warps: one accumulation pass after the other
+    const int side = warp - kEpiWarps - 1;
     const uint32_t idesc = tc::umma_idesc_bf16(kRows, kCols);
-    const uint32_t s_u = tc::smem_u32(smem);
+    const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
+    const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
     uint32_t i = 0, np = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
-      const GemmPUnit w = gemm_pol_unit(a, u);
-      for (int ks0 = 0; ks0 < w.nks && ok; ks0 += a.part_steps) {
-        const int nk = min(w.nks - ks0, a.part_steps);
-        for (int part = 0; part < 2 && ok; ++part, ++np) {
-          if (np > 0 && !tc::mbar_wait(&h.tempty, (np - 1) & 1, abort)) {
+    for (uint32_t n = 0; ok; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
+      const int nks = tc::uniform(gemm_pol_unit(a, u).nks);
+      for (int ks0 = 0; ks0 < nks && ok; ks0 += a.part_steps) {
+        const int nk = min(nks - ks0, a.part_steps);
+        for (int t = 0; t < 2 && ok; ++t, ++np) {
+          if (np > 0 && !tc::mbar_wait_warp(&h.tempty, (np - 1) & 1, abort)) {
             ok = false;
             break;
           }
           tc::tc_fence_after();
           for (int k = 0; k < nk; ++k, ++i) {
             const uint32_t st = i % kStagesP;
-            if (!tc::mbar_wait(&h.full[st], (i / kStagesP) & 1, abort)) {
+            if (!tc::mbar_wait_warp(&h.full[st], (i / kStagesP) & 1, abort)) {
               ok = false;
               break;
             }
             tc::tc_fence_after();
-            const uint32_t abase = s_u + st * kStageBytesP;
-            const uint32_t bbase = abase + kSlices * kATileBytes;
-#pragma unroll
-            for (int lev = 0; lev <= 3; ++lev) {
-#pragma unroll
-              for (int aa = 0; aa <= lev; ++aa) {
-                const uint64_t ad = tc::umma_desc(abase + aa * kATileBytes, 128, 256);
-                const uint64_t bd = tc::umma_desc(bbase + (lev - aa) * kBTileBytes, 128, 256);
-                tc::umma_bf16(tmem + lev * kCols, ad, bd, idesc, (k > 0 || aa > 0) ? 1u : 0u);
-              }
-            }
-            tc::umma_commit(&h.empty[st]);
+            const uint64_t ad = tc::umma_desc(s_u + st * kStageBytesP, 128, 256);
+            split_step<false, false>(side, utmem, ad, tc::umma_desc_add(ad, kSlices * kATileBytes),
+                              idesc, k == 0);
+            tc::umma_commit_warp(&h.empty[st]);
           }
-          if (ok) tc::umma_commit(&h.tfull);
+          if (ok) tc::umma_commit_warp(&h.tfull);
         }
       }
     }
   } else if (tid < kEpiThreads) {
     // epilogue (warps 0-7), row = TMEM lane (warp % 4: lane quarter, warp / 4: half of the
-    // columns).  No early exit: the epilogue threads must meet at every named barrier, so
-    // after an expired wait (abort) the remaining passes are walked idle.
+    // columns).  Each warp works alone; after an expired wait (abort) the remaining passes are
+    // walked idle.
     const int lane = tid & 31;
     const int row0 = (warp & 3) << 5;              // this warp's 32 rows (its TMEM lane quarter)
     const int row = row0 + lane;
@@ -398,23 +394,22 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
     double* stg = reinterpret_cast<double*>(smem + (size_t)kStagesP * kStageBytesP) +
                   (size_t)warp * kStgWarpDoubles;
     uint32_t np = 0;
-    for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
+    for (uint32_t n = 0;; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
       const GemmPUnit w = gemm_pol_unit(a, u);
       if (w.nks == 0) continue;
-      {
-        const int* eb[2] = {w.field == 0 ? a.EBQ : a.EBU, w.field == 0 ? a.EBU : a.EBQ};
-        const int bpar[2] = {w.p, 1 - w.p};
-        int e[2] = {0, 0};
-        if (tid < kCols)
-          for (int part = 0; part < 2; ++part)
-            e[part] =
-                eb[part][(((long long)w.qi * 2 + bpar[part]) * a.ngroups + w.g) * kCols + tid];
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-        if (tid < kCols)
-          for (int part = 0; part < 2; ++part)
-            s_ce[part][tid] = (e[part] == kEmptyExp) ? kEmptyExp : e[part] - 12;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      __syncwarp();
+      for (int x = lane; x < kCols; x += 32) {
+        const int part = x >> 6, c = x & 63;
+        const int comp = part == 0 ? tgt : 1 - tgt;     // the accumulator half read in this pass
+        const int* eb = (w.field == 0) == (part == 0) ? a.EBQ : a.EBU;
+        const int bpar = part == 0 ? w.p : 1 - w.p;
+        const int e =
+            eb[(((long long)w.qi * 2 + bpar) * a.ngroups + w.g) * kCols + comp * (kCols / 2) + c];
+        s_ce[warp][part][c] = (short)((e == kEmptyExp) ? kEmptyExp : e - 12);
       }
+      __syncwarp();
       const int l = w.lt0 + w.p + 2 * row;
       const bool rowok = l <= a.lmax;
       float rh = 0.f, rl = 0.f;
@@ -427,8 +422,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
       double* alm = w.field == 0 ? a.almE : a.almB;
       for (int ks0 = 0; ks0 < w.nks; ks0 += a.part_steps) {
         for (int part = 0; part < 2; ++part) {
-          bool ok = tc::mbar_wait(&h.tfull, np & 1, abort);
-          ok = __all_sync(0xffffffffu, ok);
+          const bool ok = tc::mbar_wait_warp(&h.tfull, np & 1, abort);
           ++np;
           if (!ok) continue;
           tc::tc_fence_after();
@@ -455,14 +449,14 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
               combine_levels_pair(v0[j], v1[j], v2[j], v3[j], hh[c + j], ll[c + j]);
           }
           tc::tc_fence_before();
-          tc::mbar_arrive(&h.tempty);
+          tc::mbar_arrive_warp(&h.tempty);
 #pragma unroll
           for (int cr = 0; cr < kCols / 2; cr += 16) {
             const int c0 = cbeg + cr;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
               const double uu =
-                  rowok ? pair_scaled(hh[cr + j], ll[cr + j], rh, rl, re + s_ce[part][c0 + j])
+                  rowok ? pair_scaled(hh[cr + j], ll[cr + j], rh, rl, re + s_ce[warp][part][cr + j])
                         : 0.0;
               stg[stg_at(lane, j)] = neg ? -uu : uu;
             }
@@ -492,8 +486,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
       }
     }
   }
-  if (tid == kEpiThreads + 32) {
-    tc::umma_commit(&h.fin);
+  if (warp > kEpiWarps) {
+    tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
   }
@@ -669,7 +663,7 @@ __global__ void __launch_bounds__(128) k_lambda_digits_T_pol(LamTPArgs a) {
 // accumulators, each one (lambda part, alm field, parity) product added to G_N and G_S with
 // its factor c in {-1, -i, +i} and south sign.
 struct SynthPArgs {
-  int lmax, nnorth, ngroups, q0, nrbmax, eag, nunits;
+  int lmax, nnorth, ngroups, q0, q1, nrbmax, eag, nunits;
   size_t row_bytes;
   const int* ring_i0;
   const long long* lam_offT;
@@ -707,7 +701,7 @@ __device__ __forceinline__ SynthPUnit synth_pol_unit(const SynthPArgs& a, int u)
   w.f = r & 1;
   r >>= 1;
   w.rb = r % a.nrbmax;
-  w.qi = r / a.nrbmax;
+  w.qi = wave_order(a.q0, a.q1, r / a.nrbmax) - a.q0;
   w.m = m_of_q(a.q0 + w.qi, a.lmax);
   w.i0 = a.ring_i0[w.m];
   w.K = a.nnorth - w.i0;
@@ -744,19 +738,22 @@ __device__ __forceinline__ void synth_pol_pass(int f, int t, int& part, int& fld
 __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ SynthPSmemHdr h;
-  __shared__ int s_ce[4][kCols];       // column exponents EAG + e - 12 per pass
+  __shared__ UnitQueue uq;
+  // per warp: the exponents EAG + e - 12 of its columns in each pass
+  __shared__ short s_ce[kEpiWarps][4][kCols / 2];
 
   const int tid = threadIdx.x;
-  const int warp = tid >> 5;
+  const int warp = tc::warp_index();
   volatile int* abort = &h.abort;
   if (tid == 0) {
     for (int s = 0; s < kStagesSP; ++s) {
       tc::mbar_init(&h.full[s], 1);
-      tc::mbar_init(&h.empty[s], 1);
+      tc::mbar_init(&h.empty[s], 2);                       // both UMMA warps
     }
-    tc::mbar_init(&h.tfull, 1);
-    tc::mbar_init(&h.tempty, kEpiThreads);
-    tc::mbar_init(&h.fin, 1);
+    tc::mbar_init(&h.tfull, 2);
+    tc::mbar_init(&h.tempty, kEpiWarps);
+    tc::mbar_init(&h.fin, 2);
+    uq_init(uq, kEpiWarps + 2);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -769,23 +766,19 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
   uint32_t n_loaded = 0;
   if (tid == kEpiThreads) {
     uint32_t i = 0;
-    bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
+    uq_walk(uq, a.nunits, 0, abort, [&](int u) -> bool {
       const SynthPUnit w = synth_pol_unit(a, u);
-      if (w.nkl == 0) continue;
+      if (w.nkl == 0) return true;
       const unsigned char* lam =
           a.lbuf + (size_t)(2 * (a.lam_offT[a.q0 + w.qi] - a.lam_offT[a.q0])) * kSlices * kATileBytes;
-      for (int kl0 = 0; kl0 < w.nkl && ok; kl0 += kPartStepsSP) {
+      for (int kl0 = 0; kl0 < w.nkl; kl0 += kPartStepsSP) {
         const int nk = min(w.nkl - kl0, kPartStepsSP);
-        for (int t = 0; t < 4 && ok; ++t) {
+        for (int t = 0; t < 4; ++t) {
           int part, fld, par, c, sg;
           synth_pol_pass(w.f, t, part, fld, par, c, sg);
           for (int kk = kl0; kk < kl0 + nk; ++kk, ++i) {
             const uint32_t st = i % kStagesSP;
-            if (!tc::mbar_wait(&h.empty[st], ((i / kStagesSP) & 1) ^ 1, abort)) {
-              ok = false;
-              break;
-            }
+            if (!tc::mbar_wait(&h.empty[st], ((i / kStagesSP) & 1) ^ 1, abort)) return false;
             unsigned char* dst = smem + st * kStageBytesSP;
             const unsigned char* asrc =
                 lam + ((((size_t)(part * 2 + par) * w.nrb + w.rb) * w.nkl + kk) * kSlices) *
@@ -801,77 +794,67 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
           }
         }
       }
-    }
-  } else if (tid == kEpiThreads + 32) {
+      return true;
+    });
+  } else if (warp > kEpiWarps) {
+    // UMMA warps: one accumulation pass after the other
+    const int side = warp - kEpiWarps - 1;
     const uint32_t idesc = tc::umma_idesc_bf16(kRows, kCols);
-    const uint32_t s_u = tc::smem_u32(smem);
+    const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
+    const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
     uint32_t i = 0, np = 0;
     bool ok = true;
-    for (int u = blockIdx.x; u < a.nunits && ok && !*abort; u += gridDim.x) {
-      const SynthPUnit w = synth_pol_unit(a, u);
-      for (int kl0 = 0; kl0 < w.nkl && ok; kl0 += kPartStepsSP) {
-        const int nk = min(w.nkl - kl0, kPartStepsSP);
+    for (uint32_t n = 0; ok; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
+      const int nks = tc::uniform(synth_pol_unit(a, u).nkl);
+      for (int ks0 = 0; ks0 < nks && ok; ks0 += kPartStepsSP) {
+        const int nk = min(nks - ks0, kPartStepsSP);
         for (int t = 0; t < 4 && ok; ++t, ++np) {
-          if (np > 0 && !tc::mbar_wait(&h.tempty, (np - 1) & 1, abort)) {
+          if (np > 0 && !tc::mbar_wait_warp(&h.tempty, (np - 1) & 1, abort)) {
             ok = false;
             break;
           }
           tc::tc_fence_after();
           for (int k = 0; k < nk; ++k, ++i) {
             const uint32_t st = i % kStagesSP;
-            if (!tc::mbar_wait(&h.full[st], (i / kStagesSP) & 1, abort)) {
+            if (!tc::mbar_wait_warp(&h.full[st], (i / kStagesSP) & 1, abort)) {
               ok = false;
               break;
             }
             tc::tc_fence_after();
-            const uint32_t abase = s_u + st * kStageBytesSP;
-            const uint32_t bbase = abase + kSlices * kATileBytes;
-#pragma unroll
-            for (int lev = 0; lev <= 3; ++lev) {
-#pragma unroll
-              for (int aa = 0; aa <= lev; ++aa) {
-                const uint64_t ad = tc::umma_desc(abase + aa * kATileBytes, 128, 256);
-                const uint64_t bd = tc::umma_desc(bbase + (lev - aa) * kBTileBytes, 128, 256);
-                tc::umma_bf16(tmem + lev * kCols, ad, bd, idesc, (k > 0 || aa > 0) ? 1u : 0u);
-              }
-            }
-#pragma unroll
-            for (int aa = 1; aa <= 3; ++aa) {
-              const uint64_t ad = tc::umma_desc(abase + aa * kATileBytes, 128, 256);
-              const uint64_t bd =
-                  tc::umma_desc(bbase + (kSlices - 1 + (4 - aa)) * kBTileBytes, 128, 256);
-              tc::umma_bf16(tmem + 3 * kCols, ad, bd, idesc, 1u);
-            }
-            tc::umma_commit(&h.empty[st]);
+            const uint64_t ad = tc::umma_desc(s_u + st * kStageBytesSP, 128, 256);
+            split_step<true, false>(side, utmem, ad, tc::umma_desc_add(ad, kSlices * kATileBytes),
+                              idesc, k == 0);
+            tc::umma_commit_warp(&h.empty[st]);
           }
-          if (ok) tc::umma_commit(&h.tfull);
+          if (ok) tc::umma_commit_warp(&h.tfull);
         }
       }
     }
   } else if (tid < kEpiThreads) {
-    // No early exit: the epilogue threads must meet at every named barrier.
+    // each warp works alone
     const int row = ((warp & 3) << 5) + (tid & 31);
     const int cbeg = (warp >> 2) * (kCols / 2);
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) << 5) << 16);
     uint32_t np = 0;
-    for (int u = blockIdx.x; u < a.nunits; u += gridDim.x) {
+    for (uint32_t n = 0;; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
       const SynthPUnit w = synth_pol_unit(a, u);
       if (w.nkl == 0) continue;
-      {
-        int e[4] = {0, 0, 0, 0};
-        if (tid < kCols)
-          for (int t = 0; t < 4; ++t) {
-            int part, fld, par, c, sg;
-            synth_pol_pass(w.f, t, part, fld, par, c, sg);
-            const int* eb = fld ? a.EBB : a.EBE;
-            e[t] = eb[(((long long)w.qi * 2 + par) * a.ngroups + w.g) * kCols + tid];
-          }
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
-        if (tid < kCols)
-          for (int t = 0; t < 4; ++t)
-            s_ce[t][tid] = (e[t] == kEmptyExp) ? kEmptyExp : a.eag + e[t] - 12;
-        asm volatile("bar.sync 1, %0;" ::"n"(kEpiThreads) : "memory");
+      __syncwarp();
+#pragma unroll 1
+      for (int t = 0; t < 4; ++t) {
+        int part, fld, par, c, sg;
+        synth_pol_pass(w.f, t, part, fld, par, c, sg);
+        const int* eb = fld ? a.EBB : a.EBE;
+        for (int x = tid & 31; x < kCols / 2; x += 32) {
+          const int e = eb[(((long long)w.qi * 2 + par) * a.ngroups + w.g) * kCols + cbeg + x];
+          s_ce[warp][t][x] = (short)((e == kEmptyExp) ? kEmptyExp : a.eag + e - 12);
+        }
       }
+      __syncwarp();
       const int rr = w.rb * kSCRings + row;
       const bool rowok = rr < w.K;
       const int i = w.i0 + rr;
@@ -880,8 +863,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
         for (int t = 0; t < 4; ++t) {
           int part, fld, par, c, sg;
           synth_pol_pass(w.f, t, part, fld, par, c, sg);
-          bool ok = tc::mbar_wait(&h.tfull, np & 1, abort);
-          ok = __all_sync(0xffffffffu, ok);
+          const bool ok = tc::mbar_wait_warp(&h.tfull, np & 1, abort);
           ++np;
           if (!ok) continue;
           tc::tc_fence_after();
@@ -895,7 +877,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
             tc::tmem_wait_ld();
             if (c0 == cbeg + kCols / 2 - 16) {
               tc::tc_fence_before();
-              tc::mbar_arrive(&h.tempty);
+              tc::mbar_arrive_warp(&h.tempty);
             }
             const int comp = c0 >> 6;
             // c D: -1: (-D.x, -D.y);  -i: (D.y, -D.x);  +i: (-D.y, D.x)
@@ -915,7 +897,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
               const int k = w.g * kGroupMaps + (cc & 63);
               if (k < a.kc) {
                 const double uu =
-                    levels_scaled(v0[j], v1[j], v2[j], v3[j], 1.f, 0.f, s_ce[t][cc]);
+                    levels_scaled(v0[j], v1[j], v2[j], v3[j], 1.f, 0.f, s_ce[warp][t][cc - cbeg]);
                 const double v = neg ? -uu : uu;
                 double* gn = Wf + ((((long long)w.m * a.nnorth + i) * a.kc + k) * 2) * 2 + tgt;
                 double* gs = gn + 2;
@@ -934,8 +916,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
       }
     }
   }
-  if (tid == kEpiThreads + 32) {
-    tc::umma_commit(&h.fin);
+  if (warp > kEpiWarps) {
+    tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
   }
@@ -997,6 +979,7 @@ int fsht_launch_split_gemm_pol(fsht_plan* p, int w, const unsigned char* WSQ, co
   a.nnorth = p->nnorth;
   a.ngroups = (kc + kGroupMaps - 1) / kGroupMaps;
   a.q0 = wv[0];
+  a.q1 = wv[1];
   a.ntmax = wv[2];
   a.accumulate = accumulate;
   a.which = which;
@@ -1021,11 +1004,7 @@ int fsht_launch_split_gemm_pol(fsht_plan* p, int w, const unsigned char* WSQ, co
       (p->split_part > 0 && p->split_part < kPartStepsP) ? p->split_part : kPartStepsP;
   const size_t sm = (size_t)kStagesP * kStageBytesP + kStgBytes;
   FSHT_TRY(fsht_smem_limit((const void*)k_split_gemm_pol, (size_t)(sm)));
-  int dev = 0, nsm = 0;
-  FSHT_CUDA_TRY(cudaGetDevice(&dev));
-  FSHT_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const int grid = a.nunits < nsm ? a.nunits : nsm;
-  if (grid > 0) k_split_gemm_pol<<<grid, kThreadsG, sm, s>>>(a);
+  if (a.nunits > 0) k_split_gemm_pol<<<a.nunits, kThreadsG, sm, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }
@@ -1063,6 +1042,7 @@ int fsht_launch_split_synth_pol(fsht_plan* p, int w, const unsigned char* WSE, c
   a.nnorth = p->nnorth;
   a.ngroups = (kc + kGroupMaps - 1) / kGroupMaps;
   a.q0 = wv[0];
+  a.q1 = wv[1];
   a.nrbmax = wv[4];
   a.nunits = a.ngroups * 2 * a.nrbmax * (wv[1] - wv[0]);
   a.eag = std::ilogb(std::sqrt((2.0 * p->lmax + 1.0) / (4.0 * M_PI)) * (1.0 + 0x1p-30)) + 1;
@@ -1080,11 +1060,7 @@ int fsht_launch_split_synth_pol(fsht_plan* p, int w, const unsigned char* WSE, c
   a.err = p->d_err;
   const size_t sm = (size_t)kStagesSP * kStageBytesSP;
   FSHT_TRY(fsht_smem_limit((const void*)k_split_synth_pol, (size_t)(sm)));
-  int dev = 0, nsm = 0;
-  FSHT_CUDA_TRY(cudaGetDevice(&dev));
-  FSHT_CUDA_TRY(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const int grid = a.nunits < nsm ? a.nunits : nsm;
-  if (grid > 0) k_split_synth_pol<<<grid, kThreadsG, sm, s>>>(a);
+  if (a.nunits > 0) k_split_synth_pol<<<a.nunits, kThreadsG, sm, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }

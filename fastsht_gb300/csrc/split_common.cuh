@@ -24,10 +24,12 @@ constexpr uint32_t kBTileBytes = kCols * kKStep * 2;    // 4 KB per (k-step, dig
 constexpr int kSynthPlanes = 7;
 constexpr uint32_t kSynthBBytes = kSynthPlanes * kBTileBytes;   // 28 KB per l-step
 constexpr int kThreads = 192;
-// persistent analysis contractions: eight epilogue warps (two per TMEM lane quarter, one per
-// half of the columns), then the copy thread's warp and the UMMA thread's warp
+// persistent contractions: eight epilogue warps (two per TMEM lane quarter, one per half of the
+// columns), the copy thread's warp and two UMMA warps.  One warp issues about a product per 75
+// clocks, the tensor pipe takes one per 63: two warps keep it fed (levels 0 and 3, and 1 and 2).
 constexpr int kEpiThreads = 256;
-constexpr int kThreadsG = kEpiThreads + 64;
+constexpr int kEpiWarps = kEpiThreads / 32;
+constexpr int kThreadsG = kEpiThreads + 96;
 constexpr int kEmptyExp = -4000;    // column exponent of an all-zero column
 // Epilogue staging of the analysis GEMMs: each epilogue warp turns a 32-row x 16-column block
 // of results around in shared memory, so that its global stores and reductions go out as
@@ -163,6 +165,30 @@ __device__ __forceinline__ void uq_walk(UnitQueue& q, int nunits, int stride, vo
       return;
     }
     u = next;
+  }
+}
+
+// The products of one k-step issued by UMMA warp `side` of a split contraction: ten of level
+// a + b <= 3 (digit a of the tiles at ad, digit b of those at bd) into the four level
+// accumulators (first: the step starts the accumulation), and with FOLD the three level-4 products
+// through the 2^-8 planes of bd, into level 3.  SWAP: bd is the first (M side) operand.
+template <bool FOLD, bool SWAP>
+__device__ __forceinline__ void split_step(int side, uint32_t tmem, uint64_t ad, uint64_t bd,
+                                           uint32_t idesc, bool first) {
+  auto mma = [&](int lev, int da, int pb, uint32_t acc) {
+    const uint64_t x = tc::umma_desc_add(ad, da * kATileBytes);
+    const uint64_t y = tc::umma_desc_add(bd, pb * kBTileBytes);
+    tc::umma_bf16_warp(tmem + lev * kCols, SWAP ? y : x, SWAP ? x : y, idesc, acc);
+  };
+#pragma unroll
+  for (int lev = 0; lev <= 3; ++lev) {
+    if ((lev == 0 || lev == 3) != (side == 0)) continue;
+#pragma unroll
+    for (int aa = 0; aa <= lev; ++aa) mma(lev, aa, lev - aa, (!first || aa > 0) ? 1u : 0u);
+  }
+  if (FOLD && side == 0) {
+#pragma unroll
+    for (int aa = 1; aa <= 3; ++aa) mma(3, aa, kSlices - 1 + (4 - aa), 1u);
   }
 }
 
