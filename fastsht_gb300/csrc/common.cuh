@@ -296,7 +296,7 @@ int fsht_launch_analysis_fp64(fsht_plan* p, int spin, const double2* WQ,
 // (dir 0: into alm, dir 1: into the phase matrices).  A null second field means spin 0.
 int fsht_dft_tables_init(fsht_plan* p);
 int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, int kc, int k0,
-                        int cnt, double2* W, cudaStream_t s);
+                        int cnt, bool host, double2* W, cudaStream_t s);
 int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride, int kc,
                         cudaStream_t s);
 bool fsht_tc_supported(const fsht_plan* p);

@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cmath>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 namespace {
@@ -112,11 +113,10 @@ __device__ __forceinline__ double u64_scaled(unsigned long long u, bool neg, int
   int ex = 63 - lz + e + 1023;
   const unsigned long long sign = neg ? 1ull << 63 : 0ull;
   if (ex >= 2047) return __longlong_as_double((long long)(sign | 0x7FF0000000000000ull));
-  const bool low = ex <= 0;                                        // subnormal or zero
-  if (low) ex = max(ex + 128, 1);
-  const double v = __longlong_as_double(
+  if (ex <= 0)                                                     // subnormal: u 2^(ex - 12)
+    return __longlong_as_double((long long)((ex > -52 ? u >> (12 - ex) : 0ull) | sign));
+  return __longlong_as_double(
       (long long)((((unsigned long long)ex << 52) + (r - (1ull << 52))) | sign));
-  return low ? v * 0x1p-128 : v;
 }
 __device__ __forceinline__ double i64_scaled(long long a, int e) {
   return u64_scaled((unsigned long long)(a < 0 ? -a : a), a < 0, e);
@@ -771,34 +771,51 @@ __device__ __forceinline__ int dft_exp(unsigned long long mx) {
   return ef == 0x7FF ? kNanExp : ef - 1022;
 }
 
-// Ring samples -> folded digit tiles.  grid (ring of the wave, 4 maps), 256 threads = (column of
-// 8: map, north | south; 32 chunks of 8 samples): a warp reads 256 contiguous bytes per map and
-// writes whole 128-byte core matrices.  The ring's samples against its maximum with two bits to
-// spare, so the folds are exact integer sums.
+// Ring samples -> folded digit tiles.  The ring's samples against the maximum of the map's two
+// rings with two bits to spare, so the folds are exact integer sums.
+// grid (ring of the wave, MAPS maps), 256 threads = (2 MAPS columns: map, north | south; chunks of
+// eight samples).  MAPS = 4: device maps, read twice (the second time from L2), a warp reads 256
+// contiguous bytes per map and writes whole 128-byte core matrices.  MAPS = 1: maps in host memory,
+// read in place once and kept in shared memory.
+template <int MAPS>
 __global__ void __launch_bounds__(256) k_dft_slice(DftSliceArgs a) {
-  __shared__ unsigned long long s_mx[8][8];
+  constexpr int COLS = 2 * MAPS, CH = 256 / COLS;
+  constexpr bool STAGE = MAPS == 1;
+  extern __shared__ double s_x[];              // STAGE: [2][n]
+  __shared__ unsigned long long s_mx[8][COLS];
   const FshtDftRing d = a.rings[blockIdx.x];
   const int n = 4 * d.q;
-  const int col = threadIdx.x & 7, chunk = threadIdx.x >> 3;
-  const int map = blockIdx.y * 4 + (col >> 1), h = col & 1;
+  const int col = threadIdx.x & (COLS - 1), chunk = threadIdx.x / COLS;
+  const int map = blockIdx.y * MAPS + (col >> 1), h = col & 1;
   const int ip = a.nring - 1 - d.ring;
   const bool valid = map < a.cnt && !(h == 1 && ip == d.ring);
   const double* x = a.maps + (long long)map * a.map_stride +
                     ring_start(a.nside, h ? ip : d.ring);
+  if (STAGE) {
+    for (int hh = 0; hh < (ip == d.ring ? 1 : 2); ++hh) {
+      const double* g = a.maps + (long long)map * a.map_stride +
+                        ring_start(a.nside, hh ? ip : d.ring);
+#pragma unroll 4
+      for (int j = threadIdx.x; j < n; j += 256) s_x[hh * n + j] = __ldg(&g[j]);
+    }
+    __syncthreads();
+    x = s_x + h * n;
+  }
+  auto get = [&](int j) { return STAGE ? x[j] : __ldg(&x[j]); };
   unsigned long long mx = 0;
   if (valid)
-    for (int j0 = chunk * 8; j0 < n; j0 += 256) {
+    for (int j0 = chunk * 8; j0 < n; j0 += 8 * CH) {
 #pragma unroll
       for (int e = 0; e < 8; ++e)
         if (j0 + e < n)
-          mx = max(mx, (unsigned long long)__double_as_longlong(__ldg(&x[j0 + e])) &
+          mx = max(mx, (unsigned long long)__double_as_longlong(get(j0 + e)) &
                            0x7FFFFFFFFFFFFFFFull);
     }
   // one exponent for the map's two rings: their sum and difference are formed as integers
   mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-  mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
-  if ((threadIdx.x & 31) < 8) s_mx[threadIdx.x >> 5][col] = mx;
+#pragma unroll
+  for (int o = COLS; o < 32; o *= 2) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if ((threadIdx.x & 31) < COLS) s_mx[threadIdx.x >> 5][col] = mx;
   __syncthreads();
 #pragma unroll
   for (int w = 0; w < 8; ++w) mx = max(mx, s_mx[w][col]);
@@ -813,7 +830,7 @@ __global__ void __launch_bounds__(256) k_dft_slice(DftSliceArgs a) {
                        (size_t)g * d.nk * kStepBytes + (c >> 3) * 256 + (c & 7) * 16;
   const size_t tstride = (size_t)a.ngroups * d.nk * kStepBytes;
   const int kf = kFixBits - 2 - E;
-  for (int hc = chunk; hc < 2 * d.nk; hc += 32) {
+  for (int hc = chunk; hc < 2 * d.nk; hc += CH) {
     unsigned long long y[4][8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -821,10 +838,10 @@ __global__ void __launch_bounds__(256) k_dft_slice(DftSliceArgs a) {
       long long x0 = 0, x1 = 0, x2 = 0, x3 = 0;
       if (live && j < nj) {
         const bool lo = d.s == 0 && j == 0, hi = d.s == 0 && j == d.q;   // samples on an axis
-        x0 = fixed_i64(__ldg(&x[j]), kf);
-        if (!lo) x1 = fixed_i64(__ldg(&x[n - d.s - j]), kf);
-        if (!hi) x2 = fixed_i64(__ldg(&x[n / 2 - d.s - j]), kf);
-        if (!lo && !hi) x3 = fixed_i64(__ldg(&x[n / 2 + j]), kf);
+        x0 = fixed_i64(get(j), kf);
+        if (!lo) x1 = fixed_i64(get(n - d.s - j), kf);
+        if (!hi) x2 = fixed_i64(get(n / 2 - d.s - j), kf);
+        if (!lo && !hi) x3 = fixed_i64(get(n / 2 + j), kf);
       }
       const long long u = x0 + x1, u2 = x2 + x3, v = x0 - x1, v2 = x2 - x3;
       y[0][e] = (unsigned long long)(u + u2) + kBias;
@@ -1068,41 +1085,66 @@ __device__ __forceinline__ void tc_segment(const TcGemmArgs& a, const TcUnit& w,
           (size_t)((sg * 2 + lpar) * w.nt + w.t) * w.nk) * kStepBytes;
 }
 
-// acc += level sums L of one slot, 32 columns per thread: f L (an integer, or rounded to one) times
-// mul, in the high word (HI) or as a 32 x 32 + 64-bit multiply-add.  The integer comes out of
-// the mantissa of f L + 1.5 2^23, so a sum costs a float FMA, a maximum and the multiply-add (the
-// conversion instruction and its 64-bit handling took three times as long, with the UMMA warps
-// waiting); the bias 0x4B400000 stays in acc until the end of the unit.  Sums of 2^22 and more,
-// which need extreme digits throughout, take the conversion.
-constexpr uint32_t kMagic = 0x4B400000u;
-template <bool HI>
-__device__ __forceinline__ void tc_drain(uint32_t taddr, int nrow, float f, uint32_t mul,
-                                         unsigned long long (&acc)[kTcAcc]) {
+// acc += the level sums of two neighbouring slots (levels 2 PAIR and 2 PAIR + 1), 32 columns per
+// thread, times sg.  Integers come out of the mantissa of L + 1.5 2^23 (the conversion instruction
+// took three times as long, with the UMMA warps waiting), and the two levels are joined in 32 bits
+// first, so a pair costs one 64-bit multiply-add, which runs at about an eighth of the FP32 rate:
+//   PAIR 0, 1, 2: t = 256 n_a + n_b with weight 2^wt of level b; PAIR 3: the rounded
+//   2^(unit_bits - 48) (L_6 + 2^-8 L_7).
+// The constants that the mantissa trick leaves in t (kBias2, kMagic) stay in acc until the end of
+// the unit.  |L| < 2^22 holds for levels 0 and 1 over 256 summands; larger sums of the others need
+// extreme digits throughout and take the conversion.
+constexpr uint32_t kMagic = 0x4B400000u, kBias2 = 0x8B400000u;   // kBias2 = 257 kMagic mod 2^32
+template <int PAIR>
+__device__ __forceinline__ void tc_drain(uint32_t ta, uint32_t tb, int nrow, float sg,
+                                         int unit_bits, unsigned long long (&acc)[kTcAcc]) {
+  const int wt = unit_bits - 16 * PAIR - 8;                      // of the second level
+  const float f6 = sg * __int_as_float((127 + unit_bits - 48) << 23), f7 = f6 * 0x1p-8f;
+  const uint32_t mul = PAIR == 3 ? 1u : 1u << (wt >= 32 ? wt - 32 : wt);
+  const bool hi = PAIR == 0 && wt >= 32;
 #pragma unroll
-  for (int c = 0; c < kTcAcc; c += 16) {
+  for (int c = 0; c < kTcAcc; c += 8) {
     if (c >= nrow) break;
-    uint32_t v[16];
-    tc::tmem_ld16(taddr + c, v);
+    uint32_t va[8], vb[8];
+    tc::tmem_ld8(ta + c, va);
+    tc::tmem_ld8(tb + c, vb);
     tc::tmem_wait_ld();
-    float mx = 0.f;
+    auto A = [&](int j) { return __uint_as_float(va[j]); };
+    auto B = [&](int j) { return __uint_as_float(vb[j]); };
+    bool big = false;
+    if (PAIR > 0) {
+      float mx = 0.f;
 #pragma unroll
-    for (int j = 0; j < 16; ++j) mx = fmaxf(mx, fabsf(__uint_as_float(v[j])));
-    const bool big = __any_sync(0xffffffffu, mx * fabsf(f) >= 0x1p22f);
-    auto put = [&](int j, uint32_t n) {
-      if (HI)
-        acc[c + j] = ((unsigned long long)((uint32_t)(acc[c + j] >> 32) + n * mul) << 32) |
+      for (int j = 0; j < 8; ++j) mx = fmaxf(mx, fmaxf(fabsf(A(j)), fabsf(B(j))));
+      big = __any_sync(0xffffffffu, mx >= 0x1p22f);
+    }
+    auto put = [&](int j, uint32_t t) {
+      if (hi)
+        acc[c + j] = ((unsigned long long)((uint32_t)(acc[c + j] >> 32) + t * mul) << 32) |
                      (uint32_t)acc[c + j];
       else
-        acc[c + j] += (unsigned long long)n * mul;
+        acc[c + j] += (unsigned long long)t * mul;
     };
     if (!big) {
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        put(j, __float_as_uint(fmaf(__uint_as_float(v[j]), f, 12582912.f)));
+      for (int j = 0; j < 8; ++j) {
+        if (PAIR == 3)
+          put(j, __float_as_uint(fmaf(A(j), f6, B(j) * f7) + 12582912.f));
+        else
+          put(j, __float_as_uint(fmaf(A(j), sg, 12582912.f)) * 256u +
+                     __float_as_uint(fmaf(B(j), sg, 12582912.f)));
+      }
     } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j)
-        put(j, (uint32_t)__float2int_rn(__uint_as_float(v[j]) * f) + kMagic);
+      for (int j = 0; j < 8; ++j) {
+        if (PAIR == 3) {
+          acc[c + j] += (unsigned long long)(__float2ll_rn(fmaf(A(j), f6, B(j) * f7)) +
+                                             (long long)kMagic);
+        } else {
+          const long long t = (long long)__float2int_rn(A(j) * sg) * 256 + __float2int_rn(B(j) * sg);
+          acc[c + j] += (unsigned long long)(t + (long long)kBias2) * mul;
+        }
+      }
     }
   }
 }
@@ -1157,28 +1199,38 @@ __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int
     const int nr = 4 * w.d.q, cmp = w.p >= 2;
     double* d = a.out[0] + (((long long)w.m * a.w_kc + a.k_off + map) * 2 + comp) * 2;
     const long long ms = (long long)a.nnorth * a.w_kc * 4;
+    unsigned long long y[kOut];                    // bits of the values, Im F = -(sin sum)
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
       const long long o = __shfl_xor_sync(0xffffffffu, sum[j], 1);
-      v[j] = i64_scaled(comp == 0 ? sum[j] + o : o - sum[j], e);
-      if (eb == kNanExp) v[j] = __longlong_as_double(0x7FF8000000000000ll);
+      const long long t = comp == 0 ? sum[j] + o : o - sum[j];
+      y[j] = (unsigned long long)__double_as_longlong(i64_scaled(cmp ? -t : t, e));
+      if (eb == kNanExp) y[j] = 0x7FF8000000000000ull;
     }
     if (!store) return;
+    const double zero = __longlong_as_double(eb == kNanExp ? 0x7FF8000000000000ll : 0ll);
+    const unsigned long long flip = 1ull << 63;
+    auto put = [&](int m, int cp, unsigned long long b) {
+      d[(long long)m * ms + cp] = __longlong_as_double((long long)b);
+    };
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
       if (j >= cnt) break;
       const int r = dft_r(w.p, w.row0 + n0 + j);
       const bool self = r == 0 || 2 * r == nr;
-      double sg = cmp ? -v[j] : v[j];              // Im F = -(sin sum)
-      for (int m0 = 0; m0 - r <= w.d.mtop; m0 += nr) {
-        if (m0 > 0 && !self) d[(long long)(m0 - r) * ms + cmp] = cmp ? -sg : sg;
+      unsigned long long b = y[j];
+      put(r, cmp, b);
+      // the parts that no row computes: Im at r = 0, and with s = 1 Re at n / 2
+      if (r == 0) d[1] = zero;
+      if (w.d.s && w.p == 2 && 2 * r == nr) d[(long long)r * ms] = zero;
+      for (int m0 = nr; m0 - r <= w.d.mtop; m0 += nr) {            // a n - r and a n + r
+        if (w.d.s) b ^= flip;
+        if (!self) put(m0 - r, cmp, cmp ? b ^ flip : b);
         if (m0 + r <= w.d.mtop) {
-          d[(long long)(m0 + r) * ms + cmp] = sg;
-          // the parts that no row computes: Im at r = 0, and with s = 1 Re at n / 2
-          if (r == 0) d[(long long)m0 * ms + 1] = sg - sg;
-          if (w.d.s && w.p == 2 && 2 * r == nr) d[(long long)(m0 + r) * ms] = sg - sg;
+          put(m0 + r, cmp, b);
+          if (r == 0) d[(long long)m0 * ms + 1] = zero;
+          if (w.d.s && w.p == 2 && 2 * r == nr) d[(long long)(m0 + r) * ms] = zero;
         }
-        if (w.d.s) sg = -sg;
       }
     }
   } else {
@@ -1398,8 +1450,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
     const int comp = c & 1;
     const int rbeg = (warp >> 2) * kTcAcc;               // this warp's quarter of the columns
     const uint32_t tbase = tmem + ((uint32_t)((warp & 3) << 5) << 16) + rbeg;
-    // level weights 2^wt, wt = unit_bits - 8 s, as (float factor, integer multiplier): 2^32 and up
-    // in the high word, the others with multipliers <= 2^30
     uint32_t use = 0;
     for (uint32_t n = 0;; ++n) {
       const int u = uq_take(uq, n, abort);
@@ -1450,26 +1500,32 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
           }
 #pragma unroll 1
           for (int k0 = 0; k0 < w.nk; k0 += kPartK) {
-#pragma unroll 1
-            for (int lev = 0; lev < 8; ++lev) {
-              const int slot = lev & 3;
-              const bool ok = tc::mbar_wait_warp(&h.tfull[slot], use & 1, abort);
-              if (slot == 3) ++use;
-              if (!ok) continue;
+            const float sf = (float)sign;
+            // wait for a pair of slots, drain it, hand it back
+            auto pair = [&](auto P) {
+              constexpr int kP = decltype(P)::value, kS = (2 * kP) & 3;
+              const bool ok = tc::mbar_wait_warp(&h.tfull[kS], use & 1, abort) &&
+                              tc::mbar_wait_warp(&h.tfull[kS + 1], use & 1, abort);
+              if (!ok) return;
               tc::tc_fence_after();
-              const int wt = a.unit_bits - 8 * lev;      // weight 2^wt of this level
-              if (wt >= 32) {
-                tc_drain<true>(tbase + slot * kCols, nrow, (float)sign, 1u << (wt - 32), acc);
-                bias += (unsigned long long)kMagic << wt;
-              } else {
-                const int me = min(max(wt, 0), 30);
-                tc_drain<false>(tbase + slot * kCols, nrow, sign * ldexpf(1.f, wt - me), 1u << me,
-                                acc);
-                bias += (unsigned long long)kMagic << me;
-              }
+              tc_drain<kP>(tbase + kS * kCols, tbase + (kS + 1) * kCols, nrow, sf, a.unit_bits,
+                           acc);
               tc::tc_fence_before();
-              tc::mbar_arrive_warp(&h.tempty[slot]);
-            }
+              __syncwarp();
+              if (lane == 0) {
+                tc::mbar_arrive(&h.tempty[kS]);
+                tc::mbar_arrive(&h.tempty[kS + 1]);
+              }
+            };
+            pair(std::integral_constant<int, 0>{});
+            pair(std::integral_constant<int, 1>{});
+            ++use;
+            pair(std::integral_constant<int, 2>{});
+            pair(std::integral_constant<int, 3>{});
+            ++use;
+            const int b = a.unit_bits;
+            bias += ((unsigned long long)kBias2 << (b - 8)) + ((unsigned long long)kBias2 << (b - 24)) +
+                    ((unsigned long long)kBias2 << (b - 40)) + kMagic;
           }
         }
         // the phase's sums out, a few at a time: the output code exists once and the registers
@@ -1549,7 +1605,7 @@ int launch_tc_gemm(const TcGemmArgs& a, cudaStream_t s) {
 }  // namespace
 
 bool fsht_tc_supported(const fsht_plan* p) {
-  return p->nside >= 32 && tc_bits_analysis(p) >= 38 && tc_bits_synthesis(p) >= 38;
+  return p->nside >= 32 && tc_bits_analysis(p) >= 40 && tc_bits_synthesis(p) >= 40;
 }
 
 int fsht_tc_tables_init(fsht_plan* p) {
@@ -1719,9 +1775,9 @@ namespace {
 constexpr int kDftBeltMax = 256;
 constexpr int kDftWaveInts = 5;     // first entry, end, most row tiles, largest q, digit k-steps
 
-// Sums of q / 2 + 1 products against the cosines' 2^1; north and south, or the four mirrored
-// samples, are added and subtracted.
-int dft_bits(int qmax, int extra) { return std::min(46, 51 - extra - ceil_log2(qmax / 2 + 2)); }
+// Sums of at most nk <= q + 1 products against the cosines' 2^1; north and south, or the four
+// mirrored samples, are added and subtracted.  (tc_drain wants 40 bits or more.)
+int dft_bits(int nk, int extra) { return std::min(46, 51 - extra - ceil_log2((nk + 1) / 2)); }
 
 DftSliceArgs dft_slice_args(const fsht_plan* p, const int* wv, int ngroups) {
   DftSliceArgs a{};
@@ -1753,7 +1809,7 @@ TcGemmArgs dft_gemm_args(const fsht_plan* p, const int* wv, int ngroups, int cnt
   a.ngroups = ngroups;
   a.ntmax = wv[2];
   a.nnorth = p->nnorth;
-  a.unit_bits = dft_bits(p->nside, extra);
+  a.unit_bits = dft_bits(p->nside <= kDftBeltMax ? p->nside + 1 : p->nside - 1, extra);
   a.lbuf = p->d_lbuf;
   a.WS = p->d_ws;
   a.EB = p->d_eb;
@@ -1865,10 +1921,10 @@ int fsht_dft_tables_init(fsht_plan* p) {
   return FSHT_OK;
 }
 
-// Maps [k0, k0 + cnt) of a chunk of kc maps (maps: the chunk's base) -> their {S, D} of rings
-// below dft_end.
+// Maps [k0, k0 + cnt) of a chunk of kc maps (maps: the chunk's base; host: in host memory, read in
+// place) -> their {S, D} of rings below dft_end.
 int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, int kc, int k0,
-                        int cnt, double2* W, cudaStream_t s) {
+                        int cnt, bool host, double2* W, cudaStream_t s) {
   const int ngroups = tc_groups(cnt);
   for (int w = 0; w < p->ndft_waves; ++w) {
     const int* wv = p->h_dft_waves + kDftWaveInts * w;
@@ -1877,7 +1933,13 @@ int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, 
     sa.maps = maps + (long long)k0 * map_stride;
     sa.map_stride = map_stride;
     sa.cnt = cnt;
-    k_dft_slice<<<dim3(wv[1] - wv[0], (cnt + 3) / 4), 256, 0, s>>>(sa);
+    if (host) {
+      const size_t sm = sizeof(double) * 8 * (size_t)wv[3];        // two rings of 4 q samples
+      FSHT_TRY(fsht_smem_limit((const void*)k_dft_slice<1>, sm));
+      k_dft_slice<1><<<dim3(wv[1] - wv[0], cnt), 256, sm, s>>>(sa);
+    } else {
+      k_dft_slice<4><<<dim3(wv[1] - wv[0], (cnt + 3) / 4), 256, 0, s>>>(sa);
+    }
     FSHT_LAUNCH_CHECK();
     TcGemmArgs a = dft_gemm_args(p, wv, ngroups, cnt, 1);
     a.k_off = k0;

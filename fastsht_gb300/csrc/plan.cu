@@ -662,24 +662,29 @@ static bool use_tc(const fsht_plan* p, int spin) {
   return p->tc64 && p->d_lbuf && p->d_tcflag && (spin == 0 || p->d_poltab);
 }
 
-// Whether a chunk of kc device-resident maps takes the matrix form of the ring transforms for the
-// rings below dft_end (it uses the contraction's buffers).
-static bool use_dft(const fsht_plan* p, int kc) {
-  return use_tc(p, 0) && p->dft_end > 0 && kc >= 1;
+// Whether the ring transforms of a chunk of kc maps take the matrix form for the rings below
+// dft_end (it uses the contraction's buffers).  Its matrices and its tiles of 64 maps cost the same
+// for any kc up to 64, the FFT costs by the map; forward they meet near 18 maps at every nside from
+// 64 to 1024 (16 maps: 0.43 against 0.38 ms at nside 128, 4.6 against 4.8 at 512, 24.5 against
+// 23.1 at 1024), inverse near 40.
+constexpr int kDftFwdMaps = 20, kDftInvMaps = 40;
+static bool use_dft(const fsht_plan* p, int kc, int min_maps = kDftFwdMaps) {
+  return use_tc(p, 0) && p->dft_end > 0 && kc >= min_maps;
 }
 
-// Ring transforms of a whole chunk: matrix form below dft_end where it applies, FFT above.
-static int ring_fwd(fsht_plan* p, const double* maps, int kc, double2* W) {
+// Ring transforms of a whole chunk (maps on the device, or host memory read in place): matrix form
+// below dft_end where it applies, FFT above.
+static int ring_fwd(fsht_plan* p, const double* maps, int kc, double2* W, bool host = false) {
   int ring0 = 0;
   if (use_dft(p, kc)) {
-    FSHT_TRY(fsht_launch_dft_fwd(p, maps, p->npix, kc, 0, kc, W, p->stream));
+    FSHT_TRY(fsht_launch_dft_fwd(p, maps, p->npix, kc, 0, kc, host, W, p->stream));
     ring0 = p->dft_end;
   }
   return fsht_launch_ring_fft_fwd_part(p, maps, p->npix, kc, 0, kc, W, p->stream, ring0);
 }
 static int ring_inv(fsht_plan* p, const double2* W, double* maps, int kc) {
   int ring0 = 0;
-  if (use_dft(p, kc)) {
+  if (use_dft(p, kc, kDftInvMaps)) {
     FSHT_TRY(fsht_launch_dft_inv(p, W, maps, p->npix, kc, p->stream));
     ring0 = p->dft_end;
   }
@@ -1084,14 +1089,14 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
     }
     // the first lambda tiles are computed on the auxiliary stream during the FFT
     // (not beside the matrix form of the FFT, which uses the tiles' buffers)
-    const bool tc = !split && use_tc(p, 0) && ((hx && hx->direct) || !use_dft(p, kc));
+    const bool tc = !split && use_tc(p, 0) && !use_dft(p, kc);
     if (split) FSHT_TRY(lam_start(p, fsht_launch_split_lambda));
     if (tc) FSHT_TRY(lam_start(p, fsht_launch_tc_lambda));
     // the chunk's maps as the FFT reads them: device buffer, or host memory read in place
     const double* cmaps = (hx && hx->direct ? hx->direct : maps) + (size_t)c0 * p->npix;
-    if (!hx && !split) {
+    if (!split && (!hx || hx->direct)) {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
-      FSHT_TRY(ring_fwd(p, cmaps, kc, W0));
+      FSHT_TRY(ring_fwd(p, cmaps, kc, W0, hx != nullptr));
     } else if (!hx || hx->direct) {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
       // (page-locked maps mapped into the device's address space are read over the host link
@@ -1112,7 +1117,7 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
         FSHT_PROF(FSHT_KCAT_FFT_FWD);
         int ring0 = 0;
         if (use_dft(p, kc)) {
-          FSHT_TRY(fsht_launch_dft_fwd(p, cmaps, p->npix, kc, k0, cnt, W0, p->stream));
+          FSHT_TRY(fsht_launch_dft_fwd(p, cmaps, p->npix, kc, k0, cnt, false, W0, p->stream));
           ring0 = p->dft_end;
         }
         FSHT_TRY(fsht_launch_ring_fft_fwd_part(p, cmaps, p->npix, kc, k0, cnt, W0, p->stream,
