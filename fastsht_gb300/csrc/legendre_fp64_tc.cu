@@ -102,46 +102,34 @@ __device__ __forceinline__ void store_planes(unsigned char* dst, unsigned char* 
   put(7, plane_of<7>(y));
 }
 
-// The output stays off the FP64 pipe too (an FP64 addition per value was 15 clocks a warp, and
-// bound the output of the ring transforms): sums are combined as integers and rounded once.
-// Magnitude u (bit 63 - lz leading) 2^e as the nearest FP64.
-__device__ __forceinline__ double u64_scaled(unsigned long long u, bool neg, int e) {
+// Sums leave as FP64 by integer instructions (a conversion and scaling on the FP64 pipe is three
+// operations of 15 clocks a warp), combined as integers where two meet, rounded once.
+// a 2^e as the nearest FP64, over the whole exponent range.
+__device__ __forceinline__ double i64_scaled_any(long long a, int e) {
+  unsigned long long u = (unsigned long long)(a < 0 ? -a : a);
   if (u == 0) return 0.0;
   const int lz = __clzll((long long)u);
   u <<= lz;
   const unsigned long long r = (u >> 11) + ((u >> 10) & 1);       // 2^52 .. 2^53
-  int ex = 63 - lz + e + 1023;
-  const unsigned long long sign = neg ? 1ull << 63 : 0ull;
+  const int ex = 63 - lz + e + 1023;
+  const unsigned long long sign = a < 0 ? 1ull << 63 : 0ull;
   if (ex >= 2047) return __longlong_as_double((long long)(sign | 0x7FF0000000000000ull));
   if (ex <= 0)                                                     // subnormal: u 2^(ex - 12)
     return __longlong_as_double((long long)((ex > -52 ? u >> (12 - ex) : 0ull) | sign));
   return __longlong_as_double(
-      (long long)((((unsigned long long)ex << 52) + (r - (1ull << 52))) | sign));
+      (long long)((((unsigned long long)(ex - 1) << 52) + r) | sign));
 }
+// The same for |e| <= kSafeExp, without a branch, so that several values interleave.
+constexpr int kSafeExp = 900;
 __device__ __forceinline__ double i64_scaled(long long a, int e) {
-  return u64_scaled((unsigned long long)(a < 0 ? -a : a), a < 0, e);
-}
-// a f 2^e for a factor f as (64-bit mantissa fm with its top bit set, sign, exponent: f = +-fm
-// 2^fe): the high half of the product, truncated at 2^-62 of it.
-struct TcFac {
-  unsigned long long fm;
-  int fe, neg;
-};
-__device__ __forceinline__ TcFac tc_fac(double f) {
-  TcFac t;
-  const unsigned long long b = (unsigned long long)__double_as_longlong(f);
-  const int ex = (int)(b >> 52) & 0x7FF;
-  t.fm = ex ? ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 11 : 0ull;
-  t.fe = ex - 1023 - 63;
-  t.neg = (long long)b < 0;
-  return t;
-}
-__device__ __forceinline__ double i64_scaled_mul(long long a, const TcFac& f, int e) {
-  unsigned long long u = (unsigned long long)(a < 0 ? -a : a);
-  if (u == 0) return 0.0;
+  const long long s = a >> 63;
+  unsigned long long u = (unsigned long long)((a ^ s) - s);
   const int lz = __clzll((long long)u);
-  u = __umul64hi(u << lz, f.fm);                                  // times 2^(64 - lz)
-  return u64_scaled(u, (a < 0) != (f.neg != 0), e + f.fe + 64 - lz);
+  u <<= lz & 63;
+  const unsigned long long r = ((u >> 1) + 0x200) >> 10;
+  unsigned long long b = r + ((unsigned long long)(unsigned)(e + 1085 - lz) << 52);
+  b |= (unsigned long long)s & (1ull << 63);
+  return __longlong_as_double((long long)(r ? b : 0ull));
 }
 
 // ------------------------------------------------------------------ tables
@@ -1155,7 +1143,8 @@ __device__ __forceinline__ void tc_drain(uint32_t ta, uint32_t tb, int nrow, flo
 template <int DIR, int SPIN, int kOut>
 __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int ph, bool store,
                                        int c, int n0, int cnt, int map, int eb, int e,
-                                       const long long (&sum)[kOut], const TcFac* fac) {
+                                       const long long (&sum)[kOut],
+                                       const double* fac) {
   const int comp = c & 1;
   double v[kOut];
   if (DIR == 0) {
@@ -1165,13 +1154,19 @@ __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int
                                     : (L1 - w.m) * L1 + (w.row0 - w.m) + 2 * n0;
     double* d = a.out[SPIN == 2 ? w.field : 0] + row * a.ld + a.k0 + map;
     const long long ds = 2LL * a.ld;
+    // (column exponents beyond 2^+-kMaxExp never come here)
 #pragma unroll
-    for (int j = 0; j < kOut; ++j) v[j] = a.accumulate && j < cnt ? d[j * ds] : 0.0;
+    for (int j = 0; j < kOut; ++j) v[j] = i64_scaled(sum[j], e) * fac[j];
+    if (a.accumulate) {
+      double old[kOut];
 #pragma unroll
-    for (int j = 0; j < kOut; ++j) {
-      const double x = i64_scaled_mul(sum[j], fac[j], e);
-      if (j < cnt) d[j * ds] = a.accumulate ? v[j] + x : x;
+      for (int j = 0; j < kOut; ++j) old[j] = j < cnt ? d[j * ds] : 0.0;
+#pragma unroll
+      for (int j = 0; j < kOut; ++j) v[j] += old[j];
     }
+#pragma unroll
+    for (int j = 0; j < kOut; ++j)
+      if (j < cnt) d[j * ds] = v[j];
   } else if (DIR == 1) {
     if (!store) return;
     double* d = a.out[SPIN == 2 ? w.field : 0] +
@@ -1184,14 +1179,19 @@ __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int
     } else {
 #pragma unroll
       for (int j = 0; j < kOut; ++j) v[j] = j < cnt ? d[j * ds] : 0.0;
+      double x[kOut];
 #pragma unroll
       for (int j = 0; j < kOut; ++j) {
         const long long A = __double_as_longlong(v[j]);
-        if (j < cnt) {
-          d[j * ds] = i64_scaled(A + sum[j], e);
-          d[j * ds + 2] = i64_scaled(A - sum[j], e);
-        }
+        v[j] = i64_scaled(A + sum[j], e);
+        x[j] = i64_scaled(A - sum[j], e);
       }
+#pragma unroll
+      for (int j = 0; j < kOut; ++j)
+        if (j < cnt) {
+          d[j * ds] = v[j];
+          d[j * ds + 2] = x[j];
+        }
     }
   } else if (DIR == 2) {
     // {S, D} = F_N +- F_S from the lane pair (the map's north and south), then every kept order
@@ -1204,7 +1204,7 @@ __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int
     for (int j = 0; j < kOut; ++j) {
       const long long o = __shfl_xor_sync(0xffffffffu, sum[j], 1);
       const long long t = comp == 0 ? sum[j] + o : o - sum[j];
-      y[j] = (unsigned long long)__double_as_longlong(i64_scaled(cmp ? -t : t, e));
+      y[j] = (unsigned long long)__double_as_longlong(i64_scaled_any(cmp ? -t : t, e));
       if (eb == kNanExp) y[j] = 0x7FF8000000000000ull;
     }
     if (!store) return;
@@ -1261,7 +1261,7 @@ __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int
 #pragma unroll
     for (int j = 0; j < kOut; ++j) {
       if (!live(j)) continue;
-      const int ec = fac[j].fe;
+      const int ec = (int)fac[j];
       double* b = base(j);
       if (ph == 0) {
         b[j0] = keep(sum[j]);
@@ -1270,9 +1270,9 @@ __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int
         b[i2] = keep(bits(v[j]) - sum[j]);
         if (w.d.s == 0 && j0 == 0) {                       // no later phase
           b[j0] = ec == kNanExp ? keep(0x7FF8000000000000ll)
-                                : i64_scaled(bits(v[j]) + sum[j], ec + e);
+                                : i64_scaled_any(bits(v[j]) + sum[j], ec + e);
           b[i2] = ec == kNanExp ? keep(0x7FF8000000000000ll)
-                                : i64_scaled(bits(v[j]) - sum[j], ec + e);
+                                : i64_scaled_any(bits(v[j]) - sum[j], ec + e);
         }
       } else if (ph == 2) {
         b[i1] = keep(sum[j]);
@@ -1280,7 +1280,7 @@ __device__ __forceinline__ void tc_out(const TcGemmArgs& a, const TcUnit& w, int
         const long long T = bits(q[j]) + sum[j], V = bits(q[j]) - sum[j];
         const long long P = bits(v[j]), M = bits(p[j]);
         auto out = [&](long long t) {
-          return ec == kNanExp ? keep(0x7FF8000000000000ll) : i64_scaled(t, ec + e);
+          return ec == kNanExp ? keep(0x7FF8000000000000ll) : i64_scaled_any(t, ec + e);
         };
         b[j0] = out(P - T);
         b[i1] = out(P + T);
@@ -1298,8 +1298,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ TcSmemHdr h;
   __shared__ UnitQueue uq;
-  // per epilogue warp: its rows' factors (DIR 0), its columns' exponents (DIR 3: fe)
-  __shared__ TcFac s_fac[kTcEpiWarps][kTcAcc];
+  // per epilogue warp: its rows' factors (DIR 0), its columns' exponents (DIR 3)
+  __shared__ double s_fac[kTcEpiWarps][kTcAcc];
 
   const int tid = threadIdx.x;
   const int warp = tc::warp_index();
@@ -1464,7 +1464,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
         {
           const int l = w.row0 + 2 * (rbeg + lane);
           s_fac[warp][lane] =
-              tc_fac(l <= a.lmax ? a.tab[tri_off(w.m, a.lmax) + (l - w.m)].dm * a.pa : 0.0);
+              l <= a.lmax ? a.tab[tri_off(w.m, a.lmax) + (l - w.m)].dm * a.pa : 0.0;
         }
         __syncwarp();
       }
@@ -1477,7 +1477,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
       }
       if (DIR == 3) {
         __syncwarp();
-        s_fac[warp][lane].fe = a.EB[((long long)w.qi * a.ngroups + w.g) * kCols + rbeg + lane];
+        s_fac[warp][lane] = a.EB[((long long)w.qi * a.ngroups + w.g) * kCols + rbeg + lane];
         __syncwarp();
         store = c < w.nrows;                               // the lane's matrix row
       }
@@ -1531,7 +1531,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
         // the phase's sums out, a few at a time: the output code exists once and the registers
         // move down to it (unrolled over all sums it ran at the instruction fetch rate, one value
         // at a time at the latency of a load)
-        const int e = eb - 12 - a.unit_bits + (DIR == 0 ? a.eag : DIR >= 2 ? 1 : 0);
+        // (an empty column's sums are zero: any exponent does)
+        const int e = (eb == kEmptyExp ? 0 : eb) - 12 - a.unit_bits +
+                      (DIR == 0 ? a.eag : DIR >= 2 ? 1 : 0);
         constexpr int kOut = 4;
 #pragma unroll 1
         for (int c0 = 0; c0 < nrow; c0 += kOut) {
@@ -1541,7 +1543,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
 #pragma unroll
           for (int j = 0; j + kOut < kTcAcc; ++j) acc[j] = acc[j + kOut];
           tc_out<DIR, SPIN, kOut>(a, w, ph, store, c, rbeg + c0, min(kOut, nrow - c0), map, eb, e, sum,
-                            &s_fac[warp][c0]);
+                                  &s_fac[warp][c0]);
         }
       }
     }

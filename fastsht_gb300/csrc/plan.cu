@@ -664,12 +664,16 @@ static bool use_tc(const fsht_plan* p, int spin) {
 
 // Whether the ring transforms of a chunk of kc maps take the matrix form for the rings below
 // dft_end (it uses the contraction's buffers).  Its matrices and its tiles of 64 maps cost the same
-// for any kc up to 64, the FFT costs by the map; forward they meet near 18 maps at every nside from
-// 64 to 1024 (16 maps: 0.43 against 0.38 ms at nside 128, 4.6 against 4.8 at 512, 24.5 against
-// 23.1 at 1024), inverse near 40.
-constexpr int kDftFwdMaps = 20, kDftInvMaps = 40;
-static bool use_dft(const fsht_plan* p, int kc, int min_maps = kDftFwdMaps) {
-  return use_tc(p, 0) && p->dft_end > 0 && kc >= min_maps;
+// however full they are, the FFT costs by the map, so the line is on the maps per tile.  Forward
+// they meet near 18 at every nside from 64 to 1024 (16 maps: 0.43 against 0.38 ms at nside 128, 4.6
+// against 4.8 at 512, 24.5 against 23.1 at 1024).  Inverse the samples' four read-modify-writes
+// weigh more the shorter the rings are: 50 maps a tile lose at nside 64 and win at 128, 35 win at
+// 256, 32 lose at 128 and 256 and win at 512, 40 win at 1024.
+static bool use_dft(const fsht_plan* p, int kc, bool inv = false) {
+  const int fwd_maps = 20;
+  const int inv_maps = p->nside <= 64 ? 56 : p->nside <= 128 ? 42 : p->nside <= 256 ? 34 : 26;
+  const int groups = (kc + 63) / 64;
+  return use_tc(p, 0) && p->dft_end > 0 && kc >= (inv ? inv_maps : fwd_maps) * groups;
 }
 
 // Ring transforms of a whole chunk (maps on the device, or host memory read in place): matrix form
@@ -684,7 +688,7 @@ static int ring_fwd(fsht_plan* p, const double* maps, int kc, double2* W, bool h
 }
 static int ring_inv(fsht_plan* p, const double2* W, double* maps, int kc) {
   int ring0 = 0;
-  if (use_dft(p, kc, kDftInvMaps)) {
+  if (use_dft(p, kc, true)) {
     FSHT_TRY(fsht_launch_dft_inv(p, W, maps, p->npix, kc, p->stream));
     ring0 = p->dft_end;
   }
