@@ -972,7 +972,7 @@ struct TcGemmArgs {
 };
 
 struct __align__(8) TcSmemHdr {
-  uint64_t full[kTcStages], empty[kTcStages], tfull[4], tempty[4], fin;
+  uint64_t full[kTcStages], empty[kTcStages], tfull[2], tempty[2], fin;
   uint32_t tmem;
   int abort;
 };
@@ -1040,6 +1040,40 @@ __device__ __forceinline__ TcUnit tc_unit(const TcGemmArgs& a, int u) {
   }
   w.N = (w.nrows + 15) & ~15;
   return w;
+}
+
+// The products of levels L and L + 1 for one k-step into the slot pair at `slot`.  Neighbouring
+// digit planes of the second operand are neighbours in shared memory and the two levels' slots in
+// TMEM, so where the tile is wide one 256-column product a_i x {b_(L-i), b_(L+1-i)} serves both
+// levels and reads a_i once: 36 products of 128 columns read 288 KB of shared memory a k-step
+// beside the 96 KB that the copies write (3072 clocks at 128 bytes a clock against 2304 on the
+// tensor pipe, which is what a contraction without its drains took), 14 wide and 8 narrow ones 232.
+// (The two halves of an operand's planes lie in different stages: no pair spans planes 3 and 4.)
+constexpr int kWideN = 96;
+template <int L, class F>
+__device__ __forceinline__ void tc_products(uint32_t slot, const F& plane, uint32_t id1, bool wide,
+                                            bool accumulate) {
+  const uint32_t id2 = tc::umma_idesc_bf16(kRows, 2 * kCols);
+  if (wide) {
+#pragma unroll
+    for (int i = 0; i <= L + 1; ++i) {
+      const int b = L - i;
+      const uint32_t acc = accumulate || i > 0 ? 1u : 0u;
+      if (b >= 0 && b != 3) {
+        tc::umma_bf16_warp(slot, plane(i, false), plane(b, true), id2, acc);
+      } else {
+        if (b >= 0) tc::umma_bf16_warp(slot, plane(i, false), plane(b, true), id1, acc);
+        tc::umma_bf16_warp(slot + kCols, plane(i, false), plane(b + 1, true), id1, acc);
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i <= L + 1; ++i) {
+      const uint32_t acc = accumulate || i > 0 ? 1u : 0u;
+      if (i <= L) tc::umma_bf16_warp(slot, plane(i, false), plane(L - i, true), id1, acc);
+      tc::umma_bf16_warp(slot + kCols, plane(i, false), plane(L + 1 - i, true), id1, acc);
+    }
+  }
 }
 
 // Segment sg of phase ph: its column tiles, lambda tiles and sign.
@@ -1309,7 +1343,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
       tc::mbar_init(&h.full[s], 1);
       tc::mbar_init(&h.empty[s], 2);                     // both UMMA warps
     }
-    for (int s = 0; s < 4; ++s) {
+    for (int s = 0; s < 2; ++s) {
       tc::mbar_init(&h.tfull[s], 1);
       tc::mbar_init(&h.tempty[s], kTcEpiWarps);
     }
@@ -1355,56 +1389,55 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
       return true;
     });
   } else if (warp > kTcEpiWarps) {
-    // UMMA warps: slots 0 and 3, and slots 1 and 2 (5 of 10 and 13 of 26 products each)
+    // UMMA warps: warp `side` issues the products of the slot pair {2 side, 2 side + 1}
     const int side = warp - kTcEpiWarps - 1;
     const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
-    const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
+    const uint32_t slot = (uint32_t)tc::uniform((int)tmem) + 2 * side * kCols;
     uint32_t i = 0, use = 0;       // stages consumed, passes issued (one use of every slot each)
     bool ok = true;
+    auto drained = [&]() {         // the pair's sums of the pass before are out
+      if (use > 0 && !tc::mbar_wait_warp(&h.tempty[side], (use - 1) & 1, abort)) return false;
+      tc::tc_fence_after();
+      return true;
+    };
     for (uint32_t n = 0; ok; ++n) {
       const int u = uq_take(uq, n, abort);
       if (u < 0) break;
       const TcUnit w = tc_unit<DIR, SPIN>(a, u);
       // (the shuffles tell the compiler that these are warp-uniform)
-      const int unk = tc::uniform(w.nk);
-      const uint32_t idesc = tc::umma_idesc_bf16(kRows, tc::uniform(w.N));
+      const int unk = tc::uniform(w.nk), N = tc::uniform(w.N);
+      const uint32_t id1 = tc::umma_idesc_bf16(kRows, N);
+      const bool wide = N > kWideN;
       for (int s = 0; s < NPH * NSEG && ok; ++s) {
         for (int k0 = 0; k0 < unk && ok; k0 += kPartK) {
           const int nk = min(unk - k0, kPartK);
           for (int k = 0; k < nk && ok; ++k, ++i) {              // pass 0
             const uint32_t st = i % kTcStages;
-            if (!tc::mbar_wait_warp(&h.full[st], (i / kTcStages) & 1, abort)) {
+            if (!tc::mbar_wait_warp(&h.full[st], (i / kTcStages) & 1, abort) ||
+                (k == 0 && !drained())) {
               ok = false;
               break;
             }
             tc::tc_fence_after();
             const uint64_t c0 = tc::umma_desc(s_u + st * kTcStageBytes, 128, 256);
-            const uint64_t c1 = tc::umma_desc_add(c0, kHalfBytes);
-            const uint64_t ca = SWAP ? c1 : c0, ra = SWAP ? c0 : c1;
-#pragma unroll
-            for (int lev = 0; lev < 4; ++lev) {
-              if ((lev == 0 || lev == 3) != (side == 0)) continue;
-              if (k == 0 && use > 0) {
-                if (!tc::mbar_wait_warp(&h.tempty[lev], (use - 1) & 1, abort)) {
-                  ok = false;
-                  break;
-                }
-                tc::tc_fence_after();
-              }
-#pragma unroll
-              for (int aa = 0; aa <= lev; ++aa)
-                tc::umma_bf16_warp(utmem + lev * kCols, tc::umma_desc_add(ca, aa * kPlaneBytes),
-                                   tc::umma_desc_add(ra, (lev - aa) * kPlaneBytes), idesc,
-                                   (k > 0 || aa > 0) ? 1u : 0u);
-              if (k == nk - 1) tc::umma_commit_warp(&h.tfull[lev]);
+            auto plane = [&](int d, bool second) {
+              return tc::umma_desc_add(c0, (uint32_t)d * kPlaneBytes +
+                                               (second != SWAP ? kHalfBytes : 0));
+            };
+            if (side == 0) {
+              tc_products<0>(slot, plane, id1, wide, k > 0);
+            } else {
+              tc_products<2>(slot, plane, id1, wide, k > 0);
             }
-            if (ok) tc::umma_commit_warp(&h.empty[st]);
+            if (k == nk - 1) tc::umma_commit_warp(&h.tfull[side]);
+            tc::umma_commit_warp(&h.empty[st]);
           }
           ++use;
           for (int k = 0; k < nk && ok; ++k, i += 2) {           // pass 1
             const uint32_t st = i % kTcStages, st1 = (i + 1) % kTcStages;
             if (!tc::mbar_wait_warp(&h.full[st], (i / kTcStages) & 1, abort) ||
-                !tc::mbar_wait_warp(&h.full[st1], ((i + 1) / kTcStages) & 1, abort)) {
+                !tc::mbar_wait_warp(&h.full[st1], ((i + 1) / kTcStages) & 1, abort) ||
+                (k == 0 && !drained())) {
               ok = false;
               break;
             }
@@ -1416,27 +1449,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
               return tc::umma_desc_add(d < 4 ? ca : cb, (uint32_t)(d & 3) * kPlaneBytes +
                                                             (second != SWAP ? kHalfBytes : 0));
             };
-#pragma unroll
-            for (int lev = 4; lev < 8; ++lev) {
-              if ((lev == 4 || lev == 7) != (side == 0)) continue;
-              if (k == 0) {
-                if (!tc::mbar_wait_warp(&h.tempty[lev - 4], (use - 1) & 1, abort)) {
-                  ok = false;
-                  break;
-                }
-                tc::tc_fence_after();
-              }
-#pragma unroll
-              for (int aa = 0; aa <= lev; ++aa)
-                tc::umma_bf16_warp(utmem + (lev - 4) * kCols, plane(aa, false),
-                                   plane(lev - aa, true), idesc,
-                                   (k > 0 || aa > 0) ? 1u : 0u);
-              if (k == nk - 1) tc::umma_commit_warp(&h.tfull[lev - 4]);
+            if (side == 0) {
+              tc_products<4>(slot, plane, id1, wide, k > 0);
+            } else {
+              tc_products<6>(slot, plane, id1, wide, k > 0);
             }
-            if (ok) {
-              tc::umma_commit_warp(&h.empty[st]);
-              tc::umma_commit_warp(&h.empty[st1]);
-            }
+            if (k == nk - 1) tc::umma_commit_warp(&h.tfull[side]);
+            tc::umma_commit_warp(&h.empty[st]);
+            tc::umma_commit_warp(&h.empty[st1]);
           }
           ++use;
         }
@@ -1504,18 +1524,13 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
             // wait for a pair of slots, drain it, hand it back
             auto pair = [&](auto P) {
               constexpr int kP = decltype(P)::value, kS = (2 * kP) & 3;
-              const bool ok = tc::mbar_wait_warp(&h.tfull[kS], use & 1, abort) &&
-                              tc::mbar_wait_warp(&h.tfull[kS + 1], use & 1, abort);
-              if (!ok) return;
+              if (!tc::mbar_wait_warp(&h.tfull[kP & 1], use & 1, abort)) return;
               tc::tc_fence_after();
               tc_drain<kP>(tbase + kS * kCols, tbase + (kS + 1) * kCols, nrow, sf, a.unit_bits,
                            acc);
               tc::tc_fence_before();
               __syncwarp();
-              if (lane == 0) {
-                tc::mbar_arrive(&h.tempty[kS]);
-                tc::mbar_arrive(&h.tempty[kS + 1]);
-              }
+              if (lane == 0) tc::mbar_arrive(&h.tempty[kP & 1]);
             };
             pair(std::integral_constant<int, 0>{});
             pair(std::integral_constant<int, 1>{});
