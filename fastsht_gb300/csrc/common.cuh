@@ -279,8 +279,10 @@ int fsht_launch_ring_fft_inv_df(fsht_plan* p, const double2* W, double* maps,
                                 long long map_stride, int kc, cudaStream_t s);
 // Maps per CTA of the ring-FFT launches when the autotuner has not set one.
 int fsht_fft_maps_per_block(int kc, int nrings);
+// (maps [k0, k0 + kb) of the kc, all from k0 on for kb < 0; an FP64 plan's only)
 int fsht_launch_ring_fft_inv(fsht_plan* p, const double2* W, double* maps,
-                             long long map_stride, int kc, cudaStream_t s, int ring0 = 0);
+                             long long map_stride, int kc, cudaStream_t s, int ring0 = 0,
+                             int k0 = 0, int kb = -1);
 int fsht_launch_fourier_residual(fsht_plan* p, const double2* X, double2* GR, int kc,
                                  int prefix, cudaStream_t s);
 int fsht_launch_ring_skip(fsht_plan* p, cudaStream_t s);
@@ -298,7 +300,7 @@ int fsht_dft_tables_init(fsht_plan* p);
 int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, int kc, int k0,
                         int cnt, bool host, double2* W, cudaStream_t s);
 int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride, int kc,
-                        cudaStream_t s);
+                        int cnt, cudaStream_t s);
 bool fsht_tc_supported(const fsht_plan* p);
 int fsht_tc_tables_init(fsht_plan* p);
 size_t fsht_tc_ws_bytes(const fsht_plan* p, int kc, int nf);

@@ -745,7 +745,7 @@ struct DftSliceArgs {
   int nside, nring, cnt;
   // inverse
   const double2* W;
-  int kc, nnorth;
+  int kc, nnorth;               // kc: map stride of W; cnt of the maps take part
 };
 constexpr int kNanExp = kEmptyExp - 1;     // column with a non-finite sample: NaN out
 
@@ -879,9 +879,9 @@ __global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
   const int n = 4 * d.q;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int map = blockIdx.y * 16 + (lane >> 1), h = lane & 1;
-  const bool valid = map < a.kc && !(h == 1 && d.ring == a.nnorth - 1);
+  const bool valid = map < a.cnt && !(h == 1 && d.ring == a.nnorth - 1);
   const long long stride_m = (long long)a.nnorth * a.kc * 2;
-  const double2* g = a.W + ((long long)d.ring * a.kc + (map < a.kc ? map : 0)) * 2 + h;
+  const double2* g = a.W + ((long long)d.ring * a.kc + (map < a.cnt ? map : 0)) * 2 + h;
   unsigned long long mx = 0;
   if (valid)
 #pragma unroll 4
@@ -900,7 +900,7 @@ __global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
   const int E = dft_exp(mx);
   const bool live = valid && E > kEmptyExp;
   const int grp = map >> 6, c = 2 * (map & 63) + h;
-  if (map >= a.kc) return;
+  if (map >= a.cnt) return;
   if (warp == 0) a.EB[((long long)blockIdx.x * a.ngroups + grp) * kCols + c] = E;
   unsigned char* dst = a.WS + (size_t)(d.off_c * a.ngroups) * kStepBytes +
                        (size_t)grp * d.nk * kStepBytes + (c >> 3) * 256 + (c & 7) * 16;
@@ -1968,19 +1968,20 @@ int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, 
   return FSHT_OK;
 }
 
-// {G_N, G_S} of rings below dft_end -> their pixels.
+// {G_N, G_S} of rings below dft_end -> their pixels, the first cnt of kc maps.
 int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride, int kc,
-                        cudaStream_t s) {
-  const int ngroups = tc_groups(kc);
+                        int cnt, cudaStream_t s) {
+  const int ngroups = tc_groups(cnt);
   for (int w = 0; w < p->ndft_waves; ++w) {
     const int* wv = p->h_dft_waves + kDftWaveInts * w;
     FSHT_TRY(launch_dft_trig<true>(p, wv, s));
     DftSliceArgs sa = dft_slice_args(p, wv, ngroups);
     sa.W = W;
     sa.kc = kc;
-    k_dft_slice_inv<<<dim3(wv[1] - wv[0], (kc + 15) / 16), 256, 0, s>>>(sa);
+    sa.cnt = cnt;
+    k_dft_slice_inv<<<dim3(wv[1] - wv[0], (cnt + 15) / 16), 256, 0, s>>>(sa);
     FSHT_LAUNCH_CHECK();
-    TcGemmArgs a = dft_gemm_args(p, wv, ngroups, kc, 2);
+    TcGemmArgs a = dft_gemm_args(p, wv, ngroups, cnt, 2);
     a.map_stride = map_stride;
     a.out[0] = maps;
     a.nunits = ngroups * a.ntmax * (wv[1] - wv[0]);

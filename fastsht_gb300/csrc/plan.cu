@@ -662,37 +662,42 @@ static bool use_tc(const fsht_plan* p, int spin) {
   return p->tc64 && p->d_lbuf && p->d_tcflag && (spin == 0 || p->d_poltab);
 }
 
-// Whether the ring transforms of a chunk of kc maps take the matrix form for the rings below
-// dft_end (it uses the contraction's buffers).  Its matrices and its tiles of 64 maps cost the same
-// however full they are, the FFT costs by the map, so the line is on the maps per tile.  Forward
-// they meet near 18 at every nside from 64 to 1024 (16 maps: 0.43 against 0.38 ms at nside 128, 4.6
-// against 4.8 at 512, 24.5 against 23.1 at 1024).  Inverse the samples' four read-modify-writes
-// weigh more the shorter the rings are: 50 maps a tile lose at nside 64 and win at 128, 35 win at
-// 256, 32 lose at 128 and 256 and win at 512, 40 win at 1024.
-static bool use_dft(const fsht_plan* p, int kc, bool inv = false) {
-  const int fwd_maps = 20;
-  const int inv_maps = p->nside <= 64 ? 56 : p->nside <= 128 ? 42 : p->nside <= 256 ? 34 : 26;
-  const int groups = (kc + 63) / 64;
-  return use_tc(p, 0) && p->dft_end > 0 && kc >= (inv ? inv_maps : fwd_maps) * groups;
+// How many maps of a chunk of kc, counted from the first, take the matrix form of the ring
+// transforms below dft_end (it uses the contraction's buffers): whole tiles of 64 maps, and the
+// last part of a tile if it is full enough.  The matrices and a tile cost the same however full it
+// is, the FFT costs by the map.  Measured, ms (tile / FFT of 16 maps; above nside 256 both without
+// the belt's FFT): forward .062/.046 at nside 32, .136/.112 at 64, .31/.34 at 128, 1.23/1.31 at 256,
+// 2.2/3.1 at 512, 15/17 at 1024; inverse, where the samples' read-modify-writes weigh more the
+// shorter the rings are, .21/.049, .28/.115, .85/.36, 2.6/1.28, 4.5/3.3, 28/18.
+static int dft_maps(const fsht_plan* p, int kc, bool inv = false) {
+  if (!use_tc(p, 0) || p->dft_end <= 0) return 0;
+  const int fwd_maps = p->nside <= 64 ? 20 : 15;
+  const int inv_maps = p->nside <= 32 ? 60 : p->nside <= 128 ? 38 : p->nside <= 256 ? 31 : 23;
+  const int rest = kc % 64;
+  return rest >= (inv ? inv_maps : fwd_maps) ? kc : kc - rest;
 }
 
-// Ring transforms of a whole chunk (maps on the device, or host memory read in place): matrix form
-// below dft_end where it applies, FFT above.
-static int ring_fwd(fsht_plan* p, const double* maps, int kc, double2* W, bool host = false) {
-  int ring0 = 0;
-  if (use_dft(p, kc)) {
-    FSHT_TRY(fsht_launch_dft_fwd(p, maps, p->npix, kc, 0, kc, host, W, p->stream));
-    ring0 = p->dft_end;
+// Ring transforms of maps [k0, k0 + cnt) of a chunk of kc (maps on the device, or host memory read
+// in place): matrix form where it applies, FFT for the other rings and maps.
+static int ring_fwd(fsht_plan* p, const double* maps, int kc, int k0, int cnt, double2* W,
+                    bool host) {
+  const int n = std::max(0, std::min(dft_maps(p, kc) - k0, cnt));
+  if (n > 0) {
+    FSHT_TRY(fsht_launch_dft_fwd(p, maps, p->npix, kc, k0, n, host, W, p->stream));
+    FSHT_TRY(fsht_launch_ring_fft_fwd_part(p, maps, p->npix, kc, k0, n, W, p->stream,
+                                           p->dft_end));
   }
-  return fsht_launch_ring_fft_fwd_part(p, maps, p->npix, kc, 0, kc, W, p->stream, ring0);
+  if (n == cnt) return FSHT_OK;
+  return fsht_launch_ring_fft_fwd_part(p, maps, p->npix, kc, k0 + n, cnt - n, W, p->stream, 0);
 }
 static int ring_inv(fsht_plan* p, const double2* W, double* maps, int kc) {
-  int ring0 = 0;
-  if (use_dft(p, kc, true)) {
-    FSHT_TRY(fsht_launch_dft_inv(p, W, maps, p->npix, kc, p->stream));
-    ring0 = p->dft_end;
+  const int n = dft_maps(p, kc, true);
+  if (n > 0) {
+    FSHT_TRY(fsht_launch_dft_inv(p, W, maps, p->npix, kc, n, p->stream));
+    FSHT_TRY(fsht_launch_ring_fft_inv(p, W, maps, p->npix, kc, p->stream, p->dft_end, 0, n));
   }
-  return fsht_launch_ring_fft_inv(p, W, maps, p->npix, kc, p->stream, ring0);
+  if (n == kc) return FSHT_OK;
+  return fsht_launch_ring_fft_inv(p, W, maps, p->npix, kc, p->stream, 0, n, kc - n);
 }
 
 static unsigned char* lam_buf(fsht_plan* p, int w) {
@@ -1093,14 +1098,14 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
     }
     // the first lambda tiles are computed on the auxiliary stream during the FFT
     // (not beside the matrix form of the FFT, which uses the tiles' buffers)
-    const bool tc = !split && use_tc(p, 0) && !use_dft(p, kc);
+    const bool tc = !split && use_tc(p, 0) && dft_maps(p, kc) == 0;
     if (split) FSHT_TRY(lam_start(p, fsht_launch_split_lambda));
     if (tc) FSHT_TRY(lam_start(p, fsht_launch_tc_lambda));
     // the chunk's maps as the FFT reads them: device buffer, or host memory read in place
     const double* cmaps = (hx && hx->direct ? hx->direct : maps) + (size_t)c0 * p->npix;
     if (!split && (!hx || hx->direct)) {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
-      FSHT_TRY(ring_fwd(p, cmaps, kc, W0, hx != nullptr));
+      FSHT_TRY(ring_fwd(p, cmaps, kc, 0, kc, W0, hx != nullptr));
     } else if (!hx || hx->direct) {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
       // (page-locked maps mapped into the device's address space are read over the host link
@@ -1119,13 +1124,7 @@ static int t2alm_impl(fsht_plan* p, const double* maps, double* alm, int nmaps, 
         FSHT_CUDA_TRY(cudaEventRecord(p->evx[1], p->xfer));
         FSHT_CUDA_TRY(cudaStreamWaitEvent(p->stream, p->evx[1], 0));
         FSHT_PROF(FSHT_KCAT_FFT_FWD);
-        int ring0 = 0;
-        if (use_dft(p, kc)) {
-          FSHT_TRY(fsht_launch_dft_fwd(p, cmaps, p->npix, kc, k0, cnt, false, W0, p->stream));
-          ring0 = p->dft_end;
-        }
-        FSHT_TRY(fsht_launch_ring_fft_fwd_part(p, cmaps, p->npix, kc, k0, cnt, W0, p->stream,
-                                               ring0));
+        FSHT_TRY(ring_fwd(p, cmaps, kc, k0, cnt, W0, false));
       }
     }
     if (split) {
@@ -1329,16 +1328,16 @@ static int qu_analysis(fsht_plan* p, const double* Q, const double* U, double* a
     double2* WQ = work_buf(p, 0, kc);
     double2* WU = work_buf(p, 1, kc);
     const bool split = p->precision == FSHT_PREC_SPLIT;
-    const bool pre = split ? p->d_poltab != nullptr : use_tc(p, 2) && !use_dft(p, kc);
+    const bool pre = split ? p->d_poltab != nullptr : use_tc(p, 2) && dft_maps(p, kc) == 0;
     if (pre)                                                         // overlaps the FFTs
       FSHT_TRY(lam_start(p, split ? fsht_launch_split_lambda_pol : fsht_launch_tc_lambda_pol));
     {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
-      FSHT_TRY(ring_fwd(p, Q + (size_t)c0 * p->npix, kc, WQ));
+      FSHT_TRY(ring_fwd(p, Q + (size_t)c0 * p->npix, kc, 0, kc, WQ, false));
     }
     {
       FSHT_PROF(FSHT_KCAT_FFT_FWD);
-      FSHT_TRY(ring_fwd(p, U + (size_t)c0 * p->npix, kc, WU));
+      FSHT_TRY(ring_fwd(p, U + (size_t)c0 * p->npix, kc, 0, kc, WU, false));
     }
     FSHT_TRY(pol_analysis(p, WQ, WU, almE, almB, nmaps, c0, kc, 0, which, pre));
     if (niter > 0) {

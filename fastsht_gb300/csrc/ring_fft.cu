@@ -208,7 +208,9 @@ struct InvArgs {
   const double2* W;
   double* maps;
   long long map_stride;
-  int kc, maps_per_block;
+  int kc;                   // maps in this chunk (the map stride of W)
+  int k_off, k_cnt;         // the maps of this launch: [k_off, k_off + k_cnt)
+  int maps_per_block;
   int nside, lmax, nnorth, nring, ring_base;
   const FshtRingFFT* rfs;
   FftTw tw;
@@ -251,8 +253,8 @@ __global__ void __launch_bounds__(512, 2) k_ring_fft_inv(InvArgs a) {
     }
     ph[m] = make_double2(c, s);
   }
-  const int k_begin = blockIdx.y * a.maps_per_block;
-  const int k_end = min(a.kc, k_begin + a.maps_per_block);
+  const int k_begin = a.k_off + blockIdx.y * a.maps_per_block;
+  const int k_end = min(a.k_off + a.k_cnt, k_begin + a.maps_per_block);
   const double2* chirp = a.chirp + rf.chirp_off;
   const double2* bhat = a.bhat + rf.bhat_off;
   const long long stride_m = (long long)a.nnorth * a.kc * 2;
@@ -663,13 +665,15 @@ int fsht_launch_ring_fft_fwd_part(fsht_plan* p, const double* maps, long long ma
 }
 
 int fsht_launch_ring_fft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride,
-                             int kc, cudaStream_t s, int ring0) {
+                             int kc, cudaStream_t s, int ring0, int k0, int kb) {
   if (p->d_tw_df) return fsht_launch_ring_fft_inv_df(p, W, maps, map_stride, kc, s);
   InvArgs a;
   a.W = W;
   a.maps = maps;
   a.map_stride = map_stride;
   a.kc = kc;
+  a.k_off = k0;
+  a.k_cnt = kb = kb < 0 ? kc - k0 : kb;
   a.nside = p->nside;
   a.lmax = p->lmax;
   a.nnorth = p->nnorth;
@@ -681,14 +685,14 @@ int fsht_launch_ring_fft_inv(fsht_plan* p, const double2* W, double* maps, long 
   a.chirp = p->d_chirp;
   a.bhat = p->d_bhat;
   a.ring_i0 = p->d_ring_i0;
-  a.maps_per_block = p->fft_mpb > 0 ? p->fft_mpb : maps_per_block_for(kc, p->nnorth);
+  a.maps_per_block = p->fft_mpb > 0 ? p->fft_mpb : maps_per_block_for(kb, p->nnorth);
   FSHT_TRY(fsht_smem_limit((const void*)k_ring_fft_inv, (size_t)(p->fft_smem)));
   for (int sgi = 0; sgi < p->fft_nseg; ++sgi) {
     const long long* sg = p->fft_seg + 3 * sgi;
     const int r0 = sg[0] > ring0 ? (int)sg[0] : ring0;
     if (r0 >= sg[1]) continue;
     a.ring_base = r0;
-    dim3 grid((unsigned)(sg[1] - r0), (kc + a.maps_per_block - 1) / a.maps_per_block);
+    dim3 grid((unsigned)(sg[1] - r0), (kb + a.maps_per_block - 1) / a.maps_per_block);
     k_ring_fft_inv<<<grid, p->fft_threads > 0 ? p->fft_threads : 512, (size_t)sg[2], s>>>(a);
     FSHT_LAUNCH_CHECK();
   }
