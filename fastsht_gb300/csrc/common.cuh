@@ -296,6 +296,8 @@ int fsht_launch_analysis_fp64(fsht_plan* p, int spin, const double2* WQ,
 // The same contraction as exact digit products on the tensor cores (FP64 plans with tc64).
 // Per wave w: slice (phases or alm -> digit tiles WS, exponents EB), lambda (-> lbuf), gemm
 // (dir 0: into alm, dir 1: into the phase matrices).  A null second field means spin 0.
+// The waves again, for tiles of `cap` bytes (before fsht_dft_tables_init).
+int fsht_tc_wave_cap(fsht_plan* p, size_t cap);
 int fsht_dft_tables_init(fsht_plan* p);
 int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, int kc, int k0,
                         int cnt, bool host, double2* W, cudaStream_t s);
@@ -328,8 +330,10 @@ size_t fsht_split_eb_bytes(const fsht_plan* p, int kc);
 // writes the wave's lambda digit tiles into lbuf, gemm contracts them into alm (stores, or
 // adds when accumulate).
 int fsht_split_tables_init(fsht_plan* p);
-// Tile offsets per order and the waves of m, for digit tiles of `unit` bytes per k-step.
-int fsht_wave_tables_init(fsht_plan* p, size_t unit);
+// Tile offsets per order and the waves of m, for digit tiles of `unit` bytes per k-step, at most
+// `cap` bytes a wave.
+constexpr size_t kLbufCap = 2ull << 30;
+int fsht_wave_tables_init(fsht_plan* p, size_t unit, size_t cap = kLbufCap);
 int fsht_launch_split_slice(fsht_plan* p, int w, const double2* W, unsigned char* WS, int* EB,
                             int kc, cudaStream_t s);
 int fsht_launch_split_lambda(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s);

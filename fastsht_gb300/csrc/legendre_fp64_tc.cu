@@ -1638,6 +1638,8 @@ int fsht_tc_tables_init(fsht_plan* p) {
   return fsht_wave_tables_init(p, kStepBytes);
 }
 
+int fsht_tc_wave_cap(fsht_plan* p, size_t cap) { return fsht_wave_tables_init(p, kStepBytes, cap); }
+
 // Digit tiles of one wave of kc maps (nf = 2: Q and U or E and B, plain and i v), its exponents,
 // and the flags of every order.
 size_t fsht_tc_ws_bytes(const fsht_plan* p, int kc, int nf) {

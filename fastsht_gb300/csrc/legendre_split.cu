@@ -1048,7 +1048,6 @@ int fsht_launch_split_slice(fsht_plan* p, int w, const double2* W, unsigned char
 
 // ------------------------------------------------------------------ host side
 namespace {
-constexpr size_t kLbufCap = 2ull << 30;     // lambda-digit staging per wave
 
 int eag_of(int lmax) {
   const double b = std::sqrt((2.0 * lmax + 1.0) / (4.0 * M_PI)) * (1.0 + 0x1p-30);
@@ -1065,10 +1064,10 @@ int fsht_split_tables_init(fsht_plan* p) {
   return fsht_wave_tables_init(p, (size_t)kSlices * kATileBytes);
 }
 
-int fsht_wave_tables_init(fsht_plan* p, size_t unit) {
+int fsht_wave_tables_init(fsht_plan* p, size_t unit, size_t cap) {
   const int lmax = p->lmax;
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_off, sizeof(long long) * (lmax + 2)));
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_offT, sizeof(long long) * (lmax + 2)));
+  if (!p->d_lam_off) FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_off, sizeof(long long) * (lmax + 2)));
+  if (!p->d_lam_offT) FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_offT, sizeof(long long) * (lmax + 2)));
   // per q (pair order): `unit`-byte k-steps of m(q)'s analysis tiles (l-rows) and synthesis
   // tiles (ring rows)
   std::vector<long long> off(lmax + 2, 0), offT(lmax + 2, 0);
@@ -1083,7 +1082,7 @@ int fsht_wave_tables_init(fsht_plan* p, size_t unit) {
     off[q + 1] = off[q] + 2LL * ntl[q] * nkm[q];
     offT[q + 1] = offT[q] + 2LL * nrb[q] * nkl[q];
   }
-  const size_t cap_units = kLbufCap / unit;
+  const size_t cap_units = cap / unit;
   // spin-2 plans stage lambda1 and lambda2: twice the analysis tiles
   const long long fa = p->pol ? 2 : 1;
   auto span = [&](int q0, int q1) -> size_t {
@@ -1092,6 +1091,7 @@ int fsht_wave_tables_init(fsht_plan* p, size_t unit) {
   // waves: consecutive q ranges whose tiles (either layout) fit the staging buffer
   std::vector<int> waves;
   size_t lbuf_units = 0;
+  p->wave_qmax = 0;
   for (int q0 = 0; q0 <= lmax;) {
     int q1 = q0 + 1;
     while (q1 <= lmax && span(q0, q1 + 1) <= cap_units) ++q1;
@@ -1109,6 +1109,7 @@ int fsht_wave_tables_init(fsht_plan* p, size_t unit) {
     q0 = q1;
   }
   p->nwaves = (int)waves.size() / kWaveInts;
+  delete[] p->h_waves;
   p->h_waves = new (std::nothrow) int[waves.size()];
   if (!p->h_waves) {
     fsht_set_error("host allocation failed");

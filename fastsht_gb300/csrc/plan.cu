@@ -334,7 +334,6 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     return fail(rc);
   if (precision == FSHT_PREC_FP64 && fsht_tc_supported(p)) {
     if ((rc = fsht_tc_tables_init(p))) return fail(rc);
-    if ((rc = fsht_dft_tables_init(p))) return fail(rc);
     p->tc64 = 1;
   }
   // ---- workspace: nbuf phase matrices of kchunk maps (+ the sliced copy for the
@@ -358,6 +357,24 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     return b;
   };
   const bool tables_only = (flags & FSHT_FLAG_TABLES_ONLY) != 0;
+  auto tc_chunk = [&]() -> size_t {           // maps whose tiles fit the limit beside W
+    size_t k = (size_t)nmaps_max;
+    while (k > 1 && need_tc(k) > limit) k = k > 64 ? (k - 1) / 64 * 64 : k - 1;
+    return k;
+  };
+  if (p->tc64) {
+    // Waves of kLbufCap of lambda tiles, or of half of it where that saves a chunk: every chunk
+    // computes all tiles again, while half the wave costs 4 to 7 % (nside 256, lmax 767, 128 pairs
+    // of maps: 24.8 ms in two chunks, 19.3 in one; 1024/2047/64 and 256/767/67, one chunk either
+    // way: 89.9 and 25.2 against 96.6 and 26.2; a quarter of it costs 10 to 35 %)
+    auto chunks = [&](size_t k) { return ((size_t)nmaps_max + k - 1) / k; };
+    const size_t c1 = chunks(tc_chunk());
+    if (!tables_only && c1 > 1) {
+      if ((rc = fsht_tc_wave_cap(p, kLbufCap / 2))) return fail(rc);
+      if (chunks(tc_chunk()) >= c1 && (rc = fsht_tc_wave_cap(p, kLbufCap))) return fail(rc);
+    }
+    if ((rc = fsht_dft_tables_init(p))) return fail(rc);
+  }
   size_t kc = (size_t)nmaps_max;
   while (kc > 1 && need(kc) > limit) kc = (kc > 128 && kc % 128) ? kc - kc % 128 : kc - (kc > 128 ? 128 : 1);
   if (!tables_only && need(kc) > limit) {
@@ -368,8 +385,7 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     // The digit tiles share the workspace limit with the phase matrices: whole 64-map groups.
     // A limit that leaves them less than one group (and fewer maps than the FMA kernels' chunk)
     // keeps the FMA kernels, which need no tiles.
-    size_t kt = (size_t)nmaps_max;
-    while (kt > 1 && need_tc(kt) > limit) kt = kt > 64 ? (kt - 1) / 64 * 64 : kt - 1;
+    const size_t kt = tc_chunk();
     if (need_tc(kt) > limit || (kt < kc && kt < 64)) {
       p->tc64 = 0;
     } else {
