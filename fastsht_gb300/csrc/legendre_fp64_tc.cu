@@ -564,6 +564,7 @@ struct TcSliceAArgs {
 template <int NF>
 __global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
   __shared__ unsigned long long s_mx[2 * NF][2][2][64];        // [field, half][parity][comp][map]
+  __shared__ unsigned long long s_col[2][2][64];               // of the block
   const int qi = blockIdx.x, g = blockIdx.y;
   const int m = m_of_q(a.q0 + qi, a.lmax);
   const int f = NF == 1 ? 0 : (int)(threadIdx.x >> 8);
@@ -573,7 +574,8 @@ __global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
   const bool valid = k < a.kc && !(comp == 1 && m == 0);
   const long long L1 = a.lmax + 1;
   const int nh = 2 * (((a.lmax - m) / 2 + 1 + kKStep - 1) / kKStep);   // blocks of eight l
-  const int h0 = half ? nh / 2 : 0, h1 = half ? nh : nh / 2;
+  const int seg = 2 * (int)blockIdx.z + half, nseg = 2 * (int)gridDim.z;
+  const int h0 = nh * seg / nseg, h1 = nh * (seg + 1) / nseg;
   const FshtLamRow* tab = a.tab + tri_off(m, a.lmax);
   const double* col = a.alm[f] + a.k0 + k +
                       (comp == 0 ? (long long)m * L1 + m : (L1 - m) * L1) * a.ld;
@@ -604,6 +606,7 @@ __global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
   __syncthreads();
   bool flag = false;
   int Ep[2];
+  unsigned long long mxp[2];
 #pragma unroll
   for (int p = 0; p < 2; ++p) {
     unsigned long long mx = 0;
@@ -612,14 +615,22 @@ __global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
 #pragma unroll
       for (int u = 0; u < 4; ++u)
         if (NF == 2 || (u & 1) == comp) mx = max(mx, s_mx[h][u >> 1][u & 1][kl]);
+    if (f == 0 && !half) s_col[p][comp][kl] = mx;
+  }
+  mxp[0] = slice_cluster_max(&s_col[0][comp][kl]);
+  mxp[1] = slice_cluster_max(&s_col[1][comp][kl]);
+#pragma unroll
+  for (int p = 0; p < 2; ++p) {
+    const unsigned long long mx = mxp[p];
     const int ef = (int)(mx >> 52);
     const bool odd_range = mx != 0 && (ef < 1023 - kMaxExp || ef > 1023 + kMaxExp);
     flag |= odd_range;
     Ep[p] = (mx == 0 || odd_range) ? kEmptyExp : ef - 1022;
-    if (f == 0 && !half) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = Ep[p];
+    if (f == 0 && seg == 0) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = Ep[p];
   }
   const int any = __syncthreads_or(flag ? 1 : 0);
-  if (threadIdx.x < 4) a.flags[((long long)m * a.ngroups + g) * 4 + threadIdx.x] = any;
+  if (threadIdx.x < 4 && blockIdx.z == 0)
+    a.flags[((long long)m * a.ngroups + g) * 4 + threadIdx.x] = any;
   constexpr int NC = NF == 1 ? 1 : 4;
   const int cr = 2 * kl + (comp ^ 1);
 #pragma unroll 1
@@ -650,6 +661,7 @@ __global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
                             rot + (size_t)(h >> 1) * kStepBytes + (h & 1) * 128, comp == 1, y);
     }
   }
+  slice_cluster_done();
 }
 
 // ------------------------------------------------------------------ ring transforms
@@ -1696,12 +1708,9 @@ int fsht_launch_tc_slice_alm(fsht_plan* p, int w, const double* alm0, const doub
   a.EB = EB;
   a.flags = p->d_tcflag;
   const dim3 grid(wv[1] - wv[0], a.ngroups);
-  if (alm1)
-    k_tc_slice_alm<2><<<grid, 512, 0, s>>>(a);
-  else
-    k_tc_slice_alm<1><<<grid, 256, 0, s>>>(a);
-  FSHT_LAUNCH_CHECK();
-  return FSHT_OK;
+  const int cl = slice_cluster((long long)grid.x * grid.y * (alm1 ? 4 : 2), wv[5]);
+  if (alm1) return launch_slice(k_tc_slice_alm<2>, grid, 512, cl, s, a);
+  return launch_slice(k_tc_slice_alm<1>, grid, 256, cl, s, a);
 }
 
 namespace {

@@ -68,8 +68,8 @@ __global__ void __launch_bounds__(kSliceThreads, 6) k_slice_phase(SliceArgs a) {
   const int i0 = a.ring_i0[m];
   const int K = a.nnorth - i0;
   const int nks = (K + kKStep - 1) / kKStep;
-  const int ksh = (nks + 1) / 2;                   // k-steps of the first half
-  const int ks_begin = half ? ksh : 0, ks_end = half ? nks : ksh;
+  const int seg = 2 * (int)blockIdx.z + half, nseg = 2 * (int)gridDim.z;
+  const int ks_begin = nks * seg / nseg, ks_end = nks * (seg + 1) / nseg;
   const int r_begin = ks_begin * kKStep, r_end = min(K, ks_end * kKStep);
   const bool valid = k < a.kc;
   const double* col = a.W + ((((long long)m * a.nnorth + i0) * a.kc + k) * 2 + p) * 2 + comp;
@@ -97,13 +97,12 @@ __global__ void __launch_bounds__(kSliceThreads, 6) k_slice_phase(SliceArgs a) {
   if (half) s_mx[t] = mx;
   __syncthreads();
   if (!half) s_mx[t] = max(mx, s_mx[t]);
-  __syncthreads();
-  mx = s_mx[t];
+  mx = slice_cluster_max(&s_mx[t]);
   // |v| < 2^E for every value of the column (a subnormal maximum takes E = -1021; a
   // non-finite one gives an exponent its digits report as out of range)
   const int ef = (int)(mx >> 52);
   const int E = mx == 0 ? kEmptyExp : (ef == 0 ? -1021 : ef - 1022);
-  if (!half) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = E;
+  if (seg == 0) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = E;
   unsigned char* base = a.WS + ((size_t)(qi * 2 + p) * a.ngroups + g) * a.row_bytes +
                         (c >> 3) * 256 + (c & 7) * 16;
   bool bad = false;
@@ -132,6 +131,7 @@ __global__ void __launch_bounds__(kSliceThreads, 6) k_slice_phase(SliceArgs a) {
     }
   }
   if (bad) atomicOr(a.err, tc::kErrRange);
+  slice_cluster_done();
 }
 
 // ------------------------------------------------------------------ lambda digits
@@ -710,8 +710,9 @@ __global__ void __launch_bounds__(128) k_lambda_digits_T(LamTArgs a) {
   if (bad) atomicOr(a.err, tc::kErrRange);
 }
 
-// alm -> digit tiles: grid (m, parity, group), 128 threads = columns (map = c & 63,
-// Re/Im = c >> 6).  Tile (m, p, g, l-step): 128 columns x 16 l, K-major.
+// alm -> digit tiles: grid (m, parity and group, cluster), 128 threads = columns (map = c & 63,
+// Re/Im = c >> 6); each block of the cluster takes a range of l-steps.  Tile (m, p, g, l-step):
+// 128 columns x 16 l, K-major.
 struct SliceAArgs {
   const double* alm;
   int ld, k0, kc, lmax, ngroups, q0;
@@ -722,7 +723,8 @@ struct SliceAArgs {
 };
 
 __global__ void __launch_bounds__(128) k_slice_alm(SliceAArgs a) {
-  const int qi = blockIdx.x, p = blockIdx.y, g = blockIdx.z;
+  __shared__ unsigned long long s_mx[kCols];
+  const int qi = blockIdx.x, p = blockIdx.y & 1, g = blockIdx.y >> 1;
   const int m = m_of_q(a.q0 + qi, a.lmax);
   const int c = threadIdx.x;
   const int k = g * kGroupMaps + (c & 63);
@@ -731,31 +733,47 @@ __global__ void __launch_bounds__(128) k_slice_alm(SliceAArgs a) {
   const long long L1 = a.lmax + 1;
   const int cnt0 = (a.lmax - m) / 2 + 1;
   const int cnt = (p == 0) ? cnt0 : (a.lmax > m ? (a.lmax - m - 1) / 2 + 1 : 0);
-  auto val = [&](int idx) -> double {
-    if (!valid || idx >= cnt) return 0.0;
-    const int l = m + p + 2 * idx;
-    const long long row = comp == 0 ? (long long)m * L1 + l : (L1 - m) * L1 + (l - m);
-    return a.alm[row * a.ld + a.k0 + k];
+  const int nkl = (cnt0 + kKStep - 1) / kKStep;
+  const int kl0 = nkl * (int)blockIdx.z / (int)gridDim.z;
+  const int kl1 = nkl * ((int)blockIdx.z + 1) / (int)gridDim.z;
+  const double* col = a.alm + a.k0 + k +
+                      ((comp == 0 ? (long long)m * L1 + m : (L1 - m) * L1) + p) * a.ld;
+  auto load = [&](int kl, double (&v)[kKStep]) {       // an l-step's loads issued together
+#pragma unroll
+    for (int u = 0; u < kKStep; ++u) {
+      const int idx = kl * kKStep + u;
+      v[u] = valid && idx < cnt ? __ldg(&col[(long long)(2 * idx) * a.ld]) : 0.0;
+    }
   };
   // column maximum on FP64 bits with the sign cleared (integer operations, as in
   // k_slice_phase)
   unsigned long long mx = 0;
-  for (int idx = 0; idx < cnt; ++idx)
-    mx = max(mx, (unsigned long long)__double_as_longlong(val(idx)) & 0x7FFFFFFFFFFFFFFFull);
+  for (int kl = kl0; kl < kl1; ++kl) {
+    double v[kKStep];
+    load(kl, v);
+#pragma unroll
+    for (int u = 0; u < kKStep; ++u)
+      mx = max(mx, (unsigned long long)__double_as_longlong(v[u]) & 0x7FFFFFFFFFFFFFFFull);
+  }
+  s_mx[c] = mx;
+  mx = slice_cluster_max(&s_mx[c]);
   const int ef = (int)(mx >> 52);
   const int E = mx == 0 ? kEmptyExp : (ef == 0 ? -1021 : ef - 1022);
-  a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = E;
-  const int nkl = (cnt0 + kKStep - 1) / kKStep;
+  if (blockIdx.z == 0) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = E;
   unsigned char* base = a.WS +
                         ((size_t)(qi * 2 + p) * a.ngroups + g) * a.row_bytes +
                         (c >> 3) * 256 + (c & 7) * 16;
   bool bad = false;
-  for (int kl = 0; kl < nkl; ++kl) {
+  for (int kl = kl0; kl < kl1; ++kl) {
+    double v[kKStep];
+    load(kl, v);
+#pragma unroll
     for (int half = 0; half < 2; ++half) {
       uint16_t sl[kSynthPlanes][8];
+#pragma unroll
       for (int j = 0; j < 8; ++j) {
         uint16_t q4[4] = {0, 0, 0, 0};
-        if (E != kEmptyExp) bad |= tc::digits4_f(val(kl * kKStep + half * 8 + j), E, q4);
+        if (E != kEmptyExp) bad |= tc::digits4_f(v[half * 8 + j], E, q4);
         for (int d = 0; d < kSlices; ++d) sl[d][j] = q4[d];
         for (int d = 1; d < kSlices; ++d) sl[kSlices - 1 + d][j] = tc::bf16_scale_2m8(q4[d]);
       }
@@ -771,6 +789,7 @@ __global__ void __launch_bounds__(128) k_slice_alm(SliceAArgs a) {
     }
   }
   if (bad) atomicOr(a.err, tc::kErrRange);
+  slice_cluster_done();
 }
 
 // CTA = (64-map group, 128-ring block x l-chunk, q): both parities in turn through the same
@@ -1041,7 +1060,9 @@ int fsht_launch_split_slice(fsht_plan* p, int w, const double2* W, unsigned char
   sa.WS = WS;
   sa.EB = EB;
   sa.err = p->d_err;
-  k_slice_phase<<<dim3(wv[1] - wv[0], 4 * sa.ngroups), kSliceThreads, 0, s>>>(sa);
+  const dim3 grid(wv[1] - wv[0], 4 * sa.ngroups);
+  FSHT_TRY(launch_slice(k_slice_phase, grid, kSliceThreads,
+                        slice_cluster((long long)grid.x * grid.y, p->nnorth / kKStep), s, sa));
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }
@@ -1205,8 +1226,9 @@ int fsht_launch_split_slice_alm(fsht_plan* p, int w, const double* alm, unsigned
   a.WS = WS;
   a.EB = EB;
   a.err = p->d_err;
-  k_slice_alm<<<dim3(wv[1] - wv[0], 2, a.ngroups), 128, 0, s>>>(a);
-  FSHT_LAUNCH_CHECK();
+  const dim3 grid(wv[1] - wv[0], 2 * a.ngroups);
+  FSHT_TRY(launch_slice(k_slice_alm, grid, 128,
+                        slice_cluster((long long)grid.x * grid.y, wv[5]), s, a));
   return FSHT_OK;
 }
 

@@ -6,6 +6,8 @@
 #include "df64.cuh"
 #include "tcgen05.cuh"
 
+#include <cooperative_groups.h>
+
 #include <cmath>
 
 namespace {
@@ -243,5 +245,48 @@ __device__ __forceinline__ void factor_pair(double x, float& fh, float& fl) {
   fh = __double2float_rn(x);
   fl = __double2float_rn(x - (double)fh);
 }
+
+// The slicing kernels read each column twice (its maximum, then its digits) with a few loads in
+// flight per thread, so they run at the latency of memory unless many blocks share the work, and a
+// wave of a large plan holds only some sixty orders.  The blocks of a cluster (grid z) take one
+// part of the summands each and exchange the column maxima through distributed shared memory.
+// Size: enough for eight blocks an SM, while a block keeps at least four k-steps.
+inline int slice_cluster(long long blocks, int steps) {
+  int cl = 1;
+  while (cl < 8 && blocks * cl < 8 * 152 && steps >= 8 * cl) cl *= 2;
+  return cl;
+}
+template <class Args>
+int launch_slice(void (*k)(Args), dim3 grid, int threads, int cl, cudaStream_t s, const Args& a) {
+  if (cl == 1) {
+    k<<<grid, threads, 0, s>>>(a);
+    FSHT_LAUNCH_CHECK();
+    return FSHT_OK;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  grid.z = cl;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.stream = s;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = cl;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  FSHT_CUDA_TRY(cudaLaunchKernelEx(&cfg, k, a));
+  return FSHT_OK;
+}
+// The maximum over the cluster of *slot, which every thread of the block sees complete; the block
+// must not leave before slice_cluster_done.
+__device__ __forceinline__ unsigned long long slice_cluster_max(unsigned long long* slot) {
+  auto cl = cooperative_groups::this_cluster();
+  cl.sync();
+  unsigned long long mx = 0;
+  for (unsigned r = 0; r < cl.num_blocks(); ++r)
+    mx = max(mx, *cl.map_shared_rank(slot, r));
+  return mx;
+}
+__device__ __forceinline__ void slice_cluster_done() { cooperative_groups::this_cluster().sync(); }
 
 }  // namespace
