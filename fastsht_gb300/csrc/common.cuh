@@ -343,8 +343,9 @@ int fsht_launch_split_gemm(fsht_plan* p, int w, const unsigned char* WS, const i
 // Split-precision synthesis of one chunk into W = {G_N, G_S}: per wave, slice_alm cuts alm
 // into digit tiles WS / exponents EB, lambdaT writes ring-row lambda tiles, synth contracts
 // them.
+// (paired: tile columns 2 map + comp, as the spin-0 synthesis takes them; else comp * 64 + map)
 int fsht_launch_split_slice_alm(fsht_plan* p, int w, const double* alm, unsigned char* WS,
-                                int* EB, int nmaps_total, int k0, int kc, cudaStream_t s);
+                                int* EB, int nmaps_total, int k0, int kc, cudaStream_t s, bool paired);
 int fsht_launch_split_lambdaT(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s);
 // Split-precision spin-2 analysis: lambda1/lambda2 digit tiles per wave, then the E/B
 // contraction (which: bit0 E, bit1 B) against the Q and U digit tiles of k_slice_phase.

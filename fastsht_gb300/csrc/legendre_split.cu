@@ -716,6 +716,7 @@ __global__ void __launch_bounds__(128) k_lambda_digits_T(LamTArgs a) {
 struct SliceAArgs {
   const double* alm;
   int ld, k0, kc, lmax, ngroups, q0;
+  int paired;              // tile column 2 map + comp, else comp * 64 + map
   size_t row_bytes;
   unsigned char* WS;
   int* EB;
@@ -726,9 +727,9 @@ __global__ void __launch_bounds__(128) k_slice_alm(SliceAArgs a) {
   __shared__ unsigned long long s_mx[kCols];
   const int qi = blockIdx.x, p = blockIdx.y & 1, g = blockIdx.y >> 1;
   const int m = m_of_q(a.q0 + qi, a.lmax);
-  const int c = threadIdx.x;
-  const int k = g * kGroupMaps + (c & 63);
-  const int comp = c >> 6;
+  const int kl64 = threadIdx.x & 63, comp = threadIdx.x >> 6;
+  const int k = g * kGroupMaps + kl64;
+  const int c = a.paired ? 2 * kl64 + comp : (int)threadIdx.x;
   const bool valid = k < a.kc && !(comp == 1 && m == 0);
   const long long L1 = a.lmax + 1;
   const int cnt0 = (a.lmax - m) / 2 + 1;
@@ -811,6 +812,9 @@ struct SynthArgs {
 constexpr int kStagesS = 4;
 constexpr uint32_t kStageBytesS = kSlices * kATileBytes + kSynthBBytes;   // 44 KB
 constexpr int kPartStepsS = kKChunk / kKStep;
+// sixteen epilogue warps (four per TMEM lane quarter, 32 rings each), copies, two UMMA warps
+constexpr int kEpiThreadsS = 512, kEpiWarpsS = kEpiThreadsS / 32, kSRings = kSCRings / 4;
+constexpr int kThreadsS = kEpiThreadsS + 96;
 
 struct __align__(8) SynthSmemHdr {
   uint64_t full[kStagesS], empty[kStagesS], tfull, tempty, fin;
@@ -839,12 +843,13 @@ __device__ __forceinline__ SynthUnit synth_unit(const SynthArgs& a, int u) {
 
 // Persistent like k_split_gemm: one CTA per SM walks the units; per part of <= 64 l-steps
 // (1024 l keep levels 0 and 1 exact) the even-l pass then the odd-l pass run through the same
-// TMEM accumulators.  The first even pass of a unit writes G_N = G_S = E, every later pass adds
-// (+E, or +O to G_N and -O to G_S) as fire-and-forget reductions from the thread that owns the
-// element, so W needs no clearing and the result is deterministic.  Warps 0-7: epilogue (two
-// per TMEM lane quarter, one per half of the columns), warp 8 lane 0: copies, warp 9 lane 0:
-// UMMAs (13 per l-step: levels 0-3 and the level-4 fold).
-__global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
+// TMEM accumulators, which leave no slots for the next pass's products: the epilogue's time adds to
+// theirs.  So sixteen warps (32 sums a thread) drain, the even sum E stays in registers instead of
+// going through W, and a map's two lanes write {N re, N im} and {S re, S im} as one whole 32-byte
+// entry (8-byte stores of one component each touched every sector four times):
+// 4.29 -> 2.55 ms at nside 512, lmax 1023, 64 maps.
+// Warp 16 lane 0: copies, warps 17 and 18: UMMAs (13 per l-step: levels 0-3 and the level-4 fold).
+__global__ void __launch_bounds__(kThreadsS, 1) k_split_synth(SynthArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ SynthSmemHdr h;
   __shared__ UnitQueue uq;
@@ -858,9 +863,9 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
       tc::mbar_init(&h.empty[s], 2);                       // both UMMA warps
     }
     tc::mbar_init(&h.tfull, 2);
-    tc::mbar_init(&h.tempty, kEpiWarps);
+    tc::mbar_init(&h.tempty, kEpiWarpsS);
     tc::mbar_init(&h.fin, 2);
-    uq_init(uq, kEpiWarps + 2);
+    uq_init(uq, kEpiWarpsS + 2);
     h.abort = 0;
     tc::mbar_fence_init();
   }
@@ -871,7 +876,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
   const uint32_t tmem = h.tmem;
 
   uint32_t n_loaded = 0;
-  if (tid == kEpiThreads) {
+  if (tid == kEpiThreadsS) {
     uint32_t i = 0;
     uq_walk(uq, a.nunits, 0, abort, [&](int u) -> bool {
       const SynthUnit w = synth_unit(a, u);
@@ -899,10 +904,10 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
       }
       return true;
     });
-  } else if (warp > kEpiWarps) {
+  } else if (warp > kEpiWarpsS) {
     // UMMA warps: lambda tiles (rings) as the second operand, alm tiles as the first, so that the
     // map columns are on the TMEM lanes
-    const int side = warp - kEpiWarps - 1;
+    const int side = warp - kEpiWarpsS - 1;
     const uint32_t idesc = tc::umma_idesc_bf16(kRows, kCols);
     const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
     const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
@@ -939,22 +944,24 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
         }
       }
     }
-  } else if (tid < kEpiThreads) {
-    // Each warp works alone: TMEM lane = map column (its quarter), half of the rings.  The even
-    // sum E waits in the north slot, the odd one is added and subtracted by the same thread.
+  } else if (tid < kEpiThreadsS) {
+    // Each warp works alone: TMEM lane = column (2 map + comp) of its quarter, 32 of the rings.  The
+    // even sum E stays in registers until the odd one is there; the two lanes of a map exchange
+    // halves, so that one holds {N re, N im} and the other {S re, S im} and a warp stores whole
+    // 32-byte entries.
     const int lane = tid & 31;
-    const int c = ((warp & 3) << 5) + lane;            // column: comp * 64 + map
-    const int comp = c >> 6;
-    const int rbeg = (warp >> 2) * (kCols / 2);
+    const int c = ((warp & 3) << 5) + lane;
+    const int comp = c & 1;
+    const int rbeg = (warp >> 2) * kSRings;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) << 5) << 16) + rbeg;
-    const long long rs = (long long)a.kc * 4;          // doubles from ring to ring
+    const long long rs = (long long)a.kc * 2;          // double2 from ring to ring
     uint32_t np = 0;
     for (uint32_t n = 0;; ++n) {
       const int u = uq_take(uq, n, abort);
       if (u < 0) break;
       const SynthUnit w = synth_unit(a, u);
       if (w.nkl == 0) continue;
-      const int k = w.g * kGroupMaps + (c & 63);
+      const int k = w.g * kGroupMaps + (c >> 1);
       const bool ok_col = k < a.kc;
       int ce[2];
 #pragma unroll
@@ -962,64 +969,61 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth(SynthArgs a) {
         const int e = a.EB[(((long long)w.qi * 2 + pp) * a.ngroups + w.g) * kCols + c];
         ce[pp] = (e == kEmptyExp) ? kEmptyExp : a.eag + e - 12;
       }
-      const int nrow = min(kCols / 2, w.K - w.rb * kSCRings - rbeg);
-      double* base = a.W +
-                     (((long long)w.m * a.nnorth + w.i0 + w.rb * kSCRings + rbeg) * a.kc +
-                      (ok_col ? k : 0)) * 4 + comp;
+      const int nrow = min(kSRings, w.K - w.rb * kSCRings - rbeg);
+      double2* base = reinterpret_cast<double2*>(a.W) +
+                      (((long long)w.m * a.nnorth + w.i0 + w.rb * kSCRings + rbeg) * a.kc +
+                       (ok_col ? k : 0)) * 2 + comp;   // the N (even lane) or S (odd lane) half
       for (int kl0 = 0; kl0 < w.nkl; kl0 += kPartStepsS) {
-#pragma unroll 1
-        for (int par = 0; par < 2; ++par) {
+        double ev[kSRings];
+        // walks the tile's rings in steps of four: the level sums of a ring, and the slots
+        // handed back after the last load
+        auto sums = [&](int cexp, auto put) {
           const bool ok = tc::mbar_wait_warp(&h.tfull, np & 1, abort);
           ++np;
-          if (!ok) continue;
+          if (!ok) return;
           tc::tc_fence_after();
-          // mode 0: E stored in the north slot; 1: E read back, N = E + O, S = E - O; 2: a later
-          // part added to both
-          const int mode = kl0 > 0 ? 2 : par;
-          const int cexp = par ? ce[1] : ce[0];
 #pragma unroll
-          for (int c0 = 0; c0 < kCols / 2; c0 += 16) {
-            uint32_t v0[16], v1[16], v2[16], v3[16];
-            tc::tmem_ld16(lane_base + 0 * kCols + c0, v0);
-            tc::tmem_ld16(lane_base + 1 * kCols + c0, v1);
-            tc::tmem_ld16(lane_base + 2 * kCols + c0, v2);
-            tc::tmem_ld16(lane_base + 3 * kCols + c0, v3);
+          for (int c0 = 0; c0 < kSRings; c0 += 4) {
+            uint32_t v0[4], v1[4], v2[4], v3[4];
+            tc::tmem_ld4(lane_base + 0 * kCols + c0, v0);
+            tc::tmem_ld4(lane_base + 1 * kCols + c0, v1);
+            tc::tmem_ld4(lane_base + 2 * kCols + c0, v2);
+            tc::tmem_ld4(lane_base + 3 * kCols + c0, v3);
             tc::tmem_wait_ld();
-            if (c0 == kCols / 2 - 16) {
+            if (c0 == kSRings - 4) {
               tc::tc_fence_before();
               tc::mbar_arrive_warp(&h.tempty);
             }
-            if (!ok_col) continue;
-            double* d = base + (long long)c0 * rs;
-            double n0[16], s0[16];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              const bool in = c0 + j < nrow;
-              n0[j] = mode > 0 && in ? d[j * rs] : 0.0;
-              s0[j] = mode == 2 && in ? d[j * rs + 2] : n0[j];
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (c0 + j >= nrow) continue;
-              const double v = levels_scaled(v0[j], v1[j], v2[j], v3[j], 1.f, 0.f, cexp);
-              if (mode == 0) {
-                d[j * rs] = v;
-              } else {
-                d[j * rs] = n0[j] + v;
-                d[j * rs + 2] = par ? s0[j] - v : s0[j] + v;
-              }
-            }
+            for (int j = 0; j < 4; ++j)
+              put(c0 + j, levels_scaled(v0[j], v1[j], v2[j], v3[j], 1.f, 0.f, cexp));
           }
-        }
+        };
+        sums(ce[0], [&](int j, double v) { ev[j] = v; });
+        sums(ce[1], [&](int j, double v) {
+          double n = ev[j], s = ev[j];
+          double2* d = base + (long long)j * rs;
+          const bool in = ok_col && j < nrow;
+          if (kl0 > 0) {                               // a later part (lmax > 2047): adds
+            const double2 x = in ? *d : make_double2(0.0, 0.0);
+            const double o = __shfl_xor_sync(0xffffffffu, comp ? x.x : x.y, 1);
+            n += comp ? o : x.x;
+            s += comp ? x.y : o;
+          }
+          n += v;
+          s -= v;
+          const double o = __shfl_xor_sync(0xffffffffu, comp ? n : s, 1);
+          if (in) *d = comp ? make_double2(o, s) : make_double2(n, o);
+        });
       }
     }
   }
-  if (warp > kEpiWarps) {
+  if (warp > kEpiWarpsS) {
     tc::umma_commit_warp(&h.fin);
     for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
       if (tc::mbar_try_wait(&h.fin, 0)) break;
   }
-  if (tid == kEpiThreads) {
+  if (tid == kEpiThreadsS) {
     for (uint32_t d = 0; d < (uint32_t)kStagesS && d < n_loaded; ++d) {
       const uint32_t i = n_loaded - 1 - d;
       for (uint32_t it = 0; it < tc::kWaitLimit; ++it)
@@ -1212,7 +1216,7 @@ int fsht_launch_split_gemm(fsht_plan* p, int w, const unsigned char* WS, const i
 }
 
 int fsht_launch_split_slice_alm(fsht_plan* p, int w, const double* alm, unsigned char* WS,
-                                int* EB, int nmaps_total, int k0, int kc, cudaStream_t s) {
+                                int* EB, int nmaps_total, int k0, int kc, cudaStream_t s, bool paired) {
   const int* wv = p->h_waves + kWaveInts * w;
   SliceAArgs a;
   a.alm = alm;
@@ -1223,6 +1227,7 @@ int fsht_launch_split_slice_alm(fsht_plan* p, int w, const double* alm, unsigned
   a.ngroups = (kc + kGroupMaps - 1) / kGroupMaps;
   a.q0 = wv[0];
   a.row_bytes = ws_row_bytes(p->lmax, p->nnorth);
+  a.paired = paired;
   a.WS = WS;
   a.EB = EB;
   a.err = p->d_err;
@@ -1277,7 +1282,7 @@ int fsht_launch_split_synth(fsht_plan* p, int w, const unsigned char* WS, const 
   a.err = p->d_err;
   const size_t sm = (size_t)kStagesS * kStageBytesS;
   FSHT_TRY(fsht_smem_limit((const void*)k_split_synth, (size_t)(sm)));
-  if (a.nunits > 0) k_split_synth<<<a.nunits, kThreadsG, sm, s>>>(a);
+  if (a.nunits > 0) k_split_synth<<<a.nunits, kThreadsS, sm, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }

@@ -891,7 +891,7 @@ static int split_synthesis(fsht_plan* p, const double* alm, double2* W, int nmap
     {
       FSHT_PROF(FSHT_KCAT_SLICE);
       FSHT_TRY(fsht_launch_split_slice_alm(p, w, alm, p->d_ws, p->d_eb, nmaps, c0, kc,
-                                           p->stream));
+                                           p->stream, true));
     }
     unsigned char* lb = nullptr;
     FSHT_TRY(lam_ready(p, fsht_launch_split_lambdaT, w, &lb));
@@ -1321,8 +1321,10 @@ static int pol_synthesis(fsht_plan* p, const double* almE, const double* almB, d
   for (int w = 0; w < p->nwaves; ++w) {
     {
       FSHT_PROF(FSHT_KCAT_SLICE);
-      FSHT_TRY(fsht_launch_split_slice_alm(p, w, almE, wse, ebe, nmaps, c0, kc, p->stream));
-      FSHT_TRY(fsht_launch_split_slice_alm(p, w, almB, wsb, ebb, nmaps, c0, kc, p->stream));
+      FSHT_TRY(fsht_launch_split_slice_alm(p, w, almE, wse, ebe, nmaps, c0, kc, p->stream,
+                                           false));
+      FSHT_TRY(fsht_launch_split_slice_alm(p, w, almB, wsb, ebb, nmaps, c0, kc, p->stream,
+                                           false));
     }
     unsigned char* lb = nullptr;
     FSHT_TRY(lam_ready(p, fsht_launch_split_lambdaT_pol, w, &lb));
