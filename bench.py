@@ -597,7 +597,8 @@ def ours(args, rank, world, local):
                                  "frac": dp / (peak64.value * 1e12 / 2),
                                  "note": "FP64 instructions executed (radix passes, Bluestein "
                                          "chirps and filter; an FMA counts once) over the DFMA "
-                                         "instruction rate measured in this run"}
+                                         "instruction rate measured in this run; the rings "
+                                         "that take the matrix form are counted as FFTs"}
     ana_tf = fl_step * args.steps / (ana_ms / 1000.0) / 1e12 if ana_ms > 0 else None
     traffic = None          # bytes per chunk of maps (all of its launches)
     tf = ROOT / "profiles" / "traffic.json"
@@ -634,14 +635,19 @@ def ours(args, rank, world, local):
                              "(executed_*); one chunk of maps is several wave launches, traffic "
                              "is per chunk")}
     else:
-        roof_ana = {"bound": "fp64", "kernel": "k_analysis_fp64<0>", "achieved": ana_tf,
-                    "peak": peak64.value, "unit": "TFLOP/s",
-                    "frac": ana_tf / peak64.value if ana_tf else None,
-                    "peak_source": ("DFMA loop measured by bench.py on this GPU "
-                                    "(fsht_measure_fp64_peak); MEASURED_PEAKS.json holds HBM "
-                                    "and BF16 figures only"),
-                    "algorithmic_flop_per_launch": flop_per_map(nside, lmax) * kchunk,
-                    "traffic": traffic}
+        bf = peaks.get("bf16_tflops", 1900.0)
+        ex_tf = 36 * ana_tf if ana_tf else None
+        roof_ana = {"bound": "tensor", "kernel": "k_tc_gemm<0> (tcgen05 BF16 digit UMMAs)",
+                    "achieved": ana_tf, "peak": bf, "unit": "TFLOP/s",
+                    "frac": ana_tf / bf if ana_tf else None,
+                    "peak_source": ("MEASURED_PEAKS.json bf16_tflops (measured)"
+                                    if "bf16_tflops" in peaks else "fallback 1900 TFLOP/s"),
+                    "algorithmic_flop_per_chunk": flop_per_map(nside, lmax) * kchunk,
+                    "executed_tensor_tflops": ex_tf,
+                    "executed_frac": ex_tf / bf if ex_tf else None,
+                    "traffic": traffic,
+                    "note": ("achieved counts algorithmic FLOP; the kernel executes 36 BF16 digit "
+                             "products per algorithmic FMA (executed_*)")}
     if names[top] == "ring_fft_fwd" and fft_ms > 0:
         # The dominant kernel against the measured HBM copy rate (MEASURED_PEAKS.json): its
         # algorithmic bytes are the maps read and the phase matrix written, 16 npix per map.

@@ -16,6 +16,11 @@
 // "safe start" tables, plm_table/*.bin); while e < 0 the true value is below
 // 2^-300 and the tile gets 0.
 //
+// From nside 32 on the contraction runs as digit products on the tensor cores
+// (legendre_fp64_tc.cu).  These kernels serve smaller plans, plans and jobs whose
+// workspace has no room for digit tiles, and the (order, 64-map group) pairs whose
+// values the digits cannot hold (flags).
+//
 // FP64 on GB300 runs at ~1.2 TFLOP/s (DFMA) and its DMMA (mma.sync f64) is no
 // faster, so these kernels are plain register-tiled DFMA: every thread keeps an
 // accumulator tile in registers and reads shared-memory tiles laid out so that a

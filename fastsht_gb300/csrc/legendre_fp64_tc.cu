@@ -20,9 +20,10 @@
 //
 // Per wave of orders:
 //   k_tc_slice      {S, D} phases -> digit tiles and column exponents       (HBM bound)
-//   k_tc_lambda     FP64 recursion -> lambda digit tiles, once for all maps (FP64 pipe)
-//   k_tc_gemm       persistent tcgen05 contraction                          (tensor pipe)
+//   k_tc_lambda     FP64 recursion -> lambda digit tiles, once for all maps (FP64 pipe, 79 %)
+//   k_tc_gemm       persistent tcgen05 contraction         (shared-memory and L2 bandwidth)
 // and for the synthesis k_tc_slice_alm, k_tc_lambda_T and k_tc_gemm<1, *>.
+// nside 512, lmax 1023, 64 maps, each alone: 1.23, 2.8 and 3.7 ms, where the FMA kernel needs 134 at 82 % of the DFMA rate.
 #include "legendre_rec.cuh"
 #include "split_common.cuh"
 
@@ -548,8 +549,8 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
 }
 
 // ------------------------------------------------------------------ alm -> digits
-// grid (q in wave, group), 256 threads per field = (half of the l steps, comp, map): v = a_lm Dm
-// 2^EA(l), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an exponent per
+// grid (q in wave, group, cluster), 256 threads per field = (half of the block's l steps, comp,
+// map): v = a_lm Dm 2^EA(l), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an exponent per
 // column; E/B (NF = 2): one per map and order, plain and i v copies.
 struct TcSliceAArgs {
   const double* alm[2];
@@ -671,9 +672,10 @@ __global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
 // even and odd r and cos and sin take one sign pattern each: four q x q products (s = 0: up to
 // q + 1) instead of one n x n, 8 q^2 flop per real ring.  Bins r <= n/2 serve every order
 // a n +- r, by (-1)^{a s} and a conjugate.  As digit products that is 0.12 ms per map for all
-// cap rings of nside 1024 at the tensor rate, where Bluestein transforms on the FP64 pipe (two
-// FFTs of 2 n points or more per ring) took 0.90 ms.  The belt's power-of-two rings cost q^2
-// too, and from nside 512 on the FFT is the cheaper form there (kDftBeltMax).
+// cap rings of nside 1024 at the tensor rate, and 0.25 measured in tiles of 64 maps (matrices and
+// slices included), where Bluestein transforms on the FP64 pipe (two FFTs of 2 n points or more per
+// ring) took 0.90 ms.  The belt's power-of-two rings cost q^2 too, and from nside 512 on the FFT is
+// the cheaper form there (kDftBeltMax).
 // Types: 0 cos r even, 1 cos r odd, 2 sin r even (from 2), 3 sin r odd; row rho of a type is
 // r = 2 rho + {0, 1, 2, 1}.
 __device__ __forceinline__ int dft_r(int type, int rho) {
@@ -937,18 +939,23 @@ __global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
 }
 
 // ------------------------------------------------------------------ contraction
-// Persistent, one CTA per SM, units from the queue of split_common.cuh.  A unit is a 128-column (64 maps x Re/Im, the UMMA M side = TMEM
-// lanes) x N-row tile: N <= 128 l-rows of one parity (DIR 0, analysis) or rings (DIR 1,
-// synthesis), over one or two phases of one or two segments:
+// Persistent, one CTA per SM, units from the queue of split_common.cuh.  A unit is a 128-column
+// (64 maps x Re/Im, the UMMA M side = TMEM lanes) x N-row tile: N <= 128 l-rows of one parity
+// (DIR 0, analysis) or rings (DIR 1, synthesis), over one or two phases of one or two segments:
 //   DIR 0          one phase;  spin 2: lambda1 against the field, lambda2 against i x the other
 //   DIR 1          phase 0 gives A, phase 1 gives B', north = A + B', south = A - B':
 //                  T: even l, then odd l; Q/U: (lambda1 even, lambda2 odd), then (lambda1 odd,
 //                  lambda2 even), since lambda1 keeps (-1)^(l-m) and lambda2 takes the opposite
-// Each part of <= 12 k-steps runs two passes through the four 128-column TMEM accumulators:
-// levels 0..3 (digit planes 0..3) and levels 4..7 (all planes).  A level's accumulator is drained
-// into the 64-bit integers as soon as its last product is done, while the products of the other
-// levels still run, and is handed back alone: the four slots have their own barriers.
-// One lane copies (16 KB of each operand per stage), two warps issue the UMMAs.
+//   DIR 2, 3       ring transforms, forward and inverse (below)
+// Each part of <= kPartK k-steps runs two passes through the four 128-column TMEM accumulators:
+// levels 0..3 (digit planes 0..3) and levels 4..7 (all planes).  The slots form two pairs, each
+// with a UMMA warp and barriers of its own: pair 0 finishes its smaller share first and is drained
+// into the 64-bit integers while the products of pair 1 still run (without the drains the analysis
+// took 6.21 Mcycles an SM instead of 6.34).  Shorter parts cost more passes: 11 k-steps 5 % more,
+// 8 k-steps 11 %.  One lane copies (16 KB of each operand per stage).
+// What bounds it (nside 512, lmax 1023, 64 maps): shared memory, 328 KB a k-step at 128 bytes a
+// clock = 2624 clocks against 2304 on the tensor pipe, and the copies, 96 KB a k-step (8.4 TB/s
+// over all SMs, about half of it from HBM at 55 % of its rate); tensor pipe 64 % active.
 // The map columns are on the lanes, so a warp's alm stores are two 128-byte segments and its
 // phase-matrix stores whole {Re, Im} pairs, with no staging through shared memory.
 // Sixteen epilogue warps (four per TMEM lane quarter, one per 32 accumulator columns: 32 64-bit

@@ -401,8 +401,11 @@ __global__ void __launch_bounds__(32 * kResBins) k_fourier_residual(ResArgs a) {
 
 // ------------------------------------------------------------------ ring skip
 // kept(i, m): max_{m <= l <= lcap} |lambda_lm(theta_i)| >= 1e-20, evaluated with the
-// exponent-rescaled recursion (values carried as v * 2^(600 e), e <= 0).
+// exponent-rescaled recursion (values carried as v * 2^(600 e), e <= 0), a ring per lane.  The
+// coefficients depend on (l, m) only: each lane computes those of one l of 32 and the warp shares
+// them (a thread with its own divisions and square roots per step spent its time on those).
 __device__ bool ring_kept(double c, double s, double pref, int m, int lcap) {
+  const int lane = threadIdx.x & 31;
   int ex;
   double mt = frexp(s, &ex);
   double rm = 1.0, bm = mt;
@@ -415,36 +418,45 @@ __device__ bool ring_kept(double c, double s, double pref, int m, int lcap) {
   { int t; rm = frexp(rm, &t); re += t; }
   int e = (re >= -300) ? 0 : (int)floor((double)(re + 300) / 600.0);
   double cur = ldexp(rm, (int)(re - 600LL * e)), prev = 0.0;
-  if (e == 0 && fabs(cur) >= 1e-20) return true;
+  bool kept = e == 0 && fabs(cur) >= 1e-20;
   const double mm = (double)m * (double)m;
-  for (int l = m + 1; l <= lcap; ++l) {
-    const double dl = (double)l;
-    const double al = sqrt((4.0 * dl * dl - 1.0) / (dl * dl - mm));
-    const double bl = sqrt(((dl - 1.0) * (dl - 1.0) - mm) / ((2.0 * dl - 3.0) * (2.0 * dl - 1.0))) * al;
-    const double nx = al * c * cur - bl * prev;
-    prev = cur;
-    cur = nx;
-    if (e < 0 && fabs(cur) > 0x1p300) { cur *= 0x1p-600; prev *= 0x1p-600; ++e; }
-    if (e == 0 && fabs(cur) >= 1e-20) return true;
+  for (int l0 = m + 1; l0 <= lcap; l0 += 32) {
+    if (__all_sync(0xffffffffu, kept)) break;
+    const double dl = (double)(l0 + lane);
+    const double a32 = sqrt((4.0 * dl * dl - 1.0) / (dl * dl - mm));
+    const double b32 =
+        sqrt(((dl - 1.0) * (dl - 1.0) - mm) / ((2.0 * dl - 3.0) * (2.0 * dl - 1.0))) * a32;
+    const int n = min(32, lcap - l0 + 1);
+    for (int t = 0; t < n; ++t) {
+      const double al = __shfl_sync(0xffffffffu, a32, t), bl = __shfl_sync(0xffffffffu, b32, t);
+      const double nx = al * c * cur - bl * prev;
+      prev = cur;
+      cur = nx;
+      if (e < 0 && fabs(cur) > 0x1p300) { cur *= 0x1p-600; prev *= 0x1p-600; ++e; }
+      kept |= e == 0 && fabs(cur) >= 1e-20;
+    }
   }
-  return false;
+  return kept;
 }
 
 // i0(m) = first north ring kept for order m (the rule the reference's
 // SHT_ring_skip_table/<nside>.bin follows).  max_l |lambda_lm| grows toward the
-// equator, so a binary search over rings suffices; thread per m.  The host makes
-// the result non-decreasing in m.
+// equator, so a search over rings suffices; a warp per m, 32 rings a round (three rounds at nside
+// 1024, where one thread's binary search took eleven: 52 ms of the plan's creation).  The host
+// makes the result non-decreasing in m.
 __global__ void k_ring_first_kept(const double* cth, const double* sth, const double* pref,
                                   int nnorth, int lcap, int mmax, int* first) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  const int m = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (m > mmax) return;
   int lo = 0, hi = nnorth - 1;     // the equator ring is always kept for m <= lcap
   while (lo < hi) {
-    const int mid = (lo + hi) >> 1;
-    if (ring_kept(cth[mid], sth[mid], pref[m], m, lcap)) hi = mid;
-    else lo = mid + 1;
+    const int n = hi - lo, r = lo + n * lane / 32;
+    const unsigned k = __ballot_sync(0xffffffffu, ring_kept(cth[r], sth[r], pref[m], m, lcap));
+    const int f = k ? __ffs(k) - 1 : 32;             // the first probe that is kept
+    if (f < 32) hi = lo + n * f / 32;
+    if (f > 0) lo += n * (f - 1) / 32 + 1;
   }
-  first[m] = lo;
+  if (lane == 0) first[m] = lo;
 }
 
 int maps_per_block_for(int kc, int nrings_launched) {
@@ -606,7 +618,7 @@ int fsht_launch_ring_skip(fsht_plan* p, cudaStream_t s) {
   const int lcap = (4 * p->nside > p->lmax) ? 4 * p->nside : p->lmax;
   int* d_first = nullptr;
   FSHT_CUDA_TRY(cudaMalloc(&d_first, sizeof(int) * (p->lmax + 1)));
-  k_ring_first_kept<<<(p->lmax + 1 + 63) / 64, 64, 0, s>>>(p->d_cth, p->d_sth, p->d_pref,
+  k_ring_first_kept<<<(p->lmax + 1 + 3) / 4, 128, 0, s>>>(p->d_cth, p->d_sth, p->d_pref,
                                                              p->nnorth, lcap, p->lmax, d_first);
   FSHT_LAUNCH_CHECK();
   FSHT_CUDA_TRY(cudaMemcpyAsync(p->h_ring_i0, d_first, sizeof(int) * (p->lmax + 1),

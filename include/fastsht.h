@@ -55,12 +55,16 @@ enum { FSHT_FLAG_POL = 1, FSHT_FLAG_ITER = 2, FSHT_FLAG_TABLES_ONLY = 4 };
  *   nmaps_max  largest nmaps a transform call on this plan will pass
  *   flags      FSHT_FLAG_POL for spin-2 (Q/U) transforms, FSHT_FLAG_ITER for
  *              niter > 0 (each doubles the workspace, like the reference's nbuff)
- *   precision  FSHT_PREC_FP64 (plain, all FP64) or FSHT_PREC_SPLIT (the Legendre
+ *   precision  FSHT_PREC_FP64 (plain: FP64 accuracy; from nside 32 on the Legendre
+ *              contractions and, for enough maps, the ring transforms run as exact products
+ *              of 62-bit fixed-point digits on the tensor cores where the workspace has room
+ *              for the digit tiles, else as FP64 FMAs and FFTs) or FSHT_PREC_SPLIT (the Legendre
  *              contractions of t2alm, alm2t, qu2eb / qu2e / qu2b and eb2qu as BF16 slice
  *              products on the tensor cores, the ring FFTs of t2alm in df64; max relative
  *              alm error ~1e-9..3e-8 against FP64)
- *   workspace_limit_bytes  upper bound for the plan's workspace (0 = default 16 GiB,
- *              40 GiB for FSHT_PREC_SPLIT); maps are processed in chunks that fit.
+ *   workspace_limit_bytes  upper bound for the plan's workspace, digit tiles included
+ *              (0 = default 16 GiB, 80 GiB for FSHT_PREC_SPLIT); maps are processed in chunks
+ *              that fit, of whole 64-map groups where a chunk is that large.
  *   stream     cudaStream_t (NULL = legacy default stream) */
 int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precision,
                      size_t workspace_limit_bytes, void* stream, fsht_plan** plan);
