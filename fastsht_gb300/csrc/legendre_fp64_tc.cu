@@ -201,9 +201,12 @@ __global__ void __launch_bounds__(kTabThreads) k_tc_table(int lmax, FshtLamRow* 
     r.erow = ilogb(bound / dm) + 1 - r.dx;
     tab[base + j] = r;
     if (!tab2) continue;
-    r.dm = 1.0;
-    r.dx = 0;
-    r.erow = ilogb(bound) + 1;
+    // spin 2: the normalisation N_l of lambda1 and lambda2 = Dm 2^Dx stays out of the tiles too
+    // (zero below l = 2)
+    const double nl = normal_l((int)L);
+    r.dx = nl > 0.0 ? ilogb(nl) : 0;
+    r.dm = nl > 0.0 ? ldexp(nl, -r.dx) : 1.0;
+    r.erow = ilogb(bound / r.dm) + 1 - r.dx;
     tab2[base + j] = r;
     FshtPolRow c{0.0, 0.0, 0.0, 0.0};
     if (j > 0) {
@@ -212,7 +215,7 @@ __global__ void __launch_bounds__(kTabThreads) k_tc_table(int lmax, FshtLamRow* 
       c.c2 = rc.b;
     }
     c.c3 = lam_fact((int)L, m);
-    c.c4 = normal_l((int)L);
+    c.c4 = nl;
     ptab[base + j] = c;
   }
 }
@@ -364,7 +367,7 @@ __device__ __forceinline__ void tc_step(TcRing& r, double beta) {
 }
 
 // The values of step j (l = m + j) as biased fixed point against the row exponent (k: 62 minus
-// it, plus Dx for spin 0).
+// it, plus Dx).
 template <int SPIN>
 __device__ __forceinline__ void tc_value(TcRing& r, int j, double beta, const FshtPolRow& c,
                                          const PolL& pl, int k, unsigned long long& y1,
@@ -372,9 +375,10 @@ __device__ __forceinline__ void tc_value(TcRing& r, int j, double beta, const Fs
   if (SPIN == 2) {
     if (j > 0) rec_step(r.s1, r.s2, r.et, c.c1 * r.x, c.c2);
     y1 = y2 = kBias;
-    if (r.et != 0) return;
+    if (r.et != 0 || __double2hiint(c.c4) == 0) return;
+    // N_l is in the row factor: ten FP64 operations a step instead of twelve
     double l1, l2;
-    pol_lambda(r.pol, pl, r.s1, r.s2, c.c3, c.c4, l1, l2);
+    pol_lambda_raw(r.pol, pl, r.s1, r.s2, c.c3, l1, l2);
     y1 = fixed_biased(l1, k);
     y2 = fixed_biased(l2, k);
   } else {

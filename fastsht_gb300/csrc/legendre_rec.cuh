@@ -69,5 +69,16 @@ __device__ __forceinline__ void pol_lambda(const PolRing& r, const PolL& p, doub
     l2 = (prev * lf - cur * (2.0 * r.cth * p.l1)) * r.c_w * nl;
   }
 }
+// The same without the factor N_l.
+__device__ __forceinline__ void pol_lambda_raw(const PolRing& r, const PolL& p, double cur,
+                                               double prev, double lf, double& l1, double& l2) {
+  if (p.diag) {
+    l1 = p.nm * cur * r.diag1;
+    l2 = p.nm * cur * r.diag2;
+  } else {
+    l1 = prev * lf * r.b_w - cur * (r.two_on_s2 * p.lm + p.ll);
+    l2 = (prev * lf - cur * (2.0 * r.cth * p.l1)) * r.c_w;
+  }
+}
 
 }  // namespace
