@@ -8,9 +8,9 @@
 // one accumulator per level: over the 256 summands of a part the sums of levels 0..4 stay
 // within 2^24 whatever the digits are (level s >= 1: 256 (2 2^13 + (s - 1) 2^14)), so they are
 // exact integers; levels 5..7 carry weights from 2^-40 of the leading product down, where an
-// FP32 rounding is far below FP64's.  The epilogue adds every level into one 64-bit integer per output element
-// (unit 2^-unit_bits), so no FP64 instruction runs before the last conversion and the order of
-// the parts does not matter.
+// FP32 rounding is far below FP64's.  The epilogue adds every level into one 64-bit integer per
+// output element (unit 2^-unit_bits), so no FP64 instruction runs before the last conversion and
+// the order of the parts does not matter.
 //
 // What the fixed point costs: the dropped levels (8 and up) and the unit are below 2^-44 of
 // the largest operand pair.  Against long-double sums (white, smooth and constant columns,
@@ -23,7 +23,8 @@
 //   k_tc_lambda     FP64 recursion -> lambda digit tiles, once for all maps (FP64 pipe, 79 %)
 //   k_tc_gemm       persistent tcgen05 contraction         (shared-memory and L2 bandwidth)
 // and for the synthesis k_tc_slice_alm, k_tc_lambda_T and k_tc_gemm<1, *>.
-// nside 512, lmax 1023, 64 maps, each alone: 1.23, 2.8 and 3.7 ms, where the FMA kernel needs 134 at 82 % of the DFMA rate.
+// nside 512, lmax 1023, 64 maps, each alone: 1.23, 2.8 and 3.7 ms, where the FMA kernel needs 134
+// at 82 % of the DFMA rate.
 #include "legendre_rec.cuh"
 #include "split_common.cuh"
 
@@ -554,8 +555,8 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
 
 // ------------------------------------------------------------------ alm -> digits
 // grid (q in wave, group, cluster), 256 threads per field = (half of the block's l steps, comp,
-// map): v = a_lm Dm 2^EA(l), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an exponent per
-// column; E/B (NF = 2): one per map and order, plain and i v copies.
+// map): v = a_lm Dm 2^EA(l), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an
+// exponent per column; E/B (NF = 2): one per map and order, plain and i v copies.
 struct TcSliceAArgs {
   const double* alm[2];
   int ld, k0, kc, lmax, ngroups, q0;
@@ -1562,7 +1563,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
             pair(std::integral_constant<int, 3>{});
             ++use;
             const int b = a.unit_bits;
-            bias += ((unsigned long long)kBias2 << (b - 8)) + ((unsigned long long)kBias2 << (b - 24)) +
+            bias += ((unsigned long long)kBias2 << (b - 8)) +
+                    ((unsigned long long)kBias2 << (b - 24)) +
                     ((unsigned long long)kBias2 << (b - 40)) + kMagic;
           }
         }
@@ -1580,8 +1582,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_tc_gemm(TcGemmArgs a) {
           for (int j = 0; j < kOut; ++j) sum[j] = (long long)(acc[j] - bias);
 #pragma unroll
           for (int j = 0; j + kOut < kTcAcc; ++j) acc[j] = acc[j + kOut];
-          tc_out<DIR, SPIN, kOut>(a, w, ph, store, c, rbeg + c0, min(kOut, nrow - c0), map, eb, e, sum,
-                                  &s_fac[warp][c0]);
+          tc_out<DIR, SPIN, kOut>(a, w, ph, store, c, rbeg + c0, min(kOut, nrow - c0), map, eb, e,
+                                  sum, &s_fac[warp][c0]);
         }
       }
     }
@@ -1878,7 +1880,8 @@ int fsht_dft_tables_init(fsht_plan* p) {
   // the staging buffer holds at least the largest ring's matrices, and all of a small plan's
   const long long unit = kStepBytes;
   const long long nkm = (ns + 16) / 16, nrm = (ns + 128) / 128;
-  const long long want = std::max<long long>(4 * nkm * nrm, std::min<long long>(2048, 2LL * ns * ns / 16));
+  const long long want =
+      std::max<long long>(4 * nkm * nrm, std::min<long long>(2048, 2LL * ns * ns / 16));
   p->lbuf_bytes = std::max<size_t>(p->lbuf_bytes, (size_t)(want * unit));
   const long long cap_t = (long long)(p->lbuf_bytes / unit);
   const long long cap_c = (long long)(fsht_tc_ws_bytes(p, 1, 1) / unit);

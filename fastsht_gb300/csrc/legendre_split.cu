@@ -318,15 +318,15 @@ __global__ void __launch_bounds__(128) k_lambda_digits(LamArgs a) {
 }
 
 // ------------------------------------------------------------------ split GEMM
-// Persistent: one CTA per SM walks the wave's work units u = blockIdx.x, + gridDim.x, ...;
+// Persistent: one CTA per SM takes the wave's work units from the queue of split_common.cuh;
 // a unit is (q, parity, l-tile, 64-map group), the group fastest, so CTAs running at the same
 // time share lambda tiles in L2.  A unit is one 128-row x 128-column output tile over all of
 // its k-steps of 16 rings, accumulated in parts of <= 64 k-steps (1024 rings keep levels 0
 // and 1 exact in FP32): the first part's epilogue stores, later parts add as fire-and-forget
-// reductions (one thread owns each element, so the result is deterministic).  Warp 8 lane 0 streams lambda and P digit tiles (bulk async copies) through a
-// kStagesG-deep ring that runs on across parts and units, so the next tiles load while an
-// epilogue drains the accumulators; warp 9 lane 0 issues the ten level-ordered UMMAs per
-// k-step; warps 0-7 run the epilogue.  TMEM (four 128-column level accumulators) is
+// reductions (one thread owns each element, so the result is deterministic).  Warp 8 lane 0
+// streams lambda and P digit tiles (bulk async copies) through a kStagesG-deep ring that runs on
+// across parts and units, so the next tiles load while an epilogue drains the accumulators; warps 9
+// and 10 issue the ten UMMAs of a k-step, two levels each; warps 0-7 run the epilogue.  TMEM (four 128-column level accumulators) is
 // allocated once per CTA; tfull / tempty hand it between the UMMA issuer and the epilogue for
 // every part.
 constexpr int kStagesG = 6;
@@ -458,8 +458,8 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm(GemmArgs a) {
           }
           tc::tc_fence_after();
           const uint64_t ad = tc::umma_desc(s_u + st * kStageBytesG, 128, 256);
-          split_step<false, false>(side, utmem, ad, tc::umma_desc_add(ad, kSlices * kATileBytes), idesc,
-                            k == 0);
+          split_step<false, false>(side, utmem, ad,
+                                   tc::umma_desc_add(ad, kSlices * kATileBytes), idesc, k == 0);
           tc::umma_commit_warp(&h.empty[st]);
         }
         if (ok) tc::umma_commit_warp(&h.tfull);
@@ -936,8 +936,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) k_split_synth(SynthArgs a) {
             // (level 4, a1 b3, a2 b2, a3 b1, folded into the level-3 accumulator via the 2^-8
             // planes: with lambda against one scale its digits are often small, and dropping
             // level 4 would cost ~2e-7)
-            split_step<true, true>(side, utmem, ad, tc::umma_desc_add(ad, kSlices * kATileBytes), idesc,
-                             k == 0);
+            split_step<true, true>(side, utmem, ad,
+                                   tc::umma_desc_add(ad, kSlices * kATileBytes), idesc, k == 0);
             tc::umma_commit_warp(&h.empty[st]);
           }
           if (ok) tc::umma_commit_warp(&h.tfull);
@@ -1216,7 +1216,8 @@ int fsht_launch_split_gemm(fsht_plan* p, int w, const unsigned char* WS, const i
 }
 
 int fsht_launch_split_slice_alm(fsht_plan* p, int w, const double* alm, unsigned char* WS,
-                                int* EB, int nmaps_total, int k0, int kc, cudaStream_t s, bool paired) {
+                                int* EB, int nmaps_total, int k0, int kc, cudaStream_t s,
+                                bool paired) {
   const int* wv = p->h_waves + kWaveInts * w;
   SliceAArgs a;
   a.alm = alm;

@@ -25,7 +25,6 @@ constexpr uint32_t kBTileBytes = kCols * kKStep * 2;    // 4 KB per (k-step, dig
 // the level-4 products fold into the level-3 accumulator.
 constexpr int kSynthPlanes = 7;
 constexpr uint32_t kSynthBBytes = kSynthPlanes * kBTileBytes;   // 28 KB per l-step
-constexpr int kThreads = 192;
 // persistent contractions: eight epilogue warps (two per TMEM lane quarter, one per half of the
 // columns), the copy thread's warp and two UMMA warps.  One warp issues about a product per 75
 // clocks, the tensor pipe takes one per 63: two warps keep it fed (levels 0 and 3, and 1 and 2).
