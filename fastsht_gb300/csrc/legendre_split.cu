@@ -849,6 +849,11 @@ __device__ __forceinline__ SynthUnit synth_unit(const SynthArgs& a, int u) {
 // entry (8-byte stores of one component each touched every sector four times):
 // 4.29 -> 2.55 ms at nside 512, lmax 1023, 64 maps.
 // Warp 16 lane 0: copies, warps 17 and 18: UMMAs (13 per l-step: levels 0-3 and the level-4 fold).
+// FEW (up to kFewMaps maps, one group): rings on the lanes and only the maps' columns as N, since
+// with the columns on the lanes a warp runs through all of its rings for one or two live lanes
+// (one map at nside 128, lmax 320: 144 us against 43).
+constexpr int kFewCols = 16, kFewMaps = 4 * kFewCols / 2;
+template <bool FEW>
 __global__ void __launch_bounds__(kThreadsS, 1) k_split_synth(SynthArgs a) {
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ SynthSmemHdr h;
@@ -908,7 +913,8 @@ __global__ void __launch_bounds__(kThreadsS, 1) k_split_synth(SynthArgs a) {
     // UMMA warps: lambda tiles (rings) as the second operand, alm tiles as the first, so that the
     // map columns are on the TMEM lanes
     const int side = warp - kEpiWarpsS - 1;
-    const uint32_t idesc = tc::umma_idesc_bf16(kRows, kCols);
+    const uint32_t idesc =
+        tc::umma_idesc_bf16(kRows, FEW ? (2 * tc::uniform(a.kc) + 15) & ~15 : kCols);
     const uint32_t s_u = (uint32_t)tc::uniform((int)tc::smem_u32(smem));
     const uint32_t utmem = (uint32_t)tc::uniform((int)tmem);
     uint32_t i = 0, np = 0;
@@ -936,12 +942,80 @@ __global__ void __launch_bounds__(kThreadsS, 1) k_split_synth(SynthArgs a) {
             // (level 4, a1 b3, a2 b2, a3 b1, folded into the level-3 accumulator via the 2^-8
             // planes: with lambda against one scale its digits are often small, and dropping
             // level 4 would cost ~2e-7)
-            split_step<true, true>(side, utmem, ad,
+            split_step<true, !FEW>(side, utmem, ad,
                                    tc::umma_desc_add(ad, kSlices * kATileBytes), idesc, k == 0);
             tc::umma_commit_warp(&h.empty[st]);
           }
           if (ok) tc::umma_commit_warp(&h.tfull);
         }
+      }
+    }
+  } else if (FEW && tid < kEpiThreadsS) {
+    // TMEM lane = ring, sixteen columns (eight maps) per warp: a thread has both components
+    const int lane = tid & 31, row = ((warp & 3) << 5) + lane, cbeg = (warp >> 2) * kFewCols;
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) << 5) << 16) + cbeg;
+    const int nmap = min(kFewCols / 2, a.kc - cbeg / 2);
+    uint32_t np = 0;
+    for (uint32_t n = 0;; ++n) {
+      const int u = uq_take(uq, n, abort);
+      if (u < 0) break;
+      const SynthUnit w = synth_unit(a, u);
+      if (w.nkl == 0) continue;
+      const bool in = w.rb * kSCRings + row < w.K;
+      double2* d = reinterpret_cast<double2*>(a.W) +
+                   (((long long)w.m * a.nnorth + w.i0 + (in ? w.rb * kSCRings + row : 0)) * a.kc +
+                    cbeg / 2) * 2;
+      int ce[2];                                       // lane j: column j of the warp's
+#pragma unroll
+      for (int pp = 0; pp < 2; ++pp) {
+        const int e =
+            lane < 2 * nmap ? a.EB[((long long)w.qi * 2 + pp) * kCols + cbeg + lane] : kEmptyExp;
+        ce[pp] = (e == kEmptyExp) ? kEmptyExp : a.eag + e - 12;
+      }
+      for (int kl0 = 0; kl0 < w.nkl; kl0 += kPartStepsS) {
+        double ev[kFewCols];
+        auto sums = [&](int cexp, auto put) {
+          const bool ok = tc::mbar_wait_warp(&h.tfull, np & 1, abort);
+          ++np;
+          if (!ok) return;
+          tc::tc_fence_after();
+#pragma unroll
+          for (int c0 = 0; c0 < kFewCols; c0 += 4) {
+            if (c0 / 2 >= nmap) break;
+            uint32_t v0[4], v1[4], v2[4], v3[4];
+            tc::tmem_ld4(lane_base + 0 * kCols + c0, v0);
+            tc::tmem_ld4(lane_base + 1 * kCols + c0, v1);
+            tc::tmem_ld4(lane_base + 2 * kCols + c0, v2);
+            tc::tmem_ld4(lane_base + 3 * kCols + c0, v3);
+            tc::tmem_wait_ld();
+            double v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              v[j] = levels_scaled(v0[j], v1[j], v2[j], v3[j], 1.f, 0.f,
+                                   __shfl_sync(0xffffffffu, cexp, c0 + j));
+            put(c0, v);
+          }
+          tc::tc_fence_before();
+          tc::mbar_arrive_warp(&h.tempty);
+        };
+        sums(ce[0], [&](int c0, const double (&v)[4]) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ev[c0 + j] = v[j];
+        });
+        sums(ce[1], [&](int c0, const double (&v)[4]) {
+#pragma unroll
+          for (int j = 0; j < 4; j += 2) {
+            const int mp = (c0 + j) / 2;
+            if (!in || mp >= nmap) continue;
+            double2 nn = make_double2(ev[c0 + j], ev[c0 + j + 1]), ss = nn;
+            if (kl0 > 0) {
+              nn = cadd(nn, d[2 * mp]);
+              ss = cadd(ss, d[2 * mp + 1]);
+            }
+            d[2 * mp] = make_double2(nn.x + v[j], nn.y + v[j + 1]);
+            d[2 * mp + 1] = make_double2(ss.x - v[j], ss.y - v[j + 1]);
+          }
+        });
       }
     }
   } else if (tid < kEpiThreadsS) {
@@ -963,6 +1037,11 @@ __global__ void __launch_bounds__(kThreadsS, 1) k_split_synth(SynthArgs a) {
       if (w.nkl == 0) continue;
       const int k = w.g * kGroupMaps + (c >> 1);
       const bool ok_col = k < a.kc;
+      if (!__any_sync(0xffffffffu, ok_col)) {          // no maps in this quarter: hand back
+        for (int t = 0; t < 2 * ((w.nkl + kPartStepsS - 1) / kPartStepsS); ++t, ++np)
+          if (tc::mbar_wait_warp(&h.tfull, np & 1, abort)) tc::mbar_arrive_warp(&h.tempty);
+        continue;
+      }
       int ce[2];
 #pragma unroll
       for (int pp = 0; pp < 2; ++pp) {
@@ -1282,8 +1361,9 @@ int fsht_launch_split_synth(fsht_plan* p, int w, const unsigned char* WS, const 
   a.kc = kc;
   a.err = p->d_err;
   const size_t sm = (size_t)kStagesS * kStageBytesS;
-  FSHT_TRY(fsht_smem_limit((const void*)k_split_synth, (size_t)(sm)));
-  if (a.nunits > 0) k_split_synth<<<a.nunits, kThreadsS, sm, s>>>(a);
+  void (*const k)(SynthArgs) = kc <= kFewMaps ? k_split_synth<true> : k_split_synth<false>;
+  FSHT_TRY(fsht_smem_limit((const void*)k, (size_t)(sm)));
+  if (a.nunits > 0) k<<<a.nunits, kThreadsS, sm, s>>>(a);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;
 }

@@ -249,10 +249,11 @@ __device__ __forceinline__ void factor_pair(double x, float& fh, float& fl) {
 // flight per thread, so they run at the latency of memory unless many blocks share the work, and a
 // wave of a large plan holds only some sixty orders.  The blocks of a cluster (grid z) take one
 // part of the summands each and exchange the column maxima through distributed shared memory.
-// Size: enough for eight blocks an SM, while a block keeps at least four k-steps.
+// Size: enough for eight blocks an SM, while a block keeps at least eight k-steps (below that the
+// cluster's barriers cost what the shorter loops save).
 inline int slice_cluster(long long blocks, int steps) {
   int cl = 1;
-  while (cl < 8 && blocks * cl < 8 * 152 && steps >= 8 * cl) cl *= 2;
+  while (cl < 8 && blocks * cl < 8 * 152 && steps >= 16 * cl) cl *= 2;
   return cl;
 }
 template <class Args>
