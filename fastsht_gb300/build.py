@@ -52,7 +52,7 @@ def build(verbose: bool = False, force: bool = False) -> Path:
     OUT_DIR.mkdir(exist_ok=True)
     obj_dir = OUT_DIR / "obj"
     obj_dir.mkdir(exist_ok=True)
-    headers = list(CSRC.glob("*.cuh")) + list((PKG.parent / "include").glob("*.h"))
+    headers = [h for d in (CSRC, PKG.parent / "include") for e in ("*.cuh", "*.h") for h in d.glob(e)]
     srcs = sources()
     nv = nvcc()
 

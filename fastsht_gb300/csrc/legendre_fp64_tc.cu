@@ -27,6 +27,7 @@
 // at 82 % of the DFMA rate.
 #include "legendre_rec.cuh"
 #include "split_common.cuh"
+#include "tc_units.h"
 
 #include <algorithm>
 #include <cmath>
@@ -555,11 +556,11 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
 
 // ------------------------------------------------------------------ alm -> digits
 // grid (q in wave, group, cluster), 256 threads per field = (half of the block's l steps, comp,
-// map): v = a_lm Dm 2^EA(l), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an
+// map): v = a_lm Dm 2^EA(l) with `head` spare bits (tc_units.h), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an
 // exponent per column; E/B (NF = 2): one per map and order, plain and i v copies.
 struct TcSliceAArgs {
   const double* alm[2];
-  int ld, k0, kc, lmax, ngroups, q0;
+  int ld, k0, kc, lmax, ngroups, q0, head;
   size_t row_bytes;
   const FshtLamRow* tab;
   unsigned char* WS;
@@ -631,7 +632,7 @@ __global__ void __launch_bounds__(256 * NF) k_tc_slice_alm(TcSliceAArgs a) {
     const int ef = (int)(mx >> 52);
     const bool odd_range = mx != 0 && (ef < 1023 - kMaxExp || ef > 1023 + kMaxExp);
     flag |= odd_range;
-    Ep[p] = (mx == 0 || odd_range) ? kEmptyExp : ef - 1022;
+    Ep[p] = (mx == 0 || odd_range) ? kEmptyExp : ef - 1022 + a.head;
     if (f == 0 && seg == 0) a.EB[(((long long)qi * 2 + p) * a.ngroups + g) * kCols + c] = Ep[p];
   }
   const int any = __syncthreads_or(flag ? 1 : 0);
@@ -1616,27 +1617,6 @@ size_t tc_row_bytes(const fsht_plan* p) {
 }
 int tc_groups(int kc) { return (kc + kGroupMaps - 1) / kGroupMaps; }
 
-int tc_eag(int lmax) {
-  const double b = std::sqrt((2.0 * lmax + 1.0) / (4.0 * M_PI)) * (1.0 + 0x1p-30);
-  return std::ilogb(b) + 1;
-}
-int ceil_log2(long long x) {
-  int b = 0;
-  while ((1LL << b) < x) ++b;
-  return b;
-}
-// Integer units: sums in digit units are below 2^12 times the sum of |row| / scale, and the 64-bit
-// sum has 63 bits.  Analysis: sum over the north rings of |lambda| (spin 2: |lambda1| + |lambda2|)
-// is below 0.85 nside for every l and m (tests/test_tc_bounds.py), against 2^EAG.  Synthesis: the
-// sum over l of one parity of |lambda| 2^-EA(l) is below 0.4 (lmax/2 + 1) for the same reason, and
-// the two parities are added and subtracted.
-int tc_bits_analysis(const fsht_plan* p) {
-  return std::min(46, 51 - ceil_log2(p->nside) + tc_eag(p->lmax));
-}
-int tc_bits_synthesis(const fsht_plan* p) {
-  return std::min(46, 50 - ceil_log2((2LL * (p->lmax / 2 + 1) + 4) / 5 + 1));
-}
-
 template <int DIR, int SPIN>
 int launch_tc_gemm(const TcGemmArgs& a, cudaStream_t s) {
   FSHT_TRY(fsht_smem_limit((const void*)k_tc_gemm<DIR, SPIN>, kTcSmem));
@@ -1647,7 +1627,7 @@ int launch_tc_gemm(const TcGemmArgs& a, cudaStream_t s) {
 }  // namespace
 
 bool fsht_tc_supported(const fsht_plan* p) {
-  return p->nside >= 32 && tc_bits_analysis(p) >= 40 && tc_bits_synthesis(p) >= 40;
+  return fsht_tc_sizes(p->nside, p->lmax);
 }
 
 int fsht_tc_tables_init(fsht_plan* p) {
@@ -1715,6 +1695,7 @@ int fsht_launch_tc_slice_alm(fsht_plan* p, int w, const double* alm0, const doub
   a.lmax = p->lmax;
   a.ngroups = tc_groups(kc);
   a.q0 = wv[0];
+  a.head = fsht_tc_units_synthesis(p->lmax).head;
   a.row_bytes = tc_row_bytes(p);
   a.tab = alm1 ? p->d_lamtab2 : p->d_lamtab;
   a.WS = WS;
@@ -1735,7 +1716,7 @@ int launch_tc_lambda(fsht_plan* p, int w, unsigned char* lbuf, cudaStream_t s) {
   a.lmax = p->lmax;
   a.nnorth = p->nnorth;
   a.q0 = wv[0];
-  a.eag = tc_eag(p->lmax);
+  a.eag = fsht_tc_eag(p->lmax);
   a.cth = p->d_cth;
   a.sth = p->d_sth;
   a.pref = p->d_pref;
@@ -1786,8 +1767,9 @@ int fsht_launch_tc_gemm(fsht_plan* p, int w, int dir, int spin, const unsigned c
     a.field0 = which == 2 ? 1 : 0;
   }
   a.accumulate = accumulate;
-  a.unit_bits = dir == 0 ? tc_bits_analysis(p) : tc_bits_synthesis(p);
-  a.eag = tc_eag(p->lmax);
+  a.unit_bits = (dir == 0 ? fsht_tc_units_analysis(p->nside, p->lmax)
+                          : fsht_tc_units_synthesis(p->lmax)).bits;
+  a.eag = fsht_tc_eag(p->lmax);
   a.row_bytes = tc_row_bytes(p);
   a.ring_i0 = p->d_ring_i0;
   a.lam_off = dir == 0 ? p->d_lam_off : p->d_lam_offT;
@@ -1818,7 +1800,7 @@ constexpr int kDftWaveInts = 5;     // first entry, end, most row tiles, largest
 
 // Sums of at most nk <= q + 1 products against the cosines' 2^1; north and south, or the four
 // mirrored samples, are added and subtracted.  (tc_drain wants 40 bits or more.)
-int dft_bits(int nk, int extra) { return std::min(46, 51 - extra - ceil_log2((nk + 1) / 2)); }
+int dft_bits(int nk, int extra) { return std::min(46, 51 - extra - fsht_ceil_log2((nk + 1) / 2)); }
 
 DftSliceArgs dft_slice_args(const fsht_plan* p, const int* wv, int ngroups) {
   DftSliceArgs a{};
