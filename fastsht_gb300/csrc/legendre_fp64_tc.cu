@@ -556,8 +556,9 @@ __global__ void __launch_bounds__(128) k_tc_lambda_T(TcLamArgs a) {
 
 // ------------------------------------------------------------------ alm -> digits
 // grid (q in wave, group, cluster), 256 threads per field = (half of the block's l steps, comp,
-// map): v = a_lm Dm 2^EA(l) with `head` spare bits (tc_units.h), tile column c = 2 map + comp, 16 l of one parity per k-step.  T: an
-// exponent per column; E/B (NF = 2): one per map and order, plain and i v copies.
+// map): v = a_lm Dm 2^EA(l) with `head` spare bits (tc_units.h), tile column c = 2 map + comp, 16 l
+// of one parity per k-step.  T: an exponent per column; E/B (NF = 2): one per map and order, plain
+// and i v copies.
 struct TcSliceAArgs {
   const double* alm[2];
   int ld, k0, kc, lmax, ngroups, q0, head;
@@ -757,6 +758,7 @@ __global__ void __launch_bounds__(256) k_dft_trig(DftTrigArgs a) {
 struct DftSliceArgs {
   const FshtDftRing* rings;
   int ngroups;
+  int head;                     // spare bits of the columns (tc_units.h)
   unsigned char* WS;
   int* EB;                      // per (ring of the wave, group, column)
   // forward: map k of this launch at maps + k map_stride
@@ -832,12 +834,13 @@ __global__ void __launch_bounds__(256) k_dft_slice(DftSliceArgs a) {
   const int g = map >> 6, c = 2 * (map & 63) + h;
   if (map >= a.cnt) return;
   if (chunk == 0)
-    a.EB[((long long)blockIdx.x * a.ngroups + g) * kCols + c] = E > kEmptyExp ? E + 2 : E;
+    a.EB[((long long)blockIdx.x * a.ngroups + g) * kCols + c] =
+        E > kEmptyExp ? E + 2 + a.head : E;
   const int nj = d.q + (d.s == 0 ? 1 : 0);
   unsigned char* dst = a.WS + (size_t)(d.off_c * a.ngroups) * kStepBytes +
                        (size_t)g * d.nk * kStepBytes + (c >> 3) * 256 + (c & 7) * 16;
   const size_t tstride = (size_t)a.ngroups * d.nk * kStepBytes;
-  const int kf = kFixBits - 2 - E;
+  const int kf = kFixBits - 2 - a.head - E;
   for (int hc = chunk; hc < 2 * d.nk; hc += CH) {
     unsigned long long y[4][8];
 #pragma unroll
@@ -921,7 +924,8 @@ __global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
   const bool live = valid && E > kEmptyExp;
   const int grp = map >> 6, c = 2 * (map & 63) + h;
   if (map >= a.cnt) return;
-  if (warp == 0) a.EB[((long long)blockIdx.x * a.ngroups + grp) * kCols + c] = E;
+  if (warp == 0)
+    a.EB[((long long)blockIdx.x * a.ngroups + grp) * kCols + c] = E > kEmptyExp ? E + a.head : E;
   unsigned char* dst = a.WS + (size_t)(d.off_c * a.ngroups) * kStepBytes +
                        (size_t)grp * d.nk * kStepBytes + (c >> 3) * 256 + (c & 7) * 16;
   const size_t tstride = (size_t)a.ngroups * d.nk * kStepBytes;
@@ -936,7 +940,7 @@ __global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
         y[e] = kBias;
         if (live && rho < nr) {
           const double2 v = dft_bin(g, stride_m, d, dft_r(ty, rho));
-          y[e] = fixed_biased(ty < 2 ? v.x : v.y, kFixBits - E);
+          y[e] = fixed_biased(ty < 2 ? v.x : v.y, kFixBits - a.head - E);
         }
       }
       store_planes<false>(dst + ty * tstride + (size_t)(hc >> 1) * kStepBytes + (hc & 1) * 128,
@@ -1798,14 +1802,16 @@ namespace {
 constexpr int kDftBeltMax = 256;
 constexpr int kDftWaveInts = 5;     // first entry, end, most row tiles, largest q, digit k-steps
 
-// Sums of at most nk <= q + 1 products against the cosines' 2^1; north and south, or the four
-// mirrored samples, are added and subtracted.  (tc_drain wants 40 bits or more.)
-int dft_bits(int nk, int extra) { return std::min(46, 51 - extra - fsht_ceil_log2((nk + 1) / 2)); }
+// Units of the forward (two rings added: 1) and inverse transforms (four samples: 2) of a plan.
+FshtTcUnits dft_units(const fsht_plan* p, int extra) {
+  return fsht_tc_units_dft(p->nside <= kDftBeltMax ? p->nside + 1 : p->nside - 1, extra);
+}
 
-DftSliceArgs dft_slice_args(const fsht_plan* p, const int* wv, int ngroups) {
+DftSliceArgs dft_slice_args(const fsht_plan* p, const int* wv, int ngroups, int extra) {
   DftSliceArgs a{};
   a.rings = p->d_dft + wv[0];
   a.ngroups = ngroups;
+  a.head = dft_units(p, extra).head;
   a.WS = p->d_ws;
   a.EB = p->d_eb;
   a.nside = p->nside;
@@ -1832,7 +1838,7 @@ TcGemmArgs dft_gemm_args(const fsht_plan* p, const int* wv, int ngroups, int cnt
   a.ngroups = ngroups;
   a.ntmax = wv[2];
   a.nnorth = p->nnorth;
-  a.unit_bits = dft_bits(p->nside <= kDftBeltMax ? p->nside + 1 : p->nside - 1, extra);
+  a.unit_bits = dft_units(p, extra).bits;
   a.lbuf = p->d_lbuf;
   a.WS = p->d_ws;
   a.EB = p->d_eb;
@@ -1953,7 +1959,7 @@ int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, 
   for (int w = 0; w < p->ndft_waves; ++w) {
     const int* wv = p->h_dft_waves + kDftWaveInts * w;
     FSHT_TRY(launch_dft_trig<false>(p, wv, s));
-    DftSliceArgs sa = dft_slice_args(p, wv, ngroups);
+    DftSliceArgs sa = dft_slice_args(p, wv, ngroups, 1);
     sa.maps = maps + (long long)k0 * map_stride;
     sa.map_stride = map_stride;
     sa.cnt = cnt;
@@ -1982,7 +1988,7 @@ int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long 
   for (int w = 0; w < p->ndft_waves; ++w) {
     const int* wv = p->h_dft_waves + kDftWaveInts * w;
     FSHT_TRY(launch_dft_trig<true>(p, wv, s));
-    DftSliceArgs sa = dft_slice_args(p, wv, ngroups);
+    DftSliceArgs sa = dft_slice_args(p, wv, ngroups, 2);
     sa.W = W;
     sa.kc = kc;
     sa.cnt = cnt;

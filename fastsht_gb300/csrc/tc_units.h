@@ -45,3 +45,8 @@ inline FshtTcUnits fsht_tc_units_synthesis(int lmax) {
 inline bool fsht_tc_sizes(int nside, int lmax) {
   return nside >= 32 && lmax <= 5113 && fsht_tc_units_analysis(nside, lmax).head == 0;
 }
+// Ring transforms: sums of at most nk <= q + 1 products against the cosines' 2^1; 2^extra of them
+// (north and south, or the four mirrored samples) are added and subtracted.
+inline FshtTcUnits fsht_tc_units_dft(int nk, int extra) {
+  return fsht_tc_units_of(51 - extra - fsht_ceil_log2((nk + 1) / 2));
+}

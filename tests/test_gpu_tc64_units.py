@@ -91,3 +91,20 @@ def test_iterations_on_zonal_maps(ns, lmax):
         out.append(sht.t2alm(maps).reshape(2, -1).clone())
         sht.close()
     assert ((out[0] - out[1]).abs().amax(1) <= TOL * out[1].abs().amax(1)).all()
+
+
+@pytest.mark.parametrize("ns,lmax", [(1024, 1100), (2048, 1300)])
+def test_largest_inverse_ring_transforms(ns, lmax):
+    """alm2t with the cap rings in matrix form (24 maps) against the same maps by FFT (12): bins of
+    one sign at the top of their scale, and random ones."""
+    from fastsht_gb300 import SHT
+    g = torch.Generator(device="cuda").manual_seed(ns)
+    alm = torch.randn((lmax + 1, lmax + 1, 24), dtype=torch.float64, device="cuda", generator=g)
+    alm[..., ::2].abs_()
+    out = []
+    for k in (24, 12):
+        sht = SHT(ns, lmax, k, workspace_limit=64 << 30)
+        out.append(sht.alm2t(alm[..., :k].contiguous().permute(2, 1, 0)).T[:12].clone())
+        sht.close()
+    got, want = out
+    assert ((got - want).abs().amax(1) <= TOL * want.abs().amax(1)).all()

@@ -4,7 +4,7 @@ in units of 2^-bits, within 2^63.
 
 Synthesis, every lmax from 1 to 4 nside: the running sum over l of one order and ring, rows in the
 kernel's own scale (the power of two above bound / Dm for the mantissa Dm of D_l, spin 2: of N_l),
-columns of one sign at the top of their scale.
+columns of one sign at the top of their scale.  Ring transforms: all accepted nside.
 """
 import ctypes as C
 import shutil
@@ -22,6 +22,7 @@ extern "C" int synthesis(int lmax, int* head) { return put(fsht_tc_units_synthes
 extern "C" int analysis(int ns, int lmax, int* head) {
   return put(fsht_tc_units_analysis(ns, lmax), head);
 }
+extern "C" int dft(int nk, int extra, int* head) { return put(fsht_tc_units_dft(nk, extra), head); }
 """
 
 
@@ -110,3 +111,11 @@ def test_analysis_sums_fit(units, ns):
     for lmax in (1, ns, 2 * ns, 3 * ns - 1):
         eag = int(np.floor(np.log2(np.sqrt((2 * lmax + 1) / (4 * np.pi)) * (1 + 2.0 ** -30)))) + 1
         assert 0.85 * ns * 2.0 ** (12 + units("analysis", ns, lmax) - eag) < 2.0 ** 63
+
+
+@pytest.mark.parametrize("ns", [32, 64, 128, 256, 512, 1024, 2048])
+def test_ring_transform_sums_fit(units, ns):
+    # forward (folds of two rings), inverse (four mirrored samples); the matrices hold cos 2^61
+    nk = ns + 1 if ns <= 256 else ns - 1
+    for extra in (1, 2):
+        assert nk * 0.5 * 2.0 ** extra * 2.0 ** (12 + units("dft", nk, extra)) <= 2.0 ** 63
