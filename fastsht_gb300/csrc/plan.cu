@@ -154,14 +154,32 @@ void free_plan_memory(fsht_plan* p) {
   }
 }
 
-void drop_tc_buffers(fsht_plan* p) {
-  cudaFree(p->d_ws);
-  cudaFree(p->d_eb);
-  cudaFree(p->d_tcflag);
-  cudaFree(p->d_lbuf);
-  cudaFree(p->d_lbuf2);
-  p->d_ws = p->d_lbuf = p->d_lbuf2 = nullptr;
-  p->d_eb = p->d_tcflag = nullptr;
+template <class T>
+void drop(T*& d) {
+  cudaFree(d);
+  d = nullptr;
+}
+
+// Everything an FP64 plan holds for the tensor-core form, which it does not take.
+void drop_tc(fsht_plan* p) {
+  p->tc64 = 0;
+  drop(p->d_ws);
+  drop(p->d_eb);
+  drop(p->d_tcflag);
+  drop(p->d_lbuf);
+  drop(p->d_lbuf2);
+  drop(p->d_lamtab);
+  drop(p->d_lamtab2);
+  drop(p->d_poltab);
+  drop(p->d_lam_off);
+  drop(p->d_lam_offT);
+  drop(p->d_dft);
+  drop(p->d_dft_cos);
+  delete[] p->h_waves;
+  delete[] p->h_dft_waves;
+  p->h_waves = p->h_dft_waves = nullptr;
+  p->nwaves = p->wave_qmax = p->ndft_waves = p->dft_end = 0;
+  p->ws_bytes = p->lbuf_bytes = 0;
 }
 
 // theta of the first pixel of north ring i (HEALPix pix2loc, as used through
@@ -307,10 +325,15 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   auto dalloc = [&](void** ptr, size_t bytes) -> int {
     cudaError_t e = cudaMalloc(ptr, bytes);
     if (e != cudaSuccess) {
+      cudaGetLastError();             // or the next launch check of this thread would report it
       fsht_set_error("cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
       return e == cudaErrorMemoryAllocation ? FSHT_ENOMEM : FSHT_ECUDA;
     }
     return FSHT_OK;
+  };
+  // Device memory that ran out for the tables of the tensor-core form: the plan goes without it.
+  auto no_memory = [&](int code) {
+    return code != FSHT_OK && cudaGetLastError() == cudaErrorMemoryAllocation;
   };
   if ((rc = dalloc((void**)&p->d_cth, sizeof(double) * nn))) return fail(rc);
   if ((rc = dalloc((void**)&p->d_sth, sizeof(double) * nn))) return fail(rc);
@@ -333,8 +356,11 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   if (precision == FSHT_PREC_SPLIT && p->pol && (rc = fsht_split_pol_tables_init(p)))
     return fail(rc);
   if (precision == FSHT_PREC_FP64 && fsht_tc_supported(p)) {
-    if ((rc = fsht_tc_tables_init(p))) return fail(rc);
     p->tc64 = 1;
+    if ((rc = fsht_tc_tables_init(p))) {
+      if (!no_memory(rc)) return fail(rc);
+      drop_tc(p);
+    }
   }
   // ---- workspace: nbuf phase matrices of kchunk maps (+ the sliced copy for the
   // split form, sized in groups of 128 maps)
@@ -373,7 +399,10 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
       if ((rc = fsht_tc_wave_cap(p, kLbufCap / 2))) return fail(rc);
       if (chunks(tc_chunk()) >= c1 && (rc = fsht_tc_wave_cap(p, kLbufCap))) return fail(rc);
     }
-    if ((rc = fsht_dft_tables_init(p))) return fail(rc);
+    if ((rc = fsht_dft_tables_init(p))) {
+      if (!no_memory(rc)) return fail(rc);
+      drop_tc(p);
+    }
   }
   size_t kc = (size_t)nmaps_max;
   while (kc > 1 && need(kc) > limit) kc = (kc > 128 && kc % 128) ? kc - kc % 128 : kc - (kc > 128 ? 128 : 1);
@@ -386,29 +415,27 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     // A limit that leaves them less than one group (and fewer maps than the FMA kernels' chunk)
     // keeps the FMA kernels, which need no tiles.
     const size_t kt = tc_chunk();
-    if (need_tc(kt) > limit || (kt < kc && kt < 64)) {
-      p->tc64 = 0;
-    } else {
-      // two digit-tile buffers, exponents, flags, two lambda buffers; without room for them on
-      // the device the FMA kernels run
-      const size_t ws = 2 * fsht_tc_ws_bytes(p, (int)kt, tc_nf);
-      const size_t eb = 2 * fsht_tc_eb_bytes(p, (int)kt);
-      if (cudaMalloc(&p->d_ws, ws) != cudaSuccess || cudaMalloc(&p->d_eb, eb) != cudaSuccess ||
-          cudaMalloc(&p->d_tcflag, fsht_tc_flag_bytes(p, (int)kt)) != cudaSuccess ||
-          cudaMalloc(&p->d_lbuf, p->lbuf_bytes) != cudaSuccess ||
-          cudaMalloc(&p->d_lbuf2, p->lbuf_bytes) != cudaSuccess) {
-        cudaGetLastError();
-        drop_tc_buffers(p);
-        p->tc64 = 0;
-      } else {
-        p->ws_bytes = ws;
-        kc = kt;
-      }
+    bool fits = need_tc(kt) <= limit && (kt >= kc || kt >= 64);
+    if (fits) {
+      // the phase matrices, two digit-tile buffers, exponents, flags, two lambda buffers; without
+      // room for all of them on the device the FMA kernels run, on as many maps as they take
+      p->ws_bytes = 2 * fsht_tc_ws_bytes(p, (int)kt, tc_nf);
+      fits = !dalloc((void**)&p->d_work, per_map * kt) && !dalloc((void**)&p->d_ws, p->ws_bytes) &&
+             !dalloc((void**)&p->d_eb, 2 * fsht_tc_eb_bytes(p, (int)kt)) &&
+             !dalloc((void**)&p->d_tcflag, fsht_tc_flag_bytes(p, (int)kt)) &&
+             !dalloc((void**)&p->d_lbuf, p->lbuf_bytes) &&
+             !dalloc((void**)&p->d_lbuf2, p->lbuf_bytes);
+      if (!fits) drop(p->d_work);
     }
+    if (fits)
+      kc = kt;
+    else
+      drop_tc(p);
   }
   p->kchunk = tables_only ? 0 : (int)kc;
   p->work_bytes = tables_only ? 0 : per_map * kc;
-  if (!tables_only && (rc = dalloc((void**)&p->d_work, p->work_bytes))) return fail(rc);
+  if (!tables_only && !p->d_work && (rc = dalloc((void**)&p->d_work, p->work_bytes)))
+    return fail(rc);
   if ((rc = dalloc((void**)&p->d_err, sizeof(int)))) return fail(rc);
   if ((ce = cudaMemsetAsync(p->d_err, 0, sizeof(int), p->stream)) != cudaSuccess) {
     fsht_set_error("memset: %s", cudaGetErrorString(ce));

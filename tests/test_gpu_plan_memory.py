@@ -1,0 +1,33 @@
+"""What an FP64 plan does where its digit tiles find no room: the limit or the device leaves the FMA
+form, which needs the phase matrices only."""
+import pytest
+
+torch = pytest.importorskip("torch")
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from fastsht_gb300 import build
+    build.build()
+
+
+@pytest.mark.parametrize("share", [0.1, 0.14, 0.18, 0.22, 0.26, 0.3, 0.34, 0.38, 0.42, 0.46, 0.5])
+def test_plan_whose_tiles_do_not_fit_the_device(share):
+    """Phase matrices of `share` of the free memory and no limit of the plan's own: the tiles take
+    a few times as much, so they fit, fit alone but not beside the matrices, or do not fit."""
+    from fastsht_gb300 import SHT
+    ns, lmax = 256, 767
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    nsim = int(share * free / (2 * ns * (lmax + 1) * 32))
+    sht = SHT(ns, lmax, nsim, workspace_limit=1 << 50)
+    assert sht.plan_info()["maps_per_chunk"] == nsim
+    sht.close()
+    # the thread's next calls are not disturbed by the allocations that failed
+    maps = torch.ones((12 * 16 * 16, 1), dtype=torch.float64, device="cuda")
+    alm = SHT(16, 20, 1).t2alm(maps)
+    assert abs(float(alm[0, 0, 0]) - (4 * torch.pi) ** 0.5) < 1e-12
