@@ -209,6 +209,7 @@ struct fsht_plan {
   int* h_dft_waves;
   int ndft_waves, dft_end;
   FshtLamRow* d_lamtab2;           // their spin-2 recursion rows (d_poltab: integer factors)
+  size_t dev_bytes;                // device memory that the plan has allocated
 };
 
 // ---------------------------------------------------------------- status codes
@@ -220,6 +221,14 @@ void fsht_set_error(const char* fmt, ...);
 // changing a function's attributes is not a launch-path operation and can wait for that
 // function's launches in flight, which would tie the enqueueing thread to the GPU.
 int fsht_smem_limit(const void* func, size_t bytes);
+
+// cudaMalloc on a plan's account (fsht_plan_info).
+template <class T>
+cudaError_t fsht_plan_malloc(fsht_plan* p, T** ptr, size_t bytes) {
+  const cudaError_t e = cudaMalloc(reinterpret_cast<void**>(ptr), bytes);
+  if (e == cudaSuccess) p->dev_bytes += bytes;
+  return e;
+}
 
 #define FSHT_CUDA_TRY(expr)                                                   \
   do {                                                                        \

@@ -1636,10 +1636,10 @@ bool fsht_tc_supported(const fsht_plan* p) {
 
 int fsht_tc_tables_init(fsht_plan* p) {
   const size_t ntab = (size_t)tri_off(p->lmax + 1, p->lmax);
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_lamtab, sizeof(FshtLamRow) * ntab));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_lamtab, sizeof(FshtLamRow) * ntab));
   if (p->pol) {
-    FSHT_CUDA_TRY(cudaMalloc(&p->d_lamtab2, sizeof(FshtLamRow) * ntab));
-    FSHT_CUDA_TRY(cudaMalloc(&p->d_poltab, sizeof(FshtPolRow) * ntab));
+    FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_lamtab2, sizeof(FshtLamRow) * ntab));
+    FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_poltab, sizeof(FshtPolRow) * ntab));
   }
   k_tc_table<<<p->lmax + 1, kTabThreads, 0, p->stream>>>(p->lmax, p->d_lamtab, p->d_lamtab2,
                                                          p->d_poltab);
@@ -1940,8 +1940,8 @@ int fsht_dft_tables_init(fsht_plan* p) {
     return FSHT_ENOMEM;
   }
   std::copy(waves.begin(), waves.end(), p->h_dft_waves);
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_dft, sizeof(FshtDftRing) * rings.size()));
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_dft_cos, sizeof(long long) * ucos));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_dft, sizeof(FshtDftRing) * rings.size()));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_dft_cos, sizeof(long long) * ucos));
   FSHT_CUDA_TRY(cudaMemcpyAsync(p->d_dft, rings.data(), sizeof(FshtDftRing) * rings.size(),
                                 cudaMemcpyHostToDevice, p->stream));
   k_dft_cos<<<(unsigned)rings.size(), 256, 0, p->stream>>>(p->d_dft, p->d_dft_cos);

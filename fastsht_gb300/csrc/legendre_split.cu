@@ -1162,7 +1162,7 @@ int eag_of(int lmax) {
 int fsht_split_tables_init(fsht_plan* p) {
   const int lmax = p->lmax;
   const size_t ntab = (size_t)tri_off(lmax + 1, lmax);
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_lamtab, sizeof(FshtLamRow) * (ntab ? ntab : 1)));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_lamtab, sizeof(FshtLamRow) * (ntab ? ntab : 1)));
   k_lam_table<<<(lmax + 1 + 127) / 128, 128, 0, p->stream>>>(lmax, p->d_lamtab);
   FSHT_LAUNCH_CHECK();
   return fsht_wave_tables_init(p, (size_t)kSlices * kATileBytes);
@@ -1170,8 +1170,9 @@ int fsht_split_tables_init(fsht_plan* p) {
 
 int fsht_wave_tables_init(fsht_plan* p, size_t unit, size_t cap) {
   const int lmax = p->lmax;
-  if (!p->d_lam_off) FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_off, sizeof(long long) * (lmax + 2)));
-  if (!p->d_lam_offT) FSHT_CUDA_TRY(cudaMalloc(&p->d_lam_offT, sizeof(long long) * (lmax + 2)));
+  const size_t noff = sizeof(long long) * (lmax + 2);
+  if (!p->d_lam_off) FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_lam_off, noff));
+  if (!p->d_lam_offT) FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_lam_offT, noff));
   // per q (pair order): `unit`-byte k-steps of m(q)'s analysis tiles (l-rows) and synthesis
   // tiles (ring rows)
   std::vector<long long> off(lmax + 2, 0), offT(lmax + 2, 0);

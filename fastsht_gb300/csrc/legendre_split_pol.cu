@@ -939,7 +939,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
 int fsht_split_pol_tables_init(fsht_plan* p) {
   const int lmax = p->lmax;
   const size_t ntab = (size_t)tri_off(lmax + 1, lmax);
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_poltab, sizeof(FshtPolRow) * (ntab ? ntab : 1)));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_poltab, sizeof(FshtPolRow) * (ntab ? ntab : 1)));
   k_pol_table<<<(lmax + 1 + 127) / 128, 128, 0, p->stream>>>(lmax, p->d_poltab);
   FSHT_LAUNCH_CHECK();
   return FSHT_OK;

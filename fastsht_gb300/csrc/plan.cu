@@ -160,8 +160,10 @@ void drop(T*& d) {
   d = nullptr;
 }
 
-// Everything an FP64 plan holds for the tensor-core form, which it does not take.
-void drop_tc(fsht_plan* p) {
+// Everything an FP64 plan holds for the tensor-core form, which it does not take; plain: its device
+// bytes without that.
+void drop_tc(fsht_plan* p, size_t plain) {
+  p->dev_bytes = plain;
   p->tc64 = 0;
   drop(p->d_ws);
   drop(p->d_eb);
@@ -323,7 +325,7 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     pref[m] = std::sqrt(df / 4 / M_PI);
   }
   auto dalloc = [&](void** ptr, size_t bytes) -> int {
-    cudaError_t e = cudaMalloc(ptr, bytes);
+    cudaError_t e = fsht_plan_malloc(p, ptr, bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();             // or the next launch check of this thread would report it
       fsht_set_error("cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
@@ -355,11 +357,12 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   if (precision == FSHT_PREC_SPLIT && (rc = fsht_split_tables_init(p))) return fail(rc);
   if (precision == FSHT_PREC_SPLIT && p->pol && (rc = fsht_split_pol_tables_init(p)))
     return fail(rc);
+  const size_t plain = p->dev_bytes;
   if (precision == FSHT_PREC_FP64 && fsht_tc_supported(p)) {
     p->tc64 = 1;
     if ((rc = fsht_tc_tables_init(p))) {
       if (!no_memory(rc)) return fail(rc);
-      drop_tc(p);
+      drop_tc(p, plain);
     }
   }
   // ---- workspace: nbuf phase matrices of kchunk maps (+ the sliced copy for the
@@ -401,7 +404,7 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     }
     if ((rc = fsht_dft_tables_init(p))) {
       if (!no_memory(rc)) return fail(rc);
-      drop_tc(p);
+      drop_tc(p, plain);
     }
   }
   size_t kc = (size_t)nmaps_max;
@@ -430,7 +433,7 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     if (fits)
       kc = kt;
     else
-      drop_tc(p);
+      drop_tc(p, plain);
   }
   p->kchunk = tables_only ? 0 : (int)kc;
   p->work_bytes = tables_only ? 0 : per_map * kc;
@@ -526,11 +529,7 @@ int fsht_plan_set_stream(fsht_plan* p, void* stream) {
 
 int fsht_plan_info(const fsht_plan* p, size_t* device_bytes, int* maps_per_chunk) {
   FSHT_TRY(check_plan(p));
-  if (device_bytes) {
-    size_t b = p->work_bytes + p->ws_bytes + p->lbuf_bytes * (p->aux ? 2 : 1);
-    b += sizeof(double) * (2 * p->nnorth + p->lmax + 1) + sizeof(int) * (p->lmax + 1);
-    *device_bytes = b;
-  }
+  if (device_bytes) *device_bytes = p->dev_bytes;
   if (maps_per_chunk) *maps_per_chunk = p->kchunk;
   return FSHT_OK;
 }

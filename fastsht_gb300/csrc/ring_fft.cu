@@ -594,14 +594,17 @@ int fsht_fft_tables_init(fsht_plan* p) {
   p->fft_chirp_total = lay.chirp_total;
   p->fft_bhat_total = lay.bhat_total;
   p->fft_rtw_total = lay.rtw_total;
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_rfft, sizeof(FshtRingFFT) * nn));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_rfft, sizeof(FshtRingFFT) * nn));
   FSHT_CUDA_TRY(cudaMemcpyAsync(p->d_rfft, rfs.data(), sizeof(FshtRingFFT) * nn,
                                 cudaMemcpyHostToDevice, p->stream));
   const long long ntw = fsht_tw_entries(lay.Tmax, lay.P3max);
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_tw, sizeof(double2) * (ntw > 0 ? ntw : 1)));
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_chirp, sizeof(double2) * (lay.chirp_total > 0 ? lay.chirp_total : 1)));
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_bhat, sizeof(double2) * (lay.bhat_total > 0 ? lay.bhat_total : 1)));
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_rtw, sizeof(double2) * (lay.rtw_total > 0 ? lay.rtw_total : 1)));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_tw, sizeof(double2) * (ntw > 0 ? ntw : 1)));
+  FSHT_CUDA_TRY(fsht_plan_malloc(
+      p, &p->d_chirp, sizeof(double2) * (lay.chirp_total > 0 ? lay.chirp_total : 1)));
+  FSHT_CUDA_TRY(fsht_plan_malloc(
+      p, &p->d_bhat, sizeof(double2) * (lay.bhat_total > 0 ? lay.bhat_total : 1)));
+  FSHT_CUDA_TRY(fsht_plan_malloc(
+      p, &p->d_rtw, sizeof(double2) * (lay.rtw_total > 0 ? lay.rtw_total : 1)));
   int* d_rings = nullptr;
   if (lay.nblue > 0) {
     FSHT_CUDA_TRY(cudaMalloc(&d_rings, sizeof(int) * lay.nblue));

@@ -462,13 +462,13 @@ __global__ void k_twiddles16(float4* out, int logTmax) {
   }
 }
 
-int to_cdd(const double2* in, float4** out, long long n, cudaStream_t s) {
+int to_cdd(fsht_plan* p, const double2* in, float4** out, long long n) {
   const long long cnt = n > 0 ? n : 1;
-  FSHT_CUDA_TRY(cudaMalloc(out, sizeof(float4) * cnt));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, out, sizeof(float4) * cnt));
   if (n > 0) {
     long long g = (n + 255) / 256;
     if (g > 4096) g = 4096;
-    k_to_cdd<<<(unsigned)g, 256, 0, s>>>(in, *out, n);
+    k_to_cdd<<<(unsigned)g, 256, 0, p->stream>>>(in, *out, n);
     FSHT_LAUNCH_CHECK();
   }
   return FSHT_OK;
@@ -477,12 +477,12 @@ int to_cdd(const double2* in, float4** out, long long n, cudaStream_t s) {
 }  // namespace
 
 int fsht_fft_df_tables_init(fsht_plan* p) {
-  FSHT_TRY(to_cdd(p->d_tw, &p->d_tw_df, fsht_tw_entries(p->Tmax, p->P3max), p->stream));
-  FSHT_TRY(to_cdd(p->d_chirp, &p->d_chirp_df, p->fft_chirp_total, p->stream));
-  FSHT_TRY(to_cdd(p->d_bhat, &p->d_bhat_df, p->fft_bhat_total, p->stream));
-  FSHT_TRY(to_cdd(p->d_rtw, &p->d_rtw_df, p->fft_rtw_total, p->stream));
+  FSHT_TRY(to_cdd(p, p->d_tw, &p->d_tw_df, fsht_tw_entries(p->Tmax, p->P3max)));
+  FSHT_TRY(to_cdd(p, p->d_chirp, &p->d_chirp_df, p->fft_chirp_total));
+  FSHT_TRY(to_cdd(p, p->d_bhat, &p->d_bhat_df, p->fft_bhat_total));
+  FSHT_TRY(to_cdd(p, p->d_rtw, &p->d_rtw_df, p->fft_rtw_total));
   const long long n16 = fsht_tw16_entries(p->Tmax);
-  FSHT_CUDA_TRY(cudaMalloc(&p->d_tw16_df, sizeof(float4) * (n16 > 0 ? n16 : 1)));
+  FSHT_CUDA_TRY(fsht_plan_malloc(p, &p->d_tw16_df, sizeof(float4) * (n16 > 0 ? n16 : 1)));
   if (n16 > 0) {
     long long g = (n16 + 255) / 256;
     if (g > 4096) g = 4096;

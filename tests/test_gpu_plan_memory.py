@@ -31,3 +31,24 @@ def test_plan_whose_tiles_do_not_fit_the_device(share):
     maps = torch.ones((12 * 16 * 16, 1), dtype=torch.float64, device="cuda")
     alm = SHT(16, 20, 1).t2alm(maps)
     assert abs(float(alm[0, 0, 0]) - (4 * torch.pi) ** 0.5) < 1e-12
+
+
+@pytest.mark.parametrize("precision,pol,limit", [("fp64", False, 0), ("fp64", True, 0),
+                                                 ("fp64", True, 2 << 30), ("split", True, 0)])
+def test_plan_info_counts_what_the_plan_holds(precision, pol, limit):
+    """device_bytes against the device's own count: digit tiles, tables, and a limit that leaves
+    the FMA form.  (64 MiB for the blocks that the device rounds up to, and its streams.)"""
+    from fastsht_gb300 import SHT
+    ns, lmax = 256, 767
+
+    def plan():
+        return SHT(ns, lmax, 64, pol=pol, precision=precision, workspace_limit=limit)
+    plan().close()                              # kernels that load on first use
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    sht = plan()
+    torch.cuda.synchronize()
+    held = free - torch.cuda.mem_get_info()[0]
+    assert abs(held - sht.plan_info()["device_bytes"]) <= 64 << 20
+    sht.close()
