@@ -210,6 +210,7 @@ struct fsht_plan {
   int ndft_waves, dft_end;
   FshtLamRow* d_lamtab2;           // their spin-2 recursion rows (d_poltab: integer factors)
   size_t dev_bytes;                // device memory that the plan has allocated
+  int stage_maps;                  // most maps of a fsht_run_stage call (chunk without digit tiles)
 };
 
 // ---------------------------------------------------------------- status codes

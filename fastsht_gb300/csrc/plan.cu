@@ -413,6 +413,7 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     fsht_set_error("workspace limit %zu bytes is below one map's %zu bytes", limit, need(1));
     return fail(FSHT_EINVAL);
   }
+  p->stage_maps = tables_only ? 0 : (int)kc;
   if (p->tc64 && !tables_only) {
     // The digit tiles share the workspace limit with the phase matrices: whole 64-map groups.
     // A limit that leaves them less than one group (and fewer maps than the FMA kernels' chunk)
@@ -1022,8 +1023,8 @@ static int fp64_synthesis(fsht_plan* p, int spin, const double* alm0, const doub
 
 int fsht_run_stage(fsht_plan* p, int stage, const void* in, void* out, int nmaps) {
   FSHT_TRY(check_call(p, nmaps, in, out));
-  if (nmaps > p->kchunk) {
-    fsht_set_error("run_stage: nmaps %d above maps_per_chunk %d", nmaps, p->kchunk);
+  if (nmaps > p->stage_maps) {
+    fsht_set_error("run_stage: nmaps %d above this plan's %d a call", nmaps, p->stage_maps);
     return FSHT_EINVAL;
   }
   switch (stage) {

@@ -209,7 +209,9 @@ int fsht_measure_umma_rate(int n_cols, double* tflops);
  *   FSHT_STAGE_SYNTHESIS alm -> phase matrix {G_N, G_S}     (in: alm, out: W)
  *   FSHT_STAGE_FFT_INV   phase matrix -> maps               (in: W, out: maps)
  * W is laid out [m][ring][map][2] complex (double2), ring < 2 nside, m <= lmax,
- * for nmaps <= the plan's maps_per_chunk. */
+ * for nmaps <= the plan's maps_per_chunk.  FP64 plans run the general form here (ring FFTs and
+ * FMA contractions, the reference for the digit products of the whole transforms), on as many
+ * maps as fit the workspace limit without digit tiles. */
 enum { FSHT_STAGE_FFT_FWD = 0, FSHT_STAGE_ANALYSIS = 1, FSHT_STAGE_SYNTHESIS = 2,
        FSHT_STAGE_FFT_INV = 3 };
 int fsht_run_stage(fsht_plan* plan, int stage, const void* in, void* out, int nmaps);

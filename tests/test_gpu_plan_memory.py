@@ -52,3 +52,31 @@ def test_plan_info_counts_what_the_plan_holds(precision, pol, limit):
     held = free - torch.cuda.mem_get_info()[0]
     assert abs(held - sht.plan_info()["device_bytes"]) <= 64 << 20
     sht.close()
+
+
+def test_stages_take_the_maps_of_a_chunk_without_tiles():
+    """A limit that holds 640 maps' phase matrices, and 64 maps with their digit tiles: the
+    stages, which need no tiles, run on all 640."""
+    import ctypes as C
+    from fastsht_gb300 import _lib
+    ns, lmax, nsim = 64, 191, 640
+    plan = C.c_void_p()
+    _lib.call("fsht_plan_create", ns, lmax, nsim, 0, _lib.FSHT_PREC_FP64,
+              nsim * 2 * ns * (lmax + 1) * 32, None, C.byref(plan))
+    try:
+        k = C.c_int()
+        _lib.call("fsht_plan_info", plan, None, C.byref(k))
+        assert 64 <= k.value < nsim and k.value % 64 == 0
+        maps = torch.ones((nsim, 12 * ns * ns), dtype=torch.float64, device="cuda")
+        W = torch.zeros((lmax + 1, 2 * ns, nsim, 2, 2), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        _lib.call("fsht_run_stage", plan, 0, C.c_void_p(maps.data_ptr()), C.c_void_p(W.data_ptr()),
+                  nsim)
+        _lib.call("fsht_plan_sync", plan)
+        # m = 0, every ring but the equator: S = F_N + F_S = 2 n, D = 0
+        assert (W[0, :-1, :, 0, 0] > 7).all() and W[0, :-1, :, 1].abs().max() < 1e-10
+        with pytest.raises(ValueError):
+            _lib.call("fsht_run_stage", plan, 0, C.c_void_p(maps.data_ptr()),
+                      C.c_void_p(W.data_ptr()), nsim + 1)
+    finally:
+        _lib.load().fsht_plan_destroy(plan)
