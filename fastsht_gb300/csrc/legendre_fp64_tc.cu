@@ -52,10 +52,10 @@ constexpr int kMaxExp = 900;       // column maxima beyond 2^+-900 go to the FMA
 __device__ __forceinline__ unsigned long long fixed_biased(double v, int k) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const int ex = (int)(b >> 52) & 0x7FF;
-  const unsigned long long mant = (b & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-  const int sh = ex - 1075 + k;
+  const unsigned long long mant = (b & 0xFFFFFFFFFFFFFull) | (ex != 0 ? 1ull << 52 : 0ull);
+  const int sh = max(ex, 1) - 1075 + k;
   unsigned long long x = 0;
-  if (ex != 0 && sh > -53) x = sh >= 0 ? mant << min(sh, 9) : mant >> -sh;
+  if (sh > -53) x = sh >= 0 ? mant << min(sh, 9) : mant >> -sh;
   if ((long long)b < 0) x = 0ull - x;
   return x + kBias;
 }
@@ -777,8 +777,8 @@ __device__ __forceinline__ long long fixed_i64(double v, int k) {
 }
 __device__ __forceinline__ int dft_exp(unsigned long long mx) {
   const int ef = (int)(mx >> 52);
-  if (mx == 0 || ef == 0) return kEmptyExp;
-  return ef == 0x7FF ? kNanExp : ef - 1022;
+  if (mx == 0) return kEmptyExp;
+  return ef == 0x7FF ? kNanExp : max(ef, 1) - 1022;        // (1: below the normal range)
 }
 
 // Ring samples -> folded digit tiles.  The ring's samples against the maximum of the map's two
