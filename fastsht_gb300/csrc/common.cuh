@@ -210,6 +210,7 @@ struct fsht_plan {
   int ndft_waves, dft_end;
   FshtLamRow* d_lamtab2;           // their spin-2 recursion rows (d_poltab: integer factors)
   size_t dev_bytes;                // device memory that the plan has allocated
+  int nsm;                         // SMs of its device
   int stage_maps;                  // most maps of a fsht_run_stage call (chunk without digit tiles)
 };
 
@@ -309,6 +310,9 @@ int fsht_launch_analysis_fp64(fsht_plan* p, int spin, const double2* WQ,
 // The waves again, for tiles of `cap` bytes (before fsht_dft_tables_init).
 int fsht_tc_wave_cap(fsht_plan* p, size_t cap);
 int fsht_dft_tables_init(fsht_plan* p);
+// Per wave of rings: first entry, end, most row tiles of a ring, largest q, digit k-steps, row tiles
+// of all its rings.
+constexpr int kDftWaveInts = 6;
 int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, int kc, int k0,
                         int cnt, bool host, double2* W, cudaStream_t s);
 int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride, int kc,

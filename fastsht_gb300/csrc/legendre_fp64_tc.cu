@@ -1800,7 +1800,6 @@ namespace {
 // The belt takes the matrix form up to this nside: its products grow with nside^3 in all, the
 // power-of-two FFT's passes with nside^2 log nside.
 constexpr int kDftBeltMax = 256;
-constexpr int kDftWaveInts = 5;     // first entry, end, most row tiles, largest q, digit k-steps
 
 // Units of the forward (two rings added: 1) and inverse transforms (four samples: 2) of a plan.
 FshtTcUnits dft_units(const fsht_plan* p, int extra) {
@@ -1876,16 +1875,16 @@ int fsht_dft_tables_init(fsht_plan* p) {
   const int cap_r = 2 * p->wave_qmax;
   std::vector<int> waves;
   long long ut = 0, uc = 0, ucos = 0;
-  int w0 = 0, nrt = 0, qm = 0;
+  int w0 = 0, nrt = 0, qm = 0, tiles = 0;
   std::vector<long long> cls(2, -1), clsc(2, -1);                  // belt classes of this wave
   auto close = [&](int e) {
     if (e > w0) {
-      const int wv[kDftWaveInts] = {w0, e, nrt, qm, (int)uc};
+      const int wv[kDftWaveInts] = {w0, e, nrt, qm, (int)uc, tiles};
       waves.insert(waves.end(), wv, wv + kDftWaveInts);
     }
     w0 = e;
     ut = uc = 0;
-    nrt = qm = 0;
+    nrt = qm = tiles = 0;
     cls[0] = cls[1] = -1;
   };
   for (int i : order) {
@@ -1928,6 +1927,7 @@ int fsht_dft_tables_init(fsht_plan* p) {
     d.off_c = uc;
     uc += csteps;
     nrt = std::max(nrt, d.nrt);
+    tiles += d.nrt;
     qm = std::max(qm, d.q);
     rings.push_back(d);
   }

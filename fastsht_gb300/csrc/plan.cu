@@ -324,6 +324,14 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
     if (m > 0) df = df * (2 * m + 1) / 2 / m;
     pref[m] = std::sqrt(df / 4 / M_PI);
   }
+  int dev = 0;
+  cudaError_t ce = cudaGetDevice(&dev);
+  if (ce == cudaSuccess)
+    ce = cudaDeviceGetAttribute(&p->nsm, cudaDevAttrMultiProcessorCount, dev);
+  if (ce != cudaSuccess) {
+    fsht_set_error("device: %s", cudaGetErrorString(ce));
+    return fail(FSHT_ECUDA);
+  }
   auto dalloc = [&](void** ptr, size_t bytes) -> int {
     cudaError_t e = fsht_plan_malloc(p, ptr, bytes);
     if (e != cudaSuccess) {
@@ -341,7 +349,6 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   if ((rc = dalloc((void**)&p->d_sth, sizeof(double) * nn))) return fail(rc);
   if ((rc = dalloc((void**)&p->d_pref, sizeof(double) * (lmax + 1)))) return fail(rc);
   if ((rc = dalloc((void**)&p->d_ring_i0, sizeof(int) * (lmax + 1)))) return fail(rc);
-  cudaError_t ce;
   if ((ce = cudaMemcpyAsync(p->d_cth, cth.data(), sizeof(double) * nn, cudaMemcpyHostToDevice,
                             p->stream)) != cudaSuccess ||
       (ce = cudaMemcpyAsync(p->d_sth, sth.data(), sizeof(double) * nn, cudaMemcpyHostToDevice,
@@ -706,18 +713,36 @@ static bool use_tc(const fsht_plan* p, int spin) {
 }
 
 // How many maps of a chunk of kc, counted from the first, take the matrix form of the ring
-// transforms below dft_end (it uses the contraction's buffers): whole tiles of 64 maps, and the
-// last part of a tile if it is full enough.  The matrices and a tile cost the same however full it
-// is, the FFT costs by the map.  Measured, ms (tile / FFT of 16 maps; above nside 256 both without
-// the belt's FFT): forward .062/.046 at nside 32, .136/.112 at 64, .31/.34 at 128, 1.23/1.31 at 256,
-// 2.2/3.1 at 512, 15/17 at 1024; inverse, where the samples' read-modify-writes weigh more the
-// shorter the rings are, .21/.049, .28/.115, .85/.36, 2.6/1.28, 4.5/3.3, 28/18.
+// transforms below dft_end (it uses the contraction's buffers): all of them, whole tiles of 64, or
+// none.  The matrix form costs by the round: a wave of rings is one launch of (ring, row tile, 64-map
+// group) units (forward: times four types), one an SM at a time, and a unit takes as long however few
+// there are.  Plans of small lmax hold short waves: at nside 128 the 256 rings are one wave at lmax
+// 383 (64 maps: forward .39 ms, inverse .87; by FFT 1.4 and 1.4), and 59 of four to seven rings at
+// lmax 3 (2.2 and 13.3; FFT 1.15 and 1.23).  The FFT costs by the map.  tile_maps: the maps whose FFT
+// takes as long as one tile in whole waves, measured per nside with 16 to 192 maps at lmax 2 nside and
+// above; a rest of a tile costs nearly what a full one does.
 static int dft_maps(const fsht_plan* p, int kc, bool inv = false) {
   if (!use_tc(p, 0) || p->dft_end <= 0) return 0;
-  const int fwd_maps = p->nside <= 64 ? 20 : 15;
-  const int inv_maps = p->nside <= 32 ? 60 : p->nside <= 128 ? 38 : p->nside <= 256 ? 31 : 23;
-  const int rest = kc % 64;
-  return rest >= (inv ? inv_maps : fwd_maps) ? kc : kc - rest;
+  static const int fwd[] = {22, 20, 15, 15, 12, 15, 21}, bwd[] = {100, 40, 40, 31, 18, 23, 46};
+  int i = 0;                                       // nside 32 .. 2048
+  while ((32 << i) < p->nside) ++i;
+  const int tile_maps = inv ? bwd[i] : fwd[i], per = inv ? 1 : 4;
+  if (kc < tile_maps) return 0;
+  auto rounds = [&](long long units) { return (units + p->nsm - 1) / p->nsm; };
+  long long whole = 0;
+  for (int w = 0; w < p->ndft_waves; ++w) whole += p->h_dft_waves[kDftWaveInts * w + 5];
+  whole = rounds(whole * per);
+  // cost of the first n maps in matrix form, the others by FFT, in maps' FFTs times `whole`
+  auto cost = [&](int n) {
+    long long r = 0;
+    for (int w = 0; w < p->ndft_waves && n > 0; ++w)
+      r += rounds((long long)p->h_dft_waves[kDftWaveInts * w + 5] * per * ((n + 63) / 64));
+    return r * tile_maps + whole * (kc - n);
+  };
+  int best = kc;
+  for (int n : {kc - kc % 64, 0})
+    if (cost(n) < cost(best)) best = n;
+  return best;
 }
 
 // Ring transforms of maps [k0, k0 + cnt) of a chunk of kc (maps on the device, or host memory read
