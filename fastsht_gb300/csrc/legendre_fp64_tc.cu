@@ -48,14 +48,17 @@ constexpr int kMaxExp = 900;       // column maxima beyond 2^+-900 go to the FMA
 
 // v 2^k as a fixed-point integer (truncated), biased so that its eight bytes minus 128 are the
 // balanced digits d0 (top byte) .. d7.  Integer instructions only: GB300's FP64 pipe runs two
-// operations per clock per SM.  |v 2^k| < 2^62 is the caller's scale.
+// operations per clock per SM.  |v 2^k| < 2^62 is the caller's scale.  SUB: v may lie below the
+// normal range (elsewhere such a v counts as zero: it is below the scale's last bit).
+template <bool SUB = false>
 __device__ __forceinline__ unsigned long long fixed_biased(double v, int k) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const int ex = (int)(b >> 52) & 0x7FF;
-  const unsigned long long mant = (b & 0xFFFFFFFFFFFFFull) | (ex != 0 ? 1ull << 52 : 0ull);
-  const int sh = max(ex, 1) - 1075 + k;
+  const unsigned long long mant =
+      (b & 0xFFFFFFFFFFFFFull) | (!SUB || ex != 0 ? 1ull << 52 : 0ull);
+  const int sh = (SUB ? max(ex, 1) : ex) - 1075 + k;
   unsigned long long x = 0;
-  if (sh > -53) x = sh >= 0 ? mant << min(sh, 9) : mant >> -sh;
+  if ((SUB || ex != 0) && sh > -53) x = sh >= 0 ? mant << min(sh, 9) : mant >> -sh;
   if ((long long)b < 0) x = 0ull - x;
   return x + kBias;
 }
@@ -773,7 +776,7 @@ constexpr int kNanExp = kEmptyExp - 1;     // column with a non-finite sample: N
 
 // A fixed-point value without the digit bias.
 __device__ __forceinline__ long long fixed_i64(double v, int k) {
-  return (long long)(fixed_biased(v, k) - kBias);
+  return (long long)(fixed_biased<true>(v, k) - kBias);
 }
 __device__ __forceinline__ int dft_exp(unsigned long long mx) {
   const int ef = (int)(mx >> 52);
@@ -940,7 +943,7 @@ __global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
         y[e] = kBias;
         if (live && rho < nr) {
           const double2 v = dft_bin(g, stride_m, d, dft_r(ty, rho));
-          y[e] = fixed_biased(ty < 2 ? v.x : v.y, kFixBits - a.head - E);
+          y[e] = fixed_biased<true>(ty < 2 ? v.x : v.y, kFixBits - a.head - E);
         }
       }
       store_planes<false>(dst + ty * tstride + (size_t)(hc >> 1) * kStepBytes + (hc & 1) * 128,
