@@ -452,6 +452,7 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_gemm_pol(GemmPArgs a) {
           tc::mbar_arrive_warp(&h.tempty);
 #pragma unroll
           for (int cr = 0; cr < kCols / 2; cr += 16) {
+            if (w.g * kGroupMaps + cr >= a.kc) break;
             const int c0 = cbeg + cr;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
