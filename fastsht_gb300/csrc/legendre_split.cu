@@ -742,19 +742,17 @@ __global__ void __launch_bounds__(128) k_slice_alm(SliceAArgs a) {
   const int kl1 = nkl * ((int)blockIdx.z + 1) / (int)gridDim.z;
   const double* col = a.alm + a.k0 + k +
                       ((comp == 0 ? (long long)m * L1 + m : (L1 - m) * L1) + p) * a.ld;
-  auto load = [&](int kl, double (&v)[kKStep]) {       // an l-step's loads issued together
+  auto load = [&](int idx0, auto& v) {                 // loads of one l after the other, together
 #pragma unroll
-    for (int u = 0; u < kKStep; ++u) {
-      const int idx = kl * kKStep + u;
-      v[u] = valid && idx < cnt ? __ldg(&col[(long long)(2 * idx) * a.ld]) : 0.0;
-    }
+    for (int u = 0; u < (int)(sizeof(v) / sizeof(double)); ++u)
+      v[u] = valid && idx0 + u < cnt ? __ldg(&col[(long long)(2 * (idx0 + u)) * a.ld]) : 0.0;
   };
   // column maximum on FP64 bits with the sign cleared (integer operations, as in
   // k_slice_phase)
   unsigned long long mx = 0;
   for (int kl = kl0; kl < kl1; ++kl) {
     double v[kKStep];
-    load(kl, v);
+    load(kl * kKStep, v);
 #pragma unroll
     for (int u = 0; u < kKStep; ++u)
       mx = max(mx, (unsigned long long)__double_as_longlong(v[u]) & 0x7FFFFFFFFFFFFFFFull);
@@ -769,15 +767,17 @@ __global__ void __launch_bounds__(128) k_slice_alm(SliceAArgs a) {
                         (c >> 3) * 256 + (c & 7) * 16;
   bool bad = false;
   for (int kl = kl0; kl < kl1; ++kl) {
-    double v[kKStep];
-    load(kl, v);
-#pragma unroll
+    // (one copy of the digit code, eight values a turn: with both halves unrolled this kernel and the
+    // lambda kernel that runs beside it took longer together, eb2qu 64 / 191, one map 282 us, now 258)
+#pragma unroll 1
     for (int half = 0; half < 2; ++half) {
+      double v[8];
+      load(kl * kKStep + half * 8, v);
       uint16_t sl[kSynthPlanes][8];
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         uint16_t q4[4] = {0, 0, 0, 0};
-        if (E != kEmptyExp) bad |= tc::digits4_f(v[half * 8 + j], E, q4);
+        if (E != kEmptyExp) bad |= tc::digits4_f(v[j], E, q4);
         for (int d = 0; d < kSlices; ++d) sl[d][j] = q4[d];
         for (int d = 1; d < kSlices; ++d) sl[kSlices - 1 + d][j] = tc::bf16_scale_2m8(q4[d]);
       }

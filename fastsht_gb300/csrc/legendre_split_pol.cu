@@ -845,15 +845,24 @@ __global__ void __launch_bounds__(kThreadsG, 1) k_split_synth_pol(SynthPArgs a) 
       const SynthPUnit w = synth_pol_unit(a, u);
       if (w.nkl == 0) continue;
       __syncwarp();
-#pragma unroll 1
-      for (int t = 0; t < 4; ++t) {
-        int part, fld, par, c, sg;
-        synth_pol_pass(w.f, t, part, fld, par, c, sg);
-        const int* eb = fld ? a.EBB : a.EBE;
-        for (int x = tid & 31; x < kCols / 2; x += 32) {
-          const int e = eb[(((long long)w.qi * 2 + par) * a.ngroups + w.g) * kCols + cbeg + x];
-          s_ce[warp][t][x] = (short)((e == kEmptyExp) ? kEmptyExp : a.eag + e - 12);
+      {
+        int e[4][2];                                   // eight loads in flight
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          int part, fld, par, c, sg;
+          synth_pol_pass(w.f, t, part, fld, par, c, sg);
+          const int* eb = (fld ? a.EBB : a.EBE) +
+                          (((long long)w.qi * 2 + par) * a.ngroups + w.g) * kCols + cbeg +
+                          (tid & 31);
+          e[t][0] = eb[0];
+          e[t][1] = eb[32];
         }
+#pragma unroll
+        for (int t = 0; t < 4; ++t)
+#pragma unroll
+          for (int x = 0; x < 2; ++x)
+            s_ce[warp][t][(tid & 31) + 32 * x] =
+                (short)((e[t][x] == kEmptyExp) ? kEmptyExp : a.eag + e[t][x] - 12);
       }
       __syncwarp();
       const int rr = w.rb * kSCRings + row;
