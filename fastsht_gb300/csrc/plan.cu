@@ -1019,7 +1019,12 @@ static int fp64_analysis(fsht_plan* p, int spin, const double2* W0, const double
 // One chunk's FP64 synthesis into {G_N, G_S} of W0 (and W1), by the same two routes.
 static int fp64_synthesis(fsht_plan* p, int spin, const double* alm0, const double* alm1,
                           double2* W0, double2* W1, int nmaps, int c0, int kc) {
-  if (!use_tc(p, spin)) {
+  // Few maps and orders (spin 0): one FMA launch, which takes 32 l at a time, is shorter than slices,
+  // tiles, contraction and the pass over flagged columns.  alm2t with the one and the other, us:
+  // 64 / 20, one map 55 and 66, ten 106 and 118, twenty 178 and 176; 128 / 30, one 73 and 81; 128 / 39,
+  // one 98 and 88; 256 / 10, one 120 and 133; 256 / 20, one 139 and 134; 512 / 10, one 349 and 346.
+  const bool small = spin == 0 && kc <= 16 && p->lmax < (p->nside <= 128 ? 32 : 16);
+  if (small || !use_tc(p, spin)) {
     FSHT_PROF(FSHT_KCAT_SYNTHESIS);
     return fsht_launch_synthesis_fp64(p, spin, alm0, alm1, W0, W1, nmaps, c0, kc, p->stream);
   }

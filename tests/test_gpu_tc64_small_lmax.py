@@ -34,7 +34,9 @@ def _plans(ns, lmax, nsim):
 @pytest.mark.parametrize("ns,lmax,nsim", [(32, 0, 64), (32, 1, 70), (32, 16, 48), (32, 64, 128),
                                           (32, 95, 192), (64, 3, 64), (64, 16, 40), (64, 63, 129),
                                           (128, 2, 65), (128, 32, 96), (128, 128, 100),
-                                          (256, 10, 40), (256, 32, 96), (512, 15, 24)])
+                                          (256, 10, 40), (256, 32, 96), (512, 15, 24),
+                                          (32, 0, 1), (64, 31, 16), (64, 32, 16), (64, 31, 17),
+                                          (256, 15, 1), (256, 16, 1)])
 def test_small_lmax_equals_general_path(kind, ns, lmax, nsim):
     x = _input(kind, ns, lmax, nsim)
     out = []
