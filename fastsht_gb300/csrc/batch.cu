@@ -88,6 +88,7 @@ int run_job(const fsht_plan* base, const fsht_job& j, unsigned char* arena, size
   bool tc = base->tc64 && (!pol || base->d_poltab);
   int kc = j.nmaps;
   if (tc) {
+    kc = kc < kTcMaxMaps ? kc : kTcMaxMaps;
     while (kc > 1 && job_layout(base, j, kc, true).total > arena_bytes)
       kc = kc > 64 ? (kc - 1) / 64 * 64 : kc - 1;
     if (job_layout(base, j, kc, true).total > arena_bytes || (kc < j.nmaps && kc < 64)) {

@@ -318,6 +318,8 @@ int fsht_launch_dft_fwd(fsht_plan* p, const double* maps, long long map_stride, 
 int fsht_launch_dft_inv(fsht_plan* p, const double2* W, double* maps, long long map_stride, int kc,
                         int cnt, cudaStream_t s);
 bool fsht_tc_supported(const fsht_plan* p);
+// Most maps per chunk: the slices of ring samples have up to a block per map in grid y.
+constexpr int kTcMaxMaps = 65472;
 int fsht_tc_tables_init(fsht_plan* p);
 size_t fsht_tc_ws_bytes(const fsht_plan* p, int kc, int nf);
 size_t fsht_tc_eb_bytes(const fsht_plan* p, int kc);

@@ -394,7 +394,7 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   };
   const bool tables_only = (flags & FSHT_FLAG_TABLES_ONLY) != 0;
   auto tc_chunk = [&]() -> size_t {           // maps whose tiles fit the limit beside W
-    size_t k = (size_t)nmaps_max;
+    size_t k = (size_t)std::min(nmaps_max, kTcMaxMaps);
     while (k > 1 && need_tc(k) > limit) k = k > 64 ? (k - 1) / 64 * 64 : k - 1;
     return k;
   };

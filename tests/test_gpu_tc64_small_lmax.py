@@ -67,3 +67,17 @@ def test_small_lmax_is_not_slower(kind, ns, lmax, nsim):
         ms.append(min(times))
         sht.close()
     assert ms[0] <= 2.0 * ms[1]
+
+
+def test_more_maps_than_a_grid_dimension():
+    """262,208 maps of nside 32 in one call: the ring slices' grids stay within their limits."""
+    from fastsht_gb300 import SHT
+    ns, lmax, nsim = 32, 1, 262208
+    maps = torch.full((nsim, 12 * ns * ns), 2.0, dtype=torch.float64, device="cuda")
+    x = _input("t2alm", ns, lmax, 64)
+    maps[-64:] = x.T
+    sht = SHT(ns, lmax, nsim)
+    alm = sht.t2alm(maps.T)
+    want = SHT(ns, lmax, 64).t2alm(x)
+    assert ((alm[-64:] - want).abs().max() <= 1e-13 * want.abs().max())
+    assert ((alm[:-64, 0, 0] - 2.0 * (4 * torch.pi) ** 0.5).abs().max() <= 1e-12)
