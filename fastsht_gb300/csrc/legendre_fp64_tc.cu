@@ -12,18 +12,21 @@
 // output element (unit 2^-unit_bits), so no FP64 instruction runs before the last conversion and
 // the order of the parts does not matter.
 //
-// What the fixed point costs: the dropped levels (8 and up) and the unit are below 2^-44 of
-// the largest operand pair.  Against long-double sums (white, smooth and constant columns,
-// nside 64..1024) the error is 0.2..1 times that of an FP64 FMA loop for white and constant
-// columns.  Columns that the fixed point cannot hold (non-finite, or a maximum beyond 2^+-900)
-// are flagged per (order, 64-map group) and contracted by the FMA kernels (legendre_fp64.cu).
+// What the fixed point costs: levels 8 and up are dropped, levels 5..7 may round in FP32, and sums
+// have a unit of 2^-38 .. 2^-46 of the scale (tc_units.h), all below 2^-44 of the largest operand
+// pair; a column has one exponent (spin 2: one for both fields, matrix-form rings: one for a map's
+// two rings).  Against long-double sums the rms errors of white, smooth (alm falling as l^-3) and
+// constant maps at nside 32..128, lmax 3 nside - 1, are 0.94..1.1 times the FMA kernels' in the
+// analyses and 0.5..1.03 times in the syntheses.  Columns that the fixed point cannot hold
+// (non-finite, or a maximum beyond 2^+-900) are flagged per (order, 64-map group) and contracted by
+// the FMA kernels (legendre_fp64.cu).
 //
 // Per wave of orders:
 //   k_tc_slice      {S, D} phases -> digit tiles and column exponents       (HBM bound)
 //   k_tc_lambda     FP64 recursion -> lambda digit tiles, once for all maps (FP64 pipe, 79 %)
 //   k_tc_gemm       persistent tcgen05 contraction         (shared-memory and L2 bandwidth)
 // and for the synthesis k_tc_slice_alm, k_tc_lambda_T and k_tc_gemm<1, *>.
-// nside 512, lmax 1023, 64 maps, each alone: 1.23, 2.8 and 3.7 ms, where the FMA kernel needs 134
+// nside 512, lmax 1023, 64 maps, each alone: 1.24, 2.8 and 3.6 ms, where the FMA kernel needs 134
 // at 82 % of the DFMA rate.
 #include "legendre_rec.cuh"
 #include "split_common.cuh"
@@ -125,8 +128,8 @@ __device__ __forceinline__ double i64_scaled_any(long long a, int e) {
   return __longlong_as_double(
       (long long)((((unsigned long long)(ex - 1) << 52) + r) | sign));
 }
-// The same for |e| <= kSafeExp, without a branch, so that several values interleave.
-constexpr int kSafeExp = 900;
+// The same for e of -960 .. 900 (columns beyond 2^+-kMaxExp never come here), without a branch, so
+// that several values interleave.
 __device__ __forceinline__ double i64_scaled(long long a, int e) {
   const long long s = a >> 63;
   unsigned long long u = (unsigned long long)((a ^ s) - s);
@@ -963,12 +966,11 @@ __global__ void __launch_bounds__(256) k_dft_slice_inv(DftSliceArgs a) {
 // Each part of <= kPartK k-steps runs two passes through the four 128-column TMEM accumulators:
 // levels 0..3 (digit planes 0..3) and levels 4..7 (all planes).  The slots form two pairs, each
 // with a UMMA warp and barriers of its own: pair 0 finishes its smaller share first and is drained
-// into the 64-bit integers while the products of pair 1 still run (without the drains the analysis
-// took 6.21 Mcycles an SM instead of 6.34).  Shorter parts cost more passes: 11 k-steps 5 % more,
-// 8 k-steps 11 %.  One lane copies (16 KB of each operand per stage).
+// into the 64-bit integers while the products of pair 1 still run.  Shorter parts cost more passes:
+// 11 k-steps 5 % more, 8 k-steps 11 %.  One lane copies (16 KB of each operand per stage).
 // What bounds it (nside 512, lmax 1023, 64 maps): shared memory, 328 KB a k-step at 128 bytes a
 // clock = 2624 clocks against 2304 on the tensor pipe, and the copies, 96 KB a k-step (8.4 TB/s
-// over all SMs, about half of it from HBM at 55 % of its rate); tensor pipe 64 % active.
+// over all SMs, about half of it from HBM at 55 % of its rate); tensor pipe 65 % active.
 // The map columns are on the lanes, so a warp's alm stores are two 128-byte segments and its
 // phase-matrix stores whole {Re, Im} pairs, with no staging through shared memory.
 // Sixteen epilogue warps (four per TMEM lane quarter, one per 32 accumulator columns: 32 64-bit
@@ -1079,7 +1081,7 @@ __device__ __forceinline__ TcUnit tc_unit(const TcGemmArgs& a, int u) {
 // TMEM, so where the tile is wide one 256-column product a_i x {b_(L-i), b_(L+1-i)} serves both
 // levels and reads a_i once: 36 products of 128 columns read 288 KB of shared memory a k-step
 // beside the 96 KB that the copies write (3072 clocks at 128 bytes a clock against 2304 on the
-// tensor pipe, which is what a contraction without its drains took), 14 wide and 8 narrow ones 232.
+// tensor pipe), 14 wide and 8 narrow ones 232.
 // (The two halves of an operand's planes lie in different stages: no pair spans planes 3 and 4.)
 constexpr int kWideN = 96;
 template <int L, class F>
