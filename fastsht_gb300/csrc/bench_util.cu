@@ -156,7 +156,7 @@ extern "C" int fsht_measure_dmma_peak(double* tflops) {
 
 // ---------------------------------------------------------------- wait self-test
 // One thread waits, with the kernels' bounded mbarrier wait, on a barrier that nothing
-// arrives on: the wait gives up after its iteration limit (about a second), and the
+// arrives on: the wait gives up after an iteration limit of its own (about a second), and the
 // kernel raises the plan's error word exactly as an expired wait in the split-precision
 // kernels does.  No fault, no trap, no unbounded loop.
 #include "tcgen05.cuh"
@@ -172,7 +172,7 @@ __global__ void k_wait_selftest(int* err) {
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    if (!tc::mbar_wait(&bar, 0, &abort_flag)) atomicOr(err, tc::kErrTimeout);
+    if (!tc::mbar_wait<(1u << 18)>(&bar, 0, &abort_flag)) atomicOr(err, tc::kErrTimeout);
     tc::mbar_arrive(&bar);   // leave the barrier completed before the CTA exits
   }
 }

@@ -38,10 +38,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 
 // Bounded wait: returns false (and sets *abort) when the phase does not complete
 // within the iteration budget or when another thread already aborted.
+// (A poll of a phase that does not complete takes about 4 us: 2^24 are about a minute.)
 constexpr uint32_t kWaitLimit = 1u << 24;
+template <uint32_t LIMIT = kWaitLimit>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
                                           volatile int* abort) {
-  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+  for (uint32_t it = 0; it < LIMIT; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if (*abort) return false;
     if (it > 64) __nanosleep(32);
