@@ -158,7 +158,10 @@ struct fsht_plan {
   // 8 | 16); split GEMMs' ring-part length in k-steps of 16 rings (16 | 32 | 64)
   int ana_mt, ana_rc, split_part;
   struct FshtProfile* prof;        // non-null while per-kernel timing is on
-  int* d_err;                      // device error word (bounded waits that expired)
+  // error word (bounded waits that expired, values outside their digit scale) in page-locked host
+  // memory, and its device address: the host reads it without a copy
+  int* h_err;
+  int* d_err;
   // split-precision form: sliced phase tiles and their column exponents, the scaled
   // recursion rows, and the lambda-digit staging buffer with its waves of m
   unsigned char* d_ws;

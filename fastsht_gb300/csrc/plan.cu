@@ -115,7 +115,7 @@ void free_plan_memory(fsht_plan* p) {
   cudaFree(p->d_rtw_df);
   cudaFree(p->d_tw16_df);
   cudaFree(p->d_work);
-  cudaFree(p->d_err);
+  if (p->h_err) cudaFreeHost(p->h_err);
   cudaFree(p->d_ws);
   cudaFree(p->d_eb);
   cudaFree(p->d_lamtab);
@@ -217,6 +217,15 @@ double2* work_buf(fsht_plan* p, int b, int kc) {
   return p->d_work + (size_t)b * kc * (size_t)(p->lmax + 1) * p->nnorth * 2;
 }
 
+// FP64 calls do not wait for the device, so an expired wait of the tensor-core kernels is reported by
+// the plan's next call if nothing has asked before (fsht_plan_sync, fsht_plan_check).
+int check_earlier(fsht_plan* p) {
+  if (!p->tc64 || !p->aux || !*(volatile int*)p->h_err) return FSHT_OK;
+  const int rc = fsht_plan_check(p);
+  fsht_set_error("an earlier call on this plan: %s", std::string(g_last_error).c_str());
+  return rc;
+}
+
 int check_call(fsht_plan* p, int nmaps, const void* a, const void* b) {
   int rc = check_plan(p);
   if (rc) return rc;
@@ -232,7 +241,7 @@ int check_call(fsht_plan* p, int nmaps, const void* a, const void* b) {
     fsht_set_error("null array pointer");
     return FSHT_EINVAL;
   }
-  return FSHT_OK;
+  return check_earlier(p);
 }
 
 int need_bufs(fsht_plan* p, int nb) {
@@ -447,11 +456,14 @@ int fsht_plan_create(int nside, int lmax, int nmaps_max, int flags, int precisio
   p->work_bytes = tables_only ? 0 : per_map * kc;
   if (!tables_only && !p->d_work && (rc = dalloc((void**)&p->d_work, p->work_bytes)))
     return fail(rc);
-  if ((rc = dalloc((void**)&p->d_err, sizeof(int)))) return fail(rc);
-  if ((ce = cudaMemsetAsync(p->d_err, 0, sizeof(int), p->stream)) != cudaSuccess) {
-    fsht_set_error("memset: %s", cudaGetErrorString(ce));
-    return fail(FSHT_ECUDA);
+  if ((ce = cudaHostAlloc((void**)&p->h_err, sizeof(int),
+                          cudaHostAllocMapped | cudaHostAllocPortable)) != cudaSuccess ||
+      (ce = cudaHostGetDevicePointer((void**)&p->d_err, p->h_err, 0)) != cudaSuccess) {
+    cudaGetLastError();
+    fsht_set_error("error word: %s", cudaGetErrorString(ce));
+    return fail(ce == cudaErrorMemoryAllocation ? FSHT_ENOMEM : FSHT_ECUDA);
   }
+  *p->h_err = 0;
   if ((precision == FSHT_PREC_SPLIT || p->tc64) && !tables_only) {
     if (!p->tc64) {
       const size_t f = f_ws;
@@ -679,10 +691,10 @@ int fsht_plan_set_host_read(fsht_plan* p, int direct) {
 
 int fsht_plan_check(fsht_plan* p) {
   FSHT_TRY(check_plan(p));
-  int err = 0;
-  FSHT_CUDA_TRY(cudaMemcpy(&err, p->d_err, sizeof(int), cudaMemcpyDeviceToHost));
+  volatile int* word = p->h_err;
+  const int err = *word;
   if (err) {
-    FSHT_CUDA_TRY(cudaMemset(p->d_err, 0, sizeof(int)));
+    *word = 0;
     if (err & tc::kErrTimeout) {
       fsht_set_error("a bounded device-side wait expired (error word %d); results are invalid",
                      err);

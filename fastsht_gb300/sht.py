@@ -188,11 +188,13 @@ class SHT:
                     tgt.copy_(dev)
             else:
                 torch.from_numpy(np.asarray(alms_in).T).copy_(dev, non_blocking=False)
+                self._checked()
             return 0
         if as_torch:
             return dev.permute(2, 1, 0)
         out = pinned_empty((self.nsim, self.lmax + 1, self.lmax + 1))
         torch.from_numpy(out.T).copy_(dev, non_blocking=False)
+        self._checked()
         return out
 
     def _maps_out(self, dev, maps_in, as_torch):
@@ -203,12 +205,20 @@ class SHT:
                     tgt.copy_(dev)
             else:
                 torch.from_numpy(np.asarray(maps_in).T).copy_(dev, non_blocking=False)
+                self._checked()
             return 0
         if as_torch:
             return dev.T
         out = pinned_empty((self.npix, self.nsim))
         torch.from_numpy(out.T).copy_(dev, non_blocking=False)
+        self._checked()
         return out
+
+    def _checked(self):
+        """After a copy to the host has waited for the result: expired device waits raise.  (Results
+        that stay on the device are not waited for: the plan's next call raises for them.)"""
+        if self.precision == "fp64":
+            _lib.call("fsht_plan_check", self._plan)
 
     # ------------------------------------------------------------ reference API
     def set_maps(self, maps_in):

@@ -288,8 +288,9 @@ int fsht_plan_contraction(const fsht_plan* plan, int* maps_per_cta, int* rings_p
                           int* part_steps);
 
 /* Blocks until the plan's stream is idle; returns FSHT_ECUDA on an async error,
- * FSHT_ETIMEOUT when a bounded device-side wait (split-precision kernels) expired since
- * the last check, and FSHT_ERANGE when a split-form kernel met a value outside its digit
+ * FSHT_ETIMEOUT when a bounded device-side wait (tensor-core kernels) expired since
+ * the last check (of FP64 transforms the plan's next transform call returns it too, if
+ * nothing has asked before), and FSHT_ERANGE when a split-form kernel met a value outside its digit
  * scale (a non-finite input) since the last check (the error word is then cleared). */
 int fsht_plan_sync(fsht_plan* plan);
 /* The error-word check of fsht_plan_sync without synchronising any stream: call it after
