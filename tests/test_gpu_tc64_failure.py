@@ -48,3 +48,16 @@ def test_expired_wait_is_reported_with_a_host_result():
         sht.alm2t(alm)
     assert ei.value.code == _lib.FSHT_ETIMEOUT
     assert np.abs(sht.alm2t(alm) - 1 / np.sqrt(4 * np.pi)).max() < 1e-12
+
+
+def test_more_plans_than_shared_error_words():
+    """1,030 plans at once, each with a word of its own; the last one's expiry is its own."""
+    from fastsht_gb300 import SHT, _lib
+    lib = _lib.load()
+    plans = [SHT(4, 4, 1) for _ in range(1030)]
+    assert lib.fsht_selftest_wait_timeout(plans[-1]._plan) == _lib.FSHT_OK
+    torch.cuda.synchronize()
+    assert [lib.fsht_plan_check(p._plan) for p in plans] == [_lib.FSHT_OK] * 1029 + [_lib.FSHT_ETIMEOUT]
+    for p in plans:
+        p.close()
+    assert lib.fsht_plan_check(SHT(4, 4, 1)._plan) == _lib.FSHT_OK
